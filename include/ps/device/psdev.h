@@ -214,6 +214,8 @@ size_t psdev_ll_bytes(int world, int64_t ll_cap);
 
 /* Number of kernels this library has launched in this process (for reporting). */
 uint64_t psdev_launch_count(void);
+/* 1 in the checks build (-DPSDEV_CHECKS), whose kernels can set a channel's status themselves. */
+int psdev_checks_enabled(void);
 void psdev_count_launch(void);
 /* State arrays (0, 1 or 2) that the handle of `kind` needs, or -1 for an unknown kind. */
 int psdev_handle_states(int kind);

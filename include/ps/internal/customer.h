@@ -62,6 +62,11 @@ class Customer {
   // ps::Error for it instead of returning.  Used by the device plane when a kernel gave up
   // waiting for a peer; message traffic never fails a request this way.
   void FailRequest(int timestamp, const std::string& why);
+  // Brackets a request that the device plane serves: while one is outstanding, WaitRequest polls
+  // for a short time before it sleeps, because a small device request ends within microseconds
+  // and waking a sleeping thread takes as long again.
+  void RouteBegin() { on_route_.fetch_add(1, std::memory_order_relaxed); }
+  void RouteEnd() { on_route_.fetch_sub(1, std::memory_order_relaxed); }
   // Hands a received message to this customer (called by the van's receive thread).
   void Accept(const Message& recved) { recv_queue_.Push(recved); }
   // False during the first milliseconds of a customer's life (PS_HANDLE_GRACE_MS, default 20).
@@ -82,6 +87,8 @@ class Customer {
   ThreadsafePQueue recv_queue_;
   std::unique_ptr<std::thread> recv_thread_;
 
+  std::atomic<int> on_route_{0};
+  std::atomic<unsigned> progress_{0};  // counts changes of the tracker
   std::mutex tracker_mu_;
   std::condition_variable tracker_cond_;
   // tracker_[ts - tracker_base_] = (responses expected, responses received).  Requests below

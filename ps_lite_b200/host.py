@@ -108,10 +108,13 @@ def lib() -> C.CDLL:
             L.ps_capi_bworker_new.argtypes = [i, i]
             L.ps_capi_bworker_delete.argtypes = [vp]
             L.ps_capi_bworker_request.argtypes = [vp, i, i, u64p, sz, vp, sz, vp, sz, i, i]
+            L.ps_capi_bworker_request_on.argtypes = [vp, vp, i, i, vp, sz, vp, sz, vp, sz, i, i]
             L.ps_capi_bworker_wait.argtypes = [vp, i]
             f32 = C.c_float
             L.psnvl_declare_sparse.argtypes = [i, u64, i64, i, i, f32, f32, f32, f32, f32, i]
-            L.ps_capi_bworker_keyed_request.argtypes = [vp, i, i, vp, sz, vp, sz, vp, sz, vp, vp, i]
+            keyed = [i, i, vp, sz, vp, sz, vp, sz, vp, vp, i]
+            L.ps_capi_bworker_keyed_request.argtypes = [vp] + keyed
+            L.ps_capi_bworker_keyed_request_on.argtypes = [vp, vp] + keyed
             _lib = L
         return _lib
 

@@ -56,6 +56,7 @@ class Context:
                                   max(1, torch.cuda.device_count()))
         self.device = torch.device(device)
         torch.cuda.set_device(self.device)
+        self._device_index = self.device.index or 0
         # host staging buffers and copy threads next to the GPU (matters with several GPUs
         # per host: a pinned buffer on the far socket crosses the inter-socket link)
         from .utils.affinity import bind_to_gpu_cpus
@@ -77,6 +78,10 @@ class Context:
         self.worker = L.ps_capi_bworker_new(APP_ID, 0)
         if not self.worker:
             raise host.PSError(L.ps_capi_last_error().decode())
+
+    def raw_stream(self) -> int:
+        """Handle of the calling thread's current stream on this context's device."""
+        return torch._C._cuda_getCurrentRawStream(self._device_index)
 
     def new_channel(self) -> int:
         """A rendezvous channel for one more tensor; raises when all are taken."""
@@ -193,6 +198,10 @@ class KVStore:
         self.ctx = ctx or init()
         self.tables: Dict[int, DenseTable] = {}
         self._keys: Dict[int, np.ndarray] = {}
+        self._key_ptrs: Dict[int, int] = {}
+        # looked up once: small requests cost as much as the calls that make them
+        self._call = host.lib().ps_capi_bworker_request_on
+        self._wait = host.lib().ps_capi_bworker_wait
         self._alive: Dict[int, tuple] = {}
         if slice_bytes:
             host._ck(host.lib().psnvl_set_slice_bytes(int(slice_bytes)))
@@ -223,6 +232,7 @@ class KVStore:
         host._ck(L.psnvl_dense_keys(int(key), keys.ctypes.data_as(C.POINTER(C.c_uint64))))
         self.tables[key] = t
         self._keys[key] = keys
+        self._key_ptrs[key] = keys.ctypes.data
         return t
 
     def keys_of(self, key: int) -> np.ndarray:
@@ -240,10 +250,6 @@ class KVStore:
     def _request(self, key: int, push: bool, pull: bool, value: Optional[torch.Tensor],
                  out: Optional[torch.Tensor], cmd: int = 0, priority: int = 0) -> int:
         t = self.tables[key]
-        L = host.lib()
-        keys = self._keys[key]
-        cur = torch.cuda.current_stream(self.ctx.device)
-        L.psnvl_set_stream(cur.cuda_stream)
         vptr = vbytes = optr = obytes = 0
         if push:
             if value is None:
@@ -251,19 +257,18 @@ class KVStore:
             if not value.is_contiguous() or value.numel() != t.n_user or value.dtype != t.grad_dtype:
                 raise ValueError("pushed values must be a contiguous tensor of the declared "
                                  "length and gradient dtype")
-            vptr, vbytes = value.data_ptr(), value.numel() * value.element_size()
+            vptr, vbytes = value.data_ptr(), t.n_user * t.grad_size
         if pull:
             if out is None:
                 out = t.weight[: t.n_user]
             if not out.is_contiguous() or out.numel() != t.n_user or out.dtype != t.out_dtype:
                 raise ValueError("the output must be a contiguous tensor of the declared "
                                  "length and weight dtype")
-            optr, obytes = out.data_ptr(), out.numel() * out.element_size()
-        ts = L.ps_capi_bworker_request(self.ctx.worker, int(push), int(pull),
-                                       keys.ctypes.data_as(C.POINTER(C.c_uint64)), keys.size,
-                                       vptr, vbytes, optr, obytes, int(cmd), int(priority))
+            optr, obytes = out.data_ptr(), t.n_user * t.out_size
+        ts = self._call(self.ctx.worker, self.ctx.raw_stream(), push, pull, self._key_ptrs[key],
+                        self.ctx.world, vptr, vbytes, optr, obytes, cmd, priority)
         if ts < 0:
-            raise host.PSError(L.ps_capi_last_error().decode())
+            raise host.PSError(host.lib().ps_capi_last_error().decode())
         self._alive[ts] = (value, out, t)   # zero-copy: kept until the request completed
         if len(self._alive) > MAX_UNWAITED:
             self.wait(min(self._alive))   # a caller that never waits: retire the oldest
@@ -286,10 +291,9 @@ class KVStore:
 
     def wait(self, ts: int) -> None:
         """Block until request ``ts`` completed; raises if a device wait ran out."""
-        L = host.lib()
         try:
-            if L.ps_capi_bworker_wait(self.ctx.worker, int(ts)) < 0:
-                raise host.PSError(L.ps_capi_last_error().decode())
+            if self._wait(self.ctx.worker, ts) < 0:
+                raise host.PSError(host.lib().ps_capi_last_error().decode())
         finally:
             self._alive.pop(ts, None)
 
@@ -364,9 +368,8 @@ class KeyedStore:
         if lens_out is not None and lens_out.numel() != n:
             raise ValueError("lens_out needs one entry per key")
         L = host.lib()
-        L.psnvl_set_stream(torch.cuda.current_stream(self.ctx.device).cuda_stream)
-        ts = L.ps_capi_bworker_keyed_request(
-            self.worker, int(push), int(pull), keys.data_ptr(), n,
+        ts = L.ps_capi_bworker_keyed_request_on(
+            self.worker, self.ctx.raw_stream(), push, pull, keys.data_ptr(), n,
             vals.data_ptr() if push else None, vals.numel() * 4 if push else 0,
             out.data_ptr() if pull else None, out.numel() * 4 if pull else 0,
             lens.data_ptr() if (push and lens is not None) else None,

@@ -129,6 +129,7 @@ class DenseTable:
         self.nvls_max_bytes: Optional[int] = None
         gsz = torch.empty((), dtype=grad_dtype).element_size()
         osz = torch.empty((), dtype=out_dtype).element_size()
+        self.grad_size, self.out_size = gsz, osz
         self.grad_off = heap.alloc(self.n * gsz)
         self.weight_off = heap.alloc(self.n * osz)
         self.grad = heap.tensor(self.grad_off, self.n, grad_dtype)

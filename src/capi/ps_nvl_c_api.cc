@@ -174,6 +174,14 @@ int ps_capi_bworker_request(void* worker, int push, int pull, const uint64_t* ke
     return kv->ZPull(k, o, nullptr, cmd, [o]() { delete o; }, priority);
   });
 }
+int ps_capi_bworker_request_on(void* worker, void* stream, int push, int pull,
+                               const uint64_t* keys, size_t nkeys, const void* vals,
+                               size_t vals_bytes, void* outs, size_t outs_bytes, int cmd,
+                               int priority) {
+  Plane::Get()->SetStream(stream);
+  return ps_capi_bworker_request(worker, push, pull, keys, nkeys, vals, vals_bytes, outs,
+                                 outs_bytes, cmd, priority);
+}
 int ps_capi_bworker_wait(void* worker, int timestamp) {
   return Guard([&] {
     static_cast<KVWorker<char>*>(worker)->Wait(timestamp);
@@ -213,6 +221,15 @@ int ps_capi_bworker_keyed_request(void* worker, int push, int pull, const uint64
                             : nullptr;
     return kv->ZPull(k, o, lo, cmd, [o, lo]() { delete o; delete lo; });
   });
+}
+
+int ps_capi_bworker_keyed_request_on(void* worker, void* stream, int push, int pull,
+                                     const uint64_t* keys_dev, size_t nkeys, const void* vals_dev,
+                                     size_t vals_bytes, void* outs_dev, size_t outs_bytes,
+                                     const int* lens_dev, int* lens_out_dev, int cmd) {
+  Plane::Get()->SetStream(stream);
+  return ps_capi_bworker_keyed_request(worker, push, pull, keys_dev, nkeys, vals_dev, vals_bytes,
+                                       outs_dev, outs_bytes, lens_dev, lens_out_dev, cmd);
 }
 
 }  // extern "C"

@@ -64,6 +64,11 @@ int ps_capi_bworker_delete(void* worker);
 int ps_capi_bworker_request(void* worker, int push, int pull, const uint64_t* keys, size_t nkeys,
                             const void* vals, size_t vals_bytes, void* outs, size_t outs_bytes,
                             int cmd, int priority);
+/* The same with Plane::SetStream(stream) first, in one call. */
+int ps_capi_bworker_request_on(void* worker, void* stream, int push, int pull,
+                               const uint64_t* keys, size_t nkeys, const void* vals,
+                               size_t vals_bytes, void* outs, size_t outs_bytes, int cmd,
+                               int priority);
 int ps_capi_bworker_wait(void* worker, int timestamp);
 
 /* ---- keyed (sparse) tables ---- */
@@ -79,6 +84,10 @@ int ps_capi_bworker_keyed_request(void* worker, int push, int pull, const uint64
                                   size_t nkeys, const void* vals_dev, size_t vals_bytes,
                                   void* outs_dev, size_t outs_bytes, const int* lens_dev,
                                   int* lens_out_dev, int cmd);
+int ps_capi_bworker_keyed_request_on(void* worker, void* stream, int push, int pull,
+                                     const uint64_t* keys_dev, size_t nkeys, const void* vals_dev,
+                                     size_t vals_bytes, void* outs_dev, size_t outs_bytes,
+                                     const int* lens_dev, int* lens_out_dev, int cmd);
 
 #ifdef __cplusplus
 }

@@ -1,9 +1,11 @@
 #include "ps/internal/customer.h"
 
+#include <algorithm>
 #include <chrono>
 #include <climits>
 
 #include "ps/internal/postoffice.h"
+#include "ps/internal/spin.h"
 
 namespace ps {
 
@@ -52,6 +54,17 @@ bool Customer::WaitRequestFor(int timestamp, int timeout_ms) {
     return e.first <= e.second;
   };
   bool finished = true;
+  if (on_route_.load(std::memory_order_relaxed) > 0 && !done()) {
+    const auto until = std::chrono::steady_clock::now() +
+        std::chrono::microseconds(timeout_ms < 0 ? SpinMicros() :
+                                  std::min<int64_t>(SpinMicros(), int64_t(timeout_ms) * 1000));
+    do {
+      const unsigned seen = progress_.load(std::memory_order_relaxed);
+      lk.unlock();
+      SpinUntil(until, [&] { return progress_.load(std::memory_order_relaxed) != seen; });
+      lk.lock();
+    } while (!done() && std::chrono::steady_clock::now() < until);
+  }
   if (timeout_ms < 0) {
     tracker_cond_.wait(lk, done);
   } else {
@@ -77,6 +90,7 @@ void Customer::FailRequest(int timestamp, const std::string& why) {
     auto& e = tracker_[timestamp - tracker_base_];
     e.second = e.first;
   }
+  progress_.fetch_add(1, std::memory_order_relaxed);
   tracker_cond_.notify_all();  // under the lock: see AddResponse
 }
 
@@ -95,6 +109,7 @@ void Customer::AddResponse(int timestamp, int num) {
     tracker_.pop_front();
     ++tracker_base_;
   }
+  progress_.fetch_add(1, std::memory_order_relaxed);
   // Notified under the lock.  The caller may be a thread that the customer does not own (the
   // device plane's completion thread): the thread released from Wait may destroy the customer
   // at once, and then must not find this thread still inside the condition variable.

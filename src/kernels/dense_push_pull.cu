@@ -340,6 +340,14 @@ static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op,
   return dense_dispatch_f32_f32(op, a, ctas, s);
 }
 
+extern "C" int psdev_checks_enabled(void) {
+#ifdef PSDEV_CHECKS
+  return 1;
+#else
+  return 0;
+#endif
+}
+
 extern "C" uint64_t psdev_launch_count(void) { return g_launches.load(); }
 
 // ---- flag-only device barrier -----------------------------------------------------------

@@ -33,6 +33,7 @@
 #include "ps/device/ctrl_layout.h"
 #include "ps/device/plane.h"
 #include "ps/internal/postoffice.h"
+#include "ps/internal/spin.h"
 #include "ps/simple_app.h"
 #include "van/nvl_host_sim.h"
 
@@ -89,6 +90,7 @@ struct Rt {
   int (*channel_clear)(void*, int) = nullptr;
   int (*dense_op)(const psdev_world_t*, const psdev_table_t*, int, int64_t, int64_t,
                   const psdev_opt_t*, int, int, uint64_t, int, void*) = nullptr;
+  int (*checks_enabled)() = nullptr;
   uint64_t (*launch_count)() = nullptr;
 };
 
@@ -160,6 +162,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_channel_status_on", &rt->channel_status_on);
   Bind(lib, "psdev_channel_clear", &rt->channel_clear);
   Bind(lib, "psdev_dense_op", &rt->dense_op);
+  Bind(lib, "psdev_checks_enabled", &rt->checks_enabled);
   Bind(lib, "psdev_launch_count", &rt->launch_count);
   return lib;
 }
@@ -501,8 +504,21 @@ struct Plane::Impl {
   std::vector<void*> event_pool;
   std::mutex ev_mu;
   // requests on one tensor are serialised against each other: the last event of the previous
-  // one (keyed by DenseInfo*)
-  std::map<const void*, void*> last_done;
+  // one and the stream it was recorded on (keyed by DenseInfo*)
+  struct Done {
+    void* event = nullptr;
+    void* stream = nullptr;
+  };
+  std::map<const void*, Done> last_done;
+  Done LastDone(const void* tensor) {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = last_done.find(tensor);
+    return it == last_done.end() ? Done() : it->second;
+  }
+  // Orders work on `s` after the previous request on the tensor.
+  void After(const Done& prev, void* s) {
+    if (prev.event && prev.stream != s) rt.stream_wait_event(s, prev.event);
+  }
 
   struct Pending {
     void* event = nullptr;
@@ -519,8 +535,25 @@ struct Plane::Impl {
   std::mutex q_mu;
   std::condition_variable q_cv, idle_cv;
   std::deque<Pending> queue;
-  bool stop = false;
+  std::atomic<bool> stop{false};
+  std::atomic<int> queued{0};  // entries of `queue`, for the completer to poll
+  bool asleep = false;         // the completer waits on q_cv (under q_mu)
   int in_flight = 0;
+  // a channel's status word can only change where kernels wait for peers or check indexes
+  bool status_can_change = true;
+
+  void Enqueue(Pending&& p) {
+    bool wake;
+    if (p.customer) p.customer->RouteBegin();
+    {
+      std::lock_guard<std::mutex> lk(q_mu);
+      ++in_flight;
+      queue.push_back(std::move(p));
+      queued.store(static_cast<int>(queue.size()), std::memory_order_release);
+      wake = asleep;
+    }
+    if (wake) q_cv.notify_one();
+  }
   std::thread completer;
 
   void* NewEvent() {
@@ -547,20 +580,27 @@ struct Plane::Impl {
     for (;;) {
       Pending p;
       {
+        // the next request of a worker that waits for each one follows within microseconds
+        SpinUntil(std::chrono::steady_clock::now() + std::chrono::microseconds(SpinMicros()),
+                  [&] { return queued.load(std::memory_order_acquire) > 0 || stop; });
         std::unique_lock<std::mutex> lk(q_mu);
+        asleep = true;
         q_cv.wait(lk, [&] { return stop || !queue.empty(); });
+        asleep = false;
         if (queue.empty()) return;
         p = std::move(queue.front());
         queue.pop_front();
+        queued.store(static_cast<int>(queue.size()), std::memory_order_release);
       }
       int rc = rt.event_sync(p.event);
       int32_t status = 0;
-      if (rc == 0)
+      if (rc == 0 && status_can_change)
         rc = rt.channel_status_on(ws.peer_base[rank], p.channel, s_status, &status, nullptr);
       if (p.lens_out)
         for (size_t i = 0; i < p.lens.size(); ++i) p.lens_out[i] = p.lens[i];
       if (p.on_done) p.on_done();  // before the request counts as complete, like the reference
       if (p.customer) {
+        p.customer->RouteEnd();
         if (rc != 0 || status != 0) {
           std::ostringstream why;
           why << "device plane: ";
@@ -578,7 +618,7 @@ struct Plane::Impl {
         // the event stops being the ordering point of its tensor before it is reused
         std::lock_guard<std::mutex> lk(mu);
         auto it = last_done.find(p.tensor);
-        if (it != last_done.end() && it->second == p.event) last_done.erase(it);
+        if (it != last_done.end() && it->second.event == p.event) last_done.erase(it);
       }
       RecycleEvent(p.event);
       for (void* e : p.events_to_recycle) RecycleEvent(e);
@@ -656,6 +696,7 @@ void Plane::Start(const PlaneOptions& options) {
   } else {
     m.lib = LoadRt(options.device_lib, &m.rt);
     CHECK_EQ(m.rt.set_device(options.device), 0) << "cannot select CUDA device " << options.device;
+    m.status_can_change = m.world > 1 || m.rt.checks_enabled() != 0;
   }
   m.exchange.reset(new Exchange);
   // nobody sends before every endpoint exists
@@ -788,6 +829,8 @@ void Plane::Start(const PlaneOptions& options) {
   CHECK_EQ(m.rt.stream_create(&m.s_d2h, 0), 0);
   CHECK_EQ(m.rt.stream_create(&m.s_status, 0), 0);
   m.stop = false;
+  m.asleep = false;
+  m.queued = 0;
   m.in_flight = 0;
   m.completer = std::thread(&Impl::Completing, &m);
   m.started = true;
@@ -1291,13 +1334,9 @@ void Plane::Submit(const DeviceRequest& req) {
   pend.tensor = d;
   if (req.lens_out) pend.lens = lens;
 
-  void* prev_done = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(m.mu);
-    auto it = m.last_done.find(d);
-    if (it != m.last_done.end()) prev_done = it->second;
-  }
+  const Impl::Done prev_done = m.LastDone(d);
   void* done = m.NewEvent();
+  void* done_stream = nullptr;
   const char* vals = static_cast<const char*>(req.vals);
   char* outs = static_cast<char*>(req.outs);
   char* grad = static_cast<char*>(d->grad);
@@ -1306,7 +1345,8 @@ void Plane::Submit(const DeviceRequest& req) {
   if (!staged) {
     // values already on the device: everything in order on one stream
     void* s = tls_has_stream ? tls_stream : m.s_compute;
-    if (prev_done && !m.sim) m.rt.stream_wait_event(s, prev_done);
+    done_stream = s;
+    if (!m.sim) m.After(prev_done, s);
     size_t eoff = 0;  // position in the request's value list, in elements
     for (const Run& r : runs) {
       const size_t cnt = static_cast<size_t>(r.end - r.begin);
@@ -1334,7 +1374,7 @@ void Plane::Submit(const DeviceRequest& req) {
       pend.events_to_recycle.push_back(start);
     }
     for (void* s : {m.s_h2d, m.s_compute, m.s_d2h}) {
-      if (prev_done) m.rt.stream_wait_event(s, prev_done);
+      m.After(prev_done, s);
       if (start) m.rt.stream_wait_event(s, start);
     }
     const int64_t step_g =
@@ -1415,20 +1455,16 @@ void Plane::Submit(const DeviceRequest& req) {
     m.rt.stream_wait_event(m.s_compute, tail);
     pend.events_to_recycle.push_back(tail);
     m.rt.event_record(done, m.s_compute);
+    done_stream = m.s_compute;
     if (tls_has_stream) m.rt.stream_wait_event(origin, done);
   }
   pend.event = done;
   {
     std::lock_guard<std::mutex> lk(m.mu);
     // `done` doubles as the ordering point for the next request on this tensor
-    m.last_done[d] = done;
+    m.last_done[d] = Impl::Done{done, done_stream};
   }
-  {
-    std::lock_guard<std::mutex> lk(m.q_mu);
-    ++m.in_flight;
-    m.queue.push_back(std::move(pend));
-  }
-  m.q_cv.notify_one();
+  m.Enqueue(std::move(pend));
 }
 
 // A keyed request: keys, values and outputs are device arrays.  The request is staged into the
@@ -1463,13 +1499,7 @@ void Plane::SubmitSparse(const DeviceRequest& req) {
                                                            << " bytes does not fit the request";
   }
   void* s = tls_has_stream ? tls_stream : m.s_compute;
-  void* prev_done = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(m.mu);
-    auto it = m.last_done.find(sp);
-    if (it != m.last_done.end()) prev_done = it->second;
-  }
-  if (prev_done) m.rt.stream_wait_event(s, prev_done);
+  m.After(m.LastDone(sp), s);
   const void* kptr = req.keys.data();
   if (kptr != sp->keys) {
     CHECK_EQ(m.rt.memcpy_async(sp->keys, kptr, static_cast<size_t>(n) * 8, s), 0);
@@ -1523,14 +1553,9 @@ void Plane::SubmitSparse(const DeviceRequest& req) {
   pend.tensor = sp;
   {
     std::lock_guard<std::mutex> lk(m.mu);
-    m.last_done[sp] = done;
+    m.last_done[sp] = Impl::Done{done, s};
   }
-  {
-    std::lock_guard<std::mutex> lk(m.q_mu);
-    ++m.in_flight;
-    m.queue.push_back(std::move(pend));
-  }
-  m.q_cv.notify_one();
+  m.Enqueue(std::move(pend));
 }
 
 }  // namespace device

@@ -199,6 +199,31 @@ int psdev_dense_op(const psdev_world_t* w, const psdev_table_t* t, int op,
                    int channel, int num_ctas, uint64_t timeout_ns, int sync,
                    void* stream);
 
+/* One rank (w->world == 1; PSDEV_ERR_UNSUPPORTED otherwise): `op` on elements [begin, end) with
+ * the pushed values read from `src` and the pulled values stored to `dst` as well as to the
+ * table's weight buffer, so that arrays outside the arena need no copies.  src / dst hold the
+ * value of element `begin` first and reach up to element n_valid (the rest of the range is
+ * padding); NULL names the table's own buffers.  Either may be device memory of any alignment
+ * that its type allows. */
+int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op, int64_t begin,
+                          int64_t end, const psdev_opt_t* opt, int channel, int num_ctas,
+                          void* stream, const void* src, void* dst, int64_t n_valid);
+
+/* One rank: several pieces of one table in as few launches as their number allows, the most
+ * urgent (highest priority, ties in list order) first, each with the gradient in an array of its
+ * own.  The list is host memory and is not referenced after the call. */
+#define PSDEV_MAX_LOCAL_SEGS 64
+typedef struct {
+  int64_t begin, end;  /* element range of the table, multiples of 8                       */
+  int64_t n_valid;     /* elements of the range from here on are padding (gradient 0)      */
+  int64_t priority;
+  const void* src;     /* gradient of element `begin`, or NULL: the table's gradient buffer */
+  int32_t dtype;       /* of src: PSDEV_F32 or PSDEV_BF16; rounded to the table's type first */
+} psdev_seg_t;
+int psdev_dense_op_segs(const psdev_world_t* w, const psdev_table_t* t, int op,
+                        const psdev_seg_t* segs, int nseg, const psdev_opt_t* opt, int channel,
+                        int num_ctas, void* stream);
+
 /* Several slices of one table in one launch and one rendezvous.  `segs`: device memory with
  * `nseg` (<= 1024) triples (begin, end, priority) of int64; a small kernel orders them by
  * priority (highest first, ties in submission order) and numbers the tiles across slices, so

@@ -16,6 +16,8 @@
 //
 // A user-defined server handle is any struct with the static interface of the Opt*
 // structs below; instantiate `dense_kernel<GT, OT, MyOpt, true, true>` in your own .cu.
+//
+// A job with one rank runs local_update_kernel (local_update.cuh) instead.
 #pragma once
 #include "ps/device/dev_common.cuh"
 
@@ -52,6 +54,13 @@ struct DenseArgs {
   int nseg;                 // 0: single range [begin, end)
   const long long* segs_in; // multi-slice launch: nseg x (begin, end, priority), device memory
   unsigned long long timeout_ns;
+  // one rank only (local_update.cuh): the caller's gradient and output arrays, NULL = the
+  // table's own buffers, and how far they reach; pieces with gradient arrays of their own
+  const void* src;
+  void* dst;
+  long long n_valid;
+  const psdev_seg_t* lsegs;
+  int nlsegs;
   // extents, used by the checks build (-DPSDEV_CHECKS): arena size (0 = unknown), elements of
   // the table, elements of this rank's master/state arrays
   unsigned long long heap_bytes;
@@ -275,7 +284,7 @@ __device__ __forceinline__ void channel_leave(void* const* base, int rank, int w
 }
 
 // ---- the kernel -----------------------------------------------------------------------
-// WMAX: compile-time bound on the number of ranks (1, 2, 4 or 8); the peer loops are fully
+// WMAX: compile-time bound on the number of ranks (2, 4 or 8); the peer loops are fully
 // unrolled to WMAX and predicated on the runtime world size.  Each thread handles
 // U = max(1, 4 / ... ) vectors per trip so that about 128 bytes of gradient loads per
 // thread are in flight whatever the world size.

@@ -49,6 +49,11 @@ class Table(C.Structure):
                 ("ll_off", C.c_uint64), ("ll_cap", C.c_int64)]
 
 
+class Seg(C.Structure):
+    _fields_ = [("begin", C.c_int64), ("end", C.c_int64), ("n_valid", C.c_int64),
+                ("priority", C.c_int64), ("src", C.c_void_p), ("dtype", C.c_int32)]
+
+
 class Sparse(C.Structure):
     _fields_ = [("range", C.c_uint64), ("keys_off", C.c_uint64), ("grads_off", C.c_uint64),
                 ("out_off", C.c_uint64), ("pos_off", C.c_uint64), ("acc_off", C.c_uint64),
@@ -99,6 +104,10 @@ def _declare(lib: C.CDLL) -> None:
                                  C.POINTER(Opt), i32, i32, u64, i32, vp]),
         "psdev_dense_op_multi": (i32, [C.POINTER(World), C.POINTER(Table), i32, vp, i32, vp,
                                        C.POINTER(Opt), i32, i32, u64, i32, vp]),
+        "psdev_dense_op_direct": (i32, [C.POINTER(World), C.POINTER(Table), i32, i64, i64,
+                                        C.POINTER(Opt), i32, i32, vp, vp, vp, i64]),
+        "psdev_dense_op_segs": (i32, [C.POINTER(World), C.POINTER(Table), i32, vp, i32,
+                                      C.POINTER(Opt), i32, i32, vp]),
         "psdev_sched_bytes": (sz, [i32]),
         "psdev_launch_count": (u64, []),
         "psdev_ll_bytes": (sz, [i32, i64]),

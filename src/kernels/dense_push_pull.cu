@@ -1,11 +1,13 @@
 // Host dispatch for the fused dense push / pull kernel (see ps/device/push_pull.cuh).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "ps/device/user_handle.cuh"
 
@@ -138,7 +140,9 @@ using namespace psdev;
 static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op, int64_t begin,
                          int64_t end, const psdev_opt_t* opt, int channel, int num_ctas,
                          uint64_t timeout_ns, int sync, void* stream, const int64_t* segs,
-                         int nseg, void* sched);
+                         int nseg, void* sched, const void* src = nullptr, void* dst = nullptr,
+                         int64_t n_valid = INT64_MAX, const psdev_seg_t* lsegs = nullptr,
+                         int nlsegs = 0);
 
 extern "C" int psdev_dense_op(const psdev_world_t* w, const psdev_table_t* t, int op,
                               int64_t begin, int64_t end, const psdev_opt_t* opt, int channel,
@@ -157,6 +161,44 @@ extern "C" int psdev_dense_op_multi(const psdev_world_t* w, const psdev_table_t*
   if (!segs || !sched || nseg < 1 || nseg > kMaxSegs) return PSDEV_ERR_ARG;
   return dense_op_impl(w, t, op, 0, t ? t->n : 0, opt, channel, num_ctas, timeout_ns, sync,
                        stream, segs, nseg, sched);
+}
+
+extern "C" int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op,
+                                     int64_t begin, int64_t end, const psdev_opt_t* opt,
+                                     int channel, int num_ctas, void* stream, const void* src,
+                                     void* dst, int64_t n_valid) {
+  if (!w || !t) return PSDEV_ERR_ARG;
+  if (w->world != 1) return PSDEV_ERR_UNSUPPORTED;
+  // an array of whole values: aligned to its element type
+  if (((uintptr_t)src & ((t->grad_dtype == PSDEV_F32 ? 4 : t->grad_dtype == PSDEV_BF16 ? 2 : 1) -
+                         1)) || ((uintptr_t)dst & ((t->out_dtype == PSDEV_F32 ? 4 : 2) - 1)))
+    return PSDEV_ERR_ARG;
+  return dense_op_impl(w, t, op, begin, end, opt, channel, num_ctas, 0, 0, stream, nullptr, 0,
+                       nullptr, src, dst, n_valid);
+}
+
+extern "C" int psdev_dense_op_segs(const psdev_world_t* w, const psdev_table_t* t, int op,
+                                   const psdev_seg_t* segs, int nseg, const psdev_opt_t* opt,
+                                   int channel, int num_ctas, void* stream) {
+  if (!w || !t || !segs || nseg < 1 || !(op & PSDEV_OP_PUSH)) return PSDEV_ERR_ARG;
+  if (w->world != 1 || t->grad_dtype == PSDEV_I8) return PSDEV_ERR_UNSUPPORTED;
+  std::vector<psdev_seg_t> order;
+  order.reserve(nseg);
+  for (int i = 0; i < nseg; ++i) {
+    const psdev_seg_t& g = segs[i];
+    if (g.begin < 0 || g.end > t->n || g.begin > g.end || (g.begin & 7) || (g.end & 7))
+      return PSDEV_ERR_ARG;
+    if (g.src && ((g.dtype != PSDEV_F32 && g.dtype != PSDEV_BF16) ||
+                  ((uintptr_t)g.src & (g.dtype == PSDEV_F32 ? 3 : 1))))
+      return PSDEV_ERR_ARG;
+    if (g.end > g.begin) order.push_back(g);
+  }
+  if (order.empty()) return 0;
+  std::stable_sort(order.begin(), order.end(), [](const psdev_seg_t& a, const psdev_seg_t& b) {
+    return a.priority > b.priority;
+  });
+  return dense_op_impl(w, t, op, 0, t->n, opt, channel, num_ctas, 0, 0, stream, nullptr, 0,
+                       nullptr, nullptr, nullptr, INT64_MAX, order.data(), (int)order.size());
 }
 
 extern "C" size_t psdev_ll_bytes(int world, int64_t ll_cap) {
@@ -194,7 +236,8 @@ extern "C" size_t psdev_sched_bytes(int nseg) { return sizeof(SchedEntry) * (siz
 static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op, int64_t begin,
                          int64_t end, const psdev_opt_t* opt, int channel, int num_ctas,
                          uint64_t timeout_ns, int sync, void* stream, const int64_t* segs,
-                         int nseg, void* sched) {
+                         int nseg, void* sched, const void* src, void* dst, int64_t n_valid,
+                         const psdev_seg_t* lsegs, int nlsegs) {
   if (!w || !t || w->world < 1 || w->world > PSDEV_MAX_RANKS || w->rank < 0 ||
       w->rank >= w->world)
     return PSDEV_ERR_ARG;
@@ -247,6 +290,11 @@ static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op,
     a.mc_base = nullptr;
   }
   a.timeout_ns = timeout_ns;
+  a.src = src;
+  a.dst = dst;
+  a.n_valid = n_valid;
+  a.lsegs = lsegs;
+  a.nlsegs = nlsegs;
   a.heap_bytes = w->heap_bytes;
   a.n_total = t->n;
   {

@@ -90,6 +90,9 @@ struct Rt {
   int (*channel_clear)(void*, int) = nullptr;
   int (*dense_op)(const psdev_world_t*, const psdev_table_t*, int, int64_t, int64_t,
                   const psdev_opt_t*, int, int, uint64_t, int, void*) = nullptr;
+  int (*dense_op_direct)(const psdev_world_t*, const psdev_table_t*, int, int64_t, int64_t,
+                         const psdev_opt_t*, int, int, void*, const void*, void*,
+                         int64_t) = nullptr;
   int (*checks_enabled)() = nullptr;
   uint64_t (*launch_count)() = nullptr;
 };
@@ -162,6 +165,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_channel_status_on", &rt->channel_status_on);
   Bind(lib, "psdev_channel_clear", &rt->channel_clear);
   Bind(lib, "psdev_dense_op", &rt->dense_op);
+  Bind(lib, "psdev_dense_op_direct", &rt->dense_op_direct);
   Bind(lib, "psdev_checks_enabled", &rt->checks_enabled);
   Bind(lib, "psdev_launch_count", &rt->launch_count);
   return lib;
@@ -1103,6 +1107,35 @@ inline void SplitKey(Key key, int world, int* shard, uint64_t* tensor_id) {
   *shard = static_cast<int>(s);
   *tensor_id = static_cast<uint64_t>(key) - width * s;
 }
+
+// True when two arrays share memory in another way than element for element: a kernel that reads
+// one and writes the other in the same pass would then depend on the order of its threads.
+inline bool Clash(const void* a, size_t an, size_t asz, const void* b, size_t bn, size_t bsz) {
+  const char* x = static_cast<const char*>(a);
+  const char* y = static_cast<const char*>(b);
+  return x < y + bn * bsz && y < x + an * asz && !(x == y && asz == bsz);
+}
+
+// One rank: may the kernel use the request's arrays where they are?  Not when they are aligned
+// to less than their element type, nor when an array that is read shares memory with one that
+// is written (such a request goes through the tensor's own buffers).
+bool DirectOk(const DenseInfo& d, const DeviceRequest& req, size_t gsz, size_t osz) {
+  const size_t n = static_cast<size_t>(d.n_user), nt = static_cast<size_t>(d.n);
+  const void* in = req.push ? req.vals : nullptr;
+  void* out = req.pull ? req.outs : nullptr;
+  if ((reinterpret_cast<uintptr_t>(in) & (gsz - 1)) ||
+      (reinterpret_cast<uintptr_t>(out) & (osz - 1)))
+    return false;
+  if (in && (Clash(in, n, gsz, d.weight, nt, osz) || Clash(in, n, gsz, d.table.master, nt, 4)))
+    return false;
+  if (out && (Clash(in ? in : d.grad, n, gsz, out, n, osz) ||
+              Clash(out, n, osz, d.weight, nt, osz) || Clash(out, n, osz, d.table.master, nt, 4)))
+    return false;
+  for (const float* st : {d.table.state1, d.table.state2})
+    if (st && ((in && Clash(in, n, gsz, st, nt, 4)) || (out && Clash(out, n, osz, st, nt, 4))))
+      return false;
+  return true;
+}
 }  // namespace
 
 bool Plane::Claims(int app_id, const SArray<Key>& keys) {
@@ -1350,6 +1383,16 @@ void Plane::Submit(const DeviceRequest& req) {
     size_t eoff = 0;  // position in the request's value list, in elements
     for (const Run& r : runs) {
       const size_t cnt = static_cast<size_t>(r.end - r.begin);
+      if (W == 1 && !m.sim && DirectOk(*d, req, gsz, osz)) {
+        // one rank: the kernel reads and writes the caller's arrays, nobody else needs the
+        // values in the arena
+        const char* src = req.push && vals != grad ? vals : nullptr;
+        char* dst = req.pull && outs && outs != weight ? outs : nullptr;
+        const int rc = m.rt.dense_op_direct(&m.ws, &t, op, r.begin, pad8(r.end), &opt, d->channel,
+                                            d->num_ctas, s, src, dst, d->n_user);
+        CHECK_EQ(rc, 0) << "psdev_dense_op_direct failed";
+        continue;
+      }
       if (req.push && vals + eoff * gsz != grad + r.begin * gsz) {
         CHECK_EQ(m.rt.memcpy_async(grad + r.begin * gsz, vals + eoff * gsz, cnt * gsz, s), 0);
       }

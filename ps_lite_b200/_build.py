@@ -1,11 +1,13 @@
 """In-tree build of the native libraries.
 
-Two shared objects are produced under ``ps_lite_b200/lib``:
+Three shared objects are produced under ``ps_lite_b200/lib``:
 
 * ``libpsb200_device.so`` -- the sm_100a CUDA data plane (``src/kernels``, ``src/device``),
   exported through the C ABI of ``include/ps/device/psdev.h``.
 * ``libpsb200_core.so`` -- the C++17 host runtime (``src/core``, ``src/van``, ``src/capi``):
   wire codec, vans, Postoffice, Customer, KV apps, exported through ``src/capi/ps_c_api.h``.
+* ``psb200_torch.so`` -- the Python extension module with the native gradient hooks
+  (``src/torch``), against torch's C++ API.
 
 Both are plain ``nvcc`` / ``g++`` invocations (no JIT cache): the built files sit next to
 the sources so that a snapshot of the tree is runnable as is.  The counterpart in the
@@ -60,13 +62,30 @@ def _headers_stamp(dirs=("include", "src")) -> str:
     return h.hexdigest()[:16]
 
 
+def _flags(src: Path, extra: tuple) -> list[str]:
+    return [*(NVCC_FLAGS if src.suffix == ".cu" else CXX_FLAGS), *extra]
+
+
+def _object(src: Path, stamp: str, extra: tuple = (), obj_dir: Path = OBJ_DIR) -> Path:
+    """Where the object of `src` goes; the name says what it was made from."""
+    flag_text = " ".join(_flags(src, extra)).replace(str(ROOT), "")
+    tag = hashlib.sha1(src.read_bytes() + stamp.encode() + flag_text.encode()).hexdigest()[:12]
+    return obj_dir / f"{src.stem}.{tag}.o"
+
+
+def _linked_from(out: Path, objs: list[Path]) -> bool:
+    """Whether `out` was linked from exactly these objects.  They need not exist any more: a
+    snapshot of the tree carries the libraries without the objects."""
+    manifest = out.with_suffix(".manifest")
+    return out.exists() and manifest.exists() and \
+        manifest.read_text() == "\n".join(o.name for o in objs)
+
+
 def _compile_one(src: Path, stamp: str, verbose: bool, extra: tuple = (),
                  obj_dir: Path = OBJ_DIR) -> Path:
-    flags = [*(NVCC_FLAGS if src.suffix == ".cu" else CXX_FLAGS), *extra]
-    flag_text = " ".join(flags).replace(str(ROOT), "")
-    tag = hashlib.sha1(src.read_bytes() + stamp.encode() + flag_text.encode()).hexdigest()[:12]
+    flags = _flags(src, extra)
     obj_dir.mkdir(parents=True, exist_ok=True)
-    obj = obj_dir / f"{src.stem}.{tag}.o"
+    obj = _object(src, stamp, extra, obj_dir)
     if obj.exists():
         return obj
     for old in obj_dir.glob(f"{src.stem}.*.o"):
@@ -86,9 +105,7 @@ def _compile_one(src: Path, stamp: str, verbose: bool, extra: tuple = (),
 
 
 def _link(objs: list[Path], out: Path, cuda: bool, extra: list[str]) -> None:
-    manifest = out.with_suffix(".manifest")
-    want = "\n".join(o.name for o in objs)
-    if out.exists() and manifest.exists() and manifest.read_text() == want:
+    if _linked_from(out, objs):
         return
     if cuda:
         cmd = [NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a",
@@ -106,7 +123,7 @@ def _link(objs: list[Path], out: Path, cuda: bool, extra: list[str]) -> None:
         r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
-    manifest.write_text(want)
+    out.with_suffix(".manifest").write_text("\n".join(o.name for o in objs))
 
 
 @contextlib.contextmanager
@@ -141,9 +158,11 @@ def _build_device(verbose: bool, checks: bool = False) -> Path:
     stamp = _headers_stamp(("include/ps/device", "src/kernels", "src/device"))
     extra = ("-DPSDEV_CHECKS=1",) if checks else ()
     obj_dir = ROOT / "build" / "obj_checks" if checks else OBJ_DIR
+    out = LIB_DIR / ("libpsb200_device_checks.so" if checks else "libpsb200_device.so")
+    if _linked_from(out, [_object(s, stamp, extra, obj_dir) for s in srcs]):
+        return out
     with ThreadPoolExecutor(max_workers=min(8, len(srcs) or 1)) as ex:
         objs = list(ex.map(lambda s: _compile_one(s, stamp, verbose, extra, obj_dir), srcs))
-    out = LIB_DIR / ("libpsb200_device_checks.so" if checks else "libpsb200_device.so")
     _link(objs, out, cuda=True, extra=[])
     return out
 
@@ -159,11 +178,38 @@ def _build_core(verbose: bool) -> Path | None:
     if not srcs:
         return None
     stamp = _headers_stamp()
+    out = LIB_DIR / "libpsb200_core.so"
+    if _linked_from(out, [_object(s, stamp) for s in srcs]):
+        return out
     with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
         objs = list(ex.map(lambda s: _compile_one(s, stamp, verbose), srcs))
-    out = LIB_DIR / "libpsb200_core.so"
     _link(objs, out, cuda=False, extra=[])
     return out
+
+
+def build_torch(verbose: bool = False) -> Path:
+    """Compile psb200_torch.so, the extension module that hangs native gradient hooks into torch's
+    autograd (``src/torch``)."""
+    import sysconfig
+
+    import torch
+    root = Path(torch.__file__).parent
+    with _build_lock():
+        srcs = _sources("src/torch", exts=(".cc",))
+        stamp = _headers_stamp(("include/ps/device",)) + torch.__version__
+        incs = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include",
+                sysconfig.get_paths()["include"], Path(NVCC).resolve().parent.parent / "include"]
+        extra = ("-Wno-unused", "-DTORCH_EXTENSION_NAME=psb200_torch",
+                 *(a for p in incs for a in ("-isystem", str(p))))
+        out = LIB_DIR / "psb200_torch.so"
+        if _linked_from(out, [_object(s, stamp, extra) for s in srcs]):
+            return out
+        objs = [_compile_one(s, stamp, verbose, extra) for s in srcs]
+        _link(objs, out, cuda=False,
+              extra=["-L", str(root / "lib"), f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python",
+                     "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
+                     "-L", str(Path(NVCC).resolve().parent.parent / "lib64"), "-lcudart"])
+        return out
 
 
 def build_all(verbose: bool = False) -> dict[str, str]:
@@ -171,6 +217,7 @@ def build_all(verbose: bool = False) -> dict[str, str]:
     core = build_core(verbose)
     if core:
         res["core"] = str(core)
+    res["torch"] = str(build_torch(verbose))
     return res
 
 

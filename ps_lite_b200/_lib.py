@@ -161,6 +161,27 @@ def device_lib() -> C.CDLL:
         return _device_lib
 
 
+_torch_ext = None
+
+
+def torch_ext():
+    """Load (building first if needed) the extension module with the native gradient hooks."""
+    global _torch_ext
+    with _lock:
+        if _torch_ext is None:
+            import importlib.util
+
+            from . import _build
+            path = _build.LIB_DIR / "psb200_torch.so"
+            if os.environ.get("PSB200_NO_BUILD") != "1" or not path.exists():
+                path = _build.build_torch()
+            spec = importlib.util.spec_from_file_location("psb200_torch", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _torch_ext = module
+        return _torch_ext
+
+
 def check(code: int, what: str) -> None:
     if code != 0:
         raise PsdevError(int(code), what)

@@ -12,6 +12,8 @@ and that its users build on ``KVWorker::Push/Pull`` with per-message priorities
   its slices to a priority scheduler; slices are at most ``slice_bytes`` long (4 MB by
   default) and their priority is the reverse of the layer order, so the weights the next
   forward pass needs first are exchanged first among the slices that are pending;
+* on one rank there is nothing to exchange: native hooks (src/torch/grad_exchange.cc) collect the
+  gradient tensors as they are, and the update kernel reads them where they lie;
 * slices are exchanged by fused push+pull kernels on a side stream, overlapping the rest of
   backward: as soon as ``batch_bytes`` (4 MiB by default, ``PSB200_BATCH_BYTES``) of gradients
   are pending, everything pending goes out in ONE launch whose CTAs take the slices in priority
@@ -23,7 +25,9 @@ gradient hooks fire, which is the same on every rank for the same model.
 """
 from __future__ import annotations
 
+import ctypes as C
 import heapq
+import weakref
 from typing import Iterable, List, Optional, Tuple
 
 import torch
@@ -121,9 +125,42 @@ class DistributedOptimizer:
         # a parameter's storage is its slice of the pulled-weight buffer
         for p, o in zip(self.params, self.offsets):
             p.data = self.table.weight[o:o + p.numel()].view(p.shape)
-        self._hooks = [p.register_post_accumulate_grad_hook(self._make_hook(i))
-                       for i, p in enumerate(self.params)]
+        self._hooks, self._native = [], None
+        if self._native_ok(grad_dtype):
+            self._native = self._make_native(channel, slice_bytes // gsz)
+        else:
+            self._hooks = [p.register_post_accumulate_grad_hook(self._make_hook(i))
+                           for i, p in enumerate(self.params)]
         self._pending_step = False
+
+    def _native_ok(self, grad_dtype) -> bool:
+        """One rank, gradients in a type that the update kernel reads in place, and batching on
+        (``batch_bytes=0`` asks for a launch per slice)."""
+        return (self.heap.world == 1 and not self.heap.emulated_ranks and self.batch_bytes > 0 and
+                grad_dtype in (torch.float32, torch.bfloat16) and
+                all(p.is_cuda for p in self.params))
+
+    def _make_native(self, channel: int, slice_elems: int):
+        t = self.table
+        self._opt = opt = _lib.Opt()
+        me = weakref.ref(self)   # (the native object must not keep its owner alive)
+
+        def begin_step():
+            t.step = me().steps + 1
+            C.memmove(C.byref(opt), C.byref(t._opt_struct()), C.sizeof(opt))
+
+        fn = C.cast(self.heap.lib.psdev_dense_op_segs, C.c_void_p).value
+        # reverse layer order, published parameters last (on one rank publishing is the same
+        # store into this rank's weight buffer)
+        pri = [-1 - i if self._publish[i] else len(self.params) - i
+               for i in range(len(self.params))]
+        # `num_ctas` bounds the CTAs that wait for peers while a backward pass needs the SMs; with
+        # one rank the update is a pass over memory, shortest on the whole GPU
+        return _lib.torch_ext().GradExchange(
+            self.params, self.offsets, pri, t.grad, C.addressof(t._world), C.addressof(t._table),
+            C.addressof(self._opt), fn, self.comm.cuda_stream if self.comm else 0,
+            self.comm is not None, max(1, self.batch_bytes // self._gsz),
+            max(8, int(slice_elems) & ~7), channel, begin_step)
 
     def _make_hook(self, index: int):
         n_params = len(self.params)
@@ -202,6 +239,11 @@ class DistributedOptimizer:
     def step(self) -> None:
         """Finish the exchange of this step's gradients; afterwards the parameters hold the
         weights for the next forward pass (except published ones, which their GEMM pulls)."""
+        if self._native is not None:
+            self._native.step()
+            self.launches, self.launched_slices = self._native.launches, self._native.slices
+            self.steps += 1
+            return
         self._drain()
         if self.comm is not None:
             torch.cuda.current_stream(self.heap.device).wait_stream(self.comm)
@@ -221,6 +263,9 @@ class DistributedOptimizer:
         for h in self._hooks:
             h.remove()
         self._hooks = []
+        if self._native is not None:
+            self._native.detach()
+            self._native = None
         torch.cuda.synchronize(self.heap.device)
         self.table.free()
 

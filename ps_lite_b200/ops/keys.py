@@ -5,6 +5,7 @@ Device counterparts of the reference's ``ParallelSort`` and ``ParallelOrderedMat
 operators (assign_op.h:12-21)."""
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional, Tuple
 
 import torch
@@ -18,8 +19,7 @@ def sort_keys(keys: torch.Tensor, key_bits: int = 64, return_perm: bool = False,
               check: bool = False) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """Sort uint64 keys (stored as int64 bit patterns) ascending, in place; keys must be below
     ``2**key_bits``.  With ``return_perm`` also returns the stable permutation (int32 indices
-    into the input).  ``check`` waits for the sort and raises if one of its bounded waits (a
-    tile looking back at the tiles before it) ran out."""
+    into the input).  ``check`` waits for the sort and raises if it failed."""
     assert keys.is_cuda and keys.dtype == torch.int64 and keys.is_contiguous()
     lib = _lib.device_lib()
     n = keys.numel()
@@ -37,10 +37,39 @@ def sort_keys(keys: torch.Tensor, key_bits: int = 64, return_perm: bool = False,
     return keys, perm
 
 
+def _unique_sum_fp32(keys, vals, key_bits):
+    """The native form; None when a key is wider than ``key_bits`` (only its low bits sort then)."""
+    lib, n = _lib.device_lib(), keys.numel()
+    stream = torch.cuda.current_stream(keys.device).cuda_stream
+    nbytes = lib.psdev_unique_sum_scratch_bytes(n, key_bits)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=keys.device)
+    count = C.c_int64()
+    rc = lib.psdev_unique_sum_sort(keys.data_ptr(), vals.data_ptr(), n, key_bits,
+                                   scratch.data_ptr(), nbytes, C.byref(count), stream)
+    if rc == -1:
+        return None
+    _lib.check(rc, "psdev_unique_sum_sort")
+    u = count.value
+    uk = torch.empty(u, dtype=torch.int64, device=keys.device)
+    out = torch.empty(u, dtype=torch.float32, device=keys.device)
+    _lib.check(lib.psdev_unique_sum_write(scratch.data_ptr(), n, key_bits, u, uk.data_ptr(),
+                                          out.data_ptr(), stream), "psdev_unique_sum_write")
+    return uk, out
+
+
 def sort_unique_sum(keys: torch.Tensor, vals: torch.Tensor, key_bits: int = 64
                     ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Turn arbitrary (key, value) pairs into the sorted unique keys a push needs, summing the
-    values of repeated keys."""
+    values of repeated keys; keys must be below ``2**key_bits``.  fp32 values travel with the
+    keys through the sort and are summed by a kernel of their own; other types take the sort
+    permutation and torch's ``index_add_``."""
+    n = keys.numel()
+    if (vals.dtype == torch.float32 and vals.dim() == 1 and vals.numel() == n and
+            not (vals.requires_grad and torch.is_grad_enabled()) and
+            0 < n < 1 << 30 and keys.dtype == torch.int64 and keys.is_cuda and vals.is_cuda):
+        got = _unique_sum_fp32(keys.contiguous(), vals.contiguous(), key_bits)
+        if got is not None:
+            return got
     k = keys.clone()
     k, perm = sort_keys(k, key_bits, return_perm=True)
     v = vals[perm.long()]

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <utility>
 
 #include "ps/device/psdev.h"
 
@@ -20,44 +21,48 @@ namespace psdev {
 extern std::atomic<uint64_t> g_launches;
 
 namespace sortk {
-// Least-significant-digit radix sort with 8-bit digits, one sweep per pass:
-//   digit_hist   reads the keys once and counts the digits of EVERY pass (shared-memory atomics,
-//                then one global add per digit and CTA);
-//   digit_scan   exclusive prefix of each pass's 256 totals -> where each digit's run starts;
-//   sweep        one launch per pass.  A CTA takes the next tile of 4096 keys from a counter (so
-//                every earlier tile belongs to a CTA that is already running), ranks each key
-//                among the keys of the same digit in the tile, in input order (the sort is
-//                stable), publishes the tile's 256 digit counts, and finds how many keys of each
-//                digit precede the tile by looking back over the earlier tiles' published words:
-//                a tile's own counts ("aggregate") until one is met whose word already holds the
-//                whole prefix ("inclusive").  Keys (and payloads) are then put in sorted order
-//                inside the tile in shared memory and stored, runs of equal digits to consecutive
-//                addresses.
+// Least-significant-digit radix sort with 8-bit digits.  The keys are cut into a few hundred
+// contiguous chunks, one per CTA that fits on the GPU at a time, and a pass is three launches:
+//   digit_count  counts the digits of every chunk;
+//   digit_scan   turns the counts of each digit into how many keys of the chunks before have it;
+//   scatter      takes its chunk tile by tile: ranks each key among the keys of the same digit in
+//                input order (the sort is stable), puts the tile in sorted order in shared
+//                memory and stores runs of equal digits to consecutive addresses.
 // ceil(key_bits / 8) passes: a caller that knows its keys are below 2^30 pays four passes,
-// not eight.  Per pass every key is read once and written once.
-constexpr int kThreads = 256;
+// not eight.  No CTA ever waits for another one.
+//
+// Up to some ten million keys everything stays in L2 and a pass is bound by latencies.  The
+// single-sweep form (one launch per pass, tiles finding their offsets by looking back over the
+// words that earlier tiles publish) spent a third of its time in the look-back and another third
+// in a second wave of tiles: 54 us per pass on 2^22 keys of 30 bits with a payload, against 41 us
+// for these three launches (5.5 + 2.2 + 33).  What bounds the scatter now is the shared-memory
+// pipe: some 45 wavefronts per 32 keys, half of them bank conflicts of random digits.
+constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kItems = 16;                 // keys per thread
-constexpr int kTile = kThreads * kItems;   // keys per CTA
+constexpr int kItems = 8;                  // keys per thread and tile
+constexpr int kTile = kThreads * kItems;
 constexpr int kRadixBits = 8;
 constexpr int kDigits = 1 << kRadixBits;
-constexpr int kMaxPasses = 64 / kRadixBits;
+constexpr int kMaxChunks = 2 * 148;        // two CTAs per SM
 
-// one word per (tile, digit): 2 flag bits and a 30-bit count
-constexpr unsigned int kFlagAggregate = 1u << 30;
-constexpr unsigned int kFlagInclusive = 2u << 30;
-constexpr unsigned int kCountMask = (1u << 30) - 1;
-constexpr unsigned long long kLookbackNs = 2000000000ull;  // bound of one look-back wait
-
-// Head of the scratch memory, cleared before every sort.
+// Head of the scratch memory.
 struct SortHead {
-  int error;                                   // 1: a look-back wait ran out
-  unsigned int next_tile[kMaxPasses];          // tile counter of each pass
-  unsigned int pad[23];
-  unsigned int hist[kMaxPasses * kDigits];     // digit totals, then (digit_scan) run starts
+  int too_wide;                            // 1: a key has bits beyond key_bits
 };
 
-__device__ __forceinline__ unsigned int digit_of(unsigned long long k, int shift) {
+// The chunks of n keys: `tiles` tiles each, the last ones possibly fewer.
+struct Chunks {
+  int count;
+  int tiles;
+};
+__host__ __device__ inline Chunks chunks_of(long long n) {
+  const long long ntiles = (n + kTile - 1) / kTile;
+  const long long per = (ntiles + kMaxChunks - 1) / kMaxChunks;
+  return Chunks{(int)((ntiles + per - 1) / per), (int)per};
+}
+
+template <typename K>
+__device__ __forceinline__ unsigned int digit_of(K k, int shift) {
   return (unsigned int)((k >> shift) & (kDigits - 1));
 }
 __device__ __forceinline__ unsigned int lanemask_lt() {
@@ -65,202 +70,500 @@ __device__ __forceinline__ unsigned int lanemask_lt() {
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
   return m;
 }
-__device__ __forceinline__ unsigned int ld_relaxed(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(unsigned int* p, unsigned int v) {
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 
-// Lanes of the warp whose (valid, digit) equal this lane's: one ballot per digit bit.
-__device__ __forceinline__ unsigned int peers_of(unsigned int d, bool valid) {
-  unsigned int m = __ballot_sync(0xffffffffu, valid);
-  if (!valid) m = ~m;
+// Exclusive prefix sum of one value per thread over a CTA of kThreads; `part`: kWarps words of
+// shared memory, free again after the next __syncthreads.
+__device__ __forceinline__ unsigned int cta_exclusive(unsigned int v, unsigned int* part,
+                                                      unsigned int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned int incl = v;
 #pragma unroll
-  for (int b = 0; b < kRadixBits; ++b) {
-    const bool bit = (d >> b) & 1u;
-    const unsigned int v = __ballot_sync(0xffffffffu, bit);
-    m &= bit ? v : ~v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
   }
-  return m;
-}
-
-// hist[pass * 256 + d] += keys whose digit of that pass is d
-__global__ void __launch_bounds__(kThreads)
-    digit_hist_kernel(const unsigned long long* keys, long long n, int passes, unsigned int* hist) {
-  __shared__ unsigned int s[kMaxPasses * kDigits];
-  for (int i = threadIdx.x; i < passes * kDigits; i += kThreads) s[i] = 0;
+  if (lane == 31) part[warp] = incl;
   __syncthreads();
-  // four independent loads in flight per thread
-  const long long stride = (long long)gridDim.x * kThreads;
-  for (long long i0 = blockIdx.x * (long long)kThreads + threadIdx.x; i0 < n; i0 += 4 * stride) {
-    unsigned long long k[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) k[u] = i0 + u * stride < n ? keys[i0 + u * stride] : 0ull;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (i0 + u * stride < n)
-        for (int p = 0; p < passes; ++p)
-          atomicAdd(&s[p * kDigits + digit_of(k[u], p * kRadixBits)], 1u);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < passes * kDigits; i += kThreads)
-    if (s[i]) atomicAdd(&hist[i], s[i]);
-}
-
-// One CTA per pass: totals -> exclusive prefix (the output index where each digit's run starts).
-__global__ void __launch_bounds__(kDigits) digit_scan_kernel(unsigned int* hist) {
-  __shared__ unsigned int s[kDigits];
-  unsigned int* row = hist + blockIdx.x * kDigits;
-  const unsigned int mine = row[threadIdx.x];
-  s[threadIdx.x] = mine;
-  __syncthreads();
-  unsigned int incl = mine;
-  for (int off = 1; off < kDigits; off <<= 1) {
-    const unsigned int v = threadIdx.x >= off ? s[threadIdx.x - off] : 0u;
-    __syncthreads();
-    incl += v;
-    s[threadIdx.x] = incl;
-    __syncthreads();
-  }
-  row[threadIdx.x] = incl - mine;
-}
-
-// One pass.  Shared memory: the tile's keys and payloads in sorted order, per-warp digit
-// counters, and two 256-entry tables.
-constexpr int kSweepSmem = kTile * 8 + kTile * 4 + kWarps * kDigits * 2 + 2 * kDigits * 4;
-
-__global__ void __launch_bounds__(kThreads, 4)
-    sweep_kernel(const unsigned long long* keys_in, unsigned long long* keys_out,
-                 const unsigned int* pay_in, unsigned int* pay_out, long long n, int shift,
-                 const unsigned int* run_start, unsigned int* status, unsigned int* next_tile,
-                 int* error) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  unsigned long long* skeys = reinterpret_cast<unsigned long long*>(smem_raw);
-  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + kTile * 8);
-  // cnt[w][d]: first the number of keys with digit d seen so far by warp w, afterwards the
-  // position inside the tile's digit-d run of that warp's first key with digit d
-  // (16 bits are enough: a warp holds 512 keys, a tile 4096)
-  unsigned short (*cnt)[kDigits] =
-      reinterpret_cast<unsigned short (*)[kDigits]>(smem_raw + kTile * 12);
-  unsigned int* tile_start = reinterpret_cast<unsigned int*>(smem_raw + kTile * 12 +
-                                                             kWarps * kDigits * 2);
-  unsigned int* goff = tile_start + kDigits;  // output index of sorted position q: goff[d] + q
-  __shared__ unsigned int s_tile;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) s_tile = atomicAdd(next_tile, 1u);
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) cnt[w][threadIdx.x] = 0;
-  __syncthreads();
-  const unsigned int tile = s_tile;
-  const long long tile_base = (long long)tile * kTile;
-  const long long base = tile_base + (long long)warp * (32 * kItems) + lane;
-  const int tile_n = (int)(n - tile_base < kTile ? n - tile_base : kTile);
-  unsigned long long k[kItems];
-  unsigned short rank[kItems];
-#pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    const long long i = base + j * 32;
-    k[j] = i < n ? keys_in[i] : ~0ull;
-  }
-#pragma unroll
-  for (int j = 0; j < kItems; ++j) {
-    const bool valid = base + j * 32 < n;
-    const unsigned int d = digit_of(k[j], shift);
-    const unsigned int same = peers_of(d, valid);
-    const unsigned int before = __popc(same & lanemask_lt());
-    unsigned int seen = 0;
-    if (valid) seen = cnt[warp][d];
-    __syncwarp();
-    if (valid && before == 0) cnt[warp][d] = (unsigned short)(seen + __popc(same));
-    __syncwarp();
-    rank[j] = (unsigned short)(seen + before);
-  }
-  __syncthreads();
-  // digit threadIdx.x: each warp's start inside the digit's run, and the run's length
-  unsigned int run = 0;
+  unsigned int before = 0, all = 0;
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) {
-    const unsigned int c = cnt[w][threadIdx.x];
-    cnt[w][threadIdx.x] = (unsigned short)run;
-    run += c;
+    const unsigned int t = part[w];
+    if (w < warp) before += t;
+    all += t;
   }
-  tile_start[threadIdx.x] = run;
-  // publish this tile's count of the digit, then add up the earlier tiles' counts
-  unsigned int* mine = status + (size_t)tile * kDigits + threadIdx.x;
-  unsigned int before_tile = 0;
-  if (tile == 0) {
-    st_relaxed(mine, kFlagInclusive | run);
-  } else {
-    st_relaxed(mine, kFlagAggregate | run);
-    const unsigned int* look = mine - kDigits;
-    unsigned long long t0 = 0;
-    for (unsigned int left = tile; left > 0; --left, look -= kDigits) {
-      unsigned int v = ld_relaxed(look);
-      unsigned int polls = 0;
-      while ((v >> 30) == 0) {
-        // the earlier tile's CTA is running (it took its tile before this one did) but has not
-        // ranked its keys yet
-        if ((++polls & 63u) == 0) {
-          const unsigned long long t = now_ns();
-          if (t0 == 0) t0 = t;
-          if (t - t0 > kLookbackNs) break;
-        }
-        v = ld_relaxed(look);
-      }
-      if ((v >> 30) == 0) {
-        *error = 1;  // the output of this sort is not valid
-        break;
-      }
-      before_tile += v & kCountMask;
-      if (v & kFlagInclusive) break;
-    }
-    st_relaxed(mine, kFlagInclusive | ((before_tile + run) & kCountMask));
-  }
+  if (total) *total = all;
+  return before + incl - v;
+}
+
+// counts[d * chunks + c] = keys of chunk c whose digit is d
+template <typename K>
+__global__ void __launch_bounds__(kThreads, 2)
+    digit_count_kernel(const K* __restrict__ keys, long long n, int shift, Chunks ch,
+                       int key_bits, unsigned int* counts, SortHead* head) {
+  constexpr int kSets = 4;
+  __shared__ unsigned int s[kSets][kDigits];  // four warps share a set of counters
+  unsigned int* mine = s[threadIdx.x / (kThreads / kSets)];
+  for (int i = threadIdx.x; i < kSets * kDigits; i += kThreads) s[0][i] = 0;
   __syncthreads();
-  // exclusive prefix of the run lengths over the digits (256 values, one per thread)
-  {
-    unsigned int incl = run;
-    for (int off = 1; off < kDigits; off <<= 1) {
-      const unsigned int v = threadIdx.x >= off ? tile_start[threadIdx.x - off] : 0u;
-      __syncthreads();
-      incl += v;
-      tile_start[threadIdx.x] = incl;
-      __syncthreads();
-    }
-    const unsigned int excl = incl - run;
-    __syncthreads();
-    tile_start[threadIdx.x] = excl;
-    goff[threadIdx.x] = run_start[threadIdx.x] + before_tile - excl;
+  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
+  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
+  bool wide = false;
+  for (long long base = lo + threadIdx.x; base < hi; base += kTile) {
+    K k[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; ++j)
+      k[j] = base + j * kThreads < hi ? keys[base + j * kThreads] : (K)0;
+#pragma unroll
+    for (int j = 0; j < kItems; ++j)
+      if (base + j * kThreads < hi) {
+        if (sizeof(K) == 8 && key_bits < 64) wide |= (k[j] >> (key_bits & 63)) != 0;
+        atomicAdd(&mine[digit_of(k[j], shift)], 1u);
+      }
   }
+  if (wide) head->too_wide = 1;
   __syncthreads();
+  if (threadIdx.x < kDigits) {
+    unsigned int c = 0;
+#pragma unroll
+    for (int w = 0; w < kSets; ++w) c += s[w][threadIdx.x];
+    counts[(size_t)threadIdx.x * ch.count + blockIdx.x] = c;
+  }
+}
+
+// One CTA per digit: exclusive prefix over the chunks in place, and the digit's total.
+__global__ void __launch_bounds__(kThreads)
+    digit_scan_kernel(unsigned int* counts, int chunks, unsigned int* totals) {
+  __shared__ unsigned int s_part[kWarps];
+  static_assert(kMaxChunks <= kThreads && kDigits <= kThreads, "one thread per chunk, digit");
+  unsigned int* row = counts + (size_t)blockIdx.x * chunks;
+  const unsigned int c = threadIdx.x < chunks ? row[threadIdx.x] : 0;
+  unsigned int total;
+  const unsigned int before = cta_exclusive(c, s_part, &total);
+  if (threadIdx.x < chunks) row[threadIdx.x] = before;
+  if (threadIdx.x == 0) totals[blockIdx.x] = total;
+}
+
+// What travels beside the keys of a pass.
+enum { kNoPayload = 0, kMakeIndex = 1, kPayload = 2 };
+
+template <typename KO>
+constexpr int scatter_smem(int payload) {
+  return kTile * ((int)sizeof(KO) + (payload ? 4 : 0)) +
+         2 * kWarps * kDigits * 4 + 2 * kDigits * 4;
+}
+
+// Rank of each of a thread's keys (index base + 32 j, below hi) among the keys of its warp that
+// have the same digit, in index order; cnt[d] ends up as the number of such keys.
+template <typename K>
+__device__ __forceinline__ void rank_tile(const K* k, long long base, long long hi, int shift,
+                                          unsigned int* cnt, unsigned int* lanes,
+                                          unsigned int* rank) {
 #pragma unroll
   for (int j = 0; j < kItems; ++j) {
-    const long long i = base + j * 32;
-    if (i < n) {
-      const unsigned int d = digit_of(k[j], shift);
-      const unsigned int q = tile_start[d] + cnt[warp][d] + rank[j];
-      skeys[q] = k[j];
-      if (pay_out) spay[q] = pay_in ? pay_in[i] : (unsigned int)i;
+    // the lanes that hold the same digit find each other through a mask in shared memory; the
+    // first of them advances the warp's counter for all of them
+    const bool valid = base + j * 32 < hi;
+    const unsigned int d = digit_of(k[j], shift);
+    if (valid) atomicOr(&lanes[d], 1u << (threadIdx.x & 31));
+    __syncwarp();
+    const unsigned int same = valid ? lanes[d] : 1u << (threadIdx.x & 31);
+    const unsigned int before = __popc(same & lanemask_lt());
+    unsigned int r = 0;
+    __syncwarp();
+    if (valid && before == 0) {
+      lanes[d] = 0;
+      r = cnt[d];
+      cnt[d] = r + __popc(same);
+    }
+    rank[j] = __shfl_sync(0xffffffffu, r, __ffs(same) - 1) + before;
+    __syncwarp();
+  }
+}
+
+// KI, KO: type of the keys as read and as written (a sort of short keys narrows them in its first
+// pass).  Shared memory: the tile's keys and payloads in sorted order, per-warp digit counters
+// and lane masks, and two 256-entry tables.
+template <typename KI, typename KO, int PAY>
+__global__ void __launch_bounds__(kThreads, 2)
+    scatter_kernel(const KI* __restrict__ keys_in, KO* __restrict__ keys_out,
+                   const unsigned int* __restrict__ pay_in, unsigned int* __restrict__ pay_out,
+                   long long n, int shift, Chunks ch, const unsigned int* __restrict__ prefix,
+                   const unsigned int* __restrict__ totals) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  KO* skeys = reinterpret_cast<KO*>(smem_raw);
+  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + kTile * sizeof(KO));
+  // cnt[w][d]: first the number of keys with digit d seen so far by warp w, afterwards the
+  // sorted position in the tile of that warp's first key with digit d
+  unsigned int (*cnt)[kDigits] = reinterpret_cast<unsigned int (*)[kDigits]>(
+      smem_raw + kTile * sizeof(KO) + (PAY ? kTile * 4 : 0));
+  // lanes[w][d]: lanes of warp w whose present key has digit d; zero in between
+  unsigned int (*lanes)[kDigits] = cnt + kWarps;
+  unsigned int* goff = &lanes[kWarps][0];  // output index of sorted position q: goff[d] + q
+  __shared__ unsigned int s_part[2][kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // output index of the chunk's next key with digit threadIdx.x
+  const bool digit = threadIdx.x < kDigits;
+  unsigned int next = cta_exclusive(digit ? totals[threadIdx.x] : 0, s_part[0], nullptr);
+  if (digit) next += prefix[(size_t)threadIdx.x * ch.count + blockIdx.x];
+  for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) lanes[0][i] = 0;
+  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
+  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
+  // A tile is loaded before the one before it is stored: its keys and payloads take the registers
+  // of those that have gone to shared memory.
+  KO k[kItems];
+  unsigned int pay[kItems];
+  auto load = [&](long long base) {
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      const long long i = base + j * 32;
+      k[j] = i < hi ? (KO)keys_in[i] : (KO)~0ull;
+      if constexpr (PAY == kPayload) pay[j] = i < hi ? pay_in[i] : 0u;
+      else pay[j] = (unsigned int)i;
+    }
+  };
+  load(lo + (long long)warp * (32 * kItems) + lane);
+  for (long long tile_base = lo; tile_base < hi; tile_base += kTile) {
+    const long long base = tile_base + (long long)warp * (32 * kItems) + lane;
+    const int tile_n = (int)(hi - tile_base < kTile ? hi - tile_base : kTile);
+    unsigned int rank[kItems];
+    for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) cnt[0][i] = 0;
+    __syncthreads();
+    rank_tile(k, base, hi, shift, cnt[warp], lanes[warp], rank);
+    __syncthreads();
+    // digit threadIdx.x: where its run starts in the tile, and each warp's part of it
+    unsigned int run = 0;
+    if (digit) {
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) run += cnt[w][threadIdx.x];
+    }
+    const unsigned int start = cta_exclusive(run, s_part[1], nullptr);
+    if (digit) {
+      unsigned int at = start;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const unsigned int c = cnt[w][threadIdx.x];
+        cnt[w][threadIdx.x] = at;
+        at += c;
+      }
+      goff[threadIdx.x] = next - start;
+      next += run;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      if (base + j * 32 < hi) {
+        const unsigned int q = cnt[warp][digit_of(k[j], shift)] + rank[j];
+        skeys[q] = k[j];
+        if constexpr (PAY != kNoPayload) spay[q] = pay[j];
+      }
+    }
+    load(base + kTile);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      const int q = threadIdx.x + j * kThreads;
+      if (q < tile_n) {
+        const KO key = skeys[q];
+        const unsigned int p = goff[digit_of(key, shift)] + (unsigned int)q;
+        keys_out[p] = key;
+        if constexpr (PAY != kNoPayload) pay_out[p] = spay[q];
+      }
     }
   }
-  __syncthreads();
-#pragma unroll 4
-  for (int j = 0; j < kItems; ++j) {
-    const int q = threadIdx.x + j * kThreads;
-    if (q < tile_n) {
-      const unsigned long long key = skeys[q];
-      const unsigned int p = goff[digit_of(key, shift)] + (unsigned int)q;
-      keys_out[p] = key;
-      if (pay_out) pay_out[p] = spay[q];
+}
+
+// All passes of a sort of at most one tile in one launch of one CTA (the three launches per pass of
+// the general form take longer than the work: 2^12 keys of 24 bits, with the sums of equal
+// keys, 111 us in nine launches).  `unique`: receives the number of distinct keys, or NULL.
+template <typename KI, typename K, int PAY>
+__global__ void __launch_bounds__(kThreads)
+    small_sort_kernel(const KI* keys_in, K* keys_out, const unsigned int* pay_in,
+                      unsigned int* pay_out, int n, int passes, int key_bits, SortHead* head,
+                      unsigned int* unique) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  K* skeys = reinterpret_cast<K*>(smem_raw);
+  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + kTile * sizeof(K));
+  unsigned int (*cnt)[kDigits] = reinterpret_cast<unsigned int (*)[kDigits]>(
+      smem_raw + kTile * sizeof(K) + (PAY ? kTile * 4 : 0));
+  unsigned int (*lanes)[kDigits] = cnt + kWarps;
+  __shared__ unsigned int s_part[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int base = warp * (32 * kItems) + lane;
+  bool wide = false;
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    const KI k = keys_in[i];
+    if (sizeof(KI) == 8 && key_bits < 64) wide |= (k >> (key_bits & 63)) != 0;
+    skeys[i] = (K)k;
+    if constexpr (PAY != kNoPayload) spay[i] = PAY == kPayload ? pay_in[i] : (unsigned int)i;
+  }
+  if (wide) head->too_wide = 1;
+  for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) lanes[0][i] = 0;
+  for (int pass = 0; pass < passes; ++pass) {
+    const int shift = pass * kRadixBits;
+    for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) cnt[0][i] = 0;
+    __syncthreads();
+    K k[kItems];
+    unsigned int pay[kItems], rank[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      k[j] = base + j * 32 < n ? skeys[base + j * 32] : (K)~0ull;
+      pay[j] = PAY != kNoPayload && base + j * 32 < n ? spay[base + j * 32] : 0;
     }
+    rank_tile(k, base, n, shift, cnt[warp], lanes[warp], rank);
+    __syncthreads();
+    unsigned int run = 0;
+    if (threadIdx.x < kDigits) {
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) run += cnt[w][threadIdx.x];
+    }
+    unsigned int at = cta_exclusive(run, s_part, nullptr);
+    if (threadIdx.x < kDigits) {
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const unsigned int c = cnt[w][threadIdx.x];
+        cnt[w][threadIdx.x] = at;
+        at += c;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      if (base + j * 32 < n) {
+        const unsigned int q = cnt[warp][digit_of(k[j], shift)] + rank[j];
+        skeys[q] = k[j];
+        if constexpr (PAY != kNoPayload) spay[q] = pay[j];
+      }
+    }
+    __syncthreads();
+  }
+  unsigned int heads = 0;
+  for (int i = threadIdx.x; i < n; i += kThreads) {
+    keys_out[i] = skeys[i];
+    if constexpr (PAY != kNoPayload) pay_out[i] = spay[i];
+    heads += i == 0 || skeys[i] != skeys[i - 1];
+  }
+  if (unique) {
+    unsigned int total;
+    cta_exclusive(heads, s_part, &total);
+    if (threadIdx.x == 0) *unique = total;
+  }
+}
+
+static size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// Working memory of a sort: the head and one set of counts and totals (passes follow each other
+// on one stream).
+struct SortWork {
+  SortHead* head;
+  unsigned int* counts;
+  unsigned int* totals;
+  static size_t bytes(long long n) {
+    return round256(sizeof(SortHead)) + round256((size_t)kDigits * chunks_of(n).count * 4) +
+           round256(kDigits * 4);
+  }
+  SortWork(char* p, long long n) {
+    head = reinterpret_cast<SortHead*>(p);
+    p += round256(sizeof(SortHead));
+    counts = reinterpret_cast<unsigned int*>(p);
+    p += round256((size_t)kDigits * chunks_of(n).count * 4);
+    totals = reinterpret_cast<unsigned int*>(p);
+  }
+};
+
+// Dynamic shared memory beyond the default limit, once per kernel and device.
+template <auto Kernel>
+static int allow_smem(int bytes) {
+  static std::atomic<bool> set[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!set[dev & 63].load(std::memory_order_acquire)) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return (int)e;
+    set[dev & 63].store(true, std::memory_order_release);
+  }
+  return 0;
+}
+
+template <typename KI, typename K, int PAY>
+static int small_sort(const KI* in, K* out, const unsigned int* pin, unsigned int* pout, int n,
+                      int passes, int key_bits, SortHead* head, unsigned int* unique,
+                      cudaStream_t s) {
+  if (int rc = allow_smem<small_sort_kernel<KI, K, PAY>>(scatter_smem<K>(PAY))) return rc;
+  small_sort_kernel<KI, K, PAY><<<1, kThreads, scatter_smem<K>(PAY), s>>>(
+      in, out, pin, pout, n, passes, key_bits, head, unique);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return 0;
+}
+
+template <typename KI, typename KO, int PAY>
+static int sort_pass(const KI* in, KO* out, const unsigned int* pin, unsigned int* pout,
+                     long long n, int pass, int key_bits, const SortWork& w, cudaStream_t s) {
+  if (int rc = allow_smem<scatter_kernel<KI, KO, PAY>>(scatter_smem<KO>(PAY))) return rc;
+  const Chunks ch = chunks_of(n);
+  const int shift = pass * kRadixBits;
+  digit_count_kernel<KI><<<ch.count, kThreads, 0, s>>>(in, n, shift, ch, pass ? 64 : key_bits,
+                                                       w.counts, w.head);
+  digit_scan_kernel<<<kDigits, kThreads, 0, s>>>(w.counts, ch.count, w.totals);
+  scatter_kernel<KI, KO, PAY><<<ch.count, kThreads, scatter_smem<KO>(PAY), s>>>(
+      in, out, pin, pout, n, shift, ch, w.counts, w.totals);
+  g_launches.fetch_add(3, std::memory_order_relaxed);
+  return 0;
+}
+
+// ---- sums of the values of equal keys --------------------------------------------------------
+// On sorted (key, value) pairs, in two kernels with the allocation of the outputs between them:
+// unique_count counts the first occurrences in each chunk, unique_sum writes every distinct key
+// and the sum of its values.  Their chunks are smaller than those of the sort (a CTA has little
+// to do per pair): up to 2048, as many counts as unique_sum adds up at its start.
+constexpr int kMaxUniqueChunks = 2048;
+__host__ __device__ inline Chunks unique_chunks_of(long long n) {
+  const long long ntiles = (n + kTile - 1) / kTile;
+  const long long per = (ntiles + kMaxUniqueChunks - 1) / kMaxUniqueChunks;
+  return Chunks{(int)((ntiles + per - 1) / per), (int)per};
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kThreads, 2)
+    unique_count_kernel(const K* __restrict__ keys, long long n, Chunks ch, unsigned int* counts) {
+  __shared__ unsigned int s_part[kWarps];
+  const int lane = threadIdx.x & 31;
+  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
+  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
+  unsigned int heads = 0;
+  for (long long base = lo + threadIdx.x; base - lane < hi; base += kTile) {
+    K k[kItems], before[kItems];  // before: of lane 0, the last key of the warp's neighbour
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      const long long i = base + j * kThreads;
+      k[j] = i < hi ? keys[i] : (K)0;
+      before[j] = lane == 0 && i > 0 && i < hi ? keys[i - 1] : (K)0;
+    }
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      const long long i = base + j * kThreads;
+      const K up = __shfl_up_sync(0xffffffffu, k[j], 1);
+      heads += i < hi && (i == 0 || k[j] != (lane ? up : before[j]));
+    }
+  }
+  unsigned int total;
+  cta_exclusive(heads, s_part, &total);
+  if (threadIdx.x == 0) counts[blockIdx.x] = total;
+}
+
+// Each thread walks kPer consecutive pairs of a round and adds up what belongs to one key; a
+// segmented scan over the threads carries open sums on, so that a key that fills whole chunks
+// costs no atomics inside one.  Keys that begin and end inside a round are stored; what is open at
+// either end of a round is added to its (cleared) output, two global atomics per round.
+constexpr int kUniquePer = 8;
+template <typename K>
+__global__ void __launch_bounds__(kThreads, 2)
+    unique_sum_kernel(const K* __restrict__ keys, const float* __restrict__ vals, long long n,
+                      Chunks ch, const unsigned int* __restrict__ counts,
+                      unsigned long long* out_keys, float* out_sums) {
+  constexpr int kPer = kUniquePer;
+  constexpr int kRound = kThreads * kPer;
+  constexpr int kPadded = kRound + kRound / kPer;  // (a thread's pairs start in different banks)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  K* skey = reinterpret_cast<K*>(smem_raw);
+  K* ukey = skey + kPadded;                        // distinct keys of the round, from 1
+  float* sval = reinterpret_cast<float*>(ukey + kRound + 1);
+  float* usum = sval + kPadded;                    // 0: the key that was open before the round
+  __shared__ unsigned int s_part[kWarps];
+  __shared__ float s_tail[kWarps];
+  __shared__ bool s_flag[kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // index of the chunk's first new key: what the chunks before found
+  unsigned int next;
+  {
+    unsigned int c = 0;
+    for (int i = threadIdx.x; i < blockIdx.x; i += kThreads) c += counts[i];
+    cta_exclusive(c, s_part, &next);
+  }
+  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
+  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
+  for (long long base = lo; base < hi; base += kRound) {
+    const int count = (int)(hi - base < kRound ? hi - base : kRound);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int q = threadIdx.x + j * kThreads;
+      if (q < count) {
+        skey[q + q / kPer] = keys[base + q];
+        sval[q + q / kPer] = vals[base + q];
+      }
+    }
+    __syncthreads();
+    const int q0 = threadIdx.x * kPer, p0 = q0 + threadIdx.x;
+    K prev{};
+    if (q0 < count) {
+      if (q0 > 0) prev = skey[p0 - 2];
+      else if (base > 0) prev = keys[base - 1];
+    }
+    bool head[kPer];
+    unsigned int heads = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const bool valid = q0 + j < count;
+      const K key = valid ? skey[p0 + j] : prev;
+      head[j] = valid && (base + q0 + j == 0 || key != prev);
+      heads += head[j];
+      prev = key;
+    }
+    unsigned int total;
+    unsigned int slot = cta_exclusive(heads, s_part, &total);  // slot of the key open before q0
+    // sum of what belongs to that key, then the thread's own keys; the last one stays open
+    const unsigned int first_slot = slot;
+    float lead = 0.f, sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (head[j]) {
+        if (slot == first_slot) lead = sum;
+        else usum[slot] = sum;
+        ++slot;
+        sum = 0.f;
+        ukey[slot] = skey[p0 + j];
+      }
+      if (q0 + j < count) sum += sval[p0 + j];
+    }
+    // segmented inclusive scan of (has heads, open sum) over the threads
+    const bool any = heads > 0;
+    bool f = any;
+    float v = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float pv = __shfl_up_sync(0xffffffffu, v, o);
+      const bool pf = __shfl_up_sync(0xffffffffu, f, o);
+      if (lane >= o) {
+        if (!f) v += pv;
+        f |= pf;
+      }
+    }
+    if (lane == 31) {
+      s_tail[warp] = v;
+      s_flag[warp] = f;
+    }
+    float carry = __shfl_up_sync(0xffffffffu, v, 1);
+    bool carried = __shfl_up_sync(0xffffffffu, f, 1);
+    if (lane == 0) {
+      carry = 0.f;
+      carried = false;
+    }
+    __syncthreads();
+    if (!carried)
+      for (int w = warp - 1; w >= 0; --w) {
+        carry += s_tail[w];
+        if (s_flag[w]) break;
+      }
+    if (any) usum[first_slot] = carry + lead;
+    if (threadIdx.x == kThreads - 1) usum[total] = any ? sum : carry + sum;
+    __syncthreads();
+    for (unsigned int u = threadIdx.x; u <= total; u += kThreads) {
+      if (u > 0) out_keys[next + u - 1] = (unsigned long long)ukey[u];
+      if (u > 0 && u < total) out_sums[next + u - 1] = usum[u];
+      else if (next + u > 0) atomicAdd(&out_sums[next + u - 1], usum[u]);
+    }
+    next += total;
   }
 }
 
@@ -321,13 +624,9 @@ using namespace psdev::sortk;
 
 extern "C" {
 
-static size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
-
 // Bytes of scratch psdev_sort_keys needs for n keys (with or without a payload).
 size_t psdev_sort_scratch_bytes(int64_t n, int with_payload) {
-  const size_t ntiles = (size_t)((n + kTile - 1) / kTile);
-  size_t b = round256(sizeof(SortHead));
-  b += round256(ntiles * kDigits * 4 * kMaxPasses);   // one word per (pass, tile, digit)
+  size_t b = SortWork::bytes(n > 0 ? n : 1);
   b += round256((size_t)n * 8);                        // second key buffer
   if (with_payload) b += round256((size_t)n * 4);      // second payload buffer
   return b + 256;
@@ -337,7 +636,6 @@ size_t psdev_sort_scratch_bytes(int64_t n, int with_payload) {
 // = fewer passes).  `keys` is sorted in place.  If `perm` is not NULL it receives, for every
 // output position, the index the key had in the input (a stable sort permutation).
 // `scratch` is device memory of psdev_sort_scratch_bytes(n, perm != NULL) bytes; n < 2^30.
-// psdev_sort_status(scratch) tells afterwards whether a wait inside the sort ran out.
 int psdev_sort_keys(uint64_t* keys, uint32_t* perm, int64_t n, int key_bits, void* scratch,
                     size_t scratch_bytes, void* stream) {
   if (n < 0 || key_bits < 1 || key_bits > 64 || !keys) return PSDEV_ERR_ARG;
@@ -346,52 +644,33 @@ int psdev_sort_keys(uint64_t* keys, uint32_t* perm, int64_t n, int key_bits, voi
   if (!scratch || scratch_bytes < psdev_sort_scratch_bytes(n, perm != nullptr))
     return PSDEV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  const int ntiles = (int)((n + kTile - 1) / kTile);
   const int passes = (key_bits + kRadixBits - 1) / kRadixBits;
   char* p = static_cast<char*>(scratch);
   p = reinterpret_cast<char*>(((uintptr_t)p + 255) & ~uintptr_t(255));
-  SortHead* head = reinterpret_cast<SortHead*>(p);
-  p += round256(sizeof(SortHead));
-  unsigned int* status = reinterpret_cast<unsigned int*>(p);
-  const size_t status_pass = (size_t)ntiles * kDigits;
-  // head and the status words of the passes that run are cleared together
-  const size_t clear = round256(sizeof(SortHead)) + status_pass * 4 * passes;
-  p += round256(status_pass * 4 * kMaxPasses);
-  unsigned long long* alt = reinterpret_cast<unsigned long long*>(p);
-  p += round256((size_t)n * 8);
-  unsigned int* alt_pay = nullptr;
-  if (perm) alt_pay = reinterpret_cast<unsigned int*>(p);
-  {
-    // the sweep kernel's tile buffers exceed the default limit of dynamic shared memory
-    static std::atomic<bool> attr_set[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-      cudaError_t e = cudaFuncSetAttribute(sweep_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kSweepSmem);
-      if (e != cudaSuccess) return (int)e;
-      attr_set[dev & 63].store(true, std::memory_order_release);
-    }
+  const SortWork w(p, n);
+  p += SortWork::bytes(n);
+  using K = unsigned long long;
+  K* in = reinterpret_cast<K*>(keys);
+  if (n <= kTile) {
+    const int rc = perm ? small_sort<K, K, kMakeIndex>(in, in, nullptr, perm, (int)n, passes, 64,
+                                                       w.head, nullptr, s)
+                        : small_sort<K, K, kNoPayload>(in, in, nullptr, nullptr, (int)n, passes,
+                                                       64, w.head, nullptr, s);
+    return rc ? rc : (int)cudaGetLastError();
   }
-  cudaMemsetAsync(head, 0, clear, s);
-  unsigned long long* in = reinterpret_cast<unsigned long long*>(keys);
-  unsigned long long* out = alt;
+  K* out = reinterpret_cast<K*>(p);
+  p += round256((size_t)n * 8);
   unsigned int* pin = perm;
-  unsigned int* pout = alt_pay;
-  const int hist_ctas = ntiles < 592 ? ntiles : 592;
-  digit_hist_kernel<<<hist_ctas, kThreads, 0, s>>>(in, n, passes, head->hist);
-  digit_scan_kernel<<<passes, kDigits, 0, s>>>(head->hist);
-  g_launches.fetch_add(2, std::memory_order_relaxed);
+  unsigned int* pout = perm ? reinterpret_cast<unsigned int*>(p) : nullptr;
   for (int pass = 0; pass < passes; ++pass) {
     // the first pass makes the payload: the index of every key in the input
-    sweep_kernel<<<ntiles, kThreads, kSweepSmem, s>>>(
-        in, out, pass == 0 ? nullptr : pin, pout, n, pass * kRadixBits,
-        head->hist + pass * kDigits,
-        status + status_pass * pass, &head->next_tile[pass], &head->error);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    unsigned long long* t = in; in = out; out = t;
-    unsigned int* tp = pin; pin = pout; pout = tp;
+    const int rc =
+        !perm ? sort_pass<K, K, kNoPayload>(in, out, nullptr, nullptr, n, pass, 64, w, s)
+        : pass == 0 ? sort_pass<K, K, kMakeIndex>(in, out, nullptr, pout, n, pass, 64, w, s)
+                    : sort_pass<K, K, kPayload>(in, out, pin, pout, n, pass, 64, w, s);
+    if (rc) return rc;
+    std::swap(in, out);
+    std::swap(pin, pout);
   }
   if (passes & 1) {
     // an odd number of passes leaves the result in the scratch buffers
@@ -401,17 +680,139 @@ int psdev_sort_keys(uint64_t* keys, uint32_t* perm, int64_t n, int key_bits, voi
   return (int)cudaGetLastError();
 }
 
-// 0 when the last sort that used `scratch` completed every look-back, PSDEV_ERR_TIMEOUT_ENTRY
-// when one ran out (the output of that sort is not valid).  Waits for `stream`.
+// Waits for `stream` and reports whether the sorts on it ran (the kernels have no wait of their
+// own that could run out).
 int psdev_sort_status(const void* scratch, void* stream) {
   if (!scratch) return PSDEV_ERR_ARG;
-  const char* p = reinterpret_cast<const char*>(((uintptr_t)scratch + 255) & ~uintptr_t(255));
-  int err = 0;
-  cudaError_t e = cudaMemcpyAsync(&err, p, sizeof(int), cudaMemcpyDeviceToHost,
-                                  (cudaStream_t)stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+  return (int)cudaStreamSynchronize((cudaStream_t)stream);
+}
+
+}  // extern "C"
+
+// ---- unsorted, repeated (key, value) pairs -> sorted distinct keys and sums ---------------------
+namespace {
+// Layout of the scratch memory: working memory of the sort, counts of the chunks' distinct keys,
+// then two buffers of keys (4 bytes each up to 32 bits) and of values.
+struct UniqueScratch {
+  char* work;
+  SortHead* head;        // followed by `counts`: the host reads both with one copy
+  unsigned int* counts;
+  char* keys[2];
+  unsigned int* vals[2];
+  size_t bytes;
+  UniqueScratch(void* scratch, int64_t n, int key_bits) {
+    const size_t ksz = key_bits <= 32 ? 4 : 8;
+    const uintptr_t base = ((uintptr_t)scratch + 255) & ~uintptr_t(255);
+    uintptr_t p = base;
+    work = reinterpret_cast<char*>(p);
+    p += SortWork::bytes(n);
+    head = reinterpret_cast<SortHead*>(p);
+    counts = reinterpret_cast<unsigned int*>(p + sizeof(SortHead));
+    p += round256(sizeof(SortHead) + kMaxUniqueChunks * 4);
+    for (int i = 0; i < 2; ++i) {
+      keys[i] = reinterpret_cast<char*>(p);
+      p += round256((size_t)n * ksz);
+      vals[i] = reinterpret_cast<unsigned int*>(p);
+      p += round256((size_t)n * 4);
+    }
+    bytes = p - base + 256;
+  }
+};
+
+template <typename K>
+int unique_sort(const unsigned long long* keys, const float* vals, int64_t n, int key_bits,
+                const UniqueScratch& u, const SortWork& w, cudaStream_t s) {
+  const unsigned int* v = reinterpret_cast<const unsigned int*>(vals);
+  const int passes = (key_bits + kRadixBits - 1) / kRadixBits;
+  if (n <= kTile)
+    return small_sort<unsigned long long, K, kPayload>(keys, reinterpret_cast<K*>(u.keys[0]), v,
+                                                       u.vals[0], (int)n, passes, key_bits,
+                                                       w.head, u.counts, s);
+  for (int pass = 0; pass < passes; ++pass) {
+    // buffers alternate so that the last pass writes buffer 0
+    const int to = (passes - 1 - pass) & 1;
+    K* out = reinterpret_cast<K*>(u.keys[to]);
+    const int rc =
+        pass == 0 ? sort_pass<unsigned long long, K, kPayload>(keys, out, v, u.vals[to], n, 0,
+                                                               key_bits, w, s)
+                  : sort_pass<K, K, kPayload>(reinterpret_cast<const K*>(u.keys[to ^ 1]), out,
+                                              u.vals[to ^ 1], u.vals[to], n, pass, key_bits, w, s);
+    if (rc) return rc;
+  }
+  const Chunks ch = unique_chunks_of(n);
+  unique_count_kernel<K><<<ch.count, kThreads, 0, s>>>(reinterpret_cast<const K*>(u.keys[0]), n,
+                                                       ch, u.counts);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return 0;
+}
+
+template <typename K>
+int unique_write(const UniqueScratch& u, int64_t n, unsigned long long* out_keys, float* out_sums,
+                 cudaStream_t s) {
+  // the pairs of a round (padded) and its outputs
+  constexpr int smem = (kThreads * (kUniquePer + 1) + kThreads * kUniquePer + 1) *
+                       (int)(sizeof(K) + 4);
+  if (int rc = allow_smem<unique_sum_kernel<K>>(smem)) return rc;
+  const Chunks ch = unique_chunks_of(n);
+  unique_sum_kernel<K><<<ch.count, kThreads, smem, s>>>(
+      reinterpret_cast<const K*>(u.keys[0]), reinterpret_cast<const float*>(u.vals[0]), n, ch,
+      u.counts, out_keys, out_sums);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return (int)cudaGetLastError();
+}
+}  // namespace
+
+extern "C" {
+
+size_t psdev_unique_sum_scratch_bytes(int64_t n, int key_bits) {
+  if (n < 1 || key_bits < 1 || key_bits > 64) return 0;
+  return UniqueScratch(nullptr, n, key_bits).bytes;
+}
+
+// Sorts n (key, value) pairs by key into `scratch` (psdev_unique_sum_scratch_bytes) and counts the
+// distinct keys; keys and vals are not changed.  Waits for `stream`: the outputs of
+// psdev_unique_sum_write, which follows on the same stream, are sized by the count.
+// PSDEV_ERR_ARG when a key is not below 2^key_bits.
+int psdev_unique_sum_sort(const uint64_t* keys, const float* vals, int64_t n, int key_bits,
+                          void* scratch, size_t scratch_bytes, int64_t* n_unique, void* stream) {
+  if (!keys || !vals || !n_unique || n < 1 || key_bits < 1 || key_bits > 64) return PSDEV_ERR_ARG;
+  if (n >= (int64_t)1 << 30) return PSDEV_ERR_UNSUPPORTED;
+  if (!scratch || scratch_bytes < psdev_unique_sum_scratch_bytes(n, key_bits)) return PSDEV_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  const UniqueScratch u(scratch, n, key_bits);
+  SortWork w(u.work, n);
+  w.head = u.head;
+  cudaMemsetAsync(u.head, 0, sizeof(SortHead), s);
+  const unsigned long long* k = reinterpret_cast<const unsigned long long*>(keys);
+  const int rc = key_bits <= 32 ? unique_sort<unsigned int>(k, vals, n, key_bits, u, w, s)
+                                : unique_sort<unsigned long long>(k, vals, n, key_bits, u, w, s);
+  if (rc) return rc;
+  struct {
+    SortHead head;
+    unsigned int counts[kMaxUniqueChunks];
+  } got;
+  static_assert(sizeof(SortHead) == 4, "the counts follow the head without a gap");
+  const int chunks = unique_chunks_of(n).count;
+  cudaError_t e = cudaMemcpyAsync(&got, u.head, sizeof(SortHead) + chunks * 4,
+                                  cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return (int)e;
-  return err ? PSDEV_ERR_TIMEOUT_ENTRY : 0;
+  if (got.head.too_wide) return PSDEV_ERR_ARG;
+  *n_unique = 0;
+  for (int c = 0; c < chunks; ++c) *n_unique += got.counts[c];
+  return 0;
+}
+
+// Second half: the distinct keys, ascending, and the sums of their values.
+int psdev_unique_sum_write(const void* scratch, int64_t n, int key_bits, int64_t n_unique,
+                           uint64_t* out_keys, float* out_sums, void* stream) {
+  if (!scratch || !out_keys || !out_sums || n < 1 || n_unique < 1) return PSDEV_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  const UniqueScratch u(const_cast<void*>(scratch), n, key_bits);
+  cudaMemsetAsync(out_sums, 0, (size_t)n_unique * 4, s);
+  unsigned long long* ok = reinterpret_cast<unsigned long long*>(out_keys);
+  return key_bits <= 32 ? unique_write<unsigned int>(u, n, ok, out_sums, s)
+                        : unique_write<unsigned long long>(u, n, ok, out_sums, s);
 }
 
 // dst_vals[j] op= src_vals[i] for every key present in both sorted unique lists; values have

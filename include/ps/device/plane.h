@@ -188,6 +188,7 @@ class Plane : public DeviceRoute {
 
  private:
   void SubmitSparse(const DeviceRequest& req);
+  void FinishSparse(const SparseInfo* sp, const DeviceRequest& req, void* stream);
   Plane();
   ~Plane();
   std::unique_ptr<Impl> impl_;

@@ -308,6 +308,16 @@ int psdev_sparse_apply(const psdev_world_t* w, const psdev_sparse_t* t, int num_
 int psdev_sparse_respond(const psdev_world_t* w, const psdev_sparse_t* t, int num_ctas, int sync,
                          void* stream);
 
+/* One rank (w->world == 1; PSDEV_ERR_UNSUPPORTED otherwise): a whole request in one pass on the
+ * caller's device arrays.  vals != NULL: push (`nvals` values; with lengths: lens[i] values of key
+ * i packed back to back); out != NULL: pull into `out` (`nout` values at most).  On a table with
+ * lengths a pull alone asks for the stored lengths, which lens_out receives when not NULL.
+ * Equal keys must be next to each other. */
+int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
+                       const uint64_t* keys, const float* vals, int64_t nvals,
+                       const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
+                       void* stream);
+
 /* Server role, tables with lengths: stores the length of the value of every key that a worker
  * staged (keys in its arena, cut points computed with psdev_key_shard_lookup) into that worker's
  * array of lengths; 0 for a key that was never pushed.  Used by a pull that does not know the

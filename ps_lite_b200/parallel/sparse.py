@@ -100,26 +100,54 @@ class SparseTable:
         from .dense import default_timeout_s
         t.timeout_ns = int(default_timeout_s() * 1e9)
         self._t = t
+        self._out_ptr = self.out.data_ptr()
         self.barrier_channel = barrier_channel
         self.count = 0
+
+    def _check_request(self, n: int, nv: int, lens) -> None:
+        if n > self.max_keys:
+            raise ValueError("more keys than max_keys")
+        if self.var_len:
+            if lens is None or lens.numel() != n:
+                raise ValueError("a var_len table needs one length per key")
+            if nv > self.max_vals:
+                raise ValueError("more values than the table was sized for")
+        elif nv != n * self.width:
+            raise ValueError(f"expected {self.width} values per key")
+
+    # -- one rank: a request in one pass ---------------------------------------------------------
+    def _local_ok(self, keys, grads=None, lens=None) -> bool:
+        """One rank, and tensors that the kernel can read as they are."""
+        def plain(x, *dtypes):
+            return x.is_cuda and x.dtype in dtypes and x.is_contiguous()
+        return (self.heap.world == 1 and not self.heap.emulated_ranks and
+                plain(keys, torch.int64, torch.uint64) and
+                (grads is None or (plain(grads, torch.float32) and not self._in_heap_out(grads) and
+                                   (not self.var_len or
+                                    (lens is not None and plain(lens, torch.int32))))))
+
+    def _in_heap_out(self, t: torch.Tensor) -> bool:
+        lo = self._out_ptr
+        return lo - 4 * t.numel() < t.data_ptr() < lo + 4 * self.max_vals and t.data_ptr() != lo
+
+    def _local(self, keys, n, grads=None, lens=None) -> None:
+        ask = grads is None and self.var_len   # the owner says how long the values are
+        _lib.check(self.heap.lib.psdev_sparse_local(
+            C.byref(self._world), C.byref(self._t), n, keys.data_ptr(),
+            None if grads is None else grads.data_ptr(), 0 if grads is None else grads.numel(),
+            lens.data_ptr() if self.var_len and lens is not None else None, self._out_ptr,
+            self.max_vals, self.lens.data_ptr() if ask else None,
+            torch.cuda.current_stream(self.heap.device).cuda_stream), "sparse_local")
 
     # -- the three phases; `sync=False` lets a test run all ranks' phases on one GPU ----------
     def stage(self, keys: torch.Tensor, grads: torch.Tensor,
               lens: "torch.Tensor | None" = None) -> None:
         """Copy a request into the heap buffers: sorted unique keys and their values (``width``
         per key, or ``lens[i]`` per key back to back for a ``var_len`` table)."""
-        n = keys.numel()
-        if n > self.max_keys:
-            raise ValueError("more keys than max_keys")
-        nv = grads.numel()
+        n, nv = keys.numel(), grads.numel()
+        self._check_request(n, nv, lens)
         if self.var_len:
-            if lens is None or lens.numel() != n:
-                raise ValueError("a var_len table needs one length per key")
-            if nv > self.max_vals:
-                raise ValueError("more values than the table was sized for")
             self.lens[:n].copy_(lens.to(torch.int32), non_blocking=True)
-        elif nv != n * self.width:
-            raise ValueError(f"expected {self.width} values per key")
         self.keys[:n].copy_(keys.view(torch.int64), non_blocking=True)
         self.grads[:nv].copy_(grads.reshape(-1), non_blocking=True)
         self.count, self.count_vals = n, nv
@@ -145,7 +173,14 @@ class SparseTable:
 
         Three launches: scatter; apply, which first waits for every rank's scatter; respond,
         which ends when every rank's answers have landed.  Returns a view of the heap output
-        buffer (valid until the next call), laid out like the pushed values."""
+        buffer (valid until the next call), laid out like the pushed values.  One rank: one launch
+        on the request's own tensors (``psdev_sparse_local``)."""
+        if self._local_ok(keys, grads, lens):
+            n, nv = keys.numel(), grads.numel()
+            self._check_request(n, nv, lens)
+            self._local(keys, n, grads, lens)
+            self.count, self.count_vals = n, nv
+            return self.out[:nv]
         self.stage(keys, grads, lens)
         self.scatter()
         multi = self.heap.world > 1
@@ -163,6 +198,12 @@ class SparseTable:
             raise ValueError("more keys than max_keys")
         multi = self.heap.world > 1 if sync is None else sync
         lib, s = self.heap.lib, torch.cuda.current_stream(self.heap.device)
+        if not multi and self._local_ok(keys):
+            self._local(keys, n)
+            self.count = n
+            self.count_vals = int(self.lens[:n].sum()) if self.var_len else n * self.width
+            values = self.out[: self.count_vals]
+            return (values, self.lens[:n]) if self.var_len else values
         self.keys[:n].copy_(keys.view(torch.int64), non_blocking=True)
         self.count = n
         if not self.var_len:

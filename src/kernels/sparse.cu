@@ -398,6 +398,353 @@ __global__ void __launch_bounds__(256, 8)
   }
 }
 
+// ---- one rank ----------------------------------------------------------------------------------
+// With one rank a request's worker is also the owner of every key, so nothing has to travel
+// through accumulators or wait: one pass reads a key, its value's state and gradient, applies
+// the handle and stores state and answer.  The three kernels above touch two random places of
+// memory per value and phase (accumulator and state) and copy the request into the arena first;
+// here a value costs one read and one write of its state, and the request's arrays are used
+// where they are.  2^20 Zipf keys of 2^30, FTRL: 201 us with the three kernels (and 4 copies).
+// The bound is the rate of random DRAM accesses: kLocalUnroll values per thread are looked up
+// together, so that an SM has some 64 KB of them in flight.
+struct LocalReq {
+  const unsigned long long* keys;
+  const float* vals;     // pushed values, or NULL
+  const int* lens;       // lengths that the push names, or NULL
+  float* out;            // pulled values, or NULL
+  int* lens_out;         // stored lengths of a pull, or NULL
+  long long n;           // keys
+  long long nvals;       // capacity of vals
+  long long nout;        // capacity of out
+  long long* sums;       // values per chunk (requests with lengths and many keys), or NULL
+  int blocks;            // blocks of kLenBlock keys per chunk
+};
+constexpr int kLocalUnroll = 4;
+
+// State of one value: {w, z, n} (z, n: FTRL).  GROUP: side by side, one 16-byte access.
+template <bool GROUP>
+__device__ __forceinline__ float4 load_state(const SparseArgs& a, long long e) {
+  if constexpr (GROUP) return *reinterpret_cast<const float4*>(a.w + e * 4);
+  const long long s = e * a.sstride;
+  return make_float4(a.w[s], a.kind == 2 ? a.z[s] : 0.f, a.kind == 2 ? a.nacc[s] : 0.f, 0.f);
+}
+// The handle with gradient g on a loaded state; a zero gradient changes nothing.
+template <bool GROUP>
+__device__ __forceinline__ void update_state(const SparseArgs& a, long long e, float g,
+                                             float4* v) {
+  if (g == 0.f) return;
+  if (GROUP || a.kind == 2) {
+    const float n2 = v->z + g * g;
+    const float sigma = (sqrtf(n2) - sqrtf(v->z)) / a.alpha;
+    v->y = v->y + g - sigma * v->x;
+    v->z = n2;
+    v->x = ftrl_weight(v->y, n2, a);
+  } else {
+    v->x = a.kind == 0 ? v->x + g : v->x - a.lr * g;
+  }
+  if constexpr (GROUP) {
+    *reinterpret_cast<float4*>(a.w + e * 4) = *v;
+  } else {
+    const long long s = e * a.sstride;
+    a.w[s] = v->x;
+    if (a.kind == 2) {
+      a.z[s] = v->y;
+      a.nacc[s] = v->z;
+    }
+  }
+}
+// t / d, in 32 bits where that is enough (the 64-bit division is some 80 instructions)
+__device__ __forceinline__ long long quotient(long long t, unsigned int d) {
+  return (t >> 32) == 0 ? (long long)((unsigned int)t / d) : t / d;
+}
+__device__ __forceinline__ bool below(long long at, long long end) {
+  return (unsigned long long)at < (unsigned long long)end;
+}
+
+// Every key has `width` values.  Equal keys next to each other count as one whose gradients are
+// added up: the first of them does the work of all.
+template <bool GROUP, bool ONE>
+__global__ void __launch_bounds__(256)
+    sparse_local_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ LocalReq q) {
+  const unsigned int width = ONE ? 1u : (unsigned int)a.width;
+  const long long work = q.n * width;
+  const long long first = blockIdx.x * (256ll * kLocalUnroll) + threadIdx.x;
+  long long i[kLocalUnroll], e[kLocalUnroll];  // key, value in the store (-1: none, -2: no work)
+  unsigned long long k[kLocalUnroll];
+  bool head[kLocalUnroll], again[kLocalUnroll];
+  float g[kLocalUnroll];
+  float4 v[kLocalUnroll];
+#pragma unroll
+  for (int u = 0; u < kLocalUnroll; ++u) {
+    const long long t = first + u * 256;
+    i[u] = t < work ? (ONE ? t : quotient(t, width)) : 0;
+    k[u] = 0;
+    g[u] = 0.f;
+    head[u] = again[u] = false;
+    if (t < work) {
+      k[u] = q.keys[i[u]];
+      if (q.vals) g[u] = q.vals[t];
+      head[u] = i[u] == 0 || q.keys[i[u] - 1] != k[u];
+      again[u] = i[u] + 1 < q.n && q.keys[i[u] + 1] == k[u];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kLocalUnroll; ++u) {
+    e[u] = -2;
+    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (head[u] && k[u] < a.range) {  // (a key outside the range is dropped)
+      const long long idx = state_index(a, 0, k[u], true);
+      e[u] = idx < 0 ? -1 : idx * width + (first + u * 256 - i[u] * width);
+      if (idx >= 0) v[u] = load_state<GROUP>(a, e[u]);
+      else if (a.capacity) *a.overflow = 1;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kLocalUnroll; ++u) {
+    if (e[u] == -2) continue;
+    const long long t = first + u * 256;
+    long long more = 0;  // further occurrences of the key
+    if (again[u])
+      for (long long m = i[u] + 1; m < q.n && q.keys[m] == k[u]; ++m) {
+        ++more;
+        if (q.vals) g[u] += q.vals[t + more * width];
+      }
+    if (e[u] >= 0) update_state<GROUP>(a, e[u], g[u], &v[u]);
+    if (q.out)
+      for (long long m = 0; m <= more; ++m) q.out[t + m * width] = v[u].x;
+  }
+}
+
+// Rows of a multiple of four values with one number each (sum, SGD): 16-byte accesses.
+__global__ void __launch_bounds__(256)
+    sparse_local_rows_kernel(const __grid_constant__ SparseArgs a,
+                             const __grid_constant__ LocalReq q) {
+  const unsigned int quads = (unsigned int)a.width / 4;
+  const long long work = q.n * quads;
+  const long long first = blockIdx.x * (256ll * kLocalUnroll) + threadIdx.x;
+  const float4* vals = reinterpret_cast<const float4*>(q.vals);
+  float4* out = reinterpret_cast<float4*>(q.out);
+  long long i[kLocalUnroll], idx[kLocalUnroll];
+  unsigned int j[kLocalUnroll];
+  float4 g[kLocalUnroll], w[kLocalUnroll];
+  bool again[kLocalUnroll];
+#pragma unroll
+  for (int u = 0; u < kLocalUnroll; ++u) {
+    const long long t = first + u * 256;
+    idx[u] = -2;
+    again[u] = false;
+    g[u] = w[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < work) {
+      i[u] = quotient(t, quads);
+      j[u] = (unsigned int)(t - i[u] * quads);
+      const unsigned long long k = q.keys[i[u]];
+      const bool head = i[u] == 0 || q.keys[i[u] - 1] != k;
+      again[u] = i[u] + 1 < q.n && q.keys[i[u] + 1] == k;
+      if (vals) g[u] = vals[t];
+      if (head && k < a.range) {
+        idx[u] = state_index(a, 0, k, true);
+        if (idx[u] >= 0) w[u] = reinterpret_cast<const float4*>(a.w)[idx[u] * quads + j[u]];
+        else if (a.capacity) *a.overflow = 1;
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kLocalUnroll; ++u) {
+    if (idx[u] == -2) continue;
+    long long last = i[u];
+    if (again[u]) {
+      const unsigned long long k = q.keys[i[u]];
+      while (last + 1 < q.n && q.keys[last + 1] == k) {
+        ++last;
+        if (vals) {
+          const float4 o = vals[last * quads + j[u]];
+          g[u].x += o.x; g[u].y += o.y; g[u].z += o.z; g[u].w += o.w;
+        }
+      }
+    }
+    if (idx[u] >= 0 && vals) {
+      float* x = &w[u].x;
+      const float* y = &g[u].x;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (y[c] != 0.f) x[c] = a.kind == 0 ? x[c] + y[c] : x[c] - a.lr * y[c];
+      reinterpret_cast<float4*>(a.w)[idx[u] * quads + j[u]] = w[u];
+    }
+    if (out)
+      for (long long m = i[u]; m <= last; ++m) out[m * quads + j[u]] = w[u];
+  }
+}
+
+// Values with lengths (`lens` given: a push, possibly of no value at all).  A CTA takes a chunk
+// of q.blocks x kLenBlock keys; small blocks, because a request of some thousand keys must reach
+// all SMs (4099 keys, widths up to 8: 38 us per launch with 1024 keys per CTA).  Where the
+// chunk's values start is the sum of the lengths before it: added up by the CTA itself when few
+// keys come before (kLenSelf keys at most), else from the chunk sums of a first launch (SUMS).
+constexpr int kLenBlock = 128;
+constexpr int kLenSelf = 8192;
+constexpr int kMaxLenChunks = 2048;
+
+__device__ __forceinline__ int local_len(const SparseArgs& a, const LocalReq& q, long long i) {
+  int l = 0;
+  if (q.lens) {
+    l = q.lens[i];
+  } else if (q.keys[i] < a.range) {
+    const long long idx = state_index(a, 0, q.keys[i], false);
+    if (idx >= 0) l = a.klen[idx];
+  }
+  return l < 0 ? 0 : l;
+}
+
+// Sum of the lengths of keys [lo, hi), this thread's part of it.
+__device__ __forceinline__ long long local_len_sum(const SparseArgs& a, const LocalReq& q,
+                                                   long long lo, long long hi) {
+  long long sum = 0;
+  for (long long i = lo + threadIdx.x; i < hi; i += 256 * 8) {
+    int l[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) l[u] = i + u * 256 < hi ? local_len(a, q, i + u * 256) : 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) sum += l[u];
+  }
+  return sum;
+}
+// Sum over a CTA of 256 threads, to every thread.
+__device__ __forceinline__ long long cta_sum(long long v, long long* part) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  long long all = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) all += part[w];
+  return all;
+}
+
+__global__ void __launch_bounds__(256)
+    sparse_len_sums_kernel(const __grid_constant__ SparseArgs a,
+                           const __grid_constant__ LocalReq q) {
+  __shared__ long long s_part[8];
+  const long long size = (long long)q.blocks * kLenBlock, lo = blockIdx.x * size;
+  const long long all = cta_sum(local_len_sum(a, q, lo, lo + size < q.n ? lo + size : q.n), s_part);
+  if (threadIdx.x == 0) q.sums[blockIdx.x] = all;
+}
+
+template <bool GROUP>
+__global__ void __launch_bounds__(256)
+    sparse_local_lens_kernel(const __grid_constant__ SparseArgs a,
+                             const __grid_constant__ LocalReq q) {
+  __shared__ long long s_part[8];
+  __shared__ unsigned long long s_key[kLenBlock];
+  __shared__ long long s_idx[kLenBlock];  // slot; -1: none, -2: not this key's work
+  __shared__ int s_off[kLenBlock], s_len[kLenBlock], s_warp[kLenBlock / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long chunk = (long long)blockIdx.x * q.blocks * kLenBlock;
+  long long base = 0;  // where the block's values start
+  if (q.sums) {
+    for (int c = threadIdx.x; c < blockIdx.x; c += 256) base += q.sums[c];
+  } else {
+    base = local_len_sum(a, q, 0, chunk);
+  }
+  base = cta_sum(base, s_part);
+  const unsigned int width = (unsigned int)a.width;
+  for (int b = 0; b < q.blocks; ++b) {
+    const long long lo = chunk + (long long)b * kLenBlock;
+    if (lo >= q.n) return;
+    const int count = (int)(q.n - lo < kLenBlock ? q.n - lo : kLenBlock);
+    __syncthreads();
+    int len = 0, incl = 0;
+    if (threadIdx.x < kLenBlock) {
+      if (threadIdx.x < count) {
+        const long long i = lo + threadIdx.x;
+        const unsigned long long k = q.keys[i];
+        const bool first = i == 0 || q.keys[i - 1] != k;
+        long long idx = -2;
+        if (k < a.range) idx = state_index(a, 0, k, q.lens != nullptr);
+        len = q.lens ? q.lens[i] : (idx >= 0 ? a.klen[idx] : 0);
+        if (len < 0) len = 0;
+        if (idx == -1 && a.capacity && q.lens) *a.overflow = 1;
+        if (idx >= 0 && q.lens && first && len > 0) a.klen[idx] = len < a.width ? len : a.width;
+        s_key[threadIdx.x] = k;
+        s_idx[threadIdx.x] = q.lens && !first ? -2 : idx;
+        if (q.lens_out) q.lens_out[i] = len;
+      }
+      incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (lane == 31) s_warp[warp] = incl;
+    }
+    __syncthreads();
+    int total = 0, off = incl - len;
+#pragma unroll
+    for (int w = 0; w < kLenBlock / 32; ++w) {
+      if (w < warp) off += s_warp[w];
+      total += s_warp[w];
+    }
+    if (threadIdx.x < kLenBlock) {
+      s_off[threadIdx.x] = off;
+      s_len[threadIdx.x] = len;
+    }
+    __syncthreads();
+    const unsigned int work = (unsigned int)count * width;
+    for (unsigned int t0 = threadIdx.x; t0 < work; t0 += 256 * kLocalUnroll) {
+      long long e[kLocalUnroll], at[kLocalUnroll];
+      int c[kLocalUnroll];
+      float4 v[kLocalUnroll];
+      float g[kLocalUnroll];
+#pragma unroll
+      for (int u = 0; u < kLocalUnroll; ++u) {
+        const unsigned int t = t0 + u * 256;
+        e[u] = -2;
+        g[u] = 0.f;
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < work) {
+          c[u] = (int)(t / width);
+          const int j = (int)(t - (unsigned int)c[u] * width);
+          // a value never exceeds its slot, and the request's arrays bound what is accessed
+          if (s_idx[c[u]] != -2 && j < s_len[c[u]]) {
+            at[u] = base + s_off[c[u]] + j;
+            e[u] = s_idx[c[u]] < 0 ? -1 : s_idx[c[u]] * a.width + j;
+            if (e[u] >= 0) v[u] = load_state<GROUP>(a, e[u]);
+            if (q.lens && below(at[u], q.nvals)) g[u] = q.vals[at[u]];
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kLocalUnroll; ++u) {
+        if (e[u] == -2) continue;
+        const int j = (int)(at[u] - base) - s_off[c[u]];
+        const long long i = lo + c[u];
+        // equal keys next to each other: the first adds up the gradients and answers for all
+        const bool again = q.lens && i + 1 < q.n && q.keys[i + 1] == s_key[c[u]];
+        if (again) {
+          long long m_at = base + s_off[c[u]] + s_len[c[u]];
+          for (long long m = i + 1; m < q.n && q.keys[m] == s_key[c[u]]; ++m) {
+            const int l = local_len(a, q, m);
+            if (j < l && below(m_at + j, q.nvals)) g[u] += q.vals[m_at + j];
+            m_at += l;
+          }
+        }
+        if (e[u] >= 0) update_state<GROUP>(a, e[u], g[u], &v[u]);
+        if (!q.out) continue;
+        if (below(at[u], q.nout)) q.out[at[u]] = v[u].x;
+        if (again) {
+          long long m_at = base + s_off[c[u]] + s_len[c[u]];
+          for (long long m = i + 1; m < q.n && q.keys[m] == s_key[c[u]]; ++m) {
+            const int l = local_len(a, q, m);
+            if (j < l && below(m_at + j, q.nout)) q.out[m_at + j] = v[u].x;
+            m_at += l;
+          }
+        }
+      }
+    }
+    base += total;
+  }
+}
+
 }  // namespace psdev
 
 using namespace psdev;
@@ -499,6 +846,63 @@ int psdev_sparse_scatter(const psdev_world_t* w, const psdev_sparse_t* t, int64_
   }
   // (an empty request still publishes its cut points: the servers read them)
   sparse_scatter_kernel<<<num_ctas > 0 ? num_ctas : default_ctas(), 256, 0, s>>>(a);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return (int)cudaGetLastError();
+}
+
+int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
+                       const uint64_t* keys, const float* vals, int64_t nvals,
+                       const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
+                       void* stream) {
+  SparseArgs a{};
+  int rc = fill(&a, w, t, n);
+  if (rc) return rc;
+  if (w->world != 1) return PSDEV_ERR_UNSUPPORTED;
+  if (n == 0) return 0;
+  if (!keys || (!vals && !lens && !out && !lens_out) || ((uintptr_t)keys & 7) ||
+      ((uintptr_t)vals & 3) || ((uintptr_t)out & 3) || ((uintptr_t)lens & 3) ||
+      ((uintptr_t)lens_out & 3))
+    return PSDEV_ERR_ARG;
+  const bool var = t->lens_off != 0;
+  if (!var && ((vals && nvals < n * t->width) || (out && nout < n * t->width) || lens || lens_out))
+    return PSDEV_ERR_ARG;
+  if (var && (vals ? !lens : lens && nvals > 0)) return PSDEV_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  LocalReq q{};
+  q.keys = reinterpret_cast<const unsigned long long*>(keys);
+  q.vals = vals;
+  q.lens = lens;
+  q.out = out;
+  q.lens_out = lens_out;
+  q.n = n;
+  q.nvals = nvals;
+  q.nout = nout;
+  // {w, z, n, -} side by side and aligned: one 16-byte access per value
+  const bool group = t->kind == 2 && t->state_stride == 4 && t->z == t->w + 1 &&
+                     t->n == t->w + 2 && ((uintptr_t)t->w & 15) == 0;
+  if (var) {
+    const long long blocks = (n + kLenBlock - 1) / kLenBlock;
+    q.blocks = (int)((blocks + kMaxLenChunks - 1) / kMaxLenChunks);
+    const unsigned chunks = (unsigned)((blocks + q.blocks - 1) / q.blocks);
+    if (n > kLenSelf) {
+      // (the arena's array of value offsets, unused by this form, holds the chunk sums)
+      q.sums = reinterpret_cast<long long*>(static_cast<char*>(w->peer_base[0]) + t->offs_off);
+      sparse_len_sums_kernel<<<chunks, 256, 0, s>>>(a, q);
+      g_launches.fetch_add(1, std::memory_order_relaxed);
+    }
+    if (group) sparse_local_lens_kernel<true><<<chunks, 256, 0, s>>>(a, q);
+    else sparse_local_lens_kernel<false><<<chunks, 256, 0, s>>>(a, q);
+  } else {
+    const bool rows = t->kind != 2 && t->width % 4 == 0 && a.sstride == 1 &&
+                      (((uintptr_t)vals | (uintptr_t)out | (uintptr_t)t->w) & 15) == 0;
+    const long long work = rows ? n * (t->width / 4) : n * t->width;
+    const unsigned ctas = (unsigned)((work + 256 * kLocalUnroll - 1) / (256 * kLocalUnroll));
+    if (rows) sparse_local_rows_kernel<<<ctas, 256, 0, s>>>(a, q);
+    else if (group && t->width == 1) sparse_local_kernel<true, true><<<ctas, 256, 0, s>>>(a, q);
+    else if (group) sparse_local_kernel<true, false><<<ctas, 256, 0, s>>>(a, q);
+    else if (t->width == 1) sparse_local_kernel<false, true><<<ctas, 256, 0, s>>>(a, q);
+    else sparse_local_kernel<false, false><<<ctas, 256, 0, s>>>(a, q);
+  }
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return (int)cudaGetLastError();
 }

@@ -66,6 +66,9 @@ struct Rt {
   int (*sparse_respond)(const psdev_world_t*, const psdev_sparse_t*, int, int, void*) = nullptr;
   int (*sparse_lens)(const psdev_world_t*, const psdev_sparse_t*, int, void*) = nullptr;
   int (*key_shard_lookup)(const uint64_t*, int64_t, uint64_t, int, int64_t*, void*) = nullptr;
+  int (*sparse_local)(const psdev_world_t*, const psdev_sparse_t*, int64_t, const uint64_t*,
+                      const float*, int64_t, const int32_t*, float*, int64_t, int32_t*,
+                      void*) = nullptr;
   int (*lens_to_offsets)(const int32_t*, int64_t, int64_t*, void*) = nullptr;
   int (*device_barrier)(const psdev_world_t*, int, uint64_t, void*) = nullptr;
   int (*multicast_pays)(int, uint64_t) = nullptr;
@@ -142,6 +145,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_sparse_respond", &rt->sparse_respond);
   Bind(lib, "psdev_sparse_lens", &rt->sparse_lens);
   Bind(lib, "psdev_key_shard_lookup", &rt->key_shard_lookup);
+  Bind(lib, "psdev_sparse_local", &rt->sparse_local);
   Bind(lib, "psdev_lens_to_offsets", &rt->lens_to_offsets);
   Bind(lib, "psdev_device_barrier", &rt->device_barrier);
   Bind(lib, "psdev_multicast_pays", &rt->multicast_pays);
@@ -1544,6 +1548,36 @@ void Plane::SubmitSparse(const DeviceRequest& req) {
   void* s = tls_has_stream ? tls_stream : m.s_compute;
   m.After(m.LastDone(sp), s);
   const void* kptr = req.keys.data();
+  const int* lens_in = req.push && sp->var_len ? req.lens.data() : nullptr;
+  // (an output that shares memory with what is read goes through the table's buffers)
+  auto apart = [](const void* a, size_t an, const void* b, size_t bn) {
+    return !a || !b || a == b || !Clash(a, an, 1, b, bn, 1);
+  };
+  const size_t kbytes = static_cast<size_t>(n) * 8, lbytes = static_cast<size_t>(n) * 4;
+  void* out = req.pull ? req.outs : nullptr;
+  void* lens_to = req.pull && !req.push && sp->var_len ? req.lens_out : nullptr;
+  const bool local =
+      m.world == 1 && !m.sim && (req.push || out || lens_to) && kptr != out && kptr != lens_to &&
+      apart(kptr, kbytes, out, obytes) && apart(kptr, kbytes, lens_to, lbytes) &&
+      apart(out, obytes, lens_to, lbytes) && (!out || out != lens_to) &&
+      (!req.push || (apart(req.vals, vbytes, out, obytes) && (!out || lens_in != out) &&
+                     apart(lens_in, lbytes, out, obytes))) &&
+      (!req.push || sp->var_len == (lens_in != nullptr)) &&
+      !((reinterpret_cast<uintptr_t>(kptr) & 7) |
+        ((reinterpret_cast<uintptr_t>(req.push ? req.vals : nullptr) |
+          reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(lens_in) |
+          reinterpret_cast<uintptr_t>(lens_to)) & 3));
+  if (local) {
+    // one rank: one kernel on the request's own arrays
+    if (lens_to) CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));
+    CHECK_EQ(m.rt.sparse_local(&m.ws, &t, n, static_cast<const uint64_t*>(kptr),
+                               static_cast<const float*>(req.push ? req.vals : nullptr),
+                               static_cast<int64_t>(vbytes / 4), lens_in, static_cast<float*>(out),
+                               static_cast<int64_t>(obytes / 4), static_cast<int*>(lens_to), s), 0)
+        << "psdev_sparse_local failed";
+    FinishSparse(sp, req, s);
+    return;
+  }
   if (kptr != sp->keys) {
     CHECK_EQ(m.rt.memcpy_async(sp->keys, kptr, static_cast<size_t>(n) * 8, s), 0);
   }
@@ -1584,11 +1618,17 @@ void Plane::SubmitSparse(const DeviceRequest& req) {
     CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));
     CHECK_EQ(m.rt.memcpy_async(req.lens_out, sp->lens, static_cast<size_t>(n) * 4, s), 0);
   }
+  FinishSparse(sp, req, s);
+}
+
+// The request's work has been issued on `s`: completion and the ordering point of the table.
+void Plane::FinishSparse(const SparseInfo* sp, const DeviceRequest& req, void* s) {
+  Impl& m = *impl_;
   void* done = m.NewEvent();
   m.rt.event_record(done, s);
   Impl::Pending pend;
   pend.event = done;
-  pend.channel = t.channel;
+  pend.channel = sp->table.channel;
   pend.timestamp = req.timestamp;
   pend.responses = req.responses;
   pend.customer = req.customer;

@@ -405,8 +405,7 @@ __global__ void __launch_bounds__(256, 8)
 // memory per value and phase (accumulator and state) and copy the request into the arena first;
 // here a value costs one read and one write of its state, and the request's arrays are used
 // where they are.  2^20 Zipf keys of 2^30, FTRL: 201 us with the three kernels (and 4 copies).
-// The bound is the rate of random DRAM accesses: kLocalUnroll values per thread are looked up
-// together, so that an SM has some 64 KB of them in flight.
+// 59 us with this one, which is what the random accesses alone take.
 struct LocalReq {
   const unsigned long long* keys;
   const float* vals;     // pushed values, or NULL
@@ -420,6 +419,9 @@ struct LocalReq {
   int blocks;            // blocks of kLenBlock keys per chunk
 };
 constexpr int kLocalUnroll = 4;
+// One 16-byte group per key, all of them far apart: a plain kernel that reads 2^20 such groups and
+// writes them back takes 59 us with one per thread, 63 with two, 67 with four (41 only reading).
+constexpr int kStateUnroll = 1;
 
 // State of one value: {w, z, n} (z, n: FTRL).  GROUP: side by side, one 16-byte access.
 template <bool GROUP>
@@ -466,6 +468,7 @@ __device__ __forceinline__ bool below(long long at, long long end) {
 template <bool GROUP, bool ONE>
 __global__ void __launch_bounds__(256)
     sparse_local_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ LocalReq q) {
+  constexpr int kLocalUnroll = GROUP && ONE ? kStateUnroll : psdev::kLocalUnroll;
   const unsigned int width = ONE ? 1u : (unsigned int)a.width;
   const long long work = q.n * width;
   const long long first = blockIdx.x * (256ll * kLocalUnroll) + threadIdx.x;
@@ -595,16 +598,36 @@ __device__ __forceinline__ int local_len(const SparseArgs& a, const LocalReq& q,
   return l < 0 ? 0 : l;
 }
 
-// Sum of the lengths of keys [lo, hi), this thread's part of it.
+// Sum of the lengths of keys [lo, hi), this thread's part of it.  All loads of a step are issued
+// before the first is used, and `own`, which needs loads of its own, runs among them: a request
+// of a few thousand keys is bound by the chain key -> slot -> length -> value.
+template <typename Own>
 __device__ __forceinline__ long long local_len_sum(const SparseArgs& a, const LocalReq& q,
-                                                   long long lo, long long hi) {
+                                                   long long lo, long long hi, Own&& own) {
+  constexpr int kStep = 16;
   long long sum = 0;
-  for (long long i = lo + threadIdx.x; i < hi; i += 256 * 8) {
-    int l[8];
+  bool first = true;
+  for (long long i = lo + threadIdx.x; first || i < hi; i += 256 * kStep) {
+    unsigned long long k[kStep];
+    int l[kStep];
+    if (q.lens) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) l[u] = i + u * 256 < hi ? local_len(a, q, i + u * 256) : 0;
+      for (int u = 0; u < kStep; ++u) l[u] = i + u * 256 < hi ? q.lens[i + u * 256] : 0;
+    } else {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) sum += l[u];
+      for (int u = 0; u < kStep; ++u) k[u] = i + u * 256 < hi ? q.keys[i + u * 256] : a.range;
+    }
+    if (first) own();
+    first = false;
+    if (!q.lens) {
+#pragma unroll
+      for (int u = 0; u < kStep; ++u) {
+        const long long idx = k[u] < a.range ? state_index(a, 0, k[u], false) : -1;
+        l[u] = idx >= 0 ? a.klen[idx] : 0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kStep; ++u) sum += l[u] > 0 ? l[u] : 0;
   }
   return sum;
 }
@@ -626,7 +649,8 @@ __global__ void __launch_bounds__(256)
                            const __grid_constant__ LocalReq q) {
   __shared__ long long s_part[8];
   const long long size = (long long)q.blocks * kLenBlock, lo = blockIdx.x * size;
-  const long long all = cta_sum(local_len_sum(a, q, lo, lo + size < q.n ? lo + size : q.n), s_part);
+  const long long hi = lo + size < q.n ? lo + size : q.n;
+  const long long all = cta_sum(local_len_sum(a, q, lo, hi, [] {}), s_part);
   if (threadIdx.x == 0) q.sums[blockIdx.x] = all;
 }
 
@@ -641,27 +665,41 @@ __global__ void __launch_bounds__(256)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long chunk = (long long)blockIdx.x * q.blocks * kLenBlock;
   long long base = 0;  // where the block's values start
-  if (q.sums) {
-    for (int c = threadIdx.x; c < blockIdx.x; c += 256) base += q.sums[c];
-  } else {
-    base = local_len_sum(a, q, 0, chunk);
-  }
-  base = cta_sum(base, s_part);
   const unsigned int width = (unsigned int)a.width;
   for (int b = 0; b < q.blocks; ++b) {
     const long long lo = chunk + (long long)b * kLenBlock;
     if (lo >= q.n) return;
     const int count = (int)(q.n - lo < kLenBlock ? q.n - lo : kLenBlock);
     __syncthreads();
+    const bool mine = threadIdx.x < count;
+    const long long i = lo + threadIdx.x;
+    const unsigned long long k = mine ? q.keys[i] : 0;
+    const bool first = mine && (i == 0 || q.keys[i - 1] != k);
     int len = 0, incl = 0;
+    long long idx = -2;
+    auto own = [&] {
+      if (!mine) return;
+      if (k < a.range) idx = state_index(a, 0, k, q.lens != nullptr);
+      len = q.lens ? q.lens[i] : (idx >= 0 ? a.klen[idx] : 0);
+      if (idx >= 0) {
+        // the key's values are wanted soon, by other threads
+        const char* p = reinterpret_cast<const char*>(a.w + idx * a.width * a.sstride);
+        const int bytes = a.width * a.sstride * 4;
+        for (int at = 0; at < bytes && at < 512; at += 32)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p + at));
+      }
+    };
+    if (b > 0) {
+      own();
+    } else if (q.sums) {
+      own();
+      for (int c = threadIdx.x; c < blockIdx.x; c += 256) base += q.sums[c];
+      base = cta_sum(base, s_part);
+    } else {
+      base = cta_sum(local_len_sum(a, q, 0, chunk, own), s_part);
+    }
     if (threadIdx.x < kLenBlock) {
-      if (threadIdx.x < count) {
-        const long long i = lo + threadIdx.x;
-        const unsigned long long k = q.keys[i];
-        const bool first = i == 0 || q.keys[i - 1] != k;
-        long long idx = -2;
-        if (k < a.range) idx = state_index(a, 0, k, q.lens != nullptr);
-        len = q.lens ? q.lens[i] : (idx >= 0 ? a.klen[idx] : 0);
+      if (mine) {
         if (len < 0) len = 0;
         if (idx == -1 && a.capacity && q.lens) *a.overflow = 1;
         if (idx >= 0 && q.lens && first && len > 0) a.klen[idx] = len < a.width ? len : a.width;
@@ -717,12 +755,12 @@ __global__ void __launch_bounds__(256)
       for (int u = 0; u < kLocalUnroll; ++u) {
         if (e[u] == -2) continue;
         const int j = (int)(at[u] - base) - s_off[c[u]];
-        const long long i = lo + c[u];
+        const long long ki = lo + c[u];
         // equal keys next to each other: the first adds up the gradients and answers for all
-        const bool again = q.lens && i + 1 < q.n && q.keys[i + 1] == s_key[c[u]];
+        const bool again = q.lens && ki + 1 < q.n && q.keys[ki + 1] == s_key[c[u]];
         if (again) {
           long long m_at = base + s_off[c[u]] + s_len[c[u]];
-          for (long long m = i + 1; m < q.n && q.keys[m] == s_key[c[u]]; ++m) {
+          for (long long m = ki + 1; m < q.n && q.keys[m] == s_key[c[u]]; ++m) {
             const int l = local_len(a, q, m);
             if (j < l && below(m_at + j, q.nvals)) g[u] += q.vals[m_at + j];
             m_at += l;
@@ -733,7 +771,7 @@ __global__ void __launch_bounds__(256)
         if (below(at[u], q.nout)) q.out[at[u]] = v[u].x;
         if (again) {
           long long m_at = base + s_off[c[u]] + s_len[c[u]];
-          for (long long m = i + 1; m < q.n && q.keys[m] == s_key[c[u]]; ++m) {
+          for (long long m = ki + 1; m < q.n && q.keys[m] == s_key[c[u]]; ++m) {
             const int l = local_len(a, q, m);
             if (j < l && below(m_at + j, q.nout)) q.out[m_at + j] = v[u].x;
             m_at += l;
@@ -896,7 +934,8 @@ int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t 
     const bool rows = t->kind != 2 && t->width % 4 == 0 && a.sstride == 1 &&
                       (((uintptr_t)vals | (uintptr_t)out | (uintptr_t)t->w) & 15) == 0;
     const long long work = rows ? n * (t->width / 4) : n * t->width;
-    const unsigned ctas = (unsigned)((work + 256 * kLocalUnroll - 1) / (256 * kLocalUnroll));
+    const int unroll = group && t->width == 1 ? kStateUnroll : kLocalUnroll;
+    const unsigned ctas = (unsigned)((work + 256 * unroll - 1) / (256 * unroll));
     if (rows) sparse_local_rows_kernel<<<ctas, 256, 0, s>>>(a, q);
     else if (group && t->width == 1) sparse_local_kernel<true, true><<<ctas, 256, 0, s>>>(a, q);
     else if (group) sparse_local_kernel<true, false><<<ctas, 256, 0, s>>>(a, q);

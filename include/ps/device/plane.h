@@ -175,7 +175,7 @@ class Plane : public DeviceRoute {
   // ---- DeviceRoute ---------------------------------------------------------------------------
   bool Claims(int app_id, const SArray<Key>& keys) override;
   size_t PullBytes(int app_id, const SArray<Key>& keys) override;
-  void Submit(const DeviceRequest& req) override;
+  void Submit(DeviceRequest&& req) override;
 
   // Kernels launched through the plane (for reports).
   uint64_t launches() const;
@@ -187,8 +187,8 @@ class Plane : public DeviceRoute {
   struct Impl;
 
  private:
-  void SubmitSparse(const DeviceRequest& req);
-  void FinishSparse(const SparseInfo* sp, const DeviceRequest& req, void* stream);
+  void SubmitSparse(DeviceRequest&& req);
+  void FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* stream);
   Plane();
   ~Plane();
   std::unique_ptr<Impl> impl_;

@@ -52,7 +52,7 @@ class DeviceRoute {
   virtual size_t PullBytes(int app_id, const SArray<Key>& keys) = 0;
   // Takes the request; completion is reported through req.customer (AddResponse, or
   // FailRequest when a device-side wait ran out).
-  virtual void Submit(const DeviceRequest& req) = 0;
+  virtual void Submit(DeviceRequest&& req) = 0;
 };
 
 }  // namespace ps

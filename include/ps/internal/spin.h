@@ -10,6 +10,7 @@
 
 #include <chrono>
 #include <cstdlib>
+#include <mutex>
 
 namespace ps {
 
@@ -28,6 +29,18 @@ inline void CpuPause() {
 #if defined(__x86_64__) || defined(__i386__)
   __builtin_ia32_pause();
 #endif
+}
+
+// Takes a mutex that is held for less than a microsecond at a time: a thread that went to sleep
+// on it would have to be woken by the holder, which costs either side more than the wait.
+inline std::unique_lock<std::mutex> SpinLock(std::mutex& mu) {
+  std::unique_lock<std::mutex> lk(mu, std::defer_lock);
+  for (int i = 0; i < 64; ++i) {
+    if (lk.try_lock()) return lk;
+    CpuPause();
+  }
+  lk.lock();
+  return lk;
 }
 
 // Polls `ready` until it holds or `until` has passed; returns whether it held.

@@ -200,7 +200,7 @@ class KVWorker : public SimpleApp {
   int SubmitToDevice(DeviceRoute* route, bool push, bool pull, int cmd, const SArray<Key>& keys,
                      const void* vals, size_t vals_bytes, void* outs, size_t outs_bytes,
                      const SArray<int>& lens, int* lens_out, size_t lens_out_n,
-                     const Callback& cb, int priority) {
+                     Callback cb, int priority) {
     const int ts = obj_->NewRequest(kServerGroup);
     DeviceRequest req;
     req.app_id = obj_->app_id();
@@ -220,8 +220,8 @@ class KVWorker : public SimpleApp {
     req.val_size = sizeof(Val);
     req.customer = obj_;
     req.responses = Postoffice::Get()->num_servers();
-    req.on_done = cb;
-    route->Submit(req);
+    req.on_done = std::move(cb);
+    route->Submit(std::move(req));
     return ts;
   }
 

@@ -127,6 +127,15 @@ class SArray {
     kind_ = MemKind::kHost;
   }
 
+  // A view of caller memory without an owner of any kind (nothing is allocated): the caller keeps
+  // `data` alive for as long as any view of it exists.
+  static SArray<V> View(V* data, size_t size) {
+    SArray<V> a;
+    a.data_ = data;
+    a.size_ = a.capacity_ = size;
+    return a;
+  }
+
   // Device flavour: a view of `size` elements of device memory kept alive by `owner`.
   static SArray<V> FromDevice(V* dev_ptr, size_t size, std::shared_ptr<void> owner = nullptr) {
     SArray<V> a;

@@ -79,10 +79,6 @@ class Context:
         if not self.worker:
             raise host.PSError(L.ps_capi_last_error().decode())
 
-    def raw_stream(self) -> int:
-        """Handle of the calling thread's current stream on this context's device."""
-        return torch._C._cuda_getCurrentRawStream(self._device_index)
-
     def new_channel(self) -> int:
         """A rendezvous channel for one more tensor; raises when all are taken."""
         return host._ck(host.lib().psnvl_new_channel())
@@ -198,9 +194,9 @@ class KVStore:
         self.ctx = ctx or init()
         self.tables: Dict[int, DenseTable] = {}
         self._keys: Dict[int, np.ndarray] = {}
-        self._key_ptrs: Dict[int, int] = {}
+        self._targets: Dict[int, object] = {}
         # looked up once: small requests cost as much as the calls that make them
-        self._call = host.lib().ps_capi_bworker_request_on
+        self._submit = _lib.torch_ext().request
         self._wait = host.lib().ps_capi_bworker_wait
         self._alive: Dict[int, tuple] = {}
         if slice_bytes:
@@ -232,7 +228,10 @@ class KVStore:
         host._ck(L.psnvl_dense_keys(int(key), keys.ctypes.data_as(C.POINTER(C.c_uint64))))
         self.tables[key] = t
         self._keys[key] = keys
-        self._key_ptrs[key] = keys.ctypes.data
+        fn = C.cast(L.ps_capi_bworker_request_on, C.c_void_p).value
+        self._targets[key] = _lib.torch_ext().target(
+            fn, self.ctx.worker, keys.ctypes.data, keys.size, t.n_user, t.grad_dtype, t.out_dtype,
+            t.grad.data_ptr(), t.weight.data_ptr(), self.ctx._device_index)
         return t
 
     def keys_of(self, key: int) -> np.ndarray:
@@ -249,27 +248,10 @@ class KVStore:
     # -- requests ----------------------------------------------------------------------------
     def _request(self, key: int, push: bool, pull: bool, value: Optional[torch.Tensor],
                  out: Optional[torch.Tensor], cmd: int = 0, priority: int = 0) -> int:
-        t = self.tables[key]
-        vptr = vbytes = optr = obytes = 0
-        if push:
-            if value is None:
-                value = t.grad[: t.n_user]
-            if not value.is_contiguous() or value.numel() != t.n_user or value.dtype != t.grad_dtype:
-                raise ValueError("pushed values must be a contiguous tensor of the declared "
-                                 "length and gradient dtype")
-            vptr, vbytes = value.data_ptr(), t.n_user * t.grad_size
-        if pull:
-            if out is None:
-                out = t.weight[: t.n_user]
-            if not out.is_contiguous() or out.numel() != t.n_user or out.dtype != t.out_dtype:
-                raise ValueError("the output must be a contiguous tensor of the declared "
-                                 "length and weight dtype")
-            optr, obytes = out.data_ptr(), t.n_user * t.out_size
-        ts = self._call(self.ctx.worker, self.ctx.raw_stream(), push, pull, self._key_ptrs[key],
-                        self.ctx.world, vptr, vbytes, optr, obytes, cmd, priority)
+        ts = self._submit(self._targets[key], push, pull, value, out, cmd, priority)
         if ts < 0:
             raise host.PSError(host.lib().ps_capi_last_error().decode())
-        self._alive[ts] = (value, out, t)   # zero-copy: kept until the request completed
+        self._alive[ts] = (value, out)   # zero-copy: kept until the request completed
         if len(self._alive) > MAX_UNWAITED:
             self.wait(min(self._alive))   # a caller that never waits: retire the oldest
         return ts
@@ -336,46 +318,25 @@ class KeyedStore:
         self.worker = L.ps_capi_bworker_new(self.app_id, cid)
         if not self.worker:
             raise host.PSError(L.ps_capi_last_error().decode())
+        ext = _lib.torch_ext()
+        fn = C.cast(L.ps_capi_bworker_keyed_request_on, C.c_void_p).value
+        self._submit = ext.keyed_request
+        self._target = ext.keyed_target(fn, self.worker, self.max_keys, self.var_len,
+                                        ctx._device_index)
+        self._wait = L.ps_capi_bworker_wait
         self._alive: Dict[int, tuple] = {}
         if not hasattr(ctx, "_keyed"):
             ctx._keyed = []
         ctx._keyed.append(self)   # closed with the context, before the plane stops
-
-    def _check(self, t: Optional[torch.Tensor], dtype, what: str) -> None:
-        if t is not None and not (t.is_cuda and t.is_contiguous() and t.dtype == dtype):
-            raise ValueError(f"{what} must be a contiguous {dtype} tensor on the device")
 
     def request(self, keys: torch.Tensor, vals: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None, lens: Optional[torch.Tensor] = None,
                 lens_out: Optional[torch.Tensor] = None) -> int:
         """``vals`` given: push; ``out`` given: pull; both: ``ZPushPull``.  Returns a timestamp
         for :meth:`wait`.  The tensors must stay unchanged until then."""
-        push, pull = vals is not None, out is not None
-        if not (push or pull):
-            raise ValueError("nothing to do: give vals, out or both")
-        self._check(keys, torch.int64, "keys")
-        self._check(vals, torch.float32, "vals")
-        self._check(out, torch.float32, "out")
-        self._check(lens, torch.int32, "lens")
-        self._check(lens_out, torch.int32, "lens_out")
-        n = keys.numel()
-        if n > self.max_keys:
-            raise ValueError("more keys than max_keys")
-        if push and self.var_len and (lens is None or lens.numel() != n):
-            raise ValueError("a push to a table with lengths names one length per key")
-        if not self.var_len and (lens is not None or lens_out is not None):
-            raise ValueError("this table holds fixed-width values")
-        if lens_out is not None and lens_out.numel() != n:
-            raise ValueError("lens_out needs one entry per key")
-        L = host.lib()
-        ts = L.ps_capi_bworker_keyed_request_on(
-            self.worker, self.ctx.raw_stream(), push, pull, keys.data_ptr(), n,
-            vals.data_ptr() if push else None, vals.numel() * 4 if push else 0,
-            out.data_ptr() if pull else None, out.numel() * 4 if pull else 0,
-            lens.data_ptr() if (push and lens is not None) else None,
-            lens_out.data_ptr() if (pull and not push and lens_out is not None) else None, 0)
+        ts = self._submit(self._target, keys, vals, out, lens, lens_out)
         if ts < 0:
-            raise host.PSError(L.ps_capi_last_error().decode())
+            raise host.PSError(host.lib().ps_capi_last_error().decode())
         self._alive[ts] = (keys, vals, out, lens, lens_out)
         if len(self._alive) > MAX_UNWAITED:
             self.wait(min(self._alive))
@@ -391,10 +352,9 @@ class KeyedStore:
         return self.request(keys, vals=vals, out=out, lens=lens)
 
     def wait(self, ts: int) -> None:
-        L = host.lib()
         try:
-            if L.ps_capi_bworker_wait(self.worker, int(ts)) < 0:
-                raise host.PSError(L.ps_capi_last_error().decode())
+            if self._wait(self.worker, ts) < 0:
+                raise host.PSError(host.lib().ps_capi_last_error().decode())
         finally:
             self._alive.pop(ts, None)
 
@@ -402,5 +362,5 @@ class KeyedStore:
         if self.worker:
             host._ck(host.lib().psnvl_drain())
             host.lib().ps_capi_bworker_delete(self.worker)
-            self.worker = None
+            self.worker = self._target = None
             self._alive.clear()

@@ -161,16 +161,17 @@ int ps_capi_bworker_request(void* worker, int push, int pull, const uint64_t* ke
                             int cmd, int priority) {
   return Guard([&] {
     auto* kv = static_cast<KVWorker<char>*>(worker);
-    SArray<Key> k;
-    k.CopyFrom(reinterpret_cast<const Key*>(keys), nkeys);  // a handful of keys per tensor
-    SArray<char> v(const_cast<char*>(static_cast<const char*>(vals)), vals_bytes, false);
+    // views: the caller keeps keys, values and outputs until the request has been waited for
+    const auto k = SArray<Key>::View(const_cast<Key*>(reinterpret_cast<const Key*>(keys)), nkeys);
+    const auto v =
+        SArray<char>::View(const_cast<char*>(static_cast<const char*>(vals)), vals_bytes);
     if (push && pull) {
       // the output view lives until the request has completed
-      auto* o = new SArray<char>(static_cast<char*>(outs), outs_bytes, false);
+      auto* o = new SArray<char>(SArray<char>::View(static_cast<char*>(outs), outs_bytes));
       return kv->ZPushPull(k, v, o, nullptr, cmd, [o]() { delete o; }, priority);
     }
     if (push) return kv->ZPush(k, v, {}, cmd, nullptr, priority);
-    auto* o = new SArray<char>(static_cast<char*>(outs), outs_bytes, false);
+    auto* o = new SArray<char>(SArray<char>::View(static_cast<char*>(outs), outs_bytes));
     return kv->ZPull(k, o, nullptr, cmd, [o]() { delete o; }, priority);
   });
 }

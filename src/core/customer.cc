@@ -45,7 +45,7 @@ int Customer::NewRequest(int recver) {
 void Customer::WaitRequest(int timestamp) { WaitRequestFor(timestamp, -1); }
 
 bool Customer::WaitRequestFor(int timestamp, int timeout_ms) {
-  std::unique_lock<std::mutex> lk(tracker_mu_);
+  std::unique_lock<std::mutex> lk = SpinLock(tracker_mu_);
   CHECK_GE(timestamp, 0);
   CHECK_LT(static_cast<size_t>(timestamp), tracker_base_ + tracker_.size()) << "unknown timestamp";
   auto done = [this, timestamp] {
@@ -62,7 +62,7 @@ bool Customer::WaitRequestFor(int timestamp, int timeout_ms) {
       const unsigned seen = progress_.load(std::memory_order_relaxed);
       lk.unlock();
       SpinUntil(until, [&] { return progress_.load(std::memory_order_relaxed) != seen; });
-      lk.lock();
+      lk = SpinLock(tracker_mu_);
     } while (!done() && std::chrono::steady_clock::now() < until);
   }
   if (timeout_ms < 0) {
@@ -102,7 +102,7 @@ int Customer::NumResponse(int timestamp) {
 }
 
 void Customer::AddResponse(int timestamp, int num) {
-  std::lock_guard<std::mutex> lk(tracker_mu_);
+  std::unique_lock<std::mutex> lk = SpinLock(tracker_mu_);
   if (timestamp >= tracker_base_) tracker_[timestamp - tracker_base_].second += num;
   // forget completed requests beyond the window of recent ones
   while (tracker_.size() > kTrackerWindow && tracker_.front().first <= tracker_.front().second) {

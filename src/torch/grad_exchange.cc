@@ -229,7 +229,10 @@ class GradExchange {
 
 }  // namespace
 
+void add_requests(py::module& m);  // requests.cc
+
 PYBIND11_MODULE(psb200_torch, m) {
+  add_requests(m);
   using release = py::call_guard<py::gil_scoped_release>;
   py::class_<GradExchange>(m, "GradExchange")
       .def(py::init<std::vector<at::Tensor>, std::vector<int64_t>, std::vector<int64_t>, at::Tensor,

@@ -519,7 +519,7 @@ struct Plane::Impl {
   };
   std::map<const void*, Done> last_done;
   Done LastDone(const void* tensor) {
-    std::lock_guard<std::mutex> lk(mu);
+    const auto lk = SpinLock(mu);
     auto it = last_done.find(tensor);
     return it == last_done.end() ? Done() : it->second;
   }
@@ -554,7 +554,7 @@ struct Plane::Impl {
     bool wake;
     if (p.customer) p.customer->RouteBegin();
     {
-      std::lock_guard<std::mutex> lk(q_mu);
+      const auto lk = SpinLock(q_mu);
       ++in_flight;
       queue.push_back(std::move(p));
       queued.store(static_cast<int>(queue.size()), std::memory_order_release);
@@ -566,7 +566,7 @@ struct Plane::Impl {
 
   void* NewEvent() {
     {
-      std::lock_guard<std::mutex> lk(ev_mu);
+      const auto lk = SpinLock(ev_mu);
       if (!event_pool.empty()) {
         void* e = event_pool.back();
         event_pool.pop_back();
@@ -579,7 +579,7 @@ struct Plane::Impl {
   }
   void RecycleEvent(void* e) {
     if (sim) return;
-    std::lock_guard<std::mutex> lk(ev_mu);
+    const auto lk = SpinLock(ev_mu);
     event_pool.push_back(e);
   }
 
@@ -591,10 +591,12 @@ struct Plane::Impl {
         // the next request of a worker that waits for each one follows within microseconds
         SpinUntil(std::chrono::steady_clock::now() + std::chrono::microseconds(SpinMicros()),
                   [&] { return queued.load(std::memory_order_acquire) > 0 || stop; });
-        std::unique_lock<std::mutex> lk(q_mu);
-        asleep = true;
-        q_cv.wait(lk, [&] { return stop || !queue.empty(); });
-        asleep = false;
+        std::unique_lock<std::mutex> lk = SpinLock(q_mu);
+        if (queue.empty() && !stop) {
+          asleep = true;
+          q_cv.wait(lk, [&] { return stop || !queue.empty(); });
+          asleep = false;
+        }
         if (queue.empty()) return;
         p = std::move(queue.front());
         queue.pop_front();
@@ -624,17 +626,18 @@ struct Plane::Impl {
       }
       {
         // the event stops being the ordering point of its tensor before it is reused
-        std::lock_guard<std::mutex> lk(mu);
+        const auto lk = SpinLock(mu);
         auto it = last_done.find(p.tensor);
         if (it != last_done.end() && it->second.event == p.event) last_done.erase(it);
       }
       RecycleEvent(p.event);
       for (void* e : p.events_to_recycle) RecycleEvent(e);
+      bool idle;
       {
-        std::lock_guard<std::mutex> lk(q_mu);
-        --in_flight;
+        const auto lk = SpinLock(q_mu);
+        idle = --in_flight == 0;
       }
-      idle_cv.notify_all();
+      if (idle) idle_cv.notify_all();
     }
   }
 
@@ -1071,7 +1074,7 @@ void Plane::UnregisterDense(int app_id, uint64_t tensor_id) {
 }
 
 const DenseInfo* Plane::FindDense(int app_id, uint64_t tensor_id) const {
-  std::lock_guard<std::mutex> lk(impl_->mu);
+  const auto lk = SpinLock(impl_->mu);
   auto it = impl_->dense.find(std::make_pair(app_id, tensor_id));
   return it == impl_->dense.end() ? nullptr : it->second.get();
 }
@@ -1259,7 +1262,7 @@ const SparseInfo& Plane::DeclareSparse(int app_id, uint64_t key_space, int64_t m
 }
 
 const SparseInfo* Plane::FindSparse(int app_id) const {
-  std::lock_guard<std::mutex> lk(impl_->mu);
+  const auto lk = SpinLock(impl_->mu);
   auto it = impl_->sparse.find(app_id);
   return it == impl_->sparse.end() ? nullptr : it->second.get();
 }
@@ -1272,12 +1275,12 @@ void Plane::Memcpy(void* dst, const void* src, size_t bytes) {
   CHECK_EQ(m.rt.stream_sync(m.s_status), 0);
 }
 
-void Plane::Submit(const DeviceRequest& req) {
+void Plane::Submit(DeviceRequest&& req) {
   Impl& m = *impl_;
   CHECK(m.started);
   m.rt.set_device(m.opts.device);
   if (req.keys.mem_kind() == MemKind::kDevice) {
-    SubmitSparse(req);
+    SubmitSparse(std::move(req));
     return;
   }
   const int W = m.world;
@@ -1292,8 +1295,11 @@ void Plane::Submit(const DeviceRequest& req) {
   // keys -> runs of consecutive shards -> element ranges (in user elements: the last shard's
   // share may be short)
   struct Run { int64_t begin, end; };
-  std::vector<Run> runs;
-  std::vector<int> lens(req.keys.size());
+  // (shards increase from key to key, so there are at most W of each)
+  Run runs[PSDEV_MAX_RANKS];
+  int nruns = 0;
+  int lens[PSDEV_MAX_RANKS];
+  const size_t nlens = req.keys.size();
   int prev = -2;
   for (size_t i = 0; i < req.keys.size(); ++i) {
     uint64_t id_i;
@@ -1308,12 +1314,12 @@ void Plane::Submit(const DeviceRequest& req) {
       CHECK_EQ(req.lens[static_cast<int>(i)], lens[i])
           << "length of key " << req.keys[static_cast<int>(i)] << " differs from its share";
     }
-    if (shard == prev + 1 && !runs.empty()) runs.back().end = hi;
-    else runs.push_back(Run{lo, hi});
+    if (shard == prev + 1 && nruns) runs[nruns - 1].end = hi;
+    else runs[nruns++] = Run{lo, hi};
     prev = shard;
   }
   size_t total = 0;
-  for (const Run& r : runs) total += static_cast<size_t>(r.end - r.begin);
+  for (int i = 0; i < nruns; ++i) total += static_cast<size_t>(runs[i].end - runs[i].begin);
   if (req.push) {
     CHECK(req.vals) << "push without values";
     CHECK_EQ(req.vals_bytes, total * gsz)
@@ -1323,7 +1329,7 @@ void Plane::Submit(const DeviceRequest& req) {
   if (req.pull && req.outs) {
     CHECK_EQ(req.outs_bytes, total * osz) << "output size does not match the pulled values";
   }
-  if (req.lens_out) { CHECK_EQ(req.lens_out_n, lens.size()); }
+  if (req.lens_out) { CHECK_EQ(req.lens_out_n, nlens); }
 
   // (the CPU stand-in calls "device memory" what lies in an arena)
   auto on_device = [&](const void* p) {
@@ -1366,10 +1372,10 @@ void Plane::Submit(const DeviceRequest& req) {
   pend.timestamp = req.timestamp;
   pend.responses = req.responses;
   pend.customer = req.customer;
-  pend.on_done = req.on_done;
+  pend.on_done = std::move(req.on_done);
   pend.lens_out = req.lens_out;
   pend.tensor = d;
-  if (req.lens_out) pend.lens = lens;
+  if (req.lens_out) pend.lens.assign(lens, lens + nlens);
 
   const Impl::Done prev_done = m.LastDone(d);
   void* done = m.NewEvent();
@@ -1385,7 +1391,8 @@ void Plane::Submit(const DeviceRequest& req) {
     done_stream = s;
     if (!m.sim) m.After(prev_done, s);
     size_t eoff = 0;  // position in the request's value list, in elements
-    for (const Run& r : runs) {
+    for (int ri = 0; ri < nruns; ++ri) {
+      const Run& r = runs[ri];
       const size_t cnt = static_cast<size_t>(r.end - r.begin);
       if (W == 1 && !m.sim && DirectOk(*d, req, gsz, osz)) {
         // one rank: the kernel reads and writes the caller's arrays, nobody else needs the
@@ -1448,7 +1455,8 @@ void Plane::Submit(const DeviceRequest& req) {
       CHECK_EQ(m.rt.memcpy_async(h.dst, h.src, h.bytes, m.s_d2h), 0);
     };
     size_t elem_off = 0;  // position in the request's value list
-    for (const Run& r : runs) {
+    for (int ri = 0; ri < nruns; ++ri) {
+      const Run& r = runs[ri];
       const std::vector<int64_t> cuts = SliceEnds(r.begin, r.end, small_g, step_g);
       int64_t b = r.begin;
       for (const int64_t e : cuts) {
@@ -1519,7 +1527,7 @@ void Plane::Submit(const DeviceRequest& req) {
 // apply and respond run on the caller's stream; the rendezvous of the ranks is inside the last
 // two kernels.  A push without pull still runs the respond kernel (it closes the round); a pull
 // without push scatters zeros, which changes nothing on the owners.
-void Plane::SubmitSparse(const DeviceRequest& req) {
+void Plane::SubmitSparse(DeviceRequest&& req) {
   Impl& m = *impl_;
   SparseInfo* sp = const_cast<SparseInfo*>(FindSparse(req.app_id));
   CHECK(sp) << "app " << req.app_id << " has no keyed table";
@@ -1575,7 +1583,7 @@ void Plane::SubmitSparse(const DeviceRequest& req) {
                                static_cast<int64_t>(vbytes / 4), lens_in, static_cast<float*>(out),
                                static_cast<int64_t>(obytes / 4), static_cast<int*>(lens_to), s), 0)
         << "psdev_sparse_local failed";
-    FinishSparse(sp, req, s);
+    FinishSparse(sp, std::move(req), s);
     return;
   }
   if (kptr != sp->keys) {
@@ -1618,11 +1626,11 @@ void Plane::SubmitSparse(const DeviceRequest& req) {
     CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));
     CHECK_EQ(m.rt.memcpy_async(req.lens_out, sp->lens, static_cast<size_t>(n) * 4, s), 0);
   }
-  FinishSparse(sp, req, s);
+  FinishSparse(sp, std::move(req), s);
 }
 
 // The request's work has been issued on `s`: completion and the ordering point of the table.
-void Plane::FinishSparse(const SparseInfo* sp, const DeviceRequest& req, void* s) {
+void Plane::FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* s) {
   Impl& m = *impl_;
   void* done = m.NewEvent();
   m.rt.event_record(done, s);
@@ -1632,7 +1640,7 @@ void Plane::FinishSparse(const SparseInfo* sp, const DeviceRequest& req, void* s
   pend.timestamp = req.timestamp;
   pend.responses = req.responses;
   pend.customer = req.customer;
-  pend.on_done = req.on_done;
+  pend.on_done = std::move(req.on_done);
   pend.tensor = sp;
   {
     std::lock_guard<std::mutex> lk(m.mu);

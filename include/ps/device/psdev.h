@@ -203,8 +203,8 @@ int psdev_dense_op(const psdev_world_t* w, const psdev_table_t* t, int op,
  * the pushed values read from `src` and the pulled values stored to `dst` as well as to the
  * table's weight buffer, so that arrays outside the arena need no copies.  src / dst hold the
  * value of element `begin` first and reach up to element n_valid (the rest of the range is
- * padding); NULL names the table's own buffers.  Either may be device memory of any alignment
- * that its type allows. */
+ * padding); NULL names the table's own buffers.  Either may be device memory, or page-locked host
+ * memory that the device can access, of any alignment that its type allows. */
 int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op, int64_t begin,
                           int64_t end, const psdev_opt_t* opt, int channel, int num_ctas,
                           void* stream, const void* src, void* dst, int64_t n_valid);
@@ -376,6 +376,7 @@ int psdev_rt_stream_wait_event(void* stream, void* event);
 int psdev_rt_memcpy_async(void* dst, const void* src, size_t bytes, void* stream);
 int psdev_rt_is_device_pointer(const void* p);
 int psdev_rt_is_pinned_host(const void* p);
+int psdev_rt_host_mapped(const void* p, size_t bytes, void** dev);
 int psdev_rt_host_alloc(void** p, size_t bytes);
 int psdev_rt_host_free(void* p);
 

@@ -75,6 +75,22 @@ int psdev_rt_is_pinned_host(const void* p) {
   }
   return a.type == cudaMemoryTypeHost;
 }
+// 1 if all of [p, p + bytes) is page-locked host memory that kernels can access; *dev receives
+// its address on the device.
+int psdev_rt_host_mapped(const void* p, size_t bytes, void** dev) {
+  cudaPointerAttributes a, b;
+  if (bytes == 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess ||
+      cudaPointerGetAttributes(&b, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
+      static_cast<char*>(b.devicePointer) - static_cast<char*>(a.devicePointer) !=
+          static_cast<ptrdiff_t>(bytes - 1))
+    return 0;
+  *dev = a.devicePointer;
+  return 1;
+}
 int psdev_rt_host_alloc(void** p, size_t bytes) {
   return (int)cudaHostAlloc(p, bytes, cudaHostAllocDefault);
 }

@@ -73,6 +73,7 @@ struct Rt {
   int (*device_barrier)(const psdev_world_t*, int, uint64_t, void*) = nullptr;
   int (*multicast_pays)(int, uint64_t) = nullptr;
   int (*is_device_pointer)(const void*) = nullptr;
+  int (*host_mapped)(const void*, size_t, void**) = nullptr;
   int (*heap_create)(size_t, void**, unsigned char*) = nullptr;
   int (*heap_open)(const unsigned char*, void**) = nullptr;
   int (*heap_close)(void*) = nullptr;
@@ -150,6 +151,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_device_barrier", &rt->device_barrier);
   Bind(lib, "psdev_multicast_pays", &rt->multicast_pays);
   Bind(lib, "psdev_rt_is_device_pointer", &rt->is_device_pointer);
+  Bind(lib, "psdev_rt_host_mapped", &rt->host_mapped);
   Bind(lib, "psdev_heap_create", &rt->heap_create);
   Bind(lib, "psdev_heap_open", &rt->heap_open);
   Bind(lib, "psdev_heap_close", &rt->heap_close);
@@ -1123,13 +1125,17 @@ inline bool Clash(const void* a, size_t an, size_t asz, const void* b, size_t bn
   return x < y + bn * bsz && y < x + an * asz && !(x == y && asz == bsz);
 }
 
+// One rank: the largest request whose host arrays the kernel accesses itself (both directions, one
+// direction), its CTAs, and the smallest slice of the staged form.
+constexpr size_t kZeroCopyBoth = 48u << 20, kZeroCopyOne = 16u << 20;
+constexpr int kZeroCopyCtas = 148;
+constexpr size_t kMinSlice = 4u << 20;
+
 // One rank: may the kernel use the request's arrays where they are?  Not when they are aligned
 // to less than their element type, nor when an array that is read shares memory with one that
 // is written (such a request goes through the tensor's own buffers).
-bool DirectOk(const DenseInfo& d, const DeviceRequest& req, size_t gsz, size_t osz) {
+bool DirectOk(const DenseInfo& d, const void* in, const void* out, size_t gsz, size_t osz) {
   const size_t n = static_cast<size_t>(d.n_user), nt = static_cast<size_t>(d.n);
-  const void* in = req.push ? req.vals : nullptr;
-  void* out = req.pull ? req.outs : nullptr;
   if ((reinterpret_cast<uintptr_t>(in) & (gsz - 1)) ||
       (reinterpret_cast<uintptr_t>(out) & (osz - 1)))
     return false;
@@ -1342,7 +1348,27 @@ void Plane::Submit(DeviceRequest&& req) {
   const bool out_dev = req.pull && req.outs && on_device(req.outs);
   const bool host_in = req.push && !in_dev;
   const bool host_out = req.pull && req.outs && !out_dev;
-  const bool staged = host_in || host_out;
+  bool staged = host_in || host_out;
+  // One rank, values in pinned host memory: up to a size the kernel reads and writes them over
+  // PCIe itself, a few CTAs being enough to fill the link.  One kernel has no slices to fill and
+  // drain and no hand-over between copy engine and kernel (about 10 us per slice); the copy
+  // engines move a byte faster once that no longer counts.  Both directions, device time of the
+  // best slicing against the kernel: 1 MiB 57 / 41 us, 4 MiB 163 / 119, 16 MiB 488 / 428, 32 MiB
+  // 890 / 843, 64 MiB 1638 / 1674.  One direction alone: 1213 us copied and 1314 read at 64 MiB.
+  const void* in_at = req.vals;
+  void* out_at = req.outs;
+  if (staged && W == 1 && !m.sim) {
+    const size_t limit = host_in && host_out ? kZeroCopyBoth : kZeroCopyOne;
+    void *in_map = nullptr, *out_map = nullptr;
+    if ((!host_in || (req.vals_bytes <= limit &&
+                      m.rt.host_mapped(req.vals, req.vals_bytes, &in_map))) &&
+        (!host_out || (req.outs_bytes <= limit &&
+                       m.rt.host_mapped(req.outs, req.outs_bytes, &out_map)))) {
+      if (host_in) in_at = in_map;
+      if (host_out) out_at = out_map;
+      staged = !DirectOk(*d, req.push ? in_at : nullptr, req.pull ? out_at : nullptr, gsz, osz);
+    }
+  }
   int op = (req.push ? PSDEV_OP_PUSH : 0) | (req.pull ? PSDEV_OP_PULL : 0);
   if (req.push && !req.pull && req.cmd == kCmdPublish) op |= PSDEV_OP_PUBLISH;
 
@@ -1394,13 +1420,17 @@ void Plane::Submit(DeviceRequest&& req) {
     for (int ri = 0; ri < nruns; ++ri) {
       const Run& r = runs[ri];
       const size_t cnt = static_cast<size_t>(r.end - r.begin);
-      if (W == 1 && !m.sim && DirectOk(*d, req, gsz, osz)) {
+      if (W == 1 && !m.sim && (host_in || host_out ||
+                               DirectOk(*d, req.push ? vals : nullptr, req.pull ? outs : nullptr,
+                                        gsz, osz))) {
         // one rank: the kernel reads and writes the caller's arrays, nobody else needs the
         // values in the arena
-        const char* src = req.push && vals != grad ? vals : nullptr;
-        char* dst = req.pull && outs && outs != weight ? outs : nullptr;
+        const void* src = req.push && vals != grad ? in_at : nullptr;
+        void* dst = req.pull && outs && outs != weight ? out_at : nullptr;
+        int ctas = d->num_ctas;
+        if ((host_in || host_out) && ctas <= 0) ctas = kZeroCopyCtas;
         const int rc = m.rt.dense_op_direct(&m.ws, &t, op, r.begin, pad8(r.end), &opt, d->channel,
-                                            d->num_ctas, s, src, dst, d->n_user);
+                                            ctas, s, src, dst, d->n_user);
         CHECK_EQ(rc, 0) << "psdev_dense_op_direct failed";
         continue;
       }
@@ -1431,12 +1461,16 @@ void Plane::Submit(DeviceRequest&& req) {
       m.After(prev_done, s);
       if (start) m.rt.stream_wait_event(s, start);
     }
-    const int64_t step_g =
-        std::max<int64_t>(8, static_cast<int64_t>(m.opts.slice_bytes / gsz) & ~int64_t(7));
+    size_t slice = m.opts.slice_bytes;
+    if (W == 1) slice = std::min(slice, std::max(kMinSlice, total * gsz / 32));
+    const int64_t step_g = std::max<int64_t>(8, static_cast<int64_t>(slice / gsz) & ~int64_t(7));
     // The first slice's copy in and the last slice's copy out overlap with nothing, so the
     // slices grow from 1/16 of the configured size (at least 256 KiB), doubling up to it, and
-    // shrink again the same way towards the end of a run.
-    const int64_t small_g = std::max<int64_t>(
+    // shrink again the same way towards the end of a run.  With one rank no kernel waits for a
+    // peer and equal slices are faster, as small as the hand-over between copy engine and kernel
+    // allows (64 MiB both ways: 16 MiB slices with the ramp 1937 us, equal slices of 2 / 4 / 8 MiB
+    // 1820 / 1613 / 1660; 256 MiB: 4 / 8 / 16 MiB 6063 / 6040 / 6215; plain copies 1342, 5386).
+    const int64_t small_g = W == 1 ? step_g : std::max<int64_t>(
         8, std::min<int64_t>(step_g, std::max<int64_t>(step_g / 16, (256 << 10) / gsz)) &
                ~int64_t(7));
     // A slice's copy out needs its copy in and its kernel, and the next slice's copy in ends

@@ -27,6 +27,7 @@
 #include <cuda_bf16.h>
 
 #include <atomic>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 
@@ -100,6 +101,12 @@ struct Cfg {
   static constexpr int kSmemBytes =
       kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kRingBytes;
 };
+
+}  // namespace gemm
+}  // namespace psdev
+#include "kernels/split_gemm.cuh"
+namespace psdev {
+namespace gemm {
 
 __device__ __forceinline__ void report(Scratch* s, int code) { atomicMin(&s->status, code); }
 
@@ -1342,6 +1349,66 @@ static int launch_pair(const Args& a, const CUtensorMap& tx, const CUtensorMap& 
   return launch_pair_t<false>(a, tx, tw, grid, s);
 }
 
+template <int BN, int S>
+static int launch_split_t(const SplitArgs& a, const CUtensorMap& tx, const CUtensorMap& tw,
+                          long long tiles, cudaStream_t s) {
+  static std::atomic<bool> attr_set[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(split_gemm_kernel<BN, S>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SplitCfg<BN>::kSmemBytes);
+    if (e != cudaSuccess) return (int)e;
+    attr_set[dev & 63].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(tiles * S), 1, 1);
+  cfg.blockDim = dim3(kSplitThreads, 1, 1);
+  cfg.dynamicSmemBytes = SplitCfg<BN>::kSmemBytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, split_gemm_kernel<BN, S>, a, tx, tw);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return (int)e;
+}
+template <int BN>
+static int launch_split(int split, const SplitArgs& a, const CUtensorMap& tx,
+                        const CUtensorMap& tw, long long tiles, cudaStream_t s) {
+  switch (split) {
+    case 1: return launch_split_t<BN, 1>(a, tx, tw, tiles, s);
+    case 2: return launch_split_t<BN, 2>(a, tx, tw, tiles, s);
+    case 4: return launch_split_t<BN, 4>(a, tx, tw, tiles, s);
+    case 8: return launch_split_t<BN, 8>(a, tx, tw, tiles, s);
+    default: return PSDEV_ERR_ARG;
+  }
+}
+static int run_split(const Args& a, const void* x, const void* w, int bn, int split,
+                     cudaStream_t s) {
+  CUtensorMap tx, tw;
+  int rc = make_tmap(&tx, x, a.M, a.K, BM);
+  if (rc) return rc;
+  rc = make_tmap(&tw, w, a.N, a.K, bn);
+  if (rc) return rc;
+  SplitArgs sa{};
+  sa.M = a.M;
+  sa.N = a.N;
+  sa.num_kb = (int)((a.K + BK - 1) / BK);
+  sa.tiles_m = (int)((a.M + BM - 1) / BM);
+  sa.c = a.c;
+  sa.status = &a.scratch->status;
+  sa.timeout_ns = a.timeout_ns;
+  while (split > sa.num_kb) split >>= 1;
+  const long long tiles = (long long)sa.tiles_m * ((a.N + bn - 1) / bn);
+  return bn == 64 ? launch_split<64>(split, sa, tx, tw, tiles, s)
+                  : launch_split<128>(split, sa, tx, tw, tiles, s);
+}
+
 // Output-tile height used by run(): 128 (double-buffered accumulators) or 256 (twice the
 // reuse of W per byte loaded).  0 = choose by shape.
 static std::atomic<int> g_tile_m{0};
@@ -1366,12 +1433,60 @@ static int pick_tile_m(long long M, long long N, long long K) {
   return 128;
 }
 
+// The split form (1000 * S + BN) for a product, or 0 when the persistent kernels are faster.  The
+// times below, in us, were fitted to measurements over M 64 .. 8192, N and K 256 .. 4096 (operands
+// in L2); they put the persistent kernels where 128 x 256 tiles fill the GPU and K is long:
+//                        64x256x4096  1024x1024x1024  1024x4096x1024  4096x2048x1024
+//   persistent (pairs)       23.4          11.9            12.2            18.6
+//   S = 1, BN = 64 / 128  16.9 / 20.8    7.4 / 8.3      15.7 / 11.7     28.1 / 21.2
+//   S = 4, BN = 64           10.1         21.5            34.5
+static int pick_split(long long M, long long N, long long K) {
+  const int config = g_tile_m.load();
+  if (config >= 1000) return config;
+  if (config != 0 || getenv("PSB200_GEMM_TILE")) return 0;
+  const double kb = (double)((K + BK - 1) / BK);
+  const double sms = 148;
+  auto tiles = [&](int m, int n) { return (double)(((M + m - 1) / m) * ((N + n - 1) / n)); };
+  double best;
+  const double t256 = tiles(256, 256);
+  if (M >= 256 && N >= 256 && t256 >= 74) {  // CTA pairs: whole rounds, or half of the last one
+    const double rounds = t256 / 74, whole = floor(rounds), rest = rounds - whole;
+    const double last = rest == 0 ? 0 : rest <= 0.25 ? 0.25 : rest <= 0.5 ? 0.5 : 1;
+    best = 8.0 + (whole + last) * fmax(0.327 * kb, 2.4);
+  } else {
+    const int bn = (N % 256 == 0 || N > 1024) ? 256 : 128;
+    best = 7.3 + ceil(tiles(128, bn) / sms) * fmax(0.29 * kb, 1.5);
+  }
+  int pick = 0;
+  for (int bn = 64; bn <= 128; bn += 64) {
+    for (int split = 1; split <= kMaxSplit; split *= 2) {
+      const double ctas = tiles(128, bn) * split;
+      if (split > 1 && (ctas > sms || split > kb)) break;
+      const double over = fmax(0.0, ctas / sms - 1);
+      const double base = bn == 64 ? 3.5 + 1.2 * over : 3.7 + 2.0 * over;
+      const double per_kb = bn == 64 ? fmax(0.21, 0.00117 * ctas) : fmax(0.297, 0.0016 * ctas);
+      const int l = split == 1 ? 0 : split == 2 ? 1 : split == 4 ? 2 : 3;
+      static const double exchange[2][4] = {{0, 1.7, 2.9, 3.6}, {0, 3.3, 6.7, 7.5}};
+      const double t = base + exchange[bn / 128][l] + ceil(kb / split) * per_kb;
+      if (t < best) {
+        best = t;
+        pick = 1000 * split + bn;
+      }
+    }
+  }
+  return pick;
+}
+
 static int run(Args a, const void* x, const void* w, int num_ctas, cudaStream_t s) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || (a.N & 7) || (a.K & 7)) return PSDEV_ERR_ARG;
   if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)a.c & 15)) return PSDEV_ERR_ARG;
   int err = 0;
   a.scratch = scratch_for_current_device(&err);
   if (!a.scratch) return err;
+  if (!a.fused && num_ctas <= 0) {
+    const int split = pick_split(a.M, a.N, a.K);
+    if (split) return run_split(a, x, w, split % 1000, split / 1000, s);
+  }
   const int variant = pick_tile_m(a.M, a.N, a.K);
   const bool pair = (variant == 2);
   const int tile_m = pair ? 256 : variant;  // rows of X per output tile (per pair for pairs)
@@ -1536,7 +1651,11 @@ extern "C" int64_t psdev_pull_plan_chunk(int64_t w_elem_off, int64_t nk, int blk
 // Selects the kernel variant of later GEMM launches: 128 or 256 (output-tile height of the
 // one-CTA kernels), 2 (CTA pairs, tcgen05 cta_group::2), or 0 for the built-in choice by shape.
 extern "C" int psdev_gemm_config(int tile_m) {
-  if (tile_m != 0 && tile_m != 128 && tile_m != 256 && tile_m != 2) return PSDEV_ERR_ARG;
+  const int bn = tile_m % 1000, split = tile_m / 1000;
+  const bool is_split = (bn == 64 || bn == 128) && (split == 1 || split == 2 || split == 4 ||
+                                                    split == 8);
+  if (tile_m != 0 && tile_m != 128 && tile_m != 256 && tile_m != 2 && !is_split)
+    return PSDEV_ERR_ARG;
   gemm::g_tile_m.store(tile_m);
   return 0;
 }

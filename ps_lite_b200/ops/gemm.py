@@ -9,8 +9,18 @@ import torch
 from .. import _lib
 
 
-def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
+class _Native:
+    """The native calls and the addresses they are given, resolved at the first use."""
+
+    def __getattr__(self, name):
+        lib, ext = _lib.device_lib(), _lib.torch_ext()
+        self.gemm_fn = C.cast(lib.psdev_gemm_bf16, C.c_void_p).value
+        self.pull_fn = C.cast(lib.psdev_pull_gemm_bf16, C.c_void_p).value
+        self.linear, self.pull_linear = ext.linear, ext.pull_linear
+        return self.__dict__[name]
+
+
+_native = _Native()
 
 
 def gemm_status(device) -> int:
@@ -24,16 +34,10 @@ def gemm_status(device) -> int:
 def linear_bf16(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
                 num_ctas: int = 0, timeout_s: float = 2.0) -> torch.Tensor:
     """``out[M,N] = x[M,K] @ w[N,K]^T`` (bf16 in, fp32 accumulate, bf16 out)."""
-    assert x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-    assert x.is_contiguous() and w.is_contiguous() and x.shape[-1] == w.shape[-1]
-    M, K = x.numel() // x.shape[-1], x.shape[-1]
-    N = w.shape[0]
-    if out is None:
-        out = torch.empty(*x.shape[:-1], N, dtype=torch.bfloat16, device=x.device)
-    rc = _lib.device_lib().psdev_gemm_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K,
-                                           num_ctas, int(timeout_s * 1e9), _stream(x.device))
-    _lib.check(rc, "psdev_gemm_bf16")
-    return out
+    got = _native.linear(_native.gemm_fn, x, w, out, num_ctas, int(timeout_s * 1e9))
+    if type(got) is int:
+        _lib.check(got, "psdev_gemm_bf16")
+    return got
 
 
 def pull_linear_bf16(table, w_offset: int, n_out: int, x: torch.Tensor,
@@ -45,17 +49,12 @@ def pull_linear_bf16(table, w_offset: int, n_out: int, x: torch.Tensor,
     Must follow, on the same stream, a ``table.push(..., publish=True)`` covering that range.
     Afterwards ``table.weight`` holds the complete W locally (for the backward pass).
     """
-    assert x.dtype == torch.bfloat16 and x.is_contiguous()
     assert table.out_dtype == torch.bfloat16
-    K = x.shape[-1]
-    M = x.numel() // K
-    if out is None:
-        out = torch.empty(*x.shape[:-1], n_out, dtype=torch.bfloat16, device=x.device)
-    rc = _lib.device_lib().psdev_pull_gemm_bf16(
-        C.byref(table._world), C.byref(table._table), int(w_offset), x.data_ptr(), out.data_ptr(),
-        M, n_out, K, num_copy_ctas, num_ctas, int(timeout_s * 1e9), _stream(x.device))
-    _lib.check(rc, "psdev_pull_gemm_bf16")
-    return out
+    got = _native.pull_linear(_native.pull_fn, table._world_at, table._table_at, int(w_offset),
+                              n_out, x, out, num_copy_ctas, num_ctas, int(timeout_s * 1e9))
+    if type(got) is int:
+        _lib.check(got, "psdev_pull_gemm_bf16")
+    return got
 
 
 def fusion_pays(weight_bytes: int, world: int) -> bool:

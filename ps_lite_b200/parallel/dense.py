@@ -115,7 +115,7 @@ class DenseTable:
         self.optimizer = optimizer or ServerOptimizer("sum")
         self.channel, self.num_ctas = int(channel), int(num_ctas)
         self.step = 0
-        self._opt_key, self._opt_cached = None, None
+        self._opt_key, self._opt_cached, self._opt_step, self._opt_at = None, None, -1, 0
         self._default_timeout = default_timeout_s()
         # NVSwitch multicast path: on by default from four ranks up when the heap has a
         # multicast alias (with two ranks plain peer accesses move fewer bytes per link)
@@ -153,6 +153,11 @@ class DenseTable:
         t.state2 = self.state2.data_ptr() if self.state2 is not None else None
         t.grad_dtype, t.out_dtype = _DT[grad_dtype], _DT[out_dtype]
         t.gscale_off = self.gscale_off
+        # what a call hands over, looked up once: small operations cost as much as the calls
+        self._world_at, self._table_at = C.addressof(self._world), C.addressof(t)
+        self._op_fn = C.cast(heap.lib.psdev_dense_op, C.c_void_p).value
+        self._dense_op = _lib.torch_ext().dense_op
+        self._device_index = dev.index or 0
         self.grad.zero_()
         self.weight.zero_()
         # Low-latency region for small fused requests (include/ps/device/push_pull_ll.cuh):
@@ -187,11 +192,13 @@ class DenseTable:
             raise TypeError("table was not created with grad_dtype=torch.int8")
         if begin % 256:
             raise ValueError("begin must be a multiple of 256")
-        g = grad.reshape(-1).contiguous()
-        s = torch.cuda.current_stream(self.heap.device)
+        g = grad if grad.is_contiguous() else grad.contiguous()
+        n = g.numel()
+        if begin < 0 or begin + n > self.n:
+            raise ValueError("the gradient reaches beyond the table")
         rc = self.heap.lib.psdev_filter_int8_pack(
-            g.data_ptr(), self.grad[begin:].data_ptr(), self.gscale[begin // 256:].data_ptr(),
-            g.numel(), s.cuda_stream)
+            g.data_ptr(), self.grad.data_ptr() + begin, self.gscale.data_ptr() + begin // 64, n,
+            torch._C._cuda_getCurrentRawStream(self._device_index))
         _lib.check(rc, "psdev_filter_int8_pack")
 
     # -- ownership helpers (host math mirrored by the kernels) ------------------------------
@@ -227,18 +234,17 @@ class DenseTable:
         end = self.n if end is None else end
         if op & _lib.OP_PUSH and opt_step:
             self.step += 1
-        o = self._opt_struct()
-        s = stream or torch.cuda.current_stream(self.heap.device)
+        self._opt_struct()   # (the call reads it at self._opt_at)
+        s = stream.cuda_stream if stream else torch._C._cuda_getCurrentRawStream(self._device_index)
         tmo = int((timeout_s if timeout_s is not None else self._default_timeout) * 1e9)
-        if _nvtx_enabled():
+        nvtx = _nvtx_enabled()
+        if nvtx:
             torch.cuda.nvtx.range_push(f"{_OP_NAMES.get(op, 'ps.op')}[{begin}:{end}]")
-        nvls = self.nvls and self._multicast_pays((int(end) - int(begin)) * self.grad.element_size())
-        rc = self.heap.lib.psdev_dense_op(C.byref(self._world), C.byref(self._table), op,
-                                          int(begin), int(end), C.byref(o), self.channel,
-                                          self.num_ctas, tmo,
-                                          (1 if sync else 0) | (2 if nvls else 0),
-                                          s.cuda_stream)
-        if _nvtx_enabled():
+        nvls = self.nvls and self._multicast_pays((int(end) - int(begin)) * self.grad_size)
+        rc = self._dense_op(self._op_fn, self._world_at, self._table_at, op, int(begin), int(end),
+                            self._opt_at, self.channel, self.num_ctas, tmo,
+                            (1 if sync else 0) | (2 if nvls else 0), s)
+        if nvtx:
             torch.cuda.nvtx.range_pop()
         _lib.check(rc, "psdev_dense_op")
 
@@ -251,11 +257,11 @@ class DenseTable:
         """The handle's parameters for the current step (rebuilt only when something changed:
         small requests are launch-bound, and building the structure costs microseconds)."""
         p = self.optimizer
-        key = (max(self.step, 1) if p.kind in ("adam", "adamw") else 0, p.kind, p.lr, p.momentum,
-               p.weight_decay, p.beta1, p.beta2, p.eps, p.scale, p.user_kind, p.user)
-        if key != self._opt_key:
-            self._opt_key = key
+        step = max(self.step, 1) if p.kind in ("adam", "adamw") else 0
+        if step != self._opt_step or p.__dict__ != self._opt_key:
+            self._opt_step, self._opt_key = step, dict(p.__dict__)
             self._opt_cached = p.to_struct(max(self.step, 1))
+            self._opt_at = C.addressof(self._opt_cached)
         return self._opt_cached
 
     def push(self, begin: int = 0, end: Optional[int] = None, *, sync: bool = True, stream=None,

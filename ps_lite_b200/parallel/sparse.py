@@ -100,7 +100,13 @@ class SparseTable:
         from .dense import default_timeout_s
         t.timeout_ns = int(default_timeout_s() * 1e9)
         self._t = t
-        self._out_ptr = self.out.data_ptr()
+        self._out_ptr, self._target = self.out.data_ptr(), None
+        if W == 1 and not heap.emulated_ranks:
+            ext = _lib.torch_ext()
+            self._push_pull = ext.sparse_push_pull
+            self._target = ext.sparse_target(
+                C.cast(heap.lib.psdev_sparse_local, C.c_void_p).value, C.addressof(self._world),
+                C.addressof(t), self.out, self.max_keys, self.max_vals, self.width, self.var_len)
         self.barrier_channel = barrier_channel
         self.count = 0
 
@@ -116,27 +122,11 @@ class SparseTable:
             raise ValueError(f"expected {self.width} values per key")
 
     # -- one rank: a request in one pass ---------------------------------------------------------
-    def _local_ok(self, keys, grads=None, lens=None) -> bool:
-        """One rank, and tensors that the kernel can read as they are."""
-        def plain(x, *dtypes):
-            return x.is_cuda and x.dtype in dtypes and x.is_contiguous()
-        return (self.heap.world == 1 and not self.heap.emulated_ranks and
-                plain(keys, torch.int64, torch.uint64) and
-                (grads is None or (plain(grads, torch.float32) and not self._in_heap_out(grads) and
-                                   (not self.var_len or
-                                    (lens is not None and plain(lens, torch.int32))))))
-
-    def _in_heap_out(self, t: torch.Tensor) -> bool:
-        lo = self._out_ptr
-        return lo - 4 * t.numel() < t.data_ptr() < lo + 4 * self.max_vals and t.data_ptr() != lo
-
-    def _local(self, keys, n, grads=None, lens=None) -> None:
-        ask = grads is None and self.var_len   # the owner says how long the values are
+    def _pull_local(self, keys, n) -> None:
+        # (with lengths, the owner says how long the values are)
         _lib.check(self.heap.lib.psdev_sparse_local(
-            C.byref(self._world), C.byref(self._t), n, keys.data_ptr(),
-            None if grads is None else grads.data_ptr(), 0 if grads is None else grads.numel(),
-            lens.data_ptr() if self.var_len and lens is not None else None, self._out_ptr,
-            self.max_vals, self.lens.data_ptr() if ask else None,
+            C.byref(self._world), C.byref(self._t), n, keys.data_ptr(), None, 0, None,
+            self._out_ptr, self.max_vals, self.lens.data_ptr() if self.var_len else None,
             torch.cuda.current_stream(self.heap.device).cuda_stream), "sparse_local")
 
     # -- the three phases; `sync=False` lets a test run all ranks' phases on one GPU ----------
@@ -175,12 +165,13 @@ class SparseTable:
         which ends when every rank's answers have landed.  Returns a view of the heap output
         buffer (valid until the next call), laid out like the pushed values.  One rank: one launch
         on the request's own tensors (``psdev_sparse_local``)."""
-        if self._local_ok(keys, grads, lens):
-            n, nv = keys.numel(), grads.numel()
-            self._check_request(n, nv, lens)
-            self._local(keys, n, grads, lens)
-            self.count, self.count_vals = n, nv
-            return self.out[:nv]
+        if self._target is not None:
+            got = self._push_pull(self._target, keys, grads, lens)
+            if got is not None:
+                if type(got) is int:
+                    _lib.check(got, "sparse_local")
+                self.count, self.count_vals = keys.numel(), got.numel()
+                return got
         self.stage(keys, grads, lens)
         self.scatter()
         multi = self.heap.world > 1
@@ -198,8 +189,9 @@ class SparseTable:
             raise ValueError("more keys than max_keys")
         multi = self.heap.world > 1 if sync is None else sync
         lib, s = self.heap.lib, torch.cuda.current_stream(self.heap.device)
-        if not multi and self._local_ok(keys):
-            self._local(keys, n)
+        if (not multi and self._target is not None and keys.is_cuda and keys.is_contiguous() and
+                keys.dtype in (torch.int64, torch.uint64)):
+            self._pull_local(keys, n)
             self.count = n
             self.count_vals = int(self.lens[:n].sum()) if self.var_len else n * self.width
             values = self.out[: self.count_vals]

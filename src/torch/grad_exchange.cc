@@ -230,9 +230,11 @@ class GradExchange {
 }  // namespace
 
 void add_requests(py::module& m);  // requests.cc
+void add_calls(py::module& m);     // calls.cc
 
 PYBIND11_MODULE(psb200_torch, m) {
   add_requests(m);
+  add_calls(m);
   using release = py::call_guard<py::gil_scoped_release>;
   py::class_<GradExchange>(m, "GradExchange")
       .def(py::init<std::vector<at::Tensor>, std::vector<int64_t>, std::vector<int64_t>, at::Tensor,

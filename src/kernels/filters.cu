@@ -62,29 +62,66 @@ __global__ void cast_scale_bf16_to_f32(const __nv_bfloat16* in, float* out, long
   for (long long i = vec * 8 + tid; i < n; i += nthreads) out[i] = __bfloat162float(in[i]) * s;
 }
 
-// one warp per group of 256 values (8 per lane)
-__global__ void int8_pack(const float* in, signed char* q, float* scales, long long n) {
+// One warp per group of 256 values, kPackGroups groups per warp.  Bound by HBM (5 bytes per
+// value).  With VEC a lane holds eight neighbours, so a group is one 32-byte load and one 8-byte
+// store per lane and both groups are in flight together; the CTAs are small and as many as there
+// are groups, since the hardware replaces a drained CTA faster than a loop over a fixed grid
+// comes round.  The input is read once and marked to leave L2 first: the codes stay there for
+// the push that follows.  25.6 M values: 32.9 us before,
+// 20.5 now (26.7 without the alignment).  Arrays without that
+// alignment (32 bytes in, 8 out) keep four-byte loads with neighbouring lanes on neighbouring
+// values.
+constexpr int kPackThreads = 128;
+constexpr int kPackGroups = 2;
+template <bool VEC>
+__global__ void __launch_bounds__(kPackThreads)
+    int8_pack(const float* in, signed char* q, float* scales, long long n) {
   const long long ngroups = (n + kGroup - 1) / kGroup;
   const int lane = threadIdx.x & 31;
-  for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; g < ngroups;
-       g += ((long long)gridDim.x * blockDim.x) >> 5) {
-    float v[8];
-    float m = 0.f;
+  const long long stride = (long long)gridDim.x * (kPackThreads / 32) * kPackGroups;
+  for (long long g0 = ((blockIdx.x * (long long)kPackThreads + threadIdx.x) >> 5) * kPackGroups;
+       g0 < ngroups; g0 += stride) {
+    float v[kPackGroups][8];
+    auto at = [&](int u, int j) {
+      return (g0 + u) * kGroup + (VEC ? lane * 8 + j : j * 32 + lane);
+    };
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const long long i = g * kGroup + j * 32 + lane;
-      v[j] = i < n ? in[i] : 0.f;
-      m = fmaxf(m, fabsf(v[j]));
+    for (int u = 0; u < kPackGroups; ++u) {
+      if (VEC && (g0 + u + 1) * kGroup <= n) {
+        asm volatile("ld.global.L2::evict_first.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(v[u][0]), "=f"(v[u][1]), "=f"(v[u][2]), "=f"(v[u][3]), "=f"(v[u][4]),
+                       "=f"(v[u][5]), "=f"(v[u][6]), "=f"(v[u][7])
+                     : "l"(in + at(u, 0)));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[u][j] = at(u, j) < n ? in[at(u, j)] : 0.f;
+      }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    const float scale = m > 0.f ? m / 127.f : 1.f;
-    const float inv = 1.f / scale;
-    if (lane == 0) scales[g] = scale;
+    for (int u = 0; u < kPackGroups; ++u) {
+      if (g0 + u >= ngroups) break;
+      float m = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const long long i = g * kGroup + j * 32 + lane;
-      if (i < n) q[i] = (signed char)__float2int_rn(fminf(fmaxf(v[j] * inv, -127.f), 127.f));
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(v[u][j]));
+      // floats that are not negative (and not NaN: fmaxf drops it) order as their bits do
+      m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+      const float scale = m > 0.f ? m / 127.f : 1.f;
+      const float inv = 1.f / scale;
+      if (lane == 0) scales[g0 + u] = scale;
+      int c[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        c[j] = __float2int_rn(fminf(fmaxf(v[u][j] * inv, -127.f), 127.f));
+      if (VEC && (g0 + u + 1) * kGroup <= n) {
+        uint2 w;
+        w.x = (c[0] & 0xff) | (c[1] & 0xff) << 8 | (c[2] & 0xff) << 16 | (unsigned)c[3] << 24;
+        w.y = (c[4] & 0xff) | (c[5] & 0xff) << 8 | (c[6] & 0xff) << 16 | (unsigned)c[7] << 24;
+        *reinterpret_cast<uint2*>(q + at(u, 0)) = w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (at(u, j) < n) q[at(u, j)] = (signed char)c[j];
+      }
     }
   }
 }
@@ -145,7 +182,12 @@ int psdev_filter_cast(const void* in, void* out, int64_t n, float scale, int dir
 int psdev_filter_int8_pack(const float* in, int8_t* q, float* scales, int64_t n, void* stream) {
   if (n < 0) return PSDEV_ERR_ARG;
   if (n == 0) return 0;
-  filt::int8_pack<<<592, 256, 0, (cudaStream_t)stream>>>(in, (signed char*)q, scales, n);
+  constexpr long long kPerCta = filt::kPackThreads / 32 * filt::kPackGroups * filt::kGroup;
+  const long long ctas = (n + kPerCta - 1) / kPerCta;
+  const unsigned int grid = (unsigned int)(ctas < (1ll << 30) ? ctas : 1ll << 30);
+  const bool vec = ((uintptr_t)in & 31) == 0 && ((uintptr_t)q & 7) == 0;
+  auto* kern = vec ? filt::int8_pack<true> : filt::int8_pack<false>;
+  kern<<<grid, filt::kPackThreads, 0, (cudaStream_t)stream>>>(in, (signed char*)q, scales, n);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return (int)cudaGetLastError();
 }

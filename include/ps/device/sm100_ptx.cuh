@@ -51,6 +51,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Whether the phase is complete, without waiting (try_wait may suspend the thread for thousands of
+// clocks before it says no).
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ unsigned long long gtimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -73,6 +86,38 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     if (gtimer_ns() - t0 > timeout_ns) {
       *abort_flag = 1;
       return false;
+    }
+  }
+}
+
+// What the loads have completed, for a warp that issues MMAs.  An mbarrier access behind a
+// tcgen05.commit waits until the committed MMAs are done: an issuer that looks at a barrier per
+// k-block has no MMAs queued meanwhile.  So another thread watches the barriers and counts the
+// k-blocks in place in shared memory, which the issuer reads with ordinary loads.
+__device__ __forceinline__ void st_ready(uint32_t* count, uint32_t v) {
+  asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(count)), "r"(v)
+               : "memory");
+}
+// Waits until k-block `k` is in place (`*count` > k); `*seen` gets the count.  Called by a whole
+// warp; bounded like mbar_wait_bounded.
+__device__ __forceinline__ bool wait_ready(uint32_t* count, uint32_t k, uint32_t* seen,
+                                           volatile int* abort_flag,
+                                           unsigned long long timeout_ns) {
+  unsigned long long t0 = 0;
+  for (uint32_t n = 1;; ++n) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(count))
+                 : "memory");
+    v = __shfl_sync(0xffffffffu, v, 0);
+    if (v > k) {
+      *seen = v;
+      return true;
+    }
+    if ((n & 1023) == 0) {
+      const unsigned long long t = gtimer_ns();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > timeout_ns) *abort_flag = 1;
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
     }
   }
 }
@@ -100,6 +145,16 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       " [%0], [%1, {%2, %3}], [%4];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y),
         "r"(smem_u32(bar))
+      : "memory");
+}
+
+// 2-D tiled store of this CTA's shared memory to global memory; joins the executing thread's
+// current bulk group.  Rows and columns outside the tensor are not written.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, int x, int y,
+                                             const void* smem_src) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+      ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(smem_u32(smem_src))
       : "memory");
 }
 
@@ -149,6 +204,18 @@ __device__ __forceinline__ void cp_async_commit() {
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// ---- programmatic dependent launch ----------------------------------------------------------
+// A kernel launched with programmatic stream serialization may start while the previous kernel of
+// its stream is still running: it must not touch global memory before grid_wait(), which returns
+// once that kernel has completed and its writes are visible.  grid_launch_next() lets the next
+// kernel of the stream start (as far as it was launched so) once every CTA has called it.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_launch_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---- tcgen05 ------------------------------------------------------------------------------

@@ -102,9 +102,35 @@ struct Cfg {
       kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kRingBytes;
 };
 
+// 32 accumulators of one row as bf16.  Where rows allow it, as two whole sectors of 32 bytes:
+// 16-byte pieces make half-written sectors, which cost L2 twice (16384 x 3072 x 1024 96 us with
+// them, 90 without).
+__device__ __forceinline__ void store_row32(__nv_bfloat16* row, long long N, long long col,
+                                            const uint32_t (&r)[32]) {
+  __nv_bfloat16* dst = row + col;
+  uint32_t u[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    u[j] = f2_to_bf16x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+  if (col + 32 <= N && ((uintptr_t)dst & 31) == 0) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 16 * j),
+                   "r"(u[8 * j]), "r"(u[8 * j + 1]), "r"(u[8 * j + 2]), "r"(u[8 * j + 3]),
+                   "r"(u[8 * j + 4]), "r"(u[8 * j + 5]), "r"(u[8 * j + 6]), "r"(u[8 * j + 7])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (col + j * 8 + 8 <= N)
+        *reinterpret_cast<uint4*>(dst + j * 8) =
+            make_uint4(u[4 * j], u[4 * j + 1], u[4 * j + 2], u[4 * j + 3]);
+  }
+}
 }  // namespace gemm
 }  // namespace psdev
 #include "kernels/split_gemm.cuh"
+#include "kernels/wide_gemm.cuh"
 namespace psdev {
 namespace gemm {
 
@@ -892,25 +918,20 @@ __global__ void __launch_bounds__(kThreads256, 1)
 // next tile), and the even CTA issues one M=256 MMA per K step for both.  Loads carry no
 // cluster multicast: each CTA fetches its own halves; only the completion counts and the
 // MMA-done signals cross between the two CTAs.
-// kRing: room for the pull ring of the fused form; the plain GEMM spends it on a seventh stage.
-template <bool kRing>
-struct CfgPairT {
+struct CfgPair {
   static constexpr int BN = 256;
   static constexpr int kABytes = 128 * BK * 2;  // this CTA's 128 rows of X
   static constexpr int kBBytes = 128 * BK * 2;  // this CTA's 128 rows of W
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = kRing ? 6 : 7;
+  static constexpr int kStages = 6;
   static constexpr int kTmemCols = 512;
-  static constexpr int kSmemBytes =
-      kStages * kStageBytes + 1024 + 256 + (kRing ? kRingBytes : 0);
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + kRingBytes;
 };
-using CfgPair = CfgPairT<true>;
 
-template <bool kRing>
 __device__ void gemm_role_pair(const Args& a, const CUtensorMap* tmap_x, const CUtensorMap* tmap_w,
                                int pair_idx, int num_pairs, unsigned char* smem_raw,
                                volatile int* abort_flag) {
-  using C = CfgPairT<kRing>;
+  using C = CfgPair;
   constexpr int BN = C::BN;
   static_assert(2 * C::kStages + 5 <= kRingBarIndex, "pipeline barriers overlap the ring's");
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -1019,7 +1040,9 @@ __device__ void gemm_role_pair(const Args& a, const CUtensorMap* tmap_x, const C
     __syncwarp();
   } else if (warp == 1) {
     // ================= MMA issuer (leader CTA only) =================
-    if (lane == 0 && cta == 0) {
+    if (cta == 0) {
+      // (issued by an elected thread, so that descriptors stay in uniform registers)
+      const uint64_t desc_a = make_desc_k128(smem), desc_b = make_desc_k128(smem + C::kABytes);
       int stage = 0;
       uint32_t phase = 0;
       long long local = 0;
@@ -1031,31 +1054,33 @@ __device__ void gemm_role_pair(const Args& a, const CUtensorMap* tmap_x, const C
         const uint32_t idesc = make_idesc_bf16(256, n_len);
         const int acc = (int)(local & 1);
         const uint32_t acc_phase = (uint32_t)((local >> 1) & 1);
-        if (!mbar_wait_bounded(&tmem_empty[acc], acc_phase ^ 1, abort_flag, a.timeout_ns)) {
-          ok = false;
-          break;
-        }
+        ok = mbar_wait_bounded(&tmem_empty[acc], acc_phase ^ 1, abort_flag, a.timeout_ns);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, a.timeout_ns)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          unsigned char* sa = smem + stage * C::kStageBytes;
-          const uint64_t da = make_desc_k128(sa);
-          const uint64_t db = make_desc_k128(sa + C::kABytes);
+          ok = mbar_wait_bounded(&full_bar[stage], phase, abort_flag, a.timeout_ns);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          const int cur = stage;
+          if (elect_one()) {
+            const uint64_t off = (uint64_t)(cur * (C::kStageBytes >> 4));
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
-                          (kb | k) != 0 ? 1u : 0u);
-          umma_commit_pair(&empty_bar[stage]);  // frees the stage in both CTAs
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_f16_pair(d_tmem, desc_a + off + (uint64_t)(2 * k),
+                            desc_b + off + (uint64_t)(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+          }
+          __syncwarp();
           if (++stage == C::kStages) { stage = 0; phase ^= 1; }
+          if (elect_one()) {
+            umma_commit_pair(&empty_bar[cur]);  // frees the stage in both CTAs
+            if (kb == num_kb - 1) umma_commit_pair(&tmem_full[acc]);  // wakes both epilogues
+          }
+          __syncwarp();
         }
-        if (ok) umma_commit_pair(&tmem_full[acc]);  // wakes the epilogues of both CTAs
       }
-      if (!ok) report(a.scratch, PSDEV_ERR_TIMEOUT_PIPE);
+      if (!ok && lane == 0) report(a.scratch, PSDEV_ERR_TIMEOUT_PIPE);
     }
     __syncwarp();
   } else if (warp < 6) {
@@ -1085,26 +1110,13 @@ __device__ void gemm_role_pair(const Args& a, const CUtensorMap* tmap_x, const C
         tmem_ld_32x32(taddr + (uint32_t)c0, r);
         tmem_ld_wait();
         const long long col = (long long)tn * BN + n_off + c0;
-        if (row < a.M) {
-          __nv_bfloat16* dst = a.c + row * a.N + col;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (col + j * 8 + 8 <= a.N) {
-              uint4 u;
-              u.x = f2_to_bf16x2(__uint_as_float(r[8 * j + 0]), __uint_as_float(r[8 * j + 1]));
-              u.y = f2_to_bf16x2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
-              u.z = f2_to_bf16x2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
-              u.w = f2_to_bf16x2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
-              *reinterpret_cast<uint4*>(dst + j * 8) = u;
-            }
-          }
-        }
+        if (row < a.M) store_row32(a.c + row * a.N, a.N, col, r);
       }
       tc_fence_before();
       mbar_arrive_leader(&tmem_empty[acc]);  // counted on the leader, where the MMAs are issued
     }
     if (!ok && lane == 0) report(a.scratch, PSDEV_ERR_TIMEOUT_PIPE);
-  } else if (kRing && a.fused && a.inline_copy) {
+  } else if (a.fused && a.inline_copy) {
     // warps 6 and 7: pull W while the other warps multiply
     const int cta_lin = pair_idx * 2 + (int)cta;
     if (a.ring_mode == 0)
@@ -1123,7 +1135,6 @@ __device__ void gemm_role_pair(const Args& a, const CUtensorMap* tmap_x, const C
 }
 
 // Grid: [copy CTAs (even count)][GEMM CTA pairs], clusters of 2 along x.
-template <bool kRing>
 __global__ void __launch_bounds__(kThreads, 1)
     pull_gemm_pair_kernel(const __grid_constant__ Args a,
                           const __grid_constant__ CUtensorMap tmap_x,
@@ -1137,7 +1148,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if ((int)blockIdx.x < ncopy) {
     copy_role<256>(a, (int)blockIdx.x);
   } else {
-    gemm_role_pair<kRing>(a, &tmap_x, &tmap_w, ((int)blockIdx.x - ncopy) >> 1,
+    gemm_role_pair(a, &tmap_x, &tmap_w, ((int)blockIdx.x - ncopy) >> 1,
                           ((int)gridDim.x - ncopy) >> 1, smem_raw, &s_abort);
   }
   __syncthreads();
@@ -1320,73 +1331,66 @@ static int launch256(const Args& a, const CUtensorMap& tx, const CUtensorMap& tw
   return launch_ex(pull_gemm256_kernel, a, tx, tw, grid, kThreads256, Cfg256::kSmemBytes, 1, s);
 }
 
-template <bool kRing>
-static int launch_pair_t(const Args& a, const CUtensorMap& tx, const CUtensorMap& tw, int grid,
-                         cudaStream_t s) {
+static int launch_pair(const Args& a, const CUtensorMap& tx, const CUtensorMap& tw, int grid,
+                       cudaStream_t s) {
   static std::atomic<bool> attr_set[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(pull_gemm_pair_kernel<kRing>,
+    cudaError_t e = cudaFuncSetAttribute(pull_gemm_pair_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         CfgPairT<kRing>::kSmemBytes);
+                                         CfgPair::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev & 63].store(true, std::memory_order_release);
   }
-  return launch_ex(pull_gemm_pair_kernel<kRing>, a, tx, tw, grid, kThreads,
-                   CfgPairT<kRing>::kSmemBytes, 2, s);
-}
-static int launch_pair(const Args& a, const CUtensorMap& tx, const CUtensorMap& tw, int grid,
-                       cudaStream_t s) {
-  // (the plain GEMM needs no pull ring and could spend its room on a seventh pipeline stage)
-  static const int stages_env = [] {
-    const char* e = getenv("PSB200_GEMM_PAIR_STAGES");
-    return e ? atoi(e) : 0;
-  }();
-  // measured on 16384x3072x1024: six stages 1258 TFLOP/s, seven (possible without the pull
-  // ring) 1228-1243: the seventh stage stays an option (PSB200_GEMM_PAIR_STAGES=7)
-  if (a.fused || stages_env != 7) return launch_pair_t<true>(a, tx, tw, grid, s);
-  return launch_pair_t<false>(a, tx, tw, grid, s);
+  return launch_ex(pull_gemm_pair_kernel, a, tx, tw, grid, kThreads, CfgPair::kSmemBytes, 2, s);
 }
 
-template <int BN, int S>
+template <int BN, int S, bool DEEP>
 static int launch_split_t(const SplitArgs& a, const CUtensorMap& tx, const CUtensorMap& tw,
                           long long tiles, cudaStream_t s) {
   static std::atomic<bool> attr_set[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(split_gemm_kernel<BN, S>,
+    cudaError_t e = cudaFuncSetAttribute(split_gemm_kernel<BN, S, DEEP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SplitCfg<BN>::kSmemBytes);
+                                         SplitCfg<BN, DEEP>::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev & 63].store(true, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(tiles * S), 1, 1);
   cfg.blockDim = dim3(kSplitThreads, 1, 1);
-  cfg.dynamicSmemBytes = SplitCfg<BN>::kSmemBytes;
+  cfg.dynamicSmemBytes = SplitCfg<BN, DEEP>::kSmemBytes;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = S;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = S;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = S > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, split_gemm_kernel<BN, S>, a, tx, tw);
+  cfg.numAttrs = S > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, split_gemm_kernel<BN, S, DEEP>, a, tx, tw);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return (int)e;
 }
-template <int BN>
+template <int BN, bool DEEP>
 static int launch_split(int split, const SplitArgs& a, const CUtensorMap& tx,
                         const CUtensorMap& tw, long long tiles, cudaStream_t s) {
   switch (split) {
-    case 1: return launch_split_t<BN, 1>(a, tx, tw, tiles, s);
-    case 2: return launch_split_t<BN, 2>(a, tx, tw, tiles, s);
-    case 4: return launch_split_t<BN, 4>(a, tx, tw, tiles, s);
-    case 8: return launch_split_t<BN, 8>(a, tx, tw, tiles, s);
+    case 1: return launch_split_t<BN, 1, DEEP>(a, tx, tw, tiles, s);
+    case 2: return launch_split_t<BN, 2, DEEP>(a, tx, tw, tiles, s);
+    case 4: return launch_split_t<BN, 4, DEEP>(a, tx, tw, tiles, s);
+    case 8: return launch_split_t<BN, 8, DEEP>(a, tx, tw, tiles, s);
     default: return PSDEV_ERR_ARG;
   }
+}
+// Two k-blocks per stage and one CTA per SM, where SMs would have one CTA anyway and the loop is
+// longer than the shallow form's stages.
+static bool split_deep(int bn, long long ctas, int num_kb) {
+  return ctas <= 148 && num_kb > (bn == 64 ? 4 : 3);
 }
 static int run_split(const Args& a, const void* x, const void* w, int bn, int split,
                      cudaStream_t s) {
@@ -1405,8 +1409,69 @@ static int run_split(const Args& a, const void* x, const void* w, int bn, int sp
   sa.timeout_ns = a.timeout_ns;
   while (split > sa.num_kb) split >>= 1;
   const long long tiles = (long long)sa.tiles_m * ((a.N + bn - 1) / bn);
-  return bn == 64 ? launch_split<64>(split, sa, tx, tw, tiles, s)
-                  : launch_split<128>(split, sa, tx, tw, tiles, s);
+  if (split_deep(bn, tiles * split, (sa.num_kb + split - 1) / split))
+    return bn == 64 ? launch_split<64, true>(split, sa, tx, tw, tiles, s)
+                    : launch_split<128, true>(split, sa, tx, tw, tiles, s);
+  return bn == 64 ? launch_split<64, false>(split, sa, tx, tw, tiles, s)
+                  : launch_split<128, false>(split, sa, tx, tw, tiles, s);
+}
+
+template <int NT>
+static int run_wide(const Args& a, const void* x, const void* w, int num_ctas, cudaStream_t s) {
+  CUtensorMap tx, tw, tw64, tc;
+  int rc = make_tmap(&tx, x, a.M, a.K, 128);
+  if (rc) return rc;
+  rc = make_tmap(&tw, w, a.N, a.K, 128);
+  if (rc) return rc;
+  rc = make_tmap(&tw64, w, a.N, a.K, 64);
+  if (rc) return rc;
+  rc = make_tmap(&tc, a.c, a.M, a.N, 32);
+  if (rc) return rc;
+  auto* k = wide_gemm_kernel<NT>;
+  static std::atomic<bool> attr_set[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(k,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         WideCfg<NT>::kSmemBytes);
+    if (e != cudaSuccess) return (int)e;
+    attr_set[dev & 63].store(true, std::memory_order_release);
+  }
+  WideArgs wa{};
+  wa.M = a.M;
+  wa.N = a.N;
+  wa.num_kb = (int)((a.K + BK - 1) / BK);
+  wa.tiles_m = (int)((a.M + 255) / 256);
+  wa.tiles_n = (int)((a.N + NT - 1) / NT);
+  static const int group_env = [] {
+    const char* e = getenv("PSB200_GEMM_GROUP");
+    return e ? atoi(e) : 0;
+  }();
+  wa.group = group_env > 0 ? group_env : (wa.tiles_n <= 16 ? wa.tiles_n : 8);
+  if (wa.group > wa.tiles_n) wa.group = wa.tiles_n;
+  wa.status = &a.scratch->status;
+  wa.timeout_ns = a.timeout_ns;
+  const long long tiles = (long long)wa.tiles_m * wa.tiles_n;
+  long long pairs = num_ctas / 2;
+  if (pairs > tiles * (NT / 128)) pairs = tiles * (NT / 128);
+  if (pairs < 1) pairs = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+  cfg.blockDim = dim3(kWideThreads, 1, 1);
+  cfg.dynamicSmemBytes = WideCfg<NT>::kSmemBytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, wa, tx, tw, tw64, tc);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return (int)e;
 }
 
 // Output-tile height used by run(): 128 (double-buffered accumulators) or 256 (twice the
@@ -1421,57 +1486,76 @@ static int pick_tile_m(long long M, long long N, long long K) {
   }
   if (t == 2) return (N >= 256 && M >= 256) ? 2 : 128;  // 2 = CTA pairs
   if (t == 128 || t == 256) return (t == 256 && N >= 256 && M >= 256) ? 256 : 128;
-  // by shape (measured on one B200, bf16, TFLOP/s):
-  //   16384x3072x1024: pairs 1198, 128-row tile 1070, 256-row tile 868
-  //   16384x4096x1024: pairs 1398, 128-row tile 1169
-  //   8192x8192x8192 : 256-row tile 1533, pairs 1477, 128-row tile 1341
-  // CTA pairs whenever there is at least one 256 x 256 tile per pair of SMs; the one-CTA
-  // 256-row tile for long reductions, where its exposed epilogue is amortised.
+  // Fused products (plain ones are chosen by pick_plain).  By shape, measured on one B200 without
+  // the pull, bf16, TFLOP/s: 16384x3072x1024 pairs 1198, 128-row tile 1070, 256-row tile 868;
+  // 8192x8192x8192 256-row tile 1533, pairs 1477, 128-row tile 1341.  CTA pairs whenever there is
+  // at least one 256 x 256 tile per pair of SMs; the one-CTA 256-row tile for long reductions,
+  // where its exposed epilogue is amortised.
   const long long tiles256 = ((M + 255) / 256) * ((N + 255) / 256);
   if (N >= 256 && M >= 256 && K >= 4096 && tiles256 >= 2 * 148) return 256;
   if (N >= 256 && M >= 256 && tiles256 >= 74) return 2;
   return 128;
 }
 
-// The split form (1000 * S + BN) for a product, or 0 when the persistent kernels are faster.  The
-// times below, in us, were fitted to measurements over M 64 .. 8192, N and K 256 .. 4096 (operands
-// in L2); they put the persistent kernels where 128 x 256 tiles fill the GPU and K is long:
-//                        64x256x4096  1024x1024x1024  1024x4096x1024  4096x2048x1024
-//   persistent (pairs)       23.4          11.9            12.2            18.6
-//   S = 1, BN = 64 / 128  16.9 / 20.8    7.4 / 8.3      15.7 / 11.7     28.1 / 21.2
-//   S = 4, BN = 64           10.1         21.5            34.5
-static int pick_split(long long M, long long N, long long K) {
+// The kernel of a plain product: 1000 * S + BN the split form, 2256 / 2512 pairs of CTAs with
+// tiles of 256 x 256 / 512 (wide_gemm.cuh), 0 the persistent one-CTA tiles of this file.  The
+// times below, in us, were fitted to measurements over M 64 .. 4096, N and K 256 .. 4096 (operands
+// in L2, launches back to back).  They put pairs where their tiles nearly fill the GPU or K is
+// long; the wide tile where it costs no extra round, since it moves fewer bytes per product:
+//                     1024x1024x1024  2048x2048x1024  1536x4096x1024  2048x4096x1024  2048x512x4096
+//   S = 1, BN = 64          6.0            14.9            21.1            27.8            15.3
+//   S = 1, BN = 128         6.8            11.0            18.1            20.6            17.6
+//   2256                    8.2            10.3            13.8            15.1            20.1
+//   2512                    8.7            10.9            16.0            16.2            22.4
+static int pick_plain(long long M, long long N, long long K) {
   const int config = g_tile_m.load();
   if (config >= 1000) return config;
   if (config != 0 || getenv("PSB200_GEMM_TILE")) return 0;
   const double kb = (double)((K + BK - 1) / BK);
-  const double sms = 148;
+  const double sms = 148, pairs = 74;
   auto tiles = [&](int m, int n) { return (double)(((M + m - 1) / m) * ((N + n - 1) / n)); };
-  double best;
-  const double t256 = tiles(256, 256);
-  if (M >= 256 && N >= 256 && t256 >= 74) {  // CTA pairs: whole rounds, or half of the last one
-    const double rounds = t256 / 74, whole = floor(rounds), rest = rounds - whole;
-    const double last = rest == 0 ? 0 : rest <= 0.25 ? 0.25 : rest <= 0.5 ? 0.5 : 1;
-    best = 8.0 + (whole + last) * fmax(0.327 * kb, 2.4);
-  } else {
-    const int bn = (N % 256 == 0 || N > 1024) ? 256 : 128;
-    best = 7.3 + ceil(tiles(128, bn) / sms) * fmax(0.29 * kb, 1.5);
-  }
+  const int bn = (N % 256 == 0 || N > 1024) ? 256 : 128;
+  double best = 7.3 + ceil(tiles(128, bn) / sms) * fmax(0.33 * kb, 1.6);
   int pick = 0;
-  for (int bn = 64; bn <= 128; bn += 64) {
+  if (M >= 256 && N >= 256) best = INFINITY;  // pairs are better than one-CTA tiles of that size
+  auto offer = [&](double t, int code) {
+    if (t < best) {
+      best = t;
+      pick = code;
+    }
+  };
+  if (M >= 256 && N >= 256) {
+    // a round of whole tiles, of halves and of quarters of the wide tile
+    const double t512 = fmax(0.63 * kb, 3.2), t256 = fmax(0.33 * kb, 1.6);
+    const double t128 = fmax(0.27 * kb, 0.9);
+    for (int nt = 256; nt <= 512; nt *= 2) {
+      const double rounds = tiles(256, nt) / pairs, whole = floor(rounds), rest = rounds - whole;
+      const double tile = nt == 512 ? t512 : t256;
+      double last = 0;
+      if (rest > 0) last = rest > 0.5 ? tile : nt == 256 || rest <= 0.25 ? t128 : t256;
+      const double base = whole == 0 ? (last == t128 ? 4.2 : last == t256 ? 5.3 : 5.9)
+                                     : (nt == 512 ? 5.9 : 5.3);
+      offer(base + whole * tile + last, 2000 + nt);
+    }
+  }
+  for (int n = 64; n <= 128; n += 64) {
     for (int split = 1; split <= kMaxSplit; split *= 2) {
-      const double ctas = tiles(128, bn) * split;
-      if (split > 1 && (ctas > sms || split > kb)) break;
-      const double over = fmax(0.0, ctas / sms - 1);
-      const double base = bn == 64 ? 3.5 + 1.2 * over : 3.7 + 2.0 * over;
-      const double per_kb = bn == 64 ? fmax(0.21, 0.00117 * ctas) : fmax(0.297, 0.0016 * ctas);
-      const int l = split == 1 ? 0 : split == 2 ? 1 : split == 4 ? 2 : 3;
-      static const double exchange[2][4] = {{0, 1.7, 2.9, 3.6}, {0, 3.3, 6.7, 7.5}};
-      const double t = base + exchange[bn / 128][l] + ceil(kb / split) * per_kb;
-      if (t < best) {
-        best = t;
-        pick = 1000 * split + bn;
+      const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)
+      if (split > 1 && (ctas > 2 * sms || split > kb)) break;
+      const double k = ceil(kb / split), full = fmin(ctas / sms, 1);
+      const double over = fmax(0.0, ctas / (2 * sms) - 0.9);
+      const bool deep = split_deep(n, (long long)ctas, (int)k);
+      double base, per_kb, exchange = 0;
+      if (n == 64) {
+        base = deep ? 2.2 + 0.55 * full : 1.8 + 1.95 * full + 2.7 * over;
+        per_kb = deep ? 0.203 : fmax(0.276, 0.0011 * ctas);
+        if (split > 1) exchange = 0.87 + 0.0029 * split * ctas + 0.53 * split;
+      } else {
+        base = deep ? 2.7 + 0.6 * full : 2.1 + 3.7 * full + 4.3 * over;
+        per_kb = deep ? 0.232 : fmax(0.38, 0.0015 * ctas);
+        if (split > 1) exchange = 1.36 + 0.0049 * split * ctas + 0.82 * split;
       }
+      offer(base + exchange + k * per_kb, 1000 * split + n);
     }
   }
   return pick;
@@ -1483,9 +1567,15 @@ static int run(Args a, const void* x, const void* w, int num_ctas, cudaStream_t 
   int err = 0;
   a.scratch = scratch_for_current_device(&err);
   if (!a.scratch) return err;
+  int sms = 148;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!a.fused && num_ctas <= 0) {
-    const int split = pick_split(a.M, a.N, a.K);
-    if (split) return run_split(a, x, w, split % 1000, split / 1000, s);
+    const int code = pick_plain(a.M, a.N, a.K);
+    if (code == 2256) return run_wide<256>(a, x, w, sms, s);
+    if (code == 2512) return run_wide<512>(a, x, w, sms, s);
+    if (code) return run_split(a, x, w, code % 1000, code / 1000, s);
   }
   const int variant = pick_tile_m(a.M, a.N, a.K);
   const bool pair = (variant == 2);
@@ -1498,10 +1588,6 @@ static int run(Args a, const void* x, const void* w, int num_ctas, cudaStream_t 
   if (rc) return rc;
   rc = make_tmap(&tw, w, a.N, a.K, pair ? 128 : BN);
   if (rc) return rc;
-  int sms = 148;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = ((a.M + tile_m - 1) / tile_m) * ((a.N + BN - 1) / BN);
   const int avail = num_ctas > 0 ? num_ctas : sms;
   // One launch of the chosen variant with `copy` CTAs set aside (0: ring mode or not fused).
@@ -1649,12 +1735,15 @@ extern "C" int64_t psdev_pull_plan_chunk(int64_t w_elem_off, int64_t nk, int blk
 }
 
 // Selects the kernel variant of later GEMM launches: 128 or 256 (output-tile height of the
-// one-CTA kernels), 2 (CTA pairs, tcgen05 cta_group::2), or 0 for the built-in choice by shape.
+// one-CTA kernels), 2 (CTA pairs, tcgen05 cta_group::2), 2256 or 2512 (CTA pairs of plain products
+// with tiles of so many columns), 1000 * S + BN (one 128 x BN tile per cluster of S CTAs), or 0
+// for the built-in choice by shape.
 extern "C" int psdev_gemm_config(int tile_m) {
   const int bn = tile_m % 1000, split = tile_m / 1000;
   const bool is_split = (bn == 64 || bn == 128) && (split == 1 || split == 2 || split == 4 ||
                                                     split == 8);
-  if (tile_m != 0 && tile_m != 128 && tile_m != 256 && tile_m != 2 && !is_split)
+  if (tile_m != 0 && tile_m != 128 && tile_m != 256 && tile_m != 2 && tile_m != 2256 &&
+      tile_m != 2512 && !is_split)
     return PSDEV_ERR_ARG;
   gemm::g_tile_m.store(tile_m);
   return 0;

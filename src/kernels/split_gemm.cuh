@@ -10,12 +10,18 @@
 //   warp 0      TMA producer; sets up the barriers and starts loading at once;
 //   warp 1      allocates tensor memory, issues tcgen05.mma;
 //   warps 2..5  epilogue, each its quarter of the accumulator rows.
-// About 100 KB of shared memory per CTA, so that two CTAs share an SM when there are more tiles
-// than SMs and one loads while the other stores.  (Twice the stages and one CTA per SM: 1024 x 4096
-// x 1024 16.1 us against 11.7, and no gain where there is one CTA per SM anyway.)
+// Launched with programmatic stream serialization: the prologue runs beside the end of the kernel
+// before it.
 //
-// Measured, us (this kernel / the persistent 128 x 256 kernel): 64x256x256 3.5 / 6.5,
-// 1024x1024x256 4.2 / 8.4, 1024x1024x1024 7.4 / 11.9, 64x256x4096 10.1 / 23.4 (S = 4).
+// Two forms.  With more CTAs than SMs about 100 KB of shared memory per CTA, so that two share an SM
+// and one loads while the other stores.  Otherwise (DEEP) one CTA has the SM, and a stage holds two
+// k-blocks: per stage the ring costs some 300 clocks (commit, barrier, producer) whatever it
+// carries, and 128 columns of K make up for them.  The issuer of the deep form touches no mbarrier
+// (see wait_ready).  1024 x 1024 x 4096 with BN = 64 / 128 20.9 / 24.5 us shallow, 16.5 / 18.2
+// deep; what is left is the loads, 70 bytes per clock and SM.
+//
+// Measured, us (this kernel / the persistent 128 x 256 kernel): 64x256x256 2.8 / 6.5,
+// 1024x1024x256 4.1 / 8.4, 1024x1024x1024 6.0 / 11.9, 64x256x4096 8.6 / 23.4 (S = 4).
 #pragma once
 #include "ps/device/sm100_ptx.cuh"
 
@@ -33,10 +39,12 @@ struct SplitArgs {
   unsigned long long timeout_ns;
 };
 
-template <int BN>
+template <int BN, bool DEEP>
 struct SplitCfg {
   static constexpr int kABytes = BM * BK * 2;
-  static constexpr int kStageBytes = kABytes + BN * BK * 2;
+  static constexpr int kBlockBytes = kABytes + BN * BK * 2;  // one k-block
+  static constexpr int kSub = DEEP ? 2 : 1;                  // k-blocks of a stage
+  static constexpr int kStageBytes = kSub * kBlockBytes;
   static constexpr int kStages = BN == 64 ? 4 : 3;
   static constexpr int kPitch = BN + 4;  // floats per row of the exchanged partial sums
   static constexpr int kExchange = BM * kPitch * 4;
@@ -66,17 +74,18 @@ __device__ __forceinline__ void store_bf16x8(__nv_bfloat16* p, const float* f) {
   *reinterpret_cast<uint4*>(p) = u;
 }
 
-template <int BN, int S>
+template <int BN, int S, bool DEEP>
 __global__ void __launch_bounds__(kSplitThreads)
     split_gemm_kernel(const __grid_constant__ SplitArgs a,
                       const __grid_constant__ CUtensorMap tmap_x,
                       const __grid_constant__ CUtensorMap tmap_w) {
   using namespace sm100;
-  using C = SplitCfg<BN>;
+  using C = SplitCfg<BN, DEEP>;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::kStages], empty_bar[C::kStages], done_bar;
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
+  __shared__ uint32_t s_ready;  // k-blocks in place (DEEP)
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -86,22 +95,31 @@ __global__ void __launch_bounds__(kSplitThreads)
   const int kb0 = (int)((long long)a.num_kb * part / S);
   const int nkb = (int)((long long)a.num_kb * (part + 1) / S) - kb0;
 
+  const int nst = (nkb + C::kSub - 1) / C::kSub;  // stages to fill
+
   auto load = [&](int i, int s) {
-    unsigned char* sa = smem + s * C::kStageBytes;
+    const int n = nkb - i * C::kSub < C::kSub ? nkb - i * C::kSub : C::kSub;
     uint64_t* bar = &full_bar[s];
-    mbar_arrive_expect_tx(bar, C::kStageBytes);
-    tma_load_2d(sa, &tmap_x, (kb0 + i) * BK, tm * BM, bar);
-    tma_load_2d(sa + C::kABytes, &tmap_w, (kb0 + i) * BK, tn * BN, bar);
+    mbar_arrive_expect_tx(bar, n * C::kBlockBytes);
+    for (int j = 0; j < n; ++j) {
+      unsigned char* sa = smem + s * C::kStageBytes + j * C::kBlockBytes;
+      const int x = (kb0 + i * C::kSub + j) * BK;
+      tma_load_2d(sa, &tmap_x, x, tm * BM, bar);
+      tma_load_2d(sa + C::kABytes, &tmap_w, x, tn * BN, bar);
+    }
   };
-  const int ahead = nkb < C::kStages ? nkb : C::kStages;
+  const int ahead = nst < C::kStages ? nst : C::kStages;
   if (threadIdx.x == 0) {
     s_abort = 0;
+    s_ready = 0;
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&done_bar, 1);
     fence_barrier_init();
+    grid_launch_next();
+    grid_wait();  // (all other accesses to global memory follow from these loads)
     for (int i = 0; i < ahead; ++i) load(i, i);
   }
   if (warp == 1) {
@@ -117,7 +135,7 @@ __global__ void __launch_bounds__(kSplitThreads)
   if (warp == 0) {
     int s = 0;
     uint32_t phase = 0;
-    for (int i = ahead; i < nkb; ++i) {
+    for (int i = ahead; i < nst; ++i) {
       const bool ok = mbar_wait_bounded(&empty_bar[s], phase, abort_flag, a.timeout_ns);
       if (!__all_sync(0xffffffffu, ok)) {
         // copies in flight land before shared memory is released
@@ -138,41 +156,49 @@ __global__ void __launch_bounds__(kSplitThreads)
     __syncwarp();
   } else if (warp == 1) {
     // The whole warp walks the stages and one elected thread issues, so that descriptors stay in
-    // uniform registers.  The next stage's barrier is looked at between the MMAs and their
-    // commit: an mbarrier access behind a commit waits for it.  And no fence follows the wait:
-    // operands arrive through the async proxy, whose barrier has been observed.  Clocks per 64
-    // columns of K with N = 64, operands in place: 496 (one lane loops, waits and fences), 337
-    // (elected thread), 207 (this form); the MMAs alone take 199.
+    // uniform registers.  The shallow form looks at the next stage's barrier between the MMAs and
+    // their commit: an mbarrier access behind a commit waits for it.  And no fence follows the
+    // wait: operands arrive through the async proxy, whose barrier has been observed.
     constexpr uint32_t idesc = make_idesc_bf16(BM, BN);
     const uint64_t desc_a = make_desc_k128(smem), desc_b = make_desc_k128(smem + C::kABytes);
     bool ok = true, ready = false;
-    uint32_t phase = 0;
+    uint32_t phase = 0, seen = 0;
     // (stages unrolled: their descriptors are constants away from two that stay in registers)
-    for (int i0 = 0; i0 < nkb && ok; i0 += C::kStages, phase ^= 1) {
+    for (int i0 = 0; i0 < nst && ok; i0 += C::kStages, phase ^= 1) {
 #pragma unroll
       for (int s = 0; s < C::kStages; ++s) {
         const int i = i0 + s;
-        if (i >= nkb) break;
-        if (!ready) {
+        if (i >= nst) break;
+        if constexpr (DEEP) {
+          if ((uint32_t)i >= seen)
+            ok = wait_ready(&s_ready, (uint32_t)i, &seen, abort_flag, a.timeout_ns);
+          if (!ok) break;
+        } else if (!ready) {
           ok = mbar_wait_bounded(&full_bar[s], phase, abort_flag, a.timeout_ns);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
         }
         if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_f16(tmem, desc_a + (uint64_t)(s * (C::kStageBytes >> 4) + 2 * k),
-                     desc_b + (uint64_t)(s * (C::kStageBytes >> 4) + 2 * k), idesc,
-                     (i | k) != 0 ? 1u : 0u);
+          for (int j = 0; j < C::kSub; ++j) {
+            if (j > 0 && i * C::kSub + j >= nkb) break;
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              const int off = (s * C::kStageBytes + j * C::kBlockBytes) >> 4;
+              umma_f16(tmem, desc_a + (uint64_t)(off + 2 * k), desc_b + (uint64_t)(off + 2 * k),
+                       idesc, (i | j | k) != 0 ? 1u : 0u);
+            }
+          }
         }
         __syncwarp();
         constexpr int kLast = C::kStages - 1;
-        ready = __all_sync(0xffffffffu, i + 1 < nkb &&
-                           mbar_try_wait(&full_bar[s == kLast ? 0 : s + 1],
-                                         s == kLast ? phase ^ 1 : phase));
+        if constexpr (!DEEP)
+          ready = __all_sync(0xffffffffu, i + 1 < nst &&
+                             mbar_test_wait(&full_bar[s == kLast ? 0 : s + 1],
+                                            s == kLast ? phase ^ 1 : phase));
         if (elect_one()) {
-          if (i + C::kStages < nkb) umma_commit(&empty_bar[s]);
-          if (i == nkb - 1) umma_commit(&done_bar);
+          if (i + C::kStages < nst) umma_commit(&empty_bar[s]);
+          if (i == nst - 1) umma_commit(&done_bar);
         }
         __syncwarp();
       }
@@ -181,6 +207,17 @@ __global__ void __launch_bounds__(kSplitThreads)
     __syncwarp();
   } else {
     const int q = warp & 3;  // tensor-memory lane quarter this warp may read
+    if (DEEP && warp == 2) {  // nothing to store yet: count the k-blocks in place
+      if (lane == 0) {
+        for (int i = 0; i < nst; ++i) {
+          if (!mbar_wait_bounded(&full_bar[i % C::kStages], (uint32_t)(i / C::kStages) & 1,
+                                 abort_flag, a.timeout_ns))
+            break;
+          st_ready(&s_ready, (uint32_t)i + 1);
+        }
+      }
+      __syncwarp();
+    }
     const bool ok = mbar_wait_bounded(&done_bar, 0, abort_flag, a.timeout_ns);
     __syncwarp();
     tc_fence_after();

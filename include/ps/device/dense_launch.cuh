@@ -5,6 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "ps/device/chain.cuh"
 #include "ps/device/local_update.cuh"
 #include "ps/device/push_pull_ll.cuh"
 
@@ -98,11 +99,12 @@ inline int launch_local(const DenseArgs& d, int num_ctas, cudaStream_t s) {
           list.tiles += (int)((in.end - 1) / kLocalTile - in.begin / kLocalTile + 1);
         }
         const int ctas = num_ctas > 0 && num_ctas < list.tiles ? num_ctas : list.tiles;
-        local_update_kernel<GT, OT, Opt, RED, BC, LocalSegs>
-            <<<ctas, kLocalThreads, 0, s>>>(a, list);
+        const int rc = launch_chained(local_update_kernel<GT, OT, Opt, RED, BC, LocalSegs>,
+                                      (unsigned)ctas, kLocalThreads, 0, s, 1, a, list);
         psdev_count_launch();
+        if (rc) return rc;
       }
-      return (int)cudaGetLastError();
+      return 0;
     }
     return PSDEV_ERR_UNSUPPORTED;
   }
@@ -117,10 +119,11 @@ inline int launch_local(const DenseArgs& d, int num_ctas, cudaStream_t s) {
     ntiles = d.end > d.begin ? (d.end - 1) / kLocalTile - d.begin / kLocalTile + 1 : 1;
   }
   const long long ctas = num_ctas > 0 && num_ctas < ntiles ? num_ctas : ntiles;
-  local_update_kernel<GT, OT, Opt, RED, BC, NoSegs>
-      <<<(unsigned)(ctas < (1ll << 30) ? ctas : 1ll << 30), kLocalThreads, 0, s>>>(a, NoSegs{});
+  const int rc = launch_chained(local_update_kernel<GT, OT, Opt, RED, BC, NoSegs>,
+                                (unsigned)(ctas < (1ll << 30) ? ctas : 1ll << 30), kLocalThreads, 0,
+                                s, 1, a, NoSegs{});
   psdev_count_launch();
-  return (int)cudaGetLastError();
+  return rc;
 }
 
 template <typename GT, typename OT, class Opt, bool RED, bool BC>

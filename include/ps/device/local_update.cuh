@@ -19,6 +19,7 @@
 #pragma once
 #include <type_traits>
 
+#include "ps/device/chain.cuh"
 #include "ps/device/push_pull.cuh"
 
 namespace psdev {
@@ -120,6 +121,8 @@ template <typename GT, typename OT, class Opt, bool REDUCE, bool BCAST, typename
 __global__ void __launch_bounds__(kLocalThreads)
     local_update_kernel(const __grid_constant__ LocalArgs a, const __grid_constant__ Segs segs) {
   constexpr bool kSegs = !std::is_same<Segs, NoSegs>::value;
+  grid_launch_next();
+  grid_wait();
   long long ntiles;
   if constexpr (kSegs) ntiles = segs.tiles;
   else if (a.sched) ntiles = a.sched[a.nseg].tile_begin;

@@ -206,18 +206,6 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// ---- programmatic dependent launch ----------------------------------------------------------
-// A kernel launched with programmatic stream serialization may start while the previous kernel of
-// its stream is still running: it must not touch global memory before grid_wait(), which returns
-// once that kernel has completed and its writes are visible.  grid_launch_next() lets the next
-// kernel of the stream start (as far as it was launched so) once every CTA has called it.
-__device__ __forceinline__ void grid_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void grid_launch_next() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // ---- tcgen05 ------------------------------------------------------------------------------
 // Allocates `ncols` (power of two, 32..512) tensor-memory columns; the base address is
 // written to `*smem_out`.  Must be executed by one full warp.

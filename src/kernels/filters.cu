@@ -11,6 +11,7 @@
 
 #include <atomic>
 
+#include "ps/device/chain.cuh"
 #include "ps/device/psdev.h"
 
 namespace psdev {
@@ -76,6 +77,8 @@ constexpr int kPackGroups = 2;
 template <bool VEC>
 __global__ void __launch_bounds__(kPackThreads)
     int8_pack(const float* in, signed char* q, float* scales, long long n) {
+  grid_launch_next();
+  grid_wait();
   const long long ngroups = (n + kGroup - 1) / kGroup;
   const int lane = threadIdx.x & 31;
   const long long stride = (long long)gridDim.x * (kPackThreads / 32) * kPackGroups;
@@ -187,9 +190,10 @@ int psdev_filter_int8_pack(const float* in, int8_t* q, float* scales, int64_t n,
   const unsigned int grid = (unsigned int)(ctas < (1ll << 30) ? ctas : 1ll << 30);
   const bool vec = ((uintptr_t)in & 31) == 0 && ((uintptr_t)q & 7) == 0;
   auto* kern = vec ? filt::int8_pack<true> : filt::int8_pack<false>;
-  kern<<<grid, filt::kPackThreads, 0, (cudaStream_t)stream>>>(in, (signed char*)q, scales, n);
+  const int rc = launch_chained(kern, grid, filt::kPackThreads, 0, (cudaStream_t)stream, 1, in,
+                                (signed char*)q, scales, n);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return (int)cudaGetLastError();
+  return rc;
 }
 // out[i] = (accumulate ? out[i] : 0) + q[i] * scales[i / 256]
 int psdev_filter_int8_unpack(const int8_t* q, const float* scales, float* out, int64_t n,

@@ -31,6 +31,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "ps/device/chain.cuh"
 #include "ps/device/push_pull.cuh"
 #include "ps/device/sm100_ptx.cuh"
 
@@ -1359,22 +1360,10 @@ static int launch_split_t(const SplitArgs& a, const CUtensorMap& tx, const CUten
     if (e != cudaSuccess) return (int)e;
     attr_set[dev & 63].store(true, std::memory_order_release);
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(tiles * S), 1, 1);
-  cfg.blockDim = dim3(kSplitThreads, 1, 1);
-  cfg.dynamicSmemBytes = SplitCfg<BN, DEEP>::kSmemBytes;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = S;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = S > 1 ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, split_gemm_kernel<BN, S, DEEP>, a, tx, tw);
+  const int e = launch_chained(split_gemm_kernel<BN, S, DEEP>, (unsigned)(tiles * S), kSplitThreads,
+                               SplitCfg<BN, DEEP>::kSmemBytes, s, S, a, tx, tw);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return (int)e;
+  return e;
 }
 template <int BN, bool DEEP>
 static int launch_split(int split, const SplitArgs& a, const CUtensorMap& tx,
@@ -1456,22 +1445,10 @@ static int run_wide(const Args& a, const void* x, const void* w, int num_ctas, c
   long long pairs = num_ctas / 2;
   if (pairs > tiles * (NT / 128)) pairs = tiles * (NT / 128);
   if (pairs < 1) pairs = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
-  cfg.blockDim = dim3(kWideThreads, 1, 1);
-  cfg.dynamicSmemBytes = WideCfg<NT>::kSmemBytes;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, k, wa, tx, tw, tw64, tc);
+  const int e = launch_chained(k, (unsigned)(2 * pairs), kWideThreads, WideCfg<NT>::kSmemBytes, s,
+                               2, wa, tx, tw, tw64, tc);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return (int)e;
+  return e;
 }
 
 // Output-tile height used by run(): 128 (double-buffered accumulators) or 256 (twice the

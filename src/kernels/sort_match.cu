@@ -15,6 +15,7 @@
 #include <atomic>
 #include <utility>
 
+#include "ps/device/chain.cuh"
 #include "ps/device/psdev.h"
 
 namespace psdev {
@@ -95,15 +96,21 @@ __device__ __forceinline__ unsigned int cta_exclusive(unsigned int v, unsigned i
   return before + incl - v;
 }
 
+// The kernels of a sort are chained (chain.cuh): 2^22 pairs of 30-bit keys take 249 us launched
+// one after the other and 227 chained, 2^18 of 40 bits 92 and 74.  What the kernel before has
+// written is read through L2 (__ldcg): a read-only path may not be used for it.
+
 // counts[d * chunks + c] = keys of chunk c whose digit is d
 template <typename K>
 __global__ void __launch_bounds__(kThreads, 2)
     digit_count_kernel(const K* __restrict__ keys, long long n, int shift, Chunks ch,
                        int key_bits, unsigned int* counts, SortHead* head) {
+  grid_launch_next();
   constexpr int kSets = 4;
   __shared__ unsigned int s[kSets][kDigits];  // four warps share a set of counters
   unsigned int* mine = s[threadIdx.x / (kThreads / kSets)];
   for (int i = threadIdx.x; i < kSets * kDigits; i += kThreads) s[0][i] = 0;
+  grid_wait();
   __syncthreads();
   const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
   const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
@@ -112,7 +119,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     K k[kItems];
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
-      k[j] = base + j * kThreads < hi ? keys[base + j * kThreads] : (K)0;
+      k[j] = base + j * kThreads < hi ? __ldcg(keys + base + j * kThreads) : (K)0;
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
       if (base + j * kThreads < hi) {
@@ -133,6 +140,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 // One CTA per digit: exclusive prefix over the chunks in place, and the digit's total.
 __global__ void __launch_bounds__(kThreads)
     digit_scan_kernel(unsigned int* counts, int chunks, unsigned int* totals) {
+  grid_launch_next();
+  grid_wait();
   __shared__ unsigned int s_part[kWarps];
   static_assert(kMaxChunks <= kThreads && kDigits <= kThreads, "one thread per chunk, digit");
   unsigned int* row = counts + (size_t)blockIdx.x * chunks;
@@ -189,6 +198,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                    const unsigned int* __restrict__ pay_in, unsigned int* __restrict__ pay_out,
                    long long n, int shift, Chunks ch, const unsigned int* __restrict__ prefix,
                    const unsigned int* __restrict__ totals) {
+  grid_launch_next();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   KO* skeys = reinterpret_cast<KO*>(smem_raw);
   unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + kTile * sizeof(KO));
@@ -201,11 +211,13 @@ __global__ void __launch_bounds__(kThreads, 2)
   unsigned int* goff = &lanes[kWarps][0];  // output index of sorted position q: goff[d] + q
   __shared__ unsigned int s_part[2][kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // output index of the chunk's next key with digit threadIdx.x
   const bool digit = threadIdx.x < kDigits;
-  unsigned int next = cta_exclusive(digit ? totals[threadIdx.x] : 0, s_part[0], nullptr);
-  if (digit) next += prefix[(size_t)threadIdx.x * ch.count + blockIdx.x];
   for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) lanes[0][i] = 0;
+  grid_wait();
+  // output index of the chunk's next key with digit threadIdx.x
+  unsigned int next = cta_exclusive(digit ? __ldcg(totals + threadIdx.x) : 0, s_part[0],
+                                    nullptr);
+  if (digit) next += __ldcg(prefix + (size_t)threadIdx.x * ch.count + blockIdx.x);
   const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
   const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
   // A tile is loaded before the one before it is stored: its keys and payloads take the registers
@@ -216,8 +228,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
       const long long i = base + j * 32;
-      k[j] = i < hi ? (KO)keys_in[i] : (KO)~0ull;
-      if constexpr (PAY == kPayload) pay[j] = i < hi ? pay_in[i] : 0u;
+      k[j] = i < hi ? (KO)__ldcg(keys_in + i) : (KO)~0ull;
+      if constexpr (PAY == kPayload) pay[j] = i < hi ? __ldcg(pay_in + i) : 0u;
       else pay[j] = (unsigned int)i;
     }
   };
@@ -280,6 +292,8 @@ __global__ void __launch_bounds__(kThreads)
     small_sort_kernel(const KI* keys_in, K* keys_out, const unsigned int* pay_in,
                       unsigned int* pay_out, int n, int passes, int key_bits, SortHead* head,
                       unsigned int* unique) {
+  grid_launch_next();
+  grid_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   K* skeys = reinterpret_cast<K*>(smem_raw);
   unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + kTile * sizeof(K));
@@ -390,10 +404,10 @@ static int small_sort(const KI* in, K* out, const unsigned int* pin, unsigned in
                       int passes, int key_bits, SortHead* head, unsigned int* unique,
                       cudaStream_t s) {
   if (int rc = allow_smem<small_sort_kernel<KI, K, PAY>>(scatter_smem<K>(PAY))) return rc;
-  small_sort_kernel<KI, K, PAY><<<1, kThreads, scatter_smem<K>(PAY), s>>>(
-      in, out, pin, pout, n, passes, key_bits, head, unique);
+  const int rc = launch_chained(small_sort_kernel<KI, K, PAY>, 1, kThreads, scatter_smem<K>(PAY), s,
+                                1, in, out, pin, pout, n, passes, key_bits, head, unique);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return 0;
+  return rc;
 }
 
 template <typename KI, typename KO, int PAY>
@@ -402,13 +416,16 @@ static int sort_pass(const KI* in, KO* out, const unsigned int* pin, unsigned in
   if (int rc = allow_smem<scatter_kernel<KI, KO, PAY>>(scatter_smem<KO>(PAY))) return rc;
   const Chunks ch = chunks_of(n);
   const int shift = pass * kRadixBits;
-  digit_count_kernel<KI><<<ch.count, kThreads, 0, s>>>(in, n, shift, ch, pass ? 64 : key_bits,
-                                                       w.counts, w.head);
-  digit_scan_kernel<<<kDigits, kThreads, 0, s>>>(w.counts, ch.count, w.totals);
-  scatter_kernel<KI, KO, PAY><<<ch.count, kThreads, scatter_smem<KO>(PAY), s>>>(
-      in, out, pin, pout, n, shift, ch, w.counts, w.totals);
+  int rc = launch_chained(digit_count_kernel<KI>, ch.count, kThreads, 0, s, 1, in, n, shift, ch,
+                          pass ? 64 : key_bits, w.counts, w.head);
+  if (!rc)
+    rc = launch_chained(digit_scan_kernel, kDigits, kThreads, 0, s, 1, w.counts, ch.count,
+                        w.totals);
+  if (!rc)
+    rc = launch_chained(scatter_kernel<KI, KO, PAY>, ch.count, kThreads, scatter_smem<KO>(PAY), s,
+                        1, in, out, pin, pout, n, shift, ch, w.counts, w.totals);
   g_launches.fetch_add(3, std::memory_order_relaxed);
-  return 0;
+  return rc;
 }
 
 // ---- sums of the values of equal keys --------------------------------------------------------
@@ -426,6 +443,8 @@ __host__ __device__ inline Chunks unique_chunks_of(long long n) {
 template <typename K>
 __global__ void __launch_bounds__(kThreads, 2)
     unique_count_kernel(const K* __restrict__ keys, long long n, Chunks ch, unsigned int* counts) {
+  grid_launch_next();
+  grid_wait();
   __shared__ unsigned int s_part[kWarps];
   const int lane = threadIdx.x & 31;
   const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
@@ -436,8 +455,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
       const long long i = base + j * kThreads;
-      k[j] = i < hi ? keys[i] : (K)0;
-      before[j] = lane == 0 && i > 0 && i < hi ? keys[i - 1] : (K)0;
+      k[j] = i < hi ? __ldcg(keys + i) : (K)0;
+      before[j] = lane == 0 && i > 0 && i < hi ? __ldcg(keys + i - 1) : (K)0;
     }
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
@@ -461,6 +480,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     unique_sum_kernel(const K* __restrict__ keys, const float* __restrict__ vals, long long n,
                       Chunks ch, const unsigned int* __restrict__ counts,
                       unsigned long long* out_keys, float* out_sums) {
+  grid_launch_next();
+  grid_wait();
   constexpr int kPer = kUniquePer;
   constexpr int kRound = kThreads * kPer;
   constexpr int kPadded = kRound + kRound / kPer;  // (a thread's pairs start in different banks)
@@ -477,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   unsigned int next;
   {
     unsigned int c = 0;
-    for (int i = threadIdx.x; i < blockIdx.x; i += kThreads) c += counts[i];
+    for (int i = threadIdx.x; i < blockIdx.x; i += kThreads) c += __ldcg(counts + i);
     cta_exclusive(c, s_part, &next);
   }
   const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
@@ -489,8 +510,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int j = 0; j < kPer; ++j) {
       const int q = threadIdx.x + j * kThreads;
       if (q < count) {
-        skey[q + q / kPer] = keys[base + q];
-        sval[q + q / kPer] = vals[base + q];
+        skey[q + q / kPer] = __ldcg(keys + base + q);
+        sval[q + q / kPer] = __ldcg(vals + base + q);
       }
     }
     __syncthreads();
@@ -498,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     K prev{};
     if (q0 < count) {
       if (q0 > 0) prev = skey[p0 - 2];
-      else if (base > 0) prev = keys[base - 1];
+      else if (base > 0) prev = __ldcg(keys + base - 1);
     }
     bool head[kPer];
     unsigned int heads = 0;
@@ -740,10 +761,10 @@ int unique_sort(const unsigned long long* keys, const float* vals, int64_t n, in
     if (rc) return rc;
   }
   const Chunks ch = unique_chunks_of(n);
-  unique_count_kernel<K><<<ch.count, kThreads, 0, s>>>(reinterpret_cast<const K*>(u.keys[0]), n,
-                                                       ch, u.counts);
+  const int rc = launch_chained(unique_count_kernel<K>, ch.count, kThreads, 0, s, 1,
+                                reinterpret_cast<const K*>(u.keys[0]), n, ch, u.counts);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return 0;
+  return rc;
 }
 
 template <typename K>
@@ -754,11 +775,12 @@ int unique_write(const UniqueScratch& u, int64_t n, unsigned long long* out_keys
                        (int)(sizeof(K) + 4);
   if (int rc = allow_smem<unique_sum_kernel<K>>(smem)) return rc;
   const Chunks ch = unique_chunks_of(n);
-  unique_sum_kernel<K><<<ch.count, kThreads, smem, s>>>(
-      reinterpret_cast<const K*>(u.keys[0]), reinterpret_cast<const float*>(u.vals[0]), n, ch,
-      u.counts, out_keys, out_sums);
+  const int rc = launch_chained(unique_sum_kernel<K>, ch.count, kThreads, smem, s, 1,
+                                reinterpret_cast<const K*>(u.keys[0]),
+                                reinterpret_cast<const float*>(u.vals[0]), n, ch, u.counts,
+                                out_keys, out_sums);
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return (int)cudaGetLastError();
+  return rc;
 }
 }  // namespace
 

@@ -30,6 +30,7 @@
 
 #include <atomic>
 
+#include "ps/device/chain.cuh"
 #include "ps/device/push_pull.cuh"
 
 namespace psdev {
@@ -468,6 +469,8 @@ __device__ __forceinline__ bool below(long long at, long long end) {
 template <bool GROUP, bool ONE>
 __global__ void __launch_bounds__(256)
     sparse_local_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ LocalReq q) {
+  grid_launch_next();
+  grid_wait();
   constexpr int kLocalUnroll = GROUP && ONE ? kStateUnroll : psdev::kLocalUnroll;
   const unsigned int width = ONE ? 1u : (unsigned int)a.width;
   const long long work = q.n * width;
@@ -522,6 +525,8 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     sparse_local_rows_kernel(const __grid_constant__ SparseArgs a,
                              const __grid_constant__ LocalReq q) {
+  grid_launch_next();
+  grid_wait();
   const unsigned int quads = (unsigned int)a.width / 4;
   const long long work = q.n * quads;
   const long long first = blockIdx.x * (256ll * kLocalUnroll) + threadIdx.x;
@@ -647,6 +652,8 @@ __device__ __forceinline__ long long cta_sum(long long v, long long* part) {
 __global__ void __launch_bounds__(256)
     sparse_len_sums_kernel(const __grid_constant__ SparseArgs a,
                            const __grid_constant__ LocalReq q) {
+  grid_launch_next();
+  grid_wait();
   __shared__ long long s_part[8];
   const long long size = (long long)q.blocks * kLenBlock, lo = blockIdx.x * size;
   const long long hi = lo + size < q.n ? lo + size : q.n;
@@ -658,6 +665,8 @@ template <bool GROUP>
 __global__ void __launch_bounds__(256)
     sparse_local_lens_kernel(const __grid_constant__ SparseArgs a,
                              const __grid_constant__ LocalReq q) {
+  grid_launch_next();
+  grid_wait();
   __shared__ long long s_part[8];
   __shared__ unsigned long long s_key[kLenBlock];
   __shared__ long long s_idx[kLenBlock];  // slot; -1: none, -2: not this key's work
@@ -925,25 +934,26 @@ int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t 
     if (n > kLenSelf) {
       // (the arena's array of value offsets, unused by this form, holds the chunk sums)
       q.sums = reinterpret_cast<long long*>(static_cast<char*>(w->peer_base[0]) + t->offs_off);
-      sparse_len_sums_kernel<<<chunks, 256, 0, s>>>(a, q);
+      rc = launch_chained(sparse_len_sums_kernel, chunks, 256, 0, s, 1, a, q);
       g_launches.fetch_add(1, std::memory_order_relaxed);
     }
-    if (group) sparse_local_lens_kernel<true><<<chunks, 256, 0, s>>>(a, q);
-    else sparse_local_lens_kernel<false><<<chunks, 256, 0, s>>>(a, q);
+    auto* kern = group ? sparse_local_lens_kernel<true> : sparse_local_lens_kernel<false>;
+    if (!rc) rc = launch_chained(kern, chunks, 256, 0, s, 1, a, q);
   } else {
     const bool rows = t->kind != 2 && t->width % 4 == 0 && a.sstride == 1 &&
                       (((uintptr_t)vals | (uintptr_t)out | (uintptr_t)t->w) & 15) == 0;
     const long long work = rows ? n * (t->width / 4) : n * t->width;
     const int unroll = group && t->width == 1 ? kStateUnroll : kLocalUnroll;
     const unsigned ctas = (unsigned)((work + 256 * unroll - 1) / (256 * unroll));
-    if (rows) sparse_local_rows_kernel<<<ctas, 256, 0, s>>>(a, q);
-    else if (group && t->width == 1) sparse_local_kernel<true, true><<<ctas, 256, 0, s>>>(a, q);
-    else if (group) sparse_local_kernel<true, false><<<ctas, 256, 0, s>>>(a, q);
-    else if (t->width == 1) sparse_local_kernel<false, true><<<ctas, 256, 0, s>>>(a, q);
-    else sparse_local_kernel<false, false><<<ctas, 256, 0, s>>>(a, q);
+    auto* kern = rows                    ? sparse_local_rows_kernel
+                 : group && t->width == 1 ? sparse_local_kernel<true, true>
+                 : group                  ? sparse_local_kernel<true, false>
+                 : t->width == 1          ? sparse_local_kernel<false, true>
+                                          : sparse_local_kernel<false, false>;
+    rc = launch_chained(kern, ctas, 256, 0, s, 1, a, q);
   }
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  return (int)cudaGetLastError();
+  return rc;
 }
 
 // Server role.  `sync` != 0: the kernel first waits until every rank has entered it, i.e.

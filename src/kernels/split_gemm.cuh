@@ -13,9 +13,9 @@
 // Launched with programmatic stream serialization: the prologue runs beside the end of the kernel
 // before it.
 //
-// Two forms.  With more CTAs than SMs about 100 KB of shared memory per CTA, so that two share an SM
-// and one loads while the other stores.  Otherwise (DEEP) one CTA has the SM, and a stage holds two
-// k-blocks: per stage the ring costs some 300 clocks (commit, barrier, producer) whatever it
+// Two forms.  With more CTAs than SMs about 100 KB of shared memory per CTA, so that two share an
+// SM and one loads while the other stores.  Otherwise (DEEP) one CTA has the SM, and a stage holds
+// two k-blocks: per stage the ring costs some 300 clocks (commit, barrier, producer) whatever it
 // carries, and 128 columns of K make up for them.  The issuer of the deep form touches no mbarrier
 // (see wait_ready).  1024 x 1024 x 4096 with BN = 64 / 128 20.9 / 24.5 us shallow, 16.5 / 18.2
 // deep; what is left is the loads, 70 bytes per clock and SM.

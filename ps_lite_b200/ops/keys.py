@@ -37,24 +37,19 @@ def sort_keys(keys: torch.Tensor, key_bits: int = 64, return_perm: bool = False,
     return keys, perm
 
 
-def _unique_sum_fp32(keys, vals, key_bits):
-    """The native form; None when a key is wider than ``key_bits`` (only its low bits sort then)."""
-    lib, n = _lib.device_lib(), keys.numel()
-    stream = torch.cuda.current_stream(keys.device).cuda_stream
-    nbytes = lib.psdev_unique_sum_scratch_bytes(n, key_bits)
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=keys.device)
-    count = C.c_int64()
-    rc = lib.psdev_unique_sum_sort(keys.data_ptr(), vals.data_ptr(), n, key_bits,
-                                   scratch.data_ptr(), nbytes, C.byref(count), stream)
-    if rc == -1:
-        return None
-    _lib.check(rc, "psdev_unique_sum_sort")
-    u = count.value
-    uk = torch.empty(u, dtype=torch.int64, device=keys.device)
-    out = torch.empty(u, dtype=torch.float32, device=keys.device)
-    _lib.check(lib.psdev_unique_sum_write(scratch.data_ptr(), n, key_bits, u, uk.data_ptr(),
-                                          out.data_ptr(), stream), "psdev_unique_sum_write")
-    return uk, out
+class _Native:
+    """The native call and the addresses it is given, resolved at the first use."""
+
+    def __getattr__(self, name):
+        lib, ext = _lib.device_lib(), _lib.torch_ext()
+        self.fns = tuple(C.cast(f, C.c_void_p).value for f in (
+            lib.psdev_unique_sum_scratch_bytes, lib.psdev_unique_sum_sort,
+            lib.psdev_unique_sum_write))
+        self.unique_sum = ext.unique_sum
+        return self.__dict__[name]
+
+
+_native = _Native()
 
 
 def sort_unique_sum(keys: torch.Tensor, vals: torch.Tensor, key_bits: int = 64
@@ -63,13 +58,12 @@ def sort_unique_sum(keys: torch.Tensor, vals: torch.Tensor, key_bits: int = 64
     values of repeated keys; keys must be below ``2**key_bits``.  fp32 values travel with the
     keys through the sort and are summed by a kernel of their own; other types take the sort
     permutation and torch's ``index_add_``."""
-    n = keys.numel()
-    if (vals.dtype == torch.float32 and vals.dim() == 1 and vals.numel() == n and
-            not (vals.requires_grad and torch.is_grad_enabled()) and
-            0 < n < 1 << 30 and keys.dtype == torch.int64 and keys.is_cuda and vals.is_cuda):
-        got = _unique_sum_fp32(keys.contiguous(), vals.contiguous(), key_bits)
-        if got is not None:
+    if keys.is_cuda:
+        got = _native.unique_sum(*_native.fns, keys, vals, key_bits)
+        if type(got) is tuple:
             return got
+        if got is not None:  # (None: another type, or a key wider than key_bits)
+            _lib.check(got, "psdev_unique_sum")
     k = keys.clone()
     k, perm = sort_keys(k, key_bits, return_perm=True)
     v = vals[perm.long()]

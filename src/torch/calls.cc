@@ -3,6 +3,7 @@
 // costs about 0.1 us and a ctypes call with a dozen arguments 1.5 us; a launch costs 2.5 us.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/core/GradMode.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -18,6 +19,11 @@ using DenseFn = int (*)(const psdev_world_t*, const psdev_table_t*, int, int64_t
                         const psdev_opt_t*, int, int, uint64_t, int, void*);
 using SparseFn = int (*)(const psdev_world_t*, const psdev_sparse_t*, int64_t, const uint64_t*,
                          const float*, int64_t, const int32_t*, float*, int64_t, int32_t*, void*);
+
+using UniqueBytesFn = size_t (*)(int64_t, int);
+using UniqueSortFn = int (*)(const uint64_t*, const float*, int64_t, int, void*, size_t, int64_t*,
+                             void*);
+using UniqueWriteFn = int (*)(const void*, int64_t, int, int64_t, uint64_t*, float*, void*);
 
 template <typename T>
 T address(PyObject* o) {
@@ -105,6 +111,51 @@ PyObject* pull_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// unique_sum(bytes_fn, sort_fn, write_fn, keys, vals, key_bits) -> (keys, sums), None where this
+// form does not apply (other types; a key of more than key_bits bits), or an error code
+PyObject* unique_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 6) return PyErr_Format(PyExc_TypeError, "unique_sum takes 6 arguments");
+  HANDLE_TH_ERRORS
+  const long bits = PyLong_AsLong(a[5]);
+  const auto bytes_fn = address<UniqueBytesFn>(a[0]);
+  const auto sort_fn = address<UniqueSortFn>(a[1]);
+  const auto write_fn = address<UniqueWriteFn>(a[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!THPVariable_Check(a[3]) || !THPVariable_Check(a[4])) Py_RETURN_NONE;
+  const at::Tensor &k_in = THPVariable_Unpack(a[3]), &v_in = THPVariable_Unpack(a[4]);
+  const int64_t count = k_in.numel();
+  if (k_in.scalar_type() != at::kLong || v_in.scalar_type() != at::kFloat || v_in.dim() != 1 ||
+      v_in.numel() != count || count <= 0 || count >= (int64_t{1} << 30) || !k_in.is_cuda() ||
+      !v_in.is_cuda() || (v_in.requires_grad() && c10::GradMode::is_enabled()))
+    Py_RETURN_NONE;
+  const at::Tensor k = k_in.contiguous(), v = v_in.contiguous();
+  void* stream = stream_on(k.get_device());
+  const size_t bytes = bytes_fn(count, static_cast<int>(bits));
+  const auto plain = k.options().requires_grad(false);
+  at::Tensor scratch = at::empty({static_cast<int64_t>(bytes)}, plain.dtype(at::kByte));
+  int64_t unique = 0;
+  int rc = without_gil([&] {
+    return sort_fn(static_cast<const uint64_t*>(k.data_ptr()),
+                   static_cast<const float*>(v.data_ptr()), count, static_cast<int>(bits),
+                   scratch.data_ptr(), bytes, &unique, stream);
+  });
+  if (rc == PSDEV_ERR_ARG) Py_RETURN_NONE;
+  if (rc) return PyLong_FromLong(rc);
+  at::Tensor keys = at::empty({unique}, plain), sums = at::empty({unique}, plain.dtype(at::kFloat));
+  rc = without_gil([&] {
+    return write_fn(scratch.data_ptr(), count, static_cast<int>(bits), unique,
+                    static_cast<uint64_t*>(keys.data_ptr()), static_cast<float*>(sums.data_ptr()),
+                    stream);
+  });
+  if (rc) return PyLong_FromLong(rc);
+  PyObject* pair = PyTuple_New(2);
+  if (!pair) return nullptr;
+  PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(std::move(keys)));
+  PyTuple_SET_ITEM(pair, 1, THPVariable_Wrap(std::move(sums)));
+  return pair;
+  END_HANDLE_TH_ERRORS
+}
+
 // dense_op(fn, world, table, op, begin, end, opt, channel, num_ctas, timeout_ns, sync, stream)
 PyObject* dense_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 12) return PyErr_Format(PyExc_TypeError, "dense_op takes 12 arguments");
@@ -183,6 +234,8 @@ PyMethodDef kMethods[] = {
     {"linear", fast(&linear), METH_FASTCALL, "linear(fn, x, w, out, num_ctas, timeout_ns)"},
     {"pull_linear", fast(&pull_linear), METH_FASTCALL,
      "pull_linear(fn, world, table, w_offset, n_out, x, out, copy_ctas, num_ctas, timeout_ns)"},
+    {"unique_sum", fast(&unique_sum), METH_FASTCALL,
+     "unique_sum(bytes_fn, sort_fn, write_fn, keys, vals, key_bits)"},
     {"dense_op", fast(&dense_op), METH_FASTCALL,
      "dense_op(fn, world, table, op, begin, end, opt, channel, num_ctas, timeout_ns, sync, "
      "stream)"},

@@ -486,8 +486,8 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 // Adds up the chunks' counts for the host.  A kernel that writes a word of mapped memory which the
-// host polls is cheaper than a copy and a wait for the stream (with the call from Python native: 4096
-// ids 58 us before, 41 now; 2^22 216 and 204).
+// host polls is cheaper than a copy and a wait for the stream (with the call from Python native:
+// 4096 ids 58 us before, 41 now; 2^22 216 and 204).
 __global__ void __launch_bounds__(kThreads)
     unique_total_kernel(const unsigned int* counts, int chunks, const SortHead* head,
                         unsigned long long* host) {

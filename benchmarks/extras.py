@@ -100,7 +100,7 @@ def _sparse(ctx, steps=10):
     all_ok = all(b == b"1" for b in ctx.allgather(b"1" if ok else b"0"))
     return {"metric": "sparse_lr_keys_per_s", "value": round(world * n / (ms * 1e-3)),
             "unit": "keys/s", "ms_per_step": round(ms, 4), "keys_per_worker_per_step": n,
-            "key_space": key_space, "handle": "FTRL-proximal", "launches_per_step": 3,
+            "key_space": key_space, "handle": "FTRL-proximal", "launches_per_step": 1 if world == 1 else 3,
             "first_step_matches_oracle": all_ok,
             "requests_on_keys_shared_between_workers": round(shared, 4)}
 

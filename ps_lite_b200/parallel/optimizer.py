@@ -13,7 +13,8 @@ and that its users build on ``KVWorker::Push/Pull`` with per-message priorities
   default) and their priority is the reverse of the layer order, so the weights the next
   forward pass needs first are exchanged first among the slices that are pending;
 * on one rank there is nothing to exchange: native hooks (src/torch/grad_exchange.cc) collect the
-  gradient tensors as they are, and the update kernel reads them where they lie;
+  gradient tensors as they are, and the update kernel reads them where they lie; a gradient whose
+  memory somebody else can still write (a view of a workspace, say) is copied by its hook;
 * slices are exchanged by fused push+pull kernels on a side stream, overlapping the rest of
   backward: as soon as ``batch_bytes`` (4 MiB by default, ``PSB200_BATCH_BYTES``) of gradients
   are pending, everything pending goes out in ONE launch whose CTAs take the slices in priority
@@ -149,7 +150,8 @@ class DistributedOptimizer:
             t.step = me().steps + 1
             C.memmove(C.byref(opt), C.byref(t._opt_struct()), C.sizeof(opt))
 
-        fn = C.cast(self.heap.lib.psdev_dense_op_segs, C.c_void_p).value
+        segs, cast = (C.cast(f, C.c_void_p).value for f in (self.heap.lib.psdev_dense_op_segs,
+                                                             self.heap.lib.psdev_filter_cast))
         # reverse layer order, published parameters last (on one rank publishing is the same
         # store into this rank's weight buffer)
         pri = [-1 - i if self._publish[i] else len(self.params) - i
@@ -158,7 +160,7 @@ class DistributedOptimizer:
         # one rank the update is a pass over memory, shortest on the whole GPU
         return _lib.torch_ext().GradExchange(
             self.params, self.offsets, pri, t.grad, C.addressof(t._world), C.addressof(t._table),
-            C.addressof(self._opt), fn, self.comm.cuda_stream if self.comm else 0,
+            C.addressof(self._opt), segs, cast, self.comm.cuda_stream if self.comm else 0,
             self.comm is not None, max(1, self.batch_bytes // self._gsz),
             max(8, int(slice_elems) & ~7), channel, begin_step)
 

@@ -8,6 +8,12 @@
 // lies, rounds it to the table's gradient type and updates the weights
 // (psdev_dense_op_segs, include/ps/device/local_update.cuh).
 //
+// That read comes later than the hook and on another stream, so it is made only of memory that
+// nobody else can write meanwhile (Private).  Autograd hands on a gradient without a copy as soon
+// as its tensor has one owner, even where its storage has more: a custom backward may return views
+// of a workspace that it writes again for the next layer.  Such a gradient is copied into the
+// table's gradient buffer on the stream that made it, by the hook.
+//
 // The hooks sit on the parameters' gradient accumulators, next to hooks that a program registers
 // on the parameters themselves, and run after those.  A gradient stays alive until the kernel
 // that reads it has finished: batches are kept with an event and dropped when it has fired, the
@@ -34,15 +40,18 @@ using torch::autograd::Node;
 using torch::autograd::variable_list;
 using SegsFn = int (*)(const psdev_world_t*, const psdev_table_t*, int, const psdev_seg_t*, int,
                        const psdev_opt_t*, int, int, void*);
+using CastFn = int (*)(const void*, void*, int64_t, float, int, void*);
 
 class GradExchange {
  public:
-  // `world`, `table`, `opt`, `segs_fn`: addresses of the structures and of psdev_dense_op_segs;
+  // `world`, `table`, `opt`, `segs_fn`, `cast_fn`: addresses of the structures, of
+  // psdev_dense_op_segs and of psdev_filter_cast;
   // `begin_step` refreshes *opt and is called before the first gradient of every step.
   GradExchange(std::vector<at::Tensor> params, std::vector<int64_t> offsets,
                std::vector<int64_t> priorities, at::Tensor grad_buffer, uint64_t world,
-               uint64_t table, uint64_t opt, uint64_t segs_fn, uint64_t comm_stream, bool overlap,
-               int64_t batch_elems, int64_t slice_elems, int channel, py::function begin_step)
+               uint64_t table, uint64_t opt, uint64_t segs_fn, uint64_t cast_fn,
+               uint64_t comm_stream, bool overlap, int64_t batch_elems, int64_t slice_elems,
+               int channel, py::function begin_step)
       : params_(std::move(params)),
         offsets_(std::move(offsets)),
         priorities_(std::move(priorities)),
@@ -51,6 +60,7 @@ class GradExchange {
         table_(reinterpret_cast<const psdev_table_t*>(table)),
         opt_(reinterpret_cast<const psdev_opt_t*>(opt)),
         segs_fn_(reinterpret_cast<SegsFn>(segs_fn)),
+        cast_fn_(reinterpret_cast<CastFn>(cast_fn)),
         device_(grad_buffer_.device().index()),
         overlap_(overlap),
         comm_(c10::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(comm_stream),
@@ -102,12 +112,13 @@ class GradExchange {
 
   int64_t launches() const { return launches_; }
   int64_t slices() const { return slices_; }
+  int64_t staged() const { return staged_; }  // gradients that went through the gradient buffer
 
  private:
   struct Hook : torch::autograd::FunctionPostHook {
     Hook(GradExchange* owner, size_t index) : owner(owner), index(index) {}
-    variable_list operator()(const variable_list& outputs, const variable_list&) override {
-      owner->Take(index);
+    variable_list operator()(const variable_list& outputs, const variable_list& inputs) override {
+      owner->Take(index, inputs);
       return outputs;
     }
     GradExchange* owner;
@@ -118,7 +129,51 @@ class GradExchange {
     std::vector<at::Tensor> tensors;
   };
 
-  void Take(size_t i) {
+  // Whether `grad`, taken out of its parameter, is the only way to its memory.  The tensor that
+  // autograd accumulated (`inputs`) is still alive here and may share the storage, and so may the
+  // tensor that this one is a view of (the transpose of a matrix product, for a linear layer);
+  // both go with the call that runs the hook.  Memory that is not the allocator's own may have
+  // owners that torch does not know.
+  static bool Private(const at::Tensor& grad, const variable_list& inputs) {
+    const c10::Storage& mem = grad.storage();
+    if (grad.use_count() != 1 ||
+        mem.data_ptr().get_deleter() != c10::cuda::CUDACachingAllocator::get()->raw_deleter())
+      return false;
+    size_t owners = 1;
+    for (const at::Tensor& x : inputs) {
+      if (!x.defined() || !x.has_storage() || !x.storage().is_alias_of(mem)) continue;
+      if (x.use_count() > 2) return false;  // (the engine's reference, and Python's if it has one)
+      ++owners;
+      if (x.is_view()) {
+        if (x._base().use_count() > 1) return false;  // (the view's reference)
+        ++owners;
+      }
+    }
+    return mem.use_count() == owners;
+  }
+
+  // The gradient of parameter `i` into the table's gradient buffer, on the hook's stream: a copy or
+  // a cast of its own where the layout allows it (a third of what Tensor::copy_ costs this thread).
+  void Stage(size_t i, const at::Tensor& grad, bool plain, const c10::cuda::CUDAStream& cur) {
+    ++staged_;
+    const int64_t n = params_[i].numel();
+    const auto to = grad_buffer_.scalar_type(), from = grad.scalar_type();
+    const size_t size = grad_buffer_.element_size();
+    char* dst = static_cast<char*>(grad_buffer_.data_ptr()) + offsets_[i] * size;
+    if (plain && from == to) {
+      C10_CUDA_CHECK(cudaMemcpyAsync(dst, grad.data_ptr(), n * size, cudaMemcpyDeviceToDevice,
+                                     cur.stream()));
+    } else if (plain) {
+      const int rc = cast_fn_(grad.data_ptr(), dst, n, 1.f, to == at::kBFloat16 ? 0 : 1,
+                              cur.stream());
+      TORCH_CHECK(rc == 0, "psdev_filter_cast failed with ", rc);
+    } else {
+      at::NoGradGuard no_grad;
+      grad_buffer_.narrow(0, offsets_[i], n).view(params_[i].sizes()).copy_(grad, true);
+    }
+  }
+
+  void Take(size_t i, const variable_list& inputs) {
     at::Tensor& slot = params_[i].mutable_grad();
     if (!slot.defined()) return;
     if (!in_step_.exchange(true)) {
@@ -138,15 +193,15 @@ class GradExchange {
     at::Tensor grad = std::move(slot);
     slot = at::Tensor();
     const auto dt = grad.scalar_type();
-    if (grad.layout() == at::kStrided && grad.is_contiguous() && grad.device().index() == device_ &&
-        grad.is_cuda() && (dt == at::kFloat || dt == at::kBFloat16)) {
+    const bool plain = grad.layout() == at::kStrided && grad.is_contiguous() && grad.is_cuda() &&
+                       grad.device().index() == device_ && !grad.is_neg() &&
+                       (dt == at::kFloat || dt == at::kBFloat16);
+    if (plain && Private(grad, inputs)) {
       seg.src = grad.data_ptr();
       seg.dtype = dt == at::kFloat ? PSDEV_F32 : PSDEV_BF16;
       held_.push_back(std::move(grad));
     } else {
-      // another layout or type: through the table's gradient buffer
-      at::NoGradGuard no_grad;
-      grad_buffer_.narrow(0, offsets_[i], n).view(params_[i].sizes()).copy_(grad, true);
+      Stage(i, grad, plain, cur);
     }
     segs_.push_back(seg);
     pending_ += padded;
@@ -206,6 +261,7 @@ class GradExchange {
   const psdev_table_t* table_;
   const psdev_opt_t* opt_;
   SegsFn segs_fn_;
+  CastFn cast_fn_;
   c10::DeviceIndex device_;
   bool overlap_;
   c10::cuda::CUDAStream comm_;
@@ -224,7 +280,7 @@ class GradExchange {
   cudaStream_t hook_stream_ = nullptr;
   bool other_stream_ = false;
   int64_t pending_ = 0;
-  std::atomic<int64_t> launches_{0}, slices_{0};
+  std::atomic<int64_t> launches_{0}, slices_{0}, staged_{0};
 };
 
 }  // namespace
@@ -238,10 +294,11 @@ PYBIND11_MODULE(psb200_torch, m) {
   using release = py::call_guard<py::gil_scoped_release>;
   py::class_<GradExchange>(m, "GradExchange")
       .def(py::init<std::vector<at::Tensor>, std::vector<int64_t>, std::vector<int64_t>, at::Tensor,
-                    uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, bool, int64_t, int64_t, int,
-                    py::function>())
+                    uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, bool, int64_t,
+                    int64_t, int, py::function>())
       .def("step", &GradExchange::Step, release())
       .def("detach", &GradExchange::Detach, release())
       .def_property_readonly("launches", &GradExchange::launches)
-      .def_property_readonly("slices", &GradExchange::slices);
+      .def_property_readonly("slices", &GradExchange::slices)
+      .def_property_readonly("staged", &GradExchange::staged);
 }

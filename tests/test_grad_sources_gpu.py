@@ -1,0 +1,89 @@
+"""Where the native hooks of DistributedOptimizer on one rank find a gradient: memory that belongs to
+the gradient alone is read in place, memory that somebody else can write is copied by the hook."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class _FromWorkspace(torch.autograd.Function):
+    """A layer whose backward makes its weight gradient in a workspace that all layers share."""
+
+    @staticmethod
+    def forward(ctx, x, p, value, ws):
+        ctx.value, ctx.ws, ctx.shape = value, ws, p.shape
+        return x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, g):
+        part = ctx.ws[:ctx.shape.numel()]
+        part.fill_(ctx.value)
+        return g, part.view(ctx.shape), None, None
+
+
+def _optimizer(dev, params, gdt, overlap=True, batch_bytes=1 << 22, kind="sgd"):
+    from ps_lite_b200.parallel import ServerOptimizer, SymmetricHeap
+    from ps_lite_b200.parallel.optimizer import DistributedOptimizer
+    n = sum((p.numel() + 7) & ~7 for p in params)
+    heap = SymmetricHeap(8 * n + (1 << 20), 0, 1, device=dev)
+    return heap, DistributedOptimizer(params, heap, ServerOptimizer(kind, lr=0.5, momentum=0.5),
+                                      grad_dtype=gdt, overlap=overlap, batch_bytes=batch_bytes)
+
+
+# whole numbers below 256 times powers of two: exact in bf16 and fp32
+@pytest.mark.parametrize("batch_bytes", [1, 1 << 22])
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("wdt,gdt", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16),
+                                     (torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
+def test_workspace_written_again_for_the_next_layer(cuda_device, wdt, gdt, overlap, batch_bytes):
+    shapes = [(1,), (9, 5), (1 << 18,), (513, 1025), (7,)]
+    params = [torch.nn.Parameter(torch.zeros(s, device=cuda_device, dtype=wdt)) for s in shapes]
+    heap, dopt = _optimizer(cuda_device, params, gdt, overlap, batch_bytes)
+    ws = torch.zeros(513 * 1025, device=cuda_device, dtype=wdt)
+    for step in range(3):
+        x = torch.ones(1, device=cuda_device, requires_grad=True)
+        for i, p in enumerate(params):
+            x = _FromWorkspace.apply(x, p, 2.0 * (i + 1), ws)
+        x.sum().backward()
+        ws.fill_(99.0)      # ... and once more before the step ends
+        dopt.step()
+        for i, p in enumerate(params):
+            assert torch.all(p == -(step + 1.0) * (i + 1)), (step, i)
+    assert dopt._native.staged == 3 * len(params)
+    dopt.close()
+    heap.close()
+
+
+def test_gradients_of_ordinary_layers_are_read_in_place(cuda_device):
+    torch.manual_seed(1)
+    net = torch.nn.Sequential(torch.nn.Conv2d(3, 8, 3), torch.nn.BatchNorm2d(8), torch.nn.Flatten(),
+                              torch.nn.Linear(8 * 36, 40), torch.nn.LayerNorm(40),
+                              torch.nn.Linear(40, 5, bias=False)).to(cuda_device)
+    heap, dopt = _optimizer(cuda_device, list(net.parameters()), torch.float32)
+    net(torch.randn(4, 3, 8, 8, device=cuda_device)).pow(2).sum().backward()
+    dopt.step()
+    assert dopt._native.staged == 0
+    dopt.close()
+    heap.close()
+
+
+def test_gradients_that_somebody_keeps_are_copied(cuda_device):
+    """... by a hook of the program, in a tensor that it hands over itself, or as a view."""
+    shape = (40, 50)
+    kept = []
+    params = [torch.nn.Parameter(torch.zeros(shape, device=cuda_device)) for _ in range(4)]
+    heap, dopt = _optimizer(cuda_device, params, torch.float32)
+    params[0].register_post_accumulate_grad_hook(lambda p: kept.append(p.grad))
+    params[1].grad = torch.zeros(shape, device=cuda_device)
+    kept.append(params[1].grad)
+    params[2].register_hook(lambda g: kept.append(g.view(-1)))
+    two = torch.full(shape, 2.0, device=cuda_device)
+    sum((p * two).sum() for p in params).backward()
+    for t in kept:
+        t.fill_(77.0)
+    dopt.step()
+    for p in params:
+        assert torch.all(p == -1.0)
+    assert 2 <= dopt._native.staged <= 3   # (autograd itself may copy what a tensor hook keeps)
+    dopt.close()
+    heap.close()

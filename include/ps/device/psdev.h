@@ -211,7 +211,8 @@ int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op
 
 /* One rank: several pieces of one table in as few launches as their number allows, the most
  * urgent (highest priority, ties in list order) first, each with the gradient in an array of its
- * own.  The list is host memory and is not referenced after the call. */
+ * own.  The ranges are disjoint (PSDEV_ERR_ARG otherwise).  The list is host memory and is not
+ * referenced after the call. */
 #define PSDEV_MAX_LOCAL_SEGS 64
 typedef struct {
   int64_t begin, end;  /* element range of the table, multiples of 8                       */

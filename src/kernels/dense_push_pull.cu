@@ -7,6 +7,7 @@
 
 #include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "ps/device/user_handle.cuh"
@@ -177,6 +178,21 @@ extern "C" int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t
                        nullptr, src, dst, n_valid);
 }
 
+// Whether no two ranges overlap: two CTAs would update the same values with no order between them.
+// (Gradients arrive in the reverse order of the parameters or close to it: few lists need sorting.)
+static bool disjoint(const std::vector<psdev_seg_t>& segs) {
+  bool down = true;
+  for (size_t i = 1; i < segs.size() && down; ++i) down = segs[i].end <= segs[i - 1].begin;
+  if (down) return true;
+  std::vector<std::pair<int64_t, int64_t>> r;
+  r.reserve(segs.size());
+  for (const psdev_seg_t& g : segs) r.emplace_back(g.begin, g.end);
+  std::sort(r.begin(), r.end());
+  for (size_t i = 1; i < r.size(); ++i)
+    if (r[i].first < r[i - 1].second) return false;
+  return true;
+}
+
 extern "C" int psdev_dense_op_segs(const psdev_world_t* w, const psdev_table_t* t, int op,
                                    const psdev_seg_t* segs, int nseg, const psdev_opt_t* opt,
                                    int channel, int num_ctas, void* stream) {
@@ -194,6 +210,7 @@ extern "C" int psdev_dense_op_segs(const psdev_world_t* w, const psdev_table_t* 
     if (g.end > g.begin) order.push_back(g);
   }
   if (order.empty()) return 0;
+  if (!disjoint(order)) return PSDEV_ERR_ARG;
   std::stable_sort(order.begin(), order.end(), [](const psdev_seg_t& a, const psdev_seg_t& b) {
     return a.priority > b.priority;
   });

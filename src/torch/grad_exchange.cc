@@ -27,6 +27,7 @@
 #include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <algorithm>
 #include <atomic>
 #include <deque>
 #include <mutex>
@@ -69,6 +70,7 @@ class GradExchange {
         slice_elems_(slice_elems),
         channel_(channel),
         begin_step_(std::move(begin_step)) {
+    sent_.assign(params_.size(), kNotSent);
     for (size_t i = 0; i < params_.size(); ++i) {
       auto node = torch::autograd::impl::grad_accumulator(params_[i]);
       TORCH_CHECK(node, "parameter ", i, " is no leaf that takes a gradient");
@@ -84,6 +86,7 @@ class GradExchange {
     hooks_.clear();
     std::lock_guard<std::mutex> lk(mu_);
     segs_.clear();
+    pending_ = 0;
     held_.clear();
     batches_.clear();
   }
@@ -108,6 +111,7 @@ class GradExchange {
     hook_stream_ = nullptr;
     other_stream_ = false;
     in_step_ = false;
+    std::fill(sent_.begin(), sent_.end(), kNotSent);
   }
 
   int64_t launches() const { return launches_; }
@@ -173,6 +177,17 @@ class GradExchange {
     }
   }
 
+  // Parameter `i` has a gradient once more before the step ends (two backward passes): an update of
+  // its own, after the one that the first gradient has made or will make.  Pieces of one launch
+  // must not share a range, and the gradient buffer may still be read by the launch before.
+  void Again(size_t i, const c10::cuda::CUDAStream& cur) {
+    if (sent_[i] == kPending) Drain(cur);
+    if (overlap_) {
+      fork_.record(comm_);
+      fork_.block(cur);
+    }
+  }
+
   void Take(size_t i, const variable_list& inputs) {
     at::Tensor& slot = params_[i].mutable_grad();
     if (!slot.defined()) return;
@@ -190,6 +205,7 @@ class GradExchange {
     seg.end = offsets_[i] + padded;
     seg.n_valid = offsets_[i] + n;
     seg.priority = priorities_[i];
+    if (sent_[i] != kNotSent) Again(i, cur);
     at::Tensor grad = std::move(slot);
     slot = at::Tensor();
     const auto dt = grad.scalar_type();
@@ -204,6 +220,7 @@ class GradExchange {
       Stage(i, grad, plain, cur);
     }
     segs_.push_back(seg);
+    sent_[i] = kPending;
     pending_ += padded;
     slices_ += (padded + slice_elems_ - 1) / slice_elems_;
     if (pending_ >= batch_elems_ && (pending_ >= 4 * batch_elems_ || Idle(cur))) Drain(cur);
@@ -245,6 +262,8 @@ class GradExchange {
     held_.clear();
     segs_.clear();
     pending_ = 0;
+    for (auto& state : sent_)
+      if (state == kPending) state = kLaunched;
   }
 
   void Retire() {
@@ -269,6 +288,9 @@ class GradExchange {
   int channel_;
   py::function begin_step_;
   std::vector<std::pair<std::shared_ptr<Node>, uintptr_t>> hooks_;
+
+  enum Sent : char { kNotSent, kPending, kLaunched };
+  std::vector<Sent> sent_;  // of each parameter in this step
 
   std::mutex mu_;
   std::atomic<bool> in_step_{false};

@@ -87,3 +87,49 @@ def test_gradients_that_somebody_keeps_are_copied(cuda_device):
     assert 2 <= dopt._native.staged <= 3   # (autograd itself may copy what a tensor hook keeps)
     dopt.close()
     heap.close()
+
+
+@pytest.mark.parametrize("kind", ["sgd", "momentum"])
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("batch_bytes", [1, 4096, 1 << 22])
+@pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
+def test_two_backward_passes_before_a_step(cuda_device, gdt, batch_bytes, overlap, kind):
+    """Every gradient is an update of its own, in the order of the passes: small and large tensors,
+    one of them with gradients that go through the table's buffer (channels_last)."""
+    shapes = [(3,), (1025,), (16, 8, 5, 3), (700_001,)]
+    params = [torch.nn.Parameter(torch.zeros(s, device=cuda_device)) for s in shapes]
+    want, speed = [0.0] * len(shapes), [0.0] * len(shapes)
+    heap, dopt = _optimizer(cuda_device, params, gdt, overlap, batch_bytes, kind)
+    for step in range(2):
+        for value in (2.0, 6.0, 2.0):
+            coef = [torch.full(s, value * (i + 1), device=cuda_device) for i, s in enumerate(shapes)]
+            coef[2] = coef[2].contiguous(memory_format=torch.channels_last)
+            sum((p * c).sum() for p, c in zip(params, coef)).backward()
+            for i in range(len(shapes)):
+                speed[i] = value * (i + 1) + (0.5 * speed[i] if kind == "momentum" else 0.0)
+                want[i] -= 0.5 * speed[i]
+        dopt.step()
+        for p, w in zip(params, want):
+            assert torch.all(p == w), (step, p.shape)   # halves and whole numbers: exact in fp32
+    dopt.close()
+    heap.close()
+
+
+def test_pieces_that_overlap_are_refused(cuda_device):
+    import ctypes as C
+
+    from ps_lite_b200 import _lib
+    from ps_lite_b200.parallel import DenseTable, ServerOptimizer, SymmetricHeap
+    heap = SymmetricHeap(1 << 20, 0, 1, device=cuda_device)
+    t = DenseTable(heap, 4096, optimizer=ServerOptimizer("sum"))
+    for ranges, ok in (([(0, 64), (64, 128), (256, 512)], True), ([(64, 128), (0, 72)], False),
+                       ([(512, 1024), (0, 64), (48, 56)], False), ([(8, 16), (8, 16)], False),
+                       ([(256, 512), (64, 64), (0, 256)], True)):
+        segs = (_lib.Seg * len(ranges))()
+        for s, (b, e) in zip(segs, ranges):
+            s.begin, s.end, s.n_valid = b, e, e
+        rc = _lib.device_lib().psdev_dense_op_segs(
+            C.byref(t._world), C.byref(t._table), _lib.OP_PUSHPULL, segs, len(ranges),
+            C.byref(t._opt_struct()), 0, 0, torch.cuda.current_stream().cuda_stream)
+        assert (rc == 0) == ok, (ranges, rc)
+    heap.close()

@@ -146,7 +146,9 @@ class DistributedOptimizer:
         self._opt = opt = _lib.Opt()
         me = weakref.ref(self)   # (the native object must not keep its owner alive)
 
-        def begin_step():
+        def refresh():
+            # the handle's parameters as they are at each launch: a program may change the rate
+            # between the backward pass and the step
             t.step = me().steps + 1
             C.memmove(C.byref(opt), C.byref(t._opt_struct()), C.sizeof(opt))
 
@@ -162,7 +164,7 @@ class DistributedOptimizer:
             self.params, self.offsets, pri, t.grad, C.addressof(t._world), C.addressof(t._table),
             C.addressof(self._opt), segs, cast, self.comm.cuda_stream if self.comm else 0,
             self.comm is not None, max(1, self.batch_bytes // self._gsz),
-            max(8, int(slice_elems) & ~7), channel, begin_step)
+            max(8, int(slice_elems) & ~7), channel, refresh)
 
     def _make_hook(self, index: int):
         n_params = len(self.params)

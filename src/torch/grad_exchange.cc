@@ -47,12 +47,12 @@ class GradExchange {
  public:
   // `world`, `table`, `opt`, `segs_fn`, `cast_fn`: addresses of the structures, of
   // psdev_dense_op_segs and of psdev_filter_cast;
-  // `begin_step` refreshes *opt and is called before the first gradient of every step.
+  // `refresh` brings *opt up to date and is called before every launch.
   GradExchange(std::vector<at::Tensor> params, std::vector<int64_t> offsets,
                std::vector<int64_t> priorities, at::Tensor grad_buffer, uint64_t world,
                uint64_t table, uint64_t opt, uint64_t segs_fn, uint64_t cast_fn,
                uint64_t comm_stream, bool overlap, int64_t batch_elems, int64_t slice_elems,
-               int channel, py::function begin_step)
+               int channel, py::function refresh)
       : params_(std::move(params)),
         offsets_(std::move(offsets)),
         priorities_(std::move(priorities)),
@@ -69,7 +69,7 @@ class GradExchange {
         batch_elems_(batch_elems),
         slice_elems_(slice_elems),
         channel_(channel),
-        begin_step_(std::move(begin_step)) {
+        refresh_(std::move(refresh)) {
     sent_.assign(params_.size(), kNotSent);
     for (size_t i = 0; i < params_.size(); ++i) {
       auto node = torch::autograd::impl::grad_accumulator(params_[i]);
@@ -79,7 +79,10 @@ class GradExchange {
     }
   }
 
-  ~GradExchange() { Detach(); }
+  ~GradExchange() {
+    py::gil_scoped_release no_gil;
+    Detach();
+  }
 
   void Detach() {
     for (auto& h : hooks_) h.first->del_post_hook(h.second);
@@ -93,9 +96,9 @@ class GradExchange {
 
   // End of a step: everything pending goes out, and the caller's stream waits for it.
   void Step() {
-    std::lock_guard<std::mutex> lk(mu_);
+    std::unique_lock<std::mutex> lk(mu_);
     const auto cur = at::cuda::getCurrentCUDAStream(device_);
-    Drain(cur);
+    Drain(cur, lk);
     if (overlap_) {
       fork_.record(comm_);
       fork_.block(cur);
@@ -110,7 +113,6 @@ class GradExchange {
     while (!batches_.empty()) Retire();
     hook_stream_ = nullptr;
     other_stream_ = false;
-    in_step_ = false;
     std::fill(sent_.begin(), sent_.end(), kNotSent);
   }
 
@@ -180,8 +182,8 @@ class GradExchange {
   // Parameter `i` has a gradient once more before the step ends (two backward passes): an update of
   // its own, after the one that the first gradient has made or will make.  Pieces of one launch
   // must not share a range, and the gradient buffer may still be read by the launch before.
-  void Again(size_t i, const c10::cuda::CUDAStream& cur) {
-    if (sent_[i] == kPending) Drain(cur);
+  void Again(size_t i, const c10::cuda::CUDAStream& cur, std::unique_lock<std::mutex>& lk) {
+    if (sent_[i] == kPending) Drain(cur, lk);
     if (overlap_) {
       fork_.record(comm_);
       fork_.block(cur);
@@ -191,11 +193,7 @@ class GradExchange {
   void Take(size_t i, const variable_list& inputs) {
     at::Tensor& slot = params_[i].mutable_grad();
     if (!slot.defined()) return;
-    if (!in_step_.exchange(true)) {
-      py::gil_scoped_acquire gil;
-      begin_step_();
-    }
-    std::lock_guard<std::mutex> lk(mu_);
+    std::unique_lock<std::mutex> lk(mu_);
     const auto cur = at::cuda::getCurrentCUDAStream(device_);
     if (!hook_stream_) hook_stream_ = cur.stream();
     else if (hook_stream_ != cur.stream()) other_stream_ = true;
@@ -205,7 +203,7 @@ class GradExchange {
     seg.end = offsets_[i] + padded;
     seg.n_valid = offsets_[i] + n;
     seg.priority = priorities_[i];
-    if (sent_[i] != kNotSent) Again(i, cur);
+    if (sent_[i] != kNotSent) Again(i, cur, lk);
     at::Tensor grad = std::move(slot);
     slot = at::Tensor();
     const auto dt = grad.scalar_type();
@@ -223,7 +221,7 @@ class GradExchange {
     sent_[i] = kPending;
     pending_ += padded;
     slices_ += (padded + slice_elems_ - 1) / slice_elems_;
-    if (pending_ >= batch_elems_ && (pending_ >= 4 * batch_elems_ || Idle(cur))) Drain(cur);
+    if (pending_ >= batch_elems_ && (pending_ >= 4 * batch_elems_ || Idle(cur))) Drain(cur, lk);
   }
 
   // Nothing launched earlier is still running.  While something is, what is pending would only
@@ -238,8 +236,17 @@ class GradExchange {
     return batches_.empty();
   }
 
-  void Drain(const c10::cuda::CUDAStream& cur) {
+  // `lk` holds mu_.  It is given up while Python runs: a thread that has the interpreter lock may be
+  // waiting for mu_.
+  void Drain(const c10::cuda::CUDAStream& cur, std::unique_lock<std::mutex>& lk) {
     if (segs_.empty()) return;
+    lk.unlock();
+    {
+      py::gil_scoped_acquire gil;
+      refresh_();
+    }
+    lk.lock();
+    if (segs_.empty()) return;  // another thread has sent them
     const auto& stream = overlap_ ? comm_ : cur;
     if (overlap_) {
       fork_.record(cur);
@@ -286,14 +293,13 @@ class GradExchange {
   c10::cuda::CUDAStream comm_;
   int64_t batch_elems_, slice_elems_;
   int channel_;
-  py::function begin_step_;
+  py::function refresh_;
   std::vector<std::pair<std::shared_ptr<Node>, uintptr_t>> hooks_;
 
   enum Sent : char { kNotSent, kPending, kLaunched };
   std::vector<Sent> sent_;  // of each parameter in this step
 
   std::mutex mu_;
-  std::atomic<bool> in_step_{false};
   std::vector<psdev_seg_t> segs_;
   std::vector<at::Tensor> held_;  // gradients of segs_
   std::deque<Batch> batches_;     // launched, not known to be finished

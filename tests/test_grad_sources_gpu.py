@@ -133,3 +133,44 @@ def test_pieces_that_overlap_are_refused(cuda_device):
             C.byref(t._opt_struct()), 0, 0, torch.cuda.current_stream().cuda_stream)
         assert (rc == 0) == ok, (ranges, rc)
     heap.close()
+
+
+@pytest.mark.parametrize("batch_bytes", [0, 1, 1 << 16, 1 << 22])   # 0: the hooks in Python
+def test_rate_changed_between_backward_and_step(cuda_device, batch_bytes):
+    """What is still pending goes out with the parameters of the moment: all of a model smaller than
+    a batch, or what follows the last launch of a larger one."""
+    params = [torch.nn.Parameter(torch.zeros(s, device=cuda_device)) for s in ((8,), (30_000,), (9,))]
+    heap, dopt = _optimizer(cuda_device, params, torch.float32, True, batch_bytes)
+    for step in range(2):
+        dopt.table.optimizer.lr = 0.5
+        before = [p.detach().clone() for p in params]
+        sum((p * torch.ones_like(p)).sum() for p in params).backward()
+        dopt.table.optimizer.lr = 0.25
+        dopt.step()
+        moved = [b - p.detach() for b, p in zip(before, params)]
+        for m in moved:
+            assert torch.all(m == m.flatten()[0]) and m.flatten()[0].item() in (0.5, 0.25)
+        if batch_bytes == 1 << 22:
+            assert all(m.flatten()[0].item() == 0.25 for m in moved)
+        if batch_bytes == 1 << 16:
+            # the large tensor fills a batch, whichever comes first; a small one stays behind it
+            assert 0.25 in [m.flatten()[0].item() for m in moved]
+    dopt.close()
+    heap.close()
+
+
+def test_an_error_while_the_parameters_are_read_ends_the_pass(cuda_device):
+    """... and the next pass reads them again instead of going on with the old ones."""
+    p = torch.nn.Parameter(torch.zeros(64, device=cuda_device))
+    heap, dopt = _optimizer(cuda_device, [p], torch.float32, True, 1)
+    good = dopt.table.optimizer
+    dopt.table.optimizer = None
+    with pytest.raises(Exception):
+        (p * torch.ones_like(p)).sum().backward()
+        dopt.step()
+    dopt.table.optimizer = good
+    good.lr = 0.125
+    dopt.step()
+    assert torch.all(p == -0.125)
+    dopt.close()
+    heap.close()

@@ -31,6 +31,7 @@
 #include <atomic>
 #include <deque>
 #include <mutex>
+#include <optional>
 #include <vector>
 
 #include "ps/device/psdev.h"
@@ -97,21 +98,21 @@ class GradExchange {
   // End of a step: everything pending goes out, and the caller's stream waits for it.
   void Step() {
     std::unique_lock<std::mutex> lk(mu_);
+    Drain(lk);
     const auto cur = at::cuda::getCurrentCUDAStream(device_);
-    Drain(cur, lk);
+    if (launched_on_) After(*launched_on_, cur);
     if (overlap_) {
-      fork_.record(comm_);
-      fork_.block(cur);
       // Memory given back from here on is reused on the stream the gradients were made on; that
       // is `cur`, which now comes after the kernels, or the allocator is told.
-      if (other_stream_ || hook_stream_ != cur.stream()) {
+      if (other_stream_ || (hook_stream_ && *hook_stream_ != cur)) {
         for (auto& b : batches_)
           for (auto& t : b.tensors)
             c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), comm_);
       }
     }
     while (!batches_.empty()) Retire();
-    hook_stream_ = nullptr;
+    hook_stream_.reset();
+    launched_on_.reset();
     other_stream_ = false;
     std::fill(sent_.begin(), sent_.end(), kNotSent);
   }
@@ -183,11 +184,15 @@ class GradExchange {
   // its own, after the one that the first gradient has made or will make.  Pieces of one launch
   // must not share a range, and the gradient buffer may still be read by the launch before.
   void Again(size_t i, const c10::cuda::CUDAStream& cur, std::unique_lock<std::mutex>& lk) {
-    if (sent_[i] == kPending) Drain(cur, lk);
-    if (overlap_) {
-      fork_.record(comm_);
-      fork_.block(cur);
-    }
+    if (sent_[i] == kPending) Drain(lk);
+    if (launched_on_) After(*launched_on_, cur);
+  }
+
+  // Orders work on `next` behind what has been issued on `before`.
+  void After(const c10::cuda::CUDAStream& before, const c10::cuda::CUDAStream& next) {
+    if (before == next) return;
+    fork_.record(before);
+    fork_.block(next);
   }
 
   void Take(size_t i, const variable_list& inputs) {
@@ -195,8 +200,10 @@ class GradExchange {
     if (!slot.defined()) return;
     std::unique_lock<std::mutex> lk(mu_);
     const auto cur = at::cuda::getCurrentCUDAStream(device_);
-    if (!hook_stream_) hook_stream_ = cur.stream();
-    else if (hook_stream_ != cur.stream()) other_stream_ = true;
+    // (a launch comes behind the stream of its pieces: what another stream has made goes out first)
+    if (!segs_.empty() && *pending_on_ != cur) Drain(lk);
+    if (!hook_stream_) hook_stream_ = cur;
+    else if (*hook_stream_ != cur) other_stream_ = true;
     const int64_t n = params_[i].numel(), padded = (n + 7) & ~int64_t(7);
     psdev_seg_t seg{};
     seg.begin = offsets_[i];
@@ -218,10 +225,11 @@ class GradExchange {
       Stage(i, grad, plain, cur);
     }
     segs_.push_back(seg);
+    pending_on_ = cur;
     sent_[i] = kPending;
     pending_ += padded;
     slices_ += (padded + slice_elems_ - 1) / slice_elems_;
-    if (pending_ >= batch_elems_ && (pending_ >= 4 * batch_elems_ || Idle(cur))) Drain(cur, lk);
+    if (pending_ >= batch_elems_ && (pending_ >= 4 * batch_elems_ || Idle(cur))) Drain(lk);
   }
 
   // Nothing launched earlier is still running.  While something is, what is pending would only
@@ -236,9 +244,9 @@ class GradExchange {
     return batches_.empty();
   }
 
-  // `lk` holds mu_.  It is given up while Python runs: a thread that has the interpreter lock may be
-  // waiting for mu_.
-  void Drain(const c10::cuda::CUDAStream& cur, std::unique_lock<std::mutex>& lk) {
+  // Sends what is pending, behind the stream of its hooks.  `lk` holds mu_; it is given up while
+  // Python runs, since a thread that has the interpreter lock may be waiting for mu_.
+  void Drain(std::unique_lock<std::mutex>& lk) {
     if (segs_.empty()) return;
     lk.unlock();
     {
@@ -247,11 +255,11 @@ class GradExchange {
     }
     lk.lock();
     if (segs_.empty()) return;  // another thread has sent them
-    const auto& stream = overlap_ ? comm_ : cur;
-    if (overlap_) {
-      fork_.record(cur);
-      fork_.block(comm_);
-    }
+    const auto made_on = *pending_on_;
+    const auto stream = overlap_ ? comm_ : made_on;
+    After(made_on, stream);
+    if (launched_on_) After(*launched_on_, stream);
+    launched_on_ = stream;
     const int rc = segs_fn_(world_, table_, PSDEV_OP_PUSHPULL, segs_.data(),
                             static_cast<int>(segs_.size()), opt_, channel_, 0, stream.stream());
     TORCH_CHECK(rc == 0, "psdev_dense_op_segs failed with ", rc);
@@ -305,8 +313,10 @@ class GradExchange {
   std::deque<Batch> batches_;     // launched, not known to be finished
   std::vector<Batch> spare_;
   at::cuda::CUDAEvent fork_;
-  cudaStream_t hook_stream_ = nullptr;
-  bool other_stream_ = false;
+  std::optional<c10::cuda::CUDAStream> pending_on_;   // hooks of what is pending ran here
+  std::optional<c10::cuda::CUDAStream> launched_on_;  // launches of this step
+  std::optional<c10::cuda::CUDAStream> hook_stream_;  // first hook of this step
+  bool other_stream_ = false;                         // a later one ran elsewhere
   int64_t pending_ = 0;
   std::atomic<int64_t> launches_{0}, slices_{0}, staged_{0};
 };

@@ -174,3 +174,42 @@ def test_an_error_while_the_parameters_are_read_ends_the_pass(cuda_device):
     assert torch.all(p == -0.125)
     dopt.close()
     heap.close()
+
+
+@pytest.mark.parametrize("step_on_side", [False, True])
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("batch_bytes", [1, 1 << 22])
+def test_hooks_on_two_streams(cuda_device, batch_bytes, overlap, step_on_side):
+    """Gradients accumulate on the stream that was current when the parameter first took part in a
+    graph: here the default one and another in turn."""
+    shapes = [(65,), (300_007,), (4096,), (90_000,), (3,)]
+    params = [torch.nn.Parameter(torch.zeros(s, device=cuda_device)) for s in shapes]
+    side = torch.cuda.Stream(cuda_device)
+    with torch.cuda.stream(side):
+        nodes = [p.view_as(p).grad_fn.next_functions[0][0] for p in params[1::2]]
+    heap, dopt = _optimizer(cuda_device, params, torch.float32, overlap, batch_bytes)
+    assert len(nodes) == 2
+    where = []
+    for p in params:
+        p.register_post_accumulate_grad_hook(
+            lambda q: where.append(torch.cuda.current_stream(cuda_device) == side))
+    ws = torch.zeros(max(p.numel() for p in params), device=cuda_device)
+    for step in range(4):
+        for value in (2.0, 4.0):
+            x = torch.ones(1, device=cuda_device, requires_grad=True)
+            for i, p in enumerate(params):
+                x = _FromWorkspace.apply(x, p, value * (i + 1), ws) if i == 0 else x
+            (x.sum() + sum((p * torch.full_like(p, value * (i + 1))).sum()
+                           for i, p in enumerate(params) if i)).backward()
+        if step_on_side:
+            side.wait_stream(torch.cuda.current_stream(cuda_device))
+            with torch.cuda.stream(side):
+                dopt.step()
+            torch.cuda.current_stream(cuda_device).wait_stream(side)
+        else:
+            dopt.step()
+        for i, p in enumerate(params):
+            assert torch.all(p == -3.0 * (step + 1) * (i + 1)), (step, i)
+    assert any(where) and not all(where)
+    dopt.close()
+    heap.close()

@@ -158,6 +158,11 @@ class DistributedOptimizer:
         # store into this rank's weight buffer)
         pri = [-1 - i if self._publish[i] else len(self.params) - i
                for i in range(len(self.params))]
+        # torch drops the native hooks of a tensor when the first hook in Python arrives; once it
+        # has had one, later ones are added beside them
+        for p in self.params:
+            if p._backward_hooks is None:
+                p.register_hook(lambda g: None).remove()
         # `num_ctas` bounds the CTAs that wait for peers while a backward pass needs the SMs; with
         # one rank the update is a pass over memory, shortest on the whole GPU
         return _lib.torch_ext().GradExchange(

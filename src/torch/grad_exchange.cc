@@ -15,7 +15,10 @@
 // table's gradient buffer on the stream that made it, by the hook.
 //
 // The hooks sit on the parameters' gradient accumulators, next to hooks that a program registers
-// on the parameters themselves, and run after those.  A gradient stays alive until the kernel
+// on the parameters themselves, and run after those.  An accumulator belongs to the stream that was
+// current when it was made and lives as long as the graphs that use it, so it is not held here: a
+// tensor hook, which the parameter keeps, puts the hook on each new accumulator.  (Held ones would
+// keep accumulation on the stream of the constructor, out of reach of a graph capture.)  A gradient stays alive until the kernel
 // that reads it has finished: batches are kept with an event and dropped when it has fired, the
 // rest when the step ends and the caller's stream has been ordered behind the kernels.
 #include <ATen/ATen.h>
@@ -72,11 +75,11 @@ class GradExchange {
         channel_(channel),
         refresh_(std::move(refresh)) {
     sent_.assign(params_.size(), kNotSent);
+    hooks_.resize(params_.size());
     for (size_t i = 0; i < params_.size(); ++i) {
-      auto node = torch::autograd::impl::grad_accumulator(params_[i]);
-      TORCH_CHECK(node, "parameter ", i, " is no leaf that takes a gradient");
-      const uintptr_t key = node->add_post_hook(std::make_unique<Hook>(this, i));
-      hooks_.push_back({std::move(node), key});
+      TORCH_CHECK(params_[i].is_leaf() && params_[i].requires_grad(), "parameter ", i,
+                  " is no leaf that takes a gradient");
+      hooks_[i].tensor_hook = params_[i].register_hook([this, i](const at::Tensor&) { Attach(i); });
     }
   }
 
@@ -86,7 +89,10 @@ class GradExchange {
   }
 
   void Detach() {
-    for (auto& h : hooks_) h.first->del_post_hook(h.second);
+    for (size_t i = 0; i < hooks_.size(); ++i) {
+      params_[i].remove_hook(hooks_[i].tensor_hook);
+      if (auto node = hooks_[i].node.lock()) node->del_post_hook(hooks_[i].key);
+    }
     hooks_.clear();
     std::lock_guard<std::mutex> lk(mu_);
     segs_.clear();
@@ -131,6 +137,14 @@ class GradExchange {
     GradExchange* owner;
     size_t index;
   };
+  // Before a gradient is accumulated: the accumulator has the hook.
+  void Attach(size_t i) {
+    const auto node = torch::autograd::impl::try_get_grad_accumulator(params_[i]);
+    if (!node || i >= hooks_.size() || hooks_[i].node.lock() == node) return;
+    hooks_[i].key = node->add_post_hook(std::make_unique<Hook>(this, i));
+    hooks_[i].node = node;
+  }
+
   struct Batch {
     at::cuda::CUDAEvent read;  // the kernels that read the tensors have finished
     std::vector<at::Tensor> tensors;
@@ -302,7 +316,12 @@ class GradExchange {
   int64_t batch_elems_, slice_elems_;
   int channel_;
   py::function refresh_;
-  std::vector<std::pair<std::shared_ptr<Node>, uintptr_t>> hooks_;
+  struct Attached {
+    unsigned tensor_hook = 0;
+    std::weak_ptr<Node> node;  // the accumulator that has the hook, and the hook's key there
+    uintptr_t key = 0;
+  };
+  std::vector<Attached> hooks_;
 
   enum Sent : char { kNotSent, kPending, kLaunched };
   std::vector<Sent> sent_;  // of each parameter in this step

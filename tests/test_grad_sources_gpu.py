@@ -213,3 +213,54 @@ def test_hooks_on_two_streams(cuda_device, batch_bytes, overlap, step_on_side):
     assert any(where) and not all(where)
     dopt.close()
     heap.close()
+
+
+def test_accumulation_stays_on_the_stream_of_the_forward_pass(cuda_device):
+    params = [torch.nn.Parameter(torch.zeros(40, device=cuda_device)) for _ in range(2)]
+    heap, dopt = _optimizer(cuda_device, params, torch.float32)
+    side, where = torch.cuda.Stream(cuda_device), []
+    params[0].register_post_accumulate_grad_hook(
+        lambda p: where.append(torch.cuda.current_stream(cuda_device) == side))
+    for step in range(4):
+        side.wait_stream(torch.cuda.current_stream(cuda_device))
+        with torch.cuda.stream(side if step % 2 else torch.cuda.current_stream(cuda_device)):
+            sum((p * torch.ones_like(p)).sum() for p in params).backward()
+            dopt.step()
+        torch.cuda.current_stream(cuda_device).wait_stream(side)
+    assert where == [False, True, False, True]
+    assert all(torch.all(p == -2.0) for p in params)
+    dopt.close()
+    heap.close()
+
+
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("batch_bytes", [1, 1 << 22])
+def test_a_captured_step(cuda_device, batch_bytes, overlap):
+    """Forward, backward and update in a CUDA graph, by an optimizer made outside of it."""
+    params = [torch.nn.Parameter(torch.zeros(s, device=cuda_device)) for s in ((300, 40), (7,), (90_001,))]
+    heap, dopt = _optimizer(cuda_device, params, torch.float32, overlap, batch_bytes)
+    coef = [torch.ones_like(p) for p in params]
+    ws = torch.zeros(7, device=cuda_device)
+
+    def step():
+        x = _FromWorkspace.apply(torch.ones(1, device=cuda_device, requires_grad=True), params[1], 1.0, ws)
+        (x.sum() + (params[0] * coef[0]).sum() + (params[2] * coef[2]).sum()).backward()
+        dopt.step()
+
+    side = torch.cuda.Stream(cuda_device)
+    side.wait_stream(torch.cuda.current_stream(cuda_device))
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            step()
+    torch.cuda.current_stream(cuda_device).wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for n in range(3, 8):
+        graph.replay()
+        assert all(torch.all(p == -0.5 * n) for p in params), n
+    step()
+    assert all(torch.all(p == -4.0) for p in params)
+    del graph
+    dopt.close()
+    heap.close()

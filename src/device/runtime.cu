@@ -5,6 +5,7 @@
 // binds this library at run time and reaches streams, events, copies and allocations through
 // the functions below, next to the psdev_* kernels.  Every function returns 0 or a
 // cudaError_t value.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "ps/device/psdev.h"
@@ -76,18 +77,34 @@ int psdev_rt_is_pinned_host(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 // 1 if all of [p, p + bytes) is page-locked host memory that kernels can access; *dev receives
-// its address on the device.
+// its address on the device.  The range must lie in one allocation or registration: the ends of
+// two of them say nothing about what lies between (all addresses have the same distance on host and
+// device), and the driver is asked for the bounds of the one that `p` belongs to.
 int psdev_rt_host_mapped(const void* p, size_t bytes, void** dev) {
-  cudaPointerAttributes a, b;
-  if (bytes == 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&b, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
+  cudaPointerAttributes a;
+  if (bytes == 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer ||
-      static_cast<char*>(b.devicePointer) - static_cast<char*>(a.devicePointer) !=
-          static_cast<ptrdiff_t>(bytes - 1))
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return 0;
+  static const auto attribute = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found) !=
+            cudaSuccess || found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<CUresult (*)(void*, CUpointer_attribute, CUdeviceptr)>(f);
+  }();
+  if (!attribute) return 0;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(a.devicePointer);
+  if (attribute(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+      attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
     return 0;
+  if (at < start || at - start > size || bytes > size - (at - start)) return 0;
   *dev = a.devicePointer;
   return 1;
 }

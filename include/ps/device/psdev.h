@@ -374,6 +374,7 @@ int psdev_rt_event_destroy(void* event);
 int psdev_rt_event_record(void* event, void* stream);
 int psdev_rt_event_sync(void* event);
 int psdev_rt_stream_wait_event(void* stream, void* event);
+int psdev_rt_stream_id(void* stream, unsigned long long* id);
 int psdev_rt_memcpy_async(void* dst, const void* src, size_t bytes, void* stream);
 int psdev_rt_is_device_pointer(const void* p);
 int psdev_rt_is_pinned_host(const void* p);

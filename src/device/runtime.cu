@@ -36,6 +36,12 @@ int psdev_rt_stream_create(void** stream, int priority) {
   return (int)e;
 }
 int psdev_rt_stream_destroy(void* stream) { return (int)cudaStreamDestroy((cudaStream_t)stream); }
+// An id that no other stream of the process has or will have.  Handles do not tell streams apart:
+// the per-thread default stream has one handle in all threads, and the handle of a destroyed stream
+// can come back.
+int psdev_rt_stream_id(void* stream, unsigned long long* id) {
+  return (int)cudaStreamGetId((cudaStream_t)stream, id);
+}
 int psdev_rt_stream_sync(void* stream) { return (int)cudaStreamSynchronize((cudaStream_t)stream); }
 
 int psdev_rt_event_create(void** event) {

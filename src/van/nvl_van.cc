@@ -52,6 +52,7 @@ struct Rt {
   int (*stream_create)(void**, int) = nullptr;
   int (*stream_destroy)(void*) = nullptr;
   int (*stream_sync)(void*) = nullptr;
+  int (*stream_id)(void*, unsigned long long*) = nullptr;
   int (*event_create)(void**) = nullptr;
   int (*event_destroy)(void*) = nullptr;
   int (*event_record)(void*, void*) = nullptr;
@@ -132,6 +133,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_rt_stream_create", &rt->stream_create);
   Bind(lib, "psdev_rt_stream_destroy", &rt->stream_destroy);
   Bind(lib, "psdev_rt_stream_sync", &rt->stream_sync);
+  Bind(lib, "psdev_rt_stream_id", &rt->stream_id);
   Bind(lib, "psdev_rt_event_create", &rt->event_create);
   Bind(lib, "psdev_rt_event_destroy", &rt->event_destroy);
   Bind(lib, "psdev_rt_event_record", &rt->event_record);
@@ -514,10 +516,10 @@ struct Plane::Impl {
   std::vector<void*> event_pool;
   std::mutex ev_mu;
   // requests on one tensor are serialised against each other: the last event of the previous
-  // one and the stream it was recorded on (keyed by DenseInfo*)
+  // one and the id of the stream it was recorded on (keyed by DenseInfo*)
   struct Done {
     void* event = nullptr;
-    void* stream = nullptr;
+    unsigned long long stream = 0;
   };
   std::map<const void*, Done> last_done;
   Done LastDone(const void* tensor) {
@@ -525,9 +527,16 @@ struct Plane::Impl {
     auto it = last_done.find(tensor);
     return it == last_done.end() ? Done() : it->second;
   }
-  // Orders work on `s` after the previous request on the tensor.
+  // 0 when the id cannot be had (and for the CPU stand-in): such streams are never taken for one.
+  unsigned long long StreamId(void* s) const {
+    unsigned long long id = 0;
+    return rt.stream_id && rt.stream_id(s, &id) == 0 ? id : 0;
+  }
+  // Orders work on `s` after the previous request on the tensor, unless that was on this stream too
+  // (by its id: the handles of different streams can be equal, see psdev_rt_stream_id).
   void After(const Done& prev, void* s) {
-    if (prev.event && prev.stream != s) rt.stream_wait_event(s, prev.event);
+    if (prev.event && (prev.stream == 0 || prev.stream != StreamId(s)))
+      rt.stream_wait_event(s, prev.event);
   }
 
   struct Pending {
@@ -1548,10 +1557,11 @@ void Plane::Submit(DeviceRequest&& req) {
     if (tls_has_stream) m.rt.stream_wait_event(origin, done);
   }
   pend.event = done;
+  const Impl::Done point{done, m.StreamId(done_stream)};
   {
     std::lock_guard<std::mutex> lk(m.mu);
     // `done` doubles as the ordering point for the next request on this tensor
-    m.last_done[d] = Impl::Done{done, done_stream};
+    m.last_done[d] = point;
   }
   m.Enqueue(std::move(pend));
 }
@@ -1676,9 +1686,10 @@ void Plane::FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* s) {
   pend.customer = req.customer;
   pend.on_done = std::move(req.on_done);
   pend.tensor = sp;
+  const Impl::Done point{done, m.StreamId(s)};
   {
     std::lock_guard<std::mutex> lk(m.mu);
-    m.last_done[sp] = Impl::Done{done, s};
+    m.last_done[sp] = point;
   }
   m.Enqueue(std::move(pend));
 }

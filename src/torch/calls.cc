@@ -59,12 +59,14 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   bool ok = is_bf16(a[1]) && is_bf16(a[2]) && (a[3] == Py_None || THPVariable_Check(a[3]));
   if (ok) {
     const at::Tensor &x = THPVariable_Unpack(a[1]), &w = THPVariable_Unpack(a[2]);
-    ok = x.is_cuda() && x.is_contiguous() && w.is_contiguous() && x.dim() > 0 && w.dim() > 0 &&
-         x.size(-1) == w.size(-1);
+    ok = x.is_cuda() && w.is_cuda() && x.is_contiguous() && w.is_contiguous() && x.dim() > 0 &&
+         w.dim() > 0 && x.size(-1) == w.size(-1) &&
+         (a[3] == Py_None || THPVariable_Unpack(a[3]).is_cuda());
   }
   if (!ok) {
     PyErr_SetString(PyExc_AssertionError,
-                    "x and w must be contiguous bf16 tensors on the device whose last sizes agree");
+                    "x and w must be contiguous bf16 tensors on the device whose last sizes agree, "
+                    "and the output must be on the device");
     return nullptr;
   }
   const at::Tensor &x = THPVariable_Unpack(a[1]), &w = THPVariable_Unpack(a[2]);
@@ -88,8 +90,11 @@ PyObject* pull_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 10) return PyErr_Format(PyExc_TypeError, "pull_linear takes 10 arguments");
   HANDLE_TH_ERRORS
   if (!is_bf16(a[5]) || !THPVariable_Unpack(a[5]).is_contiguous() ||
-      THPVariable_Unpack(a[5]).dim() == 0 || (a[6] != Py_None && !THPVariable_Check(a[6]))) {
-    PyErr_SetString(PyExc_AssertionError, "x must be a contiguous bf16 tensor");
+      THPVariable_Unpack(a[5]).dim() == 0 || !THPVariable_Unpack(a[5]).is_cuda() ||
+      (a[6] != Py_None &&
+       !(THPVariable_Check(a[6]) && THPVariable_Unpack(a[6]).is_cuda()))) {
+    PyErr_SetString(PyExc_AssertionError,
+                    "x must be a contiguous bf16 tensor on the device, like the output");
     return nullptr;
   }
   const at::Tensor& x = THPVariable_Unpack(a[5]);

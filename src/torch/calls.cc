@@ -35,11 +35,8 @@ cudaStream_t stream_on(c10::DeviceIndex device) {
 // A launch may wait for room in the stream: other Python threads run meanwhile.
 template <typename F>
 int without_gil(F&& f) {
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = f();
-  Py_END_ALLOW_THREADS
-  return rc;
+  py::gil_scoped_release no_gil;  // (taken back on the way of an exception as well)
+  return f();
 }
 bool is_bf16(PyObject* o) {
   return THPVariable_Check(o) && THPVariable_Unpack(o).scalar_type() == at::kBFloat16;
@@ -164,6 +161,7 @@ PyObject* unique_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // dense_op(fn, world, table, op, begin, end, opt, channel, num_ctas, timeout_ns, sync, stream)
 PyObject* dense_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 12) return PyErr_Format(PyExc_TypeError, "dense_op takes 12 arguments");
+  HANDLE_TH_ERRORS
   const auto fn = address<DenseFn>(a[0]);
   const auto* world = address<const psdev_world_t*>(a[1]);
   const auto* table = address<const psdev_table_t*>(a[2]);
@@ -179,6 +177,7 @@ PyObject* dense_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return fn(world, table, static_cast<int>(op), begin, end, opt, static_cast<int>(channel),
               static_cast<int>(ctas), timeout, static_cast<int>(sync), stream);
   }));
+  END_HANDLE_TH_ERRORS
 }
 
 // A keyed table of one rank.

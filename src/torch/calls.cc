@@ -25,6 +25,7 @@ using UniqueSortFn = int (*)(const uint64_t*, const float*, int64_t, int, void*,
                              void*);
 using UniqueWriteFn = int (*)(const void*, int64_t, int, int64_t, uint64_t*, float*, void*);
 
+// (time limits wrap like a C integer: a negative one is a very long one)
 template <typename T>
 T address(PyObject* o) {
   return reinterpret_cast<T>(PyLong_AsUnsignedLongLong(o));
@@ -70,7 +71,7 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t K = x.size(-1), M = K ? x.numel() / K : 0, N = w.size(0);
   at::Tensor out = output_for(a[3], x, N);
   const long ctas = PyLong_AsLong(a[4]);
-  const uint64_t timeout = PyLong_AsUnsignedLongLong(a[5]);
+  const uint64_t timeout = PyLong_AsUnsignedLongLongMask(a[5]);
   const auto fn = address<GemmFn>(a[0]);
   if (PyErr_Occurred()) return nullptr;
   const int rc = without_gil([&] {
@@ -98,7 +99,7 @@ PyObject* pull_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t K = x.size(-1), M = K ? x.numel() / K : 0, N = PyLong_AsLongLong(a[4]);
   const int64_t off = PyLong_AsLongLong(a[3]);
   const long copy = PyLong_AsLong(a[7]), ctas = PyLong_AsLong(a[8]);
-  const uint64_t timeout = PyLong_AsUnsignedLongLong(a[9]);
+  const uint64_t timeout = PyLong_AsUnsignedLongLongMask(a[9]);
   const auto fn = address<PullGemmFn>(a[0]);
   const auto* world = address<const psdev_world_t*>(a[1]);
   const auto* table = address<const psdev_table_t*>(a[2]);
@@ -169,7 +170,7 @@ PyObject* dense_op(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t begin = PyLong_AsLongLong(a[4]), end = PyLong_AsLongLong(a[5]);
   const auto* opt = address<const psdev_opt_t*>(a[6]);
   const long channel = PyLong_AsLong(a[7]), ctas = PyLong_AsLong(a[8]);
-  const uint64_t timeout = PyLong_AsUnsignedLongLong(a[9]);
+  const uint64_t timeout = PyLong_AsUnsignedLongLongMask(a[9]);
   const long sync = PyLong_AsLong(a[10]);
   void* stream = address<void*>(a[11]);
   if (PyErr_Occurred()) return nullptr;

@@ -73,6 +73,16 @@ int psdev_rt_is_device_pointer(const void* p) {
   }
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
+// What `p` points at: 0 host memory (pinned or pageable), 1 memory of the GPU *device, 2 managed.
+int psdev_rt_memory(const void* p, int* device) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  *device = a.device;
+  return a.type == cudaMemoryTypeManaged ? 2 : a.type == cudaMemoryTypeDevice;
+}
 // 1 if `p` is page-locked host memory that the device can copy from without staging.
 int psdev_rt_is_pinned_host(const void* p) {
   cudaPointerAttributes a;

@@ -9,6 +9,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include "ps/device/psdev.h"
+
 namespace {
 
 using RequestFn = int (*)(void*, void*, int, int, const uint64_t*, size_t, const void*, size_t,
@@ -148,11 +150,13 @@ PyObject* keyed_request(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int* lp = vals && lens ? static_cast<const int*>(lens->data_ptr()) : nullptr;
   int* lo = out && !vals && lens_out ? static_cast<int*>(lens_out->data_ptr()) : nullptr;
   const size_t vb = vals ? vals->numel() * 4 : 0, ob = out ? out->numel() * 4 : 0;
+  auto here = [&](const at::Tensor* x) { return !x || x->get_device() == t->device; };
+  const bool all = here(keys) && here(vals) && here(out) && here(lens) && here(lens_out);
   int ts;
   Py_BEGIN_ALLOW_THREADS
   ts = t->request(t->worker, stream, vals != nullptr, out != nullptr,
                   static_cast<const uint64_t*>(kp), static_cast<size_t>(n), vp, vb, op, ob, lp, lo,
-                  0);
+                  all ? PSDEV_CMD_ARRAYS_HERE : 0);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(ts);
   END_HANDLE_TH_ERRORS

@@ -73,7 +73,7 @@ struct Rt {
   int (*lens_to_offsets)(const int32_t*, int64_t, int64_t*, void*) = nullptr;
   int (*device_barrier)(const psdev_world_t*, int, uint64_t, void*) = nullptr;
   int (*multicast_pays)(int, uint64_t) = nullptr;
-  int (*is_device_pointer)(const void*) = nullptr;
+  int (*memory)(const void*, int*) = nullptr;
   int (*host_mapped)(const void*, size_t, void**) = nullptr;
   int (*heap_create)(size_t, void**, unsigned char*) = nullptr;
   int (*heap_open)(const unsigned char*, void**) = nullptr;
@@ -152,7 +152,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_lens_to_offsets", &rt->lens_to_offsets);
   Bind(lib, "psdev_device_barrier", &rt->device_barrier);
   Bind(lib, "psdev_multicast_pays", &rt->multicast_pays);
-  Bind(lib, "psdev_rt_is_device_pointer", &rt->is_device_pointer);
+  Bind(lib, "psdev_rt_memory", &rt->memory);
   Bind(lib, "psdev_rt_host_mapped", &rt->host_mapped);
   Bind(lib, "psdev_heap_create", &rt->heap_create);
   Bind(lib, "psdev_heap_open", &rt->heap_open);
@@ -531,6 +531,13 @@ struct Plane::Impl {
   unsigned long long StreamId(void* s) const {
     unsigned long long id = 0;
     return rt.stream_id && rt.stream_id(s, &id) == 0 ? id : 0;
+  }
+  // Whether `p` is device memory; *here: of this GPU.
+  bool OnDevice(const void* p, bool* here) const {
+    int device = -1;
+    const int kind = rt.memory(p, &device);
+    *here = kind == 2 || (kind == 1 && device == opts.device);
+    return kind != 0;
   }
   // Orders work on `s` after the previous request on the tensor, unless that was on this stream too
   // (by its id: the handles of different streams can be equal, see psdev_rt_stream_id).
@@ -1346,9 +1353,16 @@ void Plane::Submit(DeviceRequest&& req) {
   }
   if (req.lens_out) { CHECK_EQ(req.lens_out_n, nlens); }
 
-  // (the CPU stand-in calls "device memory" what lies in an arena)
+  // (the CPU stand-in calls "device memory" what lies in an arena.)  What lies on another GPU is
+  // copied: a kernel of this one may not be able to reach it.
+  bool near = true;
   auto on_device = [&](const void* p) {
-    if (!m.sim) return m.rt.is_device_pointer(p) != 0;
+    if (!m.sim) {
+      bool here = false;
+      const bool device = m.OnDevice(p, &here);
+      if (device && !here) near = false;
+      return device;
+    }
     const char* c = static_cast<const char*>(p);
     const char* lo = static_cast<const char*>(m.ws.peer_base[m.rank]);
     return c >= lo && c < lo + m.arena_bytes;
@@ -1375,7 +1389,8 @@ void Plane::Submit(DeviceRequest&& req) {
                        m.rt.host_mapped(req.outs, req.outs_bytes, &out_map)))) {
       if (host_in) in_at = in_map;
       if (host_out) out_at = out_map;
-      staged = !DirectOk(*d, req.push ? in_at : nullptr, req.pull ? out_at : nullptr, gsz, osz);
+      staged = !near ||
+               !DirectOk(*d, req.push ? in_at : nullptr, req.pull ? out_at : nullptr, gsz, osz);
     }
   }
   int op = (req.push ? PSDEV_OP_PUSH : 0) | (req.pull ? PSDEV_OP_PULL : 0);
@@ -1429,9 +1444,9 @@ void Plane::Submit(DeviceRequest&& req) {
     for (int ri = 0; ri < nruns; ++ri) {
       const Run& r = runs[ri];
       const size_t cnt = static_cast<size_t>(r.end - r.begin);
-      if (W == 1 && !m.sim && (host_in || host_out ||
-                               DirectOk(*d, req.push ? vals : nullptr, req.pull ? outs : nullptr,
-                                        gsz, osz))) {
+      if (W == 1 && !m.sim && near &&
+          (host_in || host_out || DirectOk(*d, req.push ? vals : nullptr,
+                                           req.pull ? outs : nullptr, gsz, osz))) {
         // one rank: the kernel reads and writes the caller's arrays, nobody else needs the
         // values in the arena
         const void* src = req.push && vals != grad ? in_at : nullptr;
@@ -1605,6 +1620,11 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
   auto apart = [](const void* a, size_t an, const void* b, size_t bn) {
     return !a || !b || a == b || !Clash(a, an, 1, b, bn, 1);
   };
+  // (and so does a request with an array on the host or on another GPU)
+  auto here = [&](const void* p) {
+    bool is = !p;
+    return is || (m.OnDevice(p, &is) && is);
+  };
   const size_t kbytes = static_cast<size_t>(n) * 8, lbytes = static_cast<size_t>(n) * 4;
   void* out = req.pull ? req.outs : nullptr;
   void* lens_to = req.pull && !req.push && sp->var_len ? req.lens_out : nullptr;
@@ -1618,7 +1638,10 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
       !((reinterpret_cast<uintptr_t>(kptr) & 7) |
         ((reinterpret_cast<uintptr_t>(req.push ? req.vals : nullptr) |
           reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(lens_in) |
-          reinterpret_cast<uintptr_t>(lens_to)) & 3));
+          reinterpret_cast<uintptr_t>(lens_to)) & 3)) &&
+      (req.cmd == PSDEV_CMD_ARRAYS_HERE ||
+       (here(kptr) && (!req.push || here(req.vals)) && here(out) && here(lens_in) &&
+        here(lens_to)));
   if (local) {
     // one rank: one kernel on the request's own arrays
     if (lens_to) CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));

@@ -2,6 +2,7 @@
 // allocation, the current stream and the library call in one function each.  A Python statement
 // costs about 0.1 us and a ctypes call with a dozen arguments 1.5 us; a launch costs 2.5 us.
 #include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/GradMode.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -114,6 +115,12 @@ PyObject* pull_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// Whether what is done to `t` is followed: by a graph, a tangent or a transform of torch.func.
+bool followed(const at::Tensor& t) {
+  return (t.requires_grad() && c10::GradMode::is_enabled()) || at::isTensorSubclassLike(t) ||
+         t._fw_grad(/*level=*/0).defined();
+}
+
 // unique_sum(bytes_fn, sort_fn, write_fn, keys, vals, key_bits) -> (keys, sums), None where this
 // form does not apply (other types; a key of more than key_bits bits), or an error code
 PyObject* unique_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -127,9 +134,10 @@ PyObject* unique_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!THPVariable_Check(a[3]) || !THPVariable_Check(a[4])) Py_RETURN_NONE;
   const at::Tensor &k_in = THPVariable_Unpack(a[3]), &v_in = THPVariable_Unpack(a[4]);
   const int64_t count = k_in.numel();
-  if (k_in.scalar_type() != at::kLong || v_in.scalar_type() != at::kFloat || v_in.dim() != 1 ||
-      v_in.numel() != count || count <= 0 || count >= (int64_t{1} << 30) || !k_in.is_cuda() ||
-      !v_in.is_cuda() || (v_in.requires_grad() && c10::GradMode::is_enabled()))
+  if (k_in.scalar_type() != at::kLong || v_in.scalar_type() != at::kFloat || k_in.dim() != 1 ||
+      v_in.dim() != 1 || v_in.numel() != count || count <= 0 || count >= (int64_t{1} << 30) ||
+      !k_in.is_cuda() || v_in.device() != k_in.device() || followed(v_in) ||
+      at::isTensorSubclassLike(k_in) || v_in.is_neg())
     Py_RETURN_NONE;
   const at::Tensor k = k_in.contiguous(), v = v_in.contiguous();
   void* stream = stream_on(k.get_device());

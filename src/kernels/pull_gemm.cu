@@ -1515,10 +1515,17 @@ static int pick_plain(long long M, long long N, long long K) {
       offer(base + whole * tile + last, 2000 + nt);
     }
   }
+  // With fewer rows or larger weights than measured (which do not stay in L2) many small tiles are
+  // not what the fit makes of them.  They are kept to one per SM up to 63 rows, where all CTAs read
+  // the same few lines of X, and to what fits at a time otherwise.  us, split form with S = 1 / what
+  // is chosen instead: 1x32768x1024 18.5 / 15.4, 1x50264x1024 31.3 / 24.6, 300x16384x4096 59.7 /
+  // 48.8, 300x16384x16384 225 / 183, 64x50264x1024 23.7 / 25.6.
+  const bool fitted = M >= 64 && (double)N * (double)K <= 4096.0 * 4096.0;
+  const double most = fitted ? INFINITY : M < 64 ? sms : 2 * sms;
   for (int n = 64; n <= 128; n += 64) {
     for (int split = 1; split <= kMaxSplit; split *= 2) {
       const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)
-      if (split > 1 && (ctas > 2 * sms || split > kb)) break;
+      if (split > 1 ? (ctas > 2 * sms || split > kb) : ctas > most) break;
       const double k = ceil(kb / split), full = fmin(ctas / sms, 1);
       const double over = fmax(0.0, ctas / (2 * sms) - 0.9);
       const bool deep = split_deep(n, (long long)ctas, (int)k);
@@ -1709,6 +1716,13 @@ extern "C" int64_t psdev_pull_plan_chunk(int64_t w_elem_off, int64_t nk, int blk
     *end = e;
   }
   return pl.n;
+}
+
+// The variant that a plain product of these sizes takes, as psdev_gemm_config names them, or 0 for
+// the one-CTA kernels.
+extern "C" int psdev_gemm_choice(int64_t M, int64_t N, int64_t K) {
+  if (M < 1 || N < 1 || K < 1) return PSDEV_ERR_ARG;
+  return gemm::pick_plain(M, N, K);
 }
 
 // Selects the kernel variant of later GEMM launches: 128 or 256 (output-tile height of the

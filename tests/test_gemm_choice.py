@@ -1,0 +1,31 @@
+"""Which kernel a plain product takes (a rule on its sizes, evaluated on the host)."""
+import pytest
+
+
+@pytest.fixture(scope="module")
+def choice():
+    from ps_lite_b200 import _lib
+    return _lib.device_lib().psdev_gemm_choice
+
+
+def _ctas(code, m, n):
+    return -(-m // 128) * -(-n // (code % 1000)) * (code // 1000)
+
+
+@pytest.mark.parametrize("m", [1, 8, 16, 63, 64, 100, 128, 200, 255, 256, 300, 511, 1024, 2048])
+@pytest.mark.parametrize("n,k", [(8192, 1024), (32768, 1024), (50264, 1024), (65536, 512),
+                                 (16384, 4096), (16384, 16384), (128, 65536), (4104, 4096)])
+def test_small_tiles_outside_of_the_measured_sizes(choice, m, n, k):
+    """No more of them than fit on the GPU, whatever the fitted times say."""
+    code = choice(m, n, k)
+    if 1000 <= code < 2000 and (m < 64 or n * k > 4096 * 4096):
+        assert _ctas(code, m, n) <= (148 if m < 64 else 296)
+    elif code >= 2000 and code not in (2256, 2512):
+        assert _ctas(code, m, n) <= 296
+
+
+@pytest.mark.parametrize("m,n,k,code", [(300, 16384, 4096, 2512), (1, 50264, 1024, 0), (16, 50264, 1024, 0),
+                                        (1024, 1024, 1024, 1064), (7572, 288, 256, 1064),
+                                        (16384, 3072, 1024, 2512), (64, 256, 4096, 4064)])
+def test_choices(choice, m, n, k, code):
+    assert choice(m, n, k) == code

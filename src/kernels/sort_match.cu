@@ -25,7 +25,8 @@ namespace sortk {
 // Least-significant-digit radix sort with 8-bit digits.  The keys are cut into a few hundred
 // contiguous chunks, one per CTA that fits on the GPU at a time, and a pass is three launches:
 //   digit_count  counts the digits of every chunk;
-//   digit_scan   turns the counts of each digit into how many keys of the chunks before have it;
+//   digit_scan   turns the counts of each digit into how many keys of the chunks before have it
+//                (left to the scatter when there are few chunks);
 //   scatter      takes its chunk tile by tile: ranks each key among the keys of the same digit in
 //                input order (the sort is stable), puts the tile in sorted order in shared
 //                memory and stores runs of equal digits to consecutive addresses.
@@ -45,6 +46,10 @@ constexpr int kTile = kThreads * kItems;
 constexpr int kRadixBits = 8;
 constexpr int kDigits = 1 << kRadixBits;
 constexpr int kMaxChunks = 2 * 148;        // two CTAs per SM
+// Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
+// number of launches (64-bit keys without payload, 2^14 / 2^16, us: 119 / 110 with three launches
+// per pass, 64 / 74 with two; the single-sweep form 97 / 101).
+constexpr int kSelfScan = 32;
 
 // Head of the scratch memory.
 struct SortHead {
@@ -225,9 +230,21 @@ __global__ void __launch_bounds__(kThreads, 2)
   for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) lanes[0][i] = 0;
   grid_wait();
   // output index of the chunk's next key with digit threadIdx.x
-  unsigned int next = cta_exclusive(digit ? __ldcg(totals + threadIdx.x) : 0, s_part[0],
-                                    nullptr);
-  if (digit) next += __ldcg(prefix + (size_t)threadIdx.x * ch.count + blockIdx.x);
+  unsigned int before = 0, total = 0;
+  if (digit) {
+    const unsigned int* row = prefix + (size_t)threadIdx.x * ch.count;
+    if (totals) {
+      before = __ldcg(row + blockIdx.x);
+      total = __ldcg(totals + threadIdx.x);
+    } else {
+      for (int c = 0; c < ch.count; ++c) {
+        const unsigned int v = __ldcg(row + c);
+        if (c < blockIdx.x) before += v;
+        total += v;
+      }
+    }
+  }
+  unsigned int next = cta_exclusive(total, s_part[0], nullptr) + before;
   const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
   const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
   // A tile is loaded before the one before it is stored: its keys and payloads take the registers
@@ -433,13 +450,15 @@ static int sort_pass(const KI* in, KO* out, const unsigned int* pin, unsigned in
   const int shift = pass * kRadixBits;
   int rc = launch_chained(digit_count_kernel<KI>, ch.count, kThreads, 0, s, 1, in, n, shift, ch,
                           pass ? 64 : key_bits, w.counts, w.head);
-  if (!rc)
+  const bool scan = ch.count > kSelfScan;
+  if (!rc && scan)
     rc = launch_chained(digit_scan_kernel, kDigits, kThreads, 0, s, 1, w.counts, ch.count,
                         w.totals);
   if (!rc)
     rc = launch_chained(scatter_kernel<KI, KO, PAY>, ch.count, kThreads, scatter_smem<KO>(PAY), s,
-                        1, in, out, pin, pout, n, shift, ch, w.counts, w.totals);
-  g_launches.fetch_add(3, std::memory_order_relaxed);
+                        1, in, out, pin, pout, n, shift, ch, w.counts,
+                        scan ? w.totals : nullptr);
+  g_launches.fetch_add(scan ? 3 : 2, std::memory_order_relaxed);
   return rc;
 }
 

@@ -189,7 +189,8 @@ class SparseTable:
             raise ValueError("more keys than max_keys")
         multi = self.heap.world > 1 if sync is None else sync
         lib, s = self.heap.lib, torch.cuda.current_stream(self.heap.device)
-        if (not multi and self._target is not None and keys.is_cuda and keys.is_contiguous() and
+        if (not multi and self._target is not None and keys.device == self.out.device and
+                keys.is_contiguous() and not keys.is_neg() and
                 keys.dtype in (torch.int64, torch.uint64)):
             self._pull_local(keys, n)
             self.count = n

@@ -201,8 +201,10 @@ struct SparseTarget {
 };
 constexpr const char* kSparseName = "psb200.sparse_target";
 
-bool plain(const at::Tensor& t, at::ScalarType type) {
-  return t.is_cuda() && t.scalar_type() == type && t.is_contiguous();
+// (what is elsewhere, or negated by torch on reading, is copied into the table's buffers)
+bool plain(const at::Tensor& t, at::ScalarType type, c10::DeviceIndex device) {
+  return t.is_cuda() && t.get_device() == device && t.scalar_type() == type &&
+         t.is_contiguous() && !t.is_neg();
 }
 
 // sparse_push_pull(target, keys, grads, lens): the pulled values (a view of the table's output),
@@ -215,14 +217,14 @@ PyObject* sparse_push_pull(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!THPVariable_Check(a[1]) || !THPVariable_Check(a[2])) Py_RETURN_NONE;
   const at::Tensor &keys = THPVariable_Unpack(a[1]), &grads = THPVariable_Unpack(a[2]);
   const int64_t nk = keys.numel(), nv = grads.numel();
-  if (!(plain(keys, at::kLong) || plain(keys, at::kUInt64)) || !plain(grads, at::kFloat) ||
-      nk > t->max_keys)
+  if (!(plain(keys, at::kLong, t->device) || plain(keys, at::kUInt64, t->device)) ||
+      !plain(grads, at::kFloat, t->device) || nk > t->max_keys)
     Py_RETURN_NONE;
   const int32_t* lens = nullptr;
   if (t->var_len) {
     if (!THPVariable_Check(a[3])) Py_RETURN_NONE;
     const at::Tensor& l = THPVariable_Unpack(a[3]);
-    if (!plain(l, at::kInt) || l.numel() != nk || nv > t->max_vals) Py_RETURN_NONE;
+    if (!plain(l, at::kInt, t->device) || l.numel() != nk || nv > t->max_vals) Py_RETURN_NONE;
     lens = static_cast<const int32_t*>(l.data_ptr());
   } else if (nv != nk * t->width) {
     Py_RETURN_NONE;

@@ -1517,11 +1517,12 @@ static int pick_plain(long long M, long long N, long long K) {
   }
   // With fewer rows or larger weights than measured (which do not stay in L2) many small tiles are
   // not what the fit makes of them.  They are kept to one per SM up to 63 rows, where all CTAs read
-  // the same few lines of X, and to what fits at a time otherwise.  us, split form with S = 1 / what
-  // is chosen instead: 1x32768x1024 18.5 / 15.4, 1x50264x1024 31.3 / 24.6, 300x16384x4096 59.7 /
-  // 48.8, 300x16384x16384 225 / 183, 64x50264x1024 23.7 / 25.6.
+  // the same few lines of X, to three per SM in one row of tiles, and to what fits at a time
+  // otherwise.  us, split form with S = 1 / what is chosen instead: 1x32768x1024 18.5 / 15.4,
+  // 1x50264x1024 31.3 / 24.6, 300x16384x4096 59.7 / 48.8, 300x16384x16384 225 / 183; in one row,
+  // with 393 and 1024 CTAs, 64x50264x1024 23.8 / 25.2 and 128x131072x256 24.0 / 21.8.
   const bool fitted = M >= 64 && (double)N * (double)K <= 4096.0 * 4096.0;
-  const double most = fitted ? INFINITY : M < 64 ? sms : 2 * sms;
+  const double most = fitted ? INFINITY : M < 64 ? sms : M <= 128 ? 3 * sms : 2 * sms;
   for (int n = 64; n <= 128; n += 64) {
     for (int split = 1; split <= kMaxSplit; split *= 2) {
       const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)

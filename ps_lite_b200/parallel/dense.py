@@ -115,7 +115,7 @@ class DenseTable:
         self.optimizer = optimizer or ServerOptimizer("sum")
         self.channel, self.num_ctas = int(channel), int(num_ctas)
         self.step = 0
-        self._opt_key, self._opt_cached, self._opt_step, self._opt_at = None, None, -1, 0
+        self._opt_key, self._opt_cached, self._opt_step = None, None, -1
         self._default_timeout = default_timeout_s()
         # NVSwitch multicast path: on by default from four ranks up when the heap has a
         # multicast alias (with two ranks plain peer accesses move fewer bytes per link)
@@ -234,7 +234,9 @@ class DenseTable:
         end = self.n if end is None else end
         if op & _lib.OP_PUSH and opt_step:
             self.step += 1
-        self._opt_struct()   # (the call reads it at self._opt_at)
+        # (kept while the call reads it: it does so without the interpreter lock, and another thread
+        # may replace the one at hand)
+        opt = self._opt_struct()
         s = stream.cuda_stream if stream else torch._C._cuda_getCurrentRawStream(self._device_index)
         tmo = int((timeout_s if timeout_s is not None else self._default_timeout) * 1e9)
         nvtx = _nvtx_enabled()
@@ -242,7 +244,7 @@ class DenseTable:
             torch.cuda.nvtx.range_push(f"{_OP_NAMES.get(op, 'ps.op')}[{begin}:{end}]")
         nvls = self.nvls and self._multicast_pays((int(end) - int(begin)) * self.grad_size)
         rc = self._dense_op(self._op_fn, self._world_at, self._table_at, op, int(begin), int(end),
-                            self._opt_at, self.channel, self.num_ctas, tmo,
+                            C.addressof(opt), self.channel, self.num_ctas, tmo,
                             (1 if sync else 0) | (2 if nvls else 0), s)
         if nvtx:
             torch.cuda.nvtx.range_pop()
@@ -261,7 +263,6 @@ class DenseTable:
         if step != self._opt_step or p.__dict__ != self._opt_key:
             self._opt_step, self._opt_key = step, dict(p.__dict__)
             self._opt_cached = p.to_struct(max(self.step, 1))
-            self._opt_at = C.addressof(self._opt_cached)
         return self._opt_cached
 
     def push(self, begin: int = 0, end: Optional[int] = None, *, sync: bool = True, stream=None,

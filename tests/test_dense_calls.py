@@ -1,0 +1,42 @@
+"""What DenseTable hands to the library, with stand-ins for the library and the streams (no GPU)."""
+import ctypes as C
+import gc
+import types
+import weakref
+
+import pytest
+import torch
+
+from ps_lite_b200 import _lib
+from ps_lite_b200.parallel.dense import DenseTable, ServerOptimizer
+
+
+@pytest.fixture
+def table(monkeypatch):
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 7, raising=False)
+    t = object.__new__(DenseTable)
+    t.optimizer, t.step, t.n, t.nvls = ServerOptimizer("adam", lr=0.5), 0, 1024, False
+    t._opt_key, t._opt_cached, t._opt_step, t._opt_at = None, None, -1, 0
+    t._default_timeout, t.grad_size, t._device_index = 1.0, 1, 0
+    t.channel = t.num_ctas = t._op_fn = t._world_at = t._table_at = 0
+    t.calls = []
+
+    def op(*args):
+        t.calls.append(_lib.Opt.from_buffer_copy(_lib.Opt.from_address(args[6])))
+        return 0
+    t._dense_op = op
+    return t
+
+
+def test_parameters_live_as_long_as_the_call(table):
+    """Another thread that changes the rate during the call replaces the structure."""
+    def op(*args):
+        at = weakref.ref(table._opt_cached)
+        assert args[6] == C.addressof(at())
+        table.optimizer.lr = 0.25
+        table._opt_struct()
+        gc.collect()
+        assert at() is not None and _lib.Opt.from_address(args[6]).lr == 0.5
+        return 0
+    table._dense_op = op
+    table.push()

@@ -260,8 +260,11 @@ class DenseTable:
         small requests are launch-bound, and building the structure costs microseconds)."""
         p = self.optimizer
         step = max(self.step, 1) if p.kind in ("adam", "adamw") else 0
-        if step != self._opt_step or p.__dict__ != self._opt_key:
-            self._opt_step, self._opt_key = step, dict(p.__dict__)
+        # (a class of the program's own may compute its fields: they are asked for one by one)
+        now = p.__dict__ if type(p) is ServerOptimizer else \
+            {f.name: getattr(p, f.name) for f in dataclasses.fields(ServerOptimizer)}
+        if step != self._opt_step or now != self._opt_key:
+            self._opt_step, self._opt_key = step, dict(now)
             self._opt_cached = p.to_struct(max(self.step, 1))
         return self._opt_cached
 

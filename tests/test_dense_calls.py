@@ -40,3 +40,26 @@ def test_parameters_live_as_long_as_the_call(table):
         return 0
     table._dense_op = op
     table.push()
+
+
+def test_parameters_that_a_class_of_the_program_computes(table):
+    class Warmup(ServerOptimizer):
+        rate = 1.0
+        lr = property(lambda self: self.rate, lambda self, value: None)
+    table.optimizer = Warmup("sgd")
+    table.push()
+    Warmup.rate = 0.125
+    table.push()
+    table.push()
+    assert [o.lr for o in table.calls] == [1.0, 0.125, 0.125]
+
+
+def test_parameters_follow_the_fields_and_the_step(table):
+    table.push()
+    table.push_pull()
+    table.optimizer.lr = 0.25
+    table.pull()
+    table.optimizer = ServerOptimizer("sgd", lr=2.0)
+    table.push()
+    assert [o.lr for o in table.calls] == [0.5, 0.5, 0.25, 2.0]
+    assert table.calls[0].bias1 != table.calls[1].bias1

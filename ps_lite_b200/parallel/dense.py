@@ -194,6 +194,8 @@ class DenseTable:
             raise ValueError("begin must be a multiple of 256")
         g = grad if grad.is_contiguous() else grad.contiguous()
         n = g.numel()
+        if begin < 0:
+            begin += self.n   # counted from the end, like an index
         if begin < 0 or begin + n > self.n:
             raise ValueError("the gradient reaches beyond the table")
         rc = self.heap.lib.psdev_filter_int8_pack(

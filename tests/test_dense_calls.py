@@ -63,3 +63,18 @@ def test_parameters_follow_the_fields_and_the_step(table):
     table.push()
     assert [o.lr for o in table.calls] == [0.5, 0.5, 0.25, 2.0]
     assert table.calls[0].bias1 != table.calls[1].bias1
+
+
+def test_a_gradient_counted_from_the_end(table):
+    """stage_int8 with a negative begin, as an index; beyond either end it is refused."""
+    got = []
+    table.gscale, table.grad = torch.zeros(4), torch.zeros(1024, dtype=torch.int8)
+    table.heap = types.SimpleNamespace(lib=types.SimpleNamespace(
+        psdev_filter_int8_pack=lambda src, dst, scale, n, stream: got.append((dst, scale, n)) or 0))
+    for begin, n in ((0, 1024), (256, 300), (-256, 256), (-1024, 5)):
+        table.stage_int8(torch.zeros(n), begin)
+        at = begin % 1024
+        assert got[-1] == (table.grad[at:].data_ptr(), table.gscale[at // 256:].data_ptr(), n)
+    for begin, n in ((0, 1025), (-256, 257), (-1280, 256), (1024, 1)):
+        with pytest.raises(ValueError):
+            table.stage_int8(torch.zeros(n), begin)

@@ -195,8 +195,8 @@ class DenseTable:
         g = grad if grad.is_contiguous() else grad.contiguous()
         n = g.numel()
         if begin < 0:
-            begin += self.n   # counted from the end, like an index
-        if begin < 0 or begin + n > self.n:
+            begin = max(begin + self.n, 0)   # counted from the end, like a slice
+        if begin + n > self.n:
             raise ValueError("the gradient reaches beyond the table")
         rc = self.heap.lib.psdev_filter_int8_pack(
             g.data_ptr(), self.grad.data_ptr() + begin, self.gscale.data_ptr() + begin // 64, n,

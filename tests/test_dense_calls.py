@@ -66,15 +66,15 @@ def test_parameters_follow_the_fields_and_the_step(table):
 
 
 def test_a_gradient_counted_from_the_end(table):
-    """stage_int8 with a negative begin, as an index; beyond either end it is refused."""
+    """stage_int8 with a negative begin, as in a slice; beyond the end it is refused."""
     got = []
     table.gscale, table.grad = torch.zeros(4), torch.zeros(1024, dtype=torch.int8)
     table.heap = types.SimpleNamespace(lib=types.SimpleNamespace(
         psdev_filter_int8_pack=lambda src, dst, scale, n, stream: got.append((dst, scale, n)) or 0))
-    for begin, n in ((0, 1024), (256, 300), (-256, 256), (-1024, 5)):
+    for begin, n in ((0, 1024), (256, 300), (-256, 256), (-1024, 5), (-1280, 256)):
         table.stage_int8(torch.zeros(n), begin)
-        at = begin % 1024
+        at = max(begin + 1024, 0) if begin < 0 else begin
         assert got[-1] == (table.grad[at:].data_ptr(), table.gscale[at // 256:].data_ptr(), n)
-    for begin, n in ((0, 1025), (-256, 257), (-1280, 256), (1024, 1)):
+    for begin, n in ((0, 1025), (-256, 257), (-1280, 1025), (1024, 1)):
         with pytest.raises(ValueError):
             table.stage_int8(torch.zeros(n), begin)

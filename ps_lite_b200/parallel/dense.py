@@ -157,7 +157,8 @@ class DenseTable:
         self._world_at, self._table_at = C.addressof(self._world), C.addressof(t)
         self._op_fn = C.cast(heap.lib.psdev_dense_op, C.c_void_p).value
         self._dense_op = _lib.torch_ext().dense_op
-        self._device_index = dev.index or 0
+        # (the heap may name its device without an index; the memory knows where it is)
+        self._device_index = self.grad.device.index
         self.grad.zero_()
         self.weight.zero_()
         # Low-latency region for small fused requests (include/ps/device/push_pull_ll.cuh):

@@ -78,3 +78,14 @@ def test_a_gradient_counted_from_the_end(table):
     for begin, n in ((0, 1025), (-256, 257), (-1280, 1025), (1024, 1)):
         with pytest.raises(ValueError):
             table.stage_int8(torch.zeros(n), begin)
+
+
+def test_streams_are_those_of_the_memory_s_device():
+    """A heap may name its device without an index."""
+    memory = types.SimpleNamespace(device=types.SimpleNamespace(index=3), zero_=lambda: None)
+    op = C.CFUNCTYPE(C.c_int)(lambda: 0)
+    heap = types.SimpleNamespace(
+        world=1, mc_base=0, emulated_ranks=False, device=torch.device("cpu"),
+        alloc=lambda nbytes: 256, tensor=lambda off, n, dtype: memory,
+        world_struct=_lib.World, lib=types.SimpleNamespace(psdev_dense_op=op))
+    assert DenseTable(heap, 64)._device_index == 3

@@ -144,7 +144,9 @@ def run_pushpull(args):
                "plain_copies_ms": round(ceiling_ms, 4),
                "ms_over_plain_copies": round(ms2 / ceiling_ms, 3),
                "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes,
-               "slice_mib": args.slice_mb,
+               # (one rank: at most a 32nd of the request, 4 MiB at least)
+               "slice_mib": args.slice_mb if world > 1 else
+               min(args.slice_mb, max(4.0, nbytes / 32 / (1 << 20))),
                "api": "KVStore.push_pull(pinned host tensor, out=pinned host tensor); wait(ts) "
                       "= KVWorker::ZPushPull + Wait through ps::Start and the device plane"}
     # the sampler ran through both timed regions (device-timed and end-to-end)

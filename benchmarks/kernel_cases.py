@@ -1,6 +1,7 @@
 """Small single-GPU cases of the kernels that have no benchmark of their own, for profiling.
 
-    python benchmarks/kernel_cases.py --case sparse|filters|sort|p3|barrier [--iters 3]
+    python benchmarks/kernel_cases.py --case sparse|sparse_one|update|filters|sort|p3|barrier
+        [--iters 3]
 
 Each case builds its inputs (larger than the 126 MB L2 where DRAM figures matter, a few GB at
 most), runs the kernels `--iters` times and prints CUDA-event times per launch group as one JSON
@@ -32,7 +33,8 @@ def timed(fn, iters):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--case", required=True, choices=["sparse", "filters", "sort", "p3", "barrier"])
+    ap.add_argument("--case", required=True, choices=[
+        "sparse", "sparse_one", "update", "filters", "sort", "p3", "barrier"])
     ap.add_argument("--iters", type=int, default=3)
     args = ap.parse_args()
     dev = torch.device("cuda", 0)
@@ -63,6 +65,25 @@ def main():
         for j, name in enumerate(("scatter_us", "apply_us", "respond_us")):
             out[name] = round(sum(e[j].elapsed_time(e[j + 1]) for e in ev) / len(ev) * 1e3, 1)
         out["keys"] = n
+        t.check()
+    elif args.case == "sparse_one":   # one rank: the request in one launch
+        key_space, n = 1 << 26, 1 << 20
+        heap = SymmetricHeap(4 * key_space + 24 * n + (64 << 20), 0, 1, device=dev)
+        t = SparseTable(heap, key_space, n, kind="ftrl")
+        # another set of keys in every launch: their states are not in L2
+        sets = [torch.sort(torch.randperm(key_space, device=dev)[:n]).values
+                for _ in range(args.iters + 1)]
+        grads = torch.randn(n, device=dev) * 0.1
+        it = iter(sets)
+        out["push_pull_2^20_keys_us"] = timed(lambda: t.push_pull(next(it), grads), args.iters)
+        t.check()
+    elif args.case == "update":   # one rank: SGD on 64 Mi fp32 values
+        n = 64 << 20
+        heap = SymmetricHeap(8 * n + (64 << 20), 0, 1, device=dev)
+        t = DenseTable(heap, n, torch.float32, torch.float32,
+                       optimizer=ServerOptimizer("sgd", lr=0.01))
+        t.grad.normal_()
+        out["push_pull_256MiB_us"] = timed(lambda: t.push_pull(), args.iters)
         t.check()
     elif args.case == "filters":
         from ps_lite_b200.ops import filters as F

@@ -2,12 +2,13 @@
 //
 // A kernel launched with launch_chained may start while the previous kernel of its stream is
 // still running, so that its launch and prologue overlap that kernel's end (2 to 3 us per launch
-// for a GEMM, about 1 us for a small kernel).  In return every thread of it calls grid_wait()
-// before its first access to global memory: that returns once the previous kernel has completed
-// and its writes are visible.  Every kernel launched so waits, on all paths, which makes the order
-// transitive.  grid_launch_next() lets the next kernel of the stream start, as far as it was
-// launched so, once every CTA has called it; in a kernel launched in the ordinary way both cost
-// nothing.
+// for a GEMM, about 1 us for a small kernel).  In return grid_wait() comes before every access that
+// it makes to global memory: that returns once the previous kernel has completed and its writes are
+// visible.  A thread with such accesses calls it itself, or makes them only after one that has
+// called it (the GEMM kernels: the threads that load wait, all else follows from what they load).
+// Every CTA of every kernel launched so waits, on all paths, which makes the order transitive.
+// grid_launch_next() lets the next kernel of the stream start, as far as it was launched so, once
+// every CTA has called it; in a kernel launched in the ordinary way both cost nothing.
 #pragma once
 #include <cuda_runtime.h>
 

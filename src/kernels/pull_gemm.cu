@@ -1477,8 +1477,9 @@ static int pick_tile_m(long long M, long long N, long long K) {
 // The kernel of a plain product: 1000 * S + BN the split form, 2256 / 2512 pairs of CTAs with
 // tiles of 256 x 256 / 512 (wide_gemm.cuh), 0 the persistent one-CTA tiles of this file.  The
 // times below, in us, were fitted to measurements over M 64 .. 4096, N and K 256 .. 4096 (operands
-// in L2, launches back to back).  They put pairs where their tiles nearly fill the GPU or K is
-// long; the wide tile where it costs no extra round, since it moves fewer bytes per product:
+// in L2, launches back to back, 148 SMs), as benchmarks/gemm_choice.py takes them.  They put pairs
+// where their tiles nearly fill the GPU or K is long; the wide tile where it costs no extra round,
+// since it moves fewer bytes per product:
 //                     1024x1024x1024  2048x2048x1024  1536x4096x1024  2048x4096x1024  2048x512x4096
 //   S = 1, BN = 64          6.0            14.9            21.1            27.8            15.3
 //   S = 1, BN = 128         6.8            11.0            18.1            20.6            17.6

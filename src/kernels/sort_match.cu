@@ -38,7 +38,7 @@ namespace sortk {
 // words that earlier tiles publish) spent a third of its time in the look-back and another third
 // in a second wave of tiles: 54 us per pass on 2^22 keys of 30 bits with a payload, against 41 us
 // for these three launches (5.5 + 2.2 + 33).  What bounds the scatter now is the shared-memory
-// pipe: some 45 wavefronts per 32 keys, half of them bank conflicts of random digits.
+// pipe: 40 wavefronts per 32 keys, half of them bank conflicts of random digits.
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kItems = 8;                  // keys per thread and tile
@@ -765,7 +765,7 @@ namespace {
 // then two buffers of keys (4 bytes each up to 32 bits) and of values.
 struct UniqueScratch {
   char* work;
-  SortHead* head;        // followed by `counts`: the host reads both with one copy
+  SortHead* head;
   unsigned int* counts;
   char* keys[2];
   unsigned int* vals[2];

@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(256, 8)
 // the handle and stores state and answer.  The three kernels above touch two random places of
 // memory per value and phase (accumulator and state) and copy the request into the arena first;
 // here a value costs one read and one write of its state, and the request's arrays are used
-// where they are.  2^20 Zipf keys of 2^30, FTRL: 201 us with the three kernels (and 4 copies).
-// 59 us with this one, which is what the random accesses alone take.
+// where they are.  2^20 Zipf keys of 2^30, FTRL, steps back to back: 201 us with the three kernels
+// (and 4 copies), 57 us with this one, bound by the rate of random DRAM accesses (kStateUnroll).
 struct LocalReq {
   const unsigned long long* keys;
   const float* vals;     // pushed values, or NULL
@@ -421,7 +421,8 @@ struct LocalReq {
 };
 constexpr int kLocalUnroll = 4;
 // One 16-byte group per key, all of them far apart: a plain kernel that reads 2^20 such groups and
-// writes them back takes 59 us with one per thread, 63 with two, 67 with four (41 only reading).
+// writes them back takes 59 us with one per thread, 63 with two, 67 with four (41 only reading),
+// each launch by itself.
 constexpr int kStateUnroll = 1;
 
 // State of one value: {w, z, n} (z, n: FTRL).  GROUP: side by side, one 16-byte access.

@@ -18,9 +18,11 @@
 // on the parameters themselves, and run after those.  An accumulator belongs to the stream that was
 // current when it was made and lives as long as the graphs that use it, so it is not held here: a
 // tensor hook, which the parameter keeps, puts the hook on each new accumulator.  (Held ones would
-// keep accumulation on the stream of the constructor, out of reach of a graph capture.)  A gradient stays alive until the kernel
-// that reads it has finished: batches are kept with an event and dropped when it has fired, the
-// rest when the step ends and the caller's stream has been ordered behind the kernels.
+// keep accumulation on the stream of the constructor, out of reach of a graph capture.)
+//
+// A gradient stays alive until the kernel that reads it has finished: batches are kept with an
+// event and dropped when it has fired, the rest when the step ends and the caller's stream has been
+// ordered behind the kernels.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>

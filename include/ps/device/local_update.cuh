@@ -117,8 +117,30 @@ __device__ __forceinline__ void load_part(const T* p, long long count, bool vec,
   }
 }
 
+// Elements [lo, hi) one by one, from and to the table's own buffers: the part of a vector that
+// belongs to a slice which starts or ends inside it (the rest is another CTA's).
+template <typename GT, typename OT, class Opt, bool REDUCE, bool BCAST>
+__device__ __forceinline__ void update_part(const LocalArgs& a, long long lo, long long hi) {
+#pragma unroll 1
+  for (long long e = lo; e < hi; ++e) {
+    float w = a.master[e];
+    if constexpr (REDUCE) {
+      float g = to_f32(reinterpret_cast<const GT*>(a.grad)[e]);
+      float m = Opt::kStates >= 1 ? a.s1[e] : 0.f;
+      float v = Opt::kStates >= 2 ? a.s2[e] : 0.f;
+      if constexpr (sizeof(GT) == 1) g *= a.gscale[e / kInt8Group];
+      Opt::apply(w, g * a.opt.scale, m, v, a.opt);
+      a.master[e] = w;
+      if (Opt::kStates >= 1) a.s1[e] = m;
+      if (Opt::kStates >= 2) a.s2[e] = v;
+    }
+    if constexpr (BCAST) from_f32(reinterpret_cast<OT*>(a.weight) + e, w);
+  }
+}
+
+// (two states per value: 56 registers, so that nine CTAs fit an SM)
 template <typename GT, typename OT, class Opt, bool REDUCE, bool BCAST, typename Segs>
-__global__ void __launch_bounds__(kLocalThreads)
+__global__ void __launch_bounds__(kLocalThreads, Opt::kStates >= 2 ? 9 : 0)
     local_update_kernel(const __grid_constant__ LocalArgs a, const __grid_constant__ Segs segs) {
   constexpr bool kSegs = !std::is_same<Segs, NoSegs>::value;
   grid_launch_next();
@@ -150,7 +172,7 @@ __global__ void __launch_bounds__(kLocalThreads)
       tl = t - a.sched[lo].tile_begin;
     }
     const long long i = (begin / kLocalTile + tl) * kLocalTile + threadIdx.x * kLocalVec;
-    if (i < begin || i >= end) continue;
+    if (i + kLocalVec <= begin || i >= end) continue;
 #ifdef PSDEV_CHECKS
     if (i + kLocalVec > a.n_total || i + kLocalVec > a.local_len ||
         (a.heap_bytes &&
@@ -160,6 +182,13 @@ __global__ void __launch_bounds__(kLocalThreads)
       continue;
     }
 #endif
+    if constexpr (!kSegs) {
+      if (i < begin || i + kLocalVec > end) {  // (slices of the device's list: any boundaries)
+        update_part<GT, OT, Opt, REDUCE, BCAST>(a, i < begin ? begin : i,
+                                                i + kLocalVec < end ? i + kLocalVec : end);
+        continue;
+      }
+    }
     float w[kLocalVec];
     if constexpr (REDUCE) {
       float g[kLocalVec], m[kLocalVec], v[kLocalVec];

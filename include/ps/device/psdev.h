@@ -228,8 +228,9 @@ int psdev_dense_op_segs(const psdev_world_t* w, const psdev_table_t* t, int op,
 /* Several slices of one table in one launch and one rendezvous.  `segs`: device memory with
  * `nseg` (<= 1024) triples (begin, end, priority) of int64; a small kernel orders them by
  * priority (highest first, ties in submission order) and numbers the tiles across slices, so
- * the CTAs work on the most urgent slice first.  `sched`: device scratch of
- * psdev_sched_bytes(nseg) bytes. */
+ * the CTAs work on the most urgent slice first.  Slices start and end at multiples of 16 bytes of
+ * gradients (of fp32 weights for a pull alone); with one rank anywhere.  `sched`: device scratch
+ * of psdev_sched_bytes(nseg) bytes. */
 int psdev_dense_op_multi(const psdev_world_t* w, const psdev_table_t* t, int op,
                          const int64_t* segs, int nseg, void* sched, const psdev_opt_t* opt,
                          int channel, int num_ctas, uint64_t timeout_ns, int sync, void* stream);

@@ -159,7 +159,7 @@ class DistributedOptimizer:
         pri = [-1 - i if self._publish[i] else len(self.params) - i
                for i in range(len(self.params))]
         # torch drops the native hooks of a tensor when the first hook in Python arrives; once it
-        # has had one, later ones are added beside them
+        # has had one, later ones are added beside the native one
         for p in self.params:
             if p._backward_hooks is None:
                 p.register_hook(lambda g: None).remove()

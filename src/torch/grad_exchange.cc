@@ -17,7 +17,8 @@
 // The hooks sit on the parameters' gradient accumulators, next to hooks that a program registers
 // on the parameters themselves, and run after those.  An accumulator belongs to the stream that was
 // current when it was made and lives as long as the graphs that use it, so it is not held here: a
-// tensor hook, which the parameter keeps, puts the hook on each new accumulator.  (Held ones would
+// tensor hook, which the parameter keeps, puts the hook on each new accumulator.  It stands behind
+// the one for the program's tensor hooks, which Tensor::register_hook would drop.  (Held ones would
 // keep accumulation on the stream of the constructor, out of reach of a graph capture.)
 //
 // A gradient stays alive until the kernel that reads it has finished: batches are kept with an
@@ -81,7 +82,10 @@ class GradExchange {
     for (size_t i = 0; i < params_.size(); ++i) {
       TORCH_CHECK(params_[i].is_leaf() && params_[i].requires_grad(), "parameter ", i,
                   " is no leaf that takes a gradient");
-      hooks_[i].tensor_hook = params_[i].register_hook([this, i](const at::Tensor&) { Attach(i); });
+      auto before = std::make_unique<BeforeAccumulation>(this, i);
+      hooks_[i].tensor_hook = before.get();
+      torch::autograd::impl::materialize_autograd_meta(params_[i])->hooks_.push_back(
+          std::move(before));
     }
   }
 
@@ -92,7 +96,12 @@ class GradExchange {
 
   void Detach() {
     for (size_t i = 0; i < hooks_.size(); ++i) {
-      params_[i].remove_hook(hooks_[i].tensor_hook);
+      auto& of_tensor = torch::autograd::impl::materialize_autograd_meta(params_[i])->hooks_;
+      of_tensor.erase(std::remove_if(of_tensor.begin(), of_tensor.end(),
+                                     [&](const auto& h) {
+                                       return h.get() == hooks_[i].tensor_hook;
+                                     }),
+                      of_tensor.end());
       if (auto node = hooks_[i].node.lock()) node->del_post_hook(hooks_[i].key);
     }
     hooks_.clear();
@@ -135,6 +144,15 @@ class GradExchange {
     variable_list operator()(const variable_list& outputs, const variable_list& inputs) override {
       owner->Take(index, inputs);
       return outputs;
+    }
+    GradExchange* owner;
+    size_t index;
+  };
+  struct BeforeAccumulation : torch::autograd::FunctionPreHook {
+    BeforeAccumulation(GradExchange* owner, size_t index) : owner(owner), index(index) {}
+    variable_list operator()(const variable_list& grads) override {
+      owner->Attach(index);
+      return grads;
     }
     GradExchange* owner;
     size_t index;
@@ -319,7 +337,7 @@ class GradExchange {
   int channel_;
   py::function refresh_;
   struct Attached {
-    unsigned tensor_hook = 0;
+    const torch::autograd::FunctionPreHook* tensor_hook = nullptr;
     std::weak_ptr<Node> node;  // the accumulator that has the hook, and the hook's key there
     uintptr_t key = 0;
   };

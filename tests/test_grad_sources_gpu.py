@@ -264,3 +264,33 @@ def test_a_captured_step(cuda_device, batch_bytes, overlap):
     del graph
     dopt.close()
     heap.close()
+
+
+@pytest.mark.parametrize("where", ["before", "after", "both"])
+def test_tensor_hooks_of_the_program(cuda_device, where):
+    """Hooks on the parameters, made before or after the optimizer, see and change the gradients."""
+    p, q = (torch.nn.Parameter(torch.zeros(300, device=cuda_device)) for _ in range(2))
+    seen = []
+
+    def hook(g):
+        seen.append(float(g[0]))
+        return 2 * g
+    first = p.register_hook(hook) if where != "after" else None
+    heap, dopt = _optimizer(cuda_device, [p, q], torch.float32)
+    second = p.register_hook(hook) if where != "before" else None
+    for _ in range(2):
+        (p.sum() + q.sum()).backward()
+        dopt.step()
+    times = 2 if where == "both" else 1
+    assert seen == [1.0, 2.0][:times] * 2
+    assert torch.all(p == -2.0 ** times) and torch.all(q == -1.0)
+    (second or first).remove()
+    (p.sum() + q.sum()).backward()
+    dopt.step()
+    assert torch.all(p == -2.0 ** times - 2.0 ** (times - 1) / 2) and torch.all(q == -1.5)
+    dopt.close()
+    if first and second:
+        first.remove()
+    (p.sum() + q.sum()).backward()
+    assert torch.all(p.grad == 1.0) and torch.all(q.grad == 1.0)
+    heap.close()

@@ -109,6 +109,7 @@ class GradExchange {
     segs_.clear();
     pending_ = 0;
     held_.clear();
+    OutliveComm();  // (without a step nobody waits for the launches)
     batches_.clear();
   }
 
@@ -121,11 +122,7 @@ class GradExchange {
     if (overlap_) {
       // Memory given back from here on is reused on the stream the gradients were made on; that
       // is `cur`, which now comes after the kernels, or the allocator is told.
-      if (other_stream_ || (hook_stream_ && *hook_stream_ != cur)) {
-        for (auto& b : batches_)
-          for (auto& t : b.tensors)
-            c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), comm_);
-      }
+      if (other_stream_ || (hook_stream_ && *hook_stream_ != cur)) OutliveComm();
     }
     while (!batches_.empty()) Retire();
     hook_stream_.reset();
@@ -220,6 +217,13 @@ class GradExchange {
   void Again(size_t i, const c10::cuda::CUDAStream& cur, std::unique_lock<std::mutex>& lk) {
     if (sent_[i] == kPending) Drain(lk);
     if (launched_on_) After(*launched_on_, cur);
+  }
+
+  // The memory of launched gradients is not used again before what runs on `comm_` has finished.
+  void OutliveComm() {
+    for (auto& b : batches_)
+      for (auto& t : b.tensors)
+        c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), comm_);
   }
 
   // Orders work on `next` behind what has been issued on `before`.

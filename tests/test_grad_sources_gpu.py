@@ -266,6 +266,27 @@ def test_a_captured_step(cuda_device, batch_bytes, overlap):
     heap.close()
 
 
+def test_closed_between_backward_and_step(cuda_device):
+    """Gradients whose update has been launched and not waited for keep their memory."""
+    n = 1 << 20
+    p = torch.nn.Parameter(torch.zeros(n, device=cuda_device))
+    heap, dopt = _optimizer(cuda_device, [p], torch.float32, batch_bytes=1)
+    at = []
+    p.register_hook(lambda g: at.append(g.data_ptr()))
+    x = torch.full((n,), 2.0, device=cuda_device)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(dopt.comm):
+        torch.cuda._sleep(400_000_000)   # the update comes behind this: some 0.2 s
+    (p * x).sum().backward()
+    assert dopt._native.launches == 1 and dopt._native.staged == 0
+    dopt._native.detach()
+    again = [torch.full((n,), 8.0, device=cuda_device) for _ in range(8)]
+    assert at[0] not in [t.data_ptr() for t in again]
+    dopt.close()
+    assert torch.all(dopt.table.weight[:n] == -1.0)
+    heap.close()
+
+
 @pytest.mark.parametrize("where", ["before", "after", "both"])
 def test_tensor_hooks_of_the_program(cuda_device, where):
     """Hooks on the parameters, made before or after the optimizer, see and change the gradients."""

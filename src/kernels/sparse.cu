@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "ps/device/chain.cuh"
 #include "ps/device/push_pull.cuh"
@@ -406,7 +407,8 @@ __global__ void __launch_bounds__(256, 8)
 // memory per value and phase (accumulator and state) and copy the request into the arena first;
 // here a value costs one read and one write of its state, and the request's arrays are used
 // where they are.  2^20 Zipf keys of 2^30, FTRL, steps back to back: 201 us with the three kernels
-// (and 4 copies), 57 us with this one, bound by the rate of random DRAM accesses (kStateUnroll).
+// (and 4 copies), 54 us with this one, bound by the rate of random DRAM accesses (kStateUnroll,
+// load_one).
 struct LocalReq {
   const unsigned long long* keys;
   const float* vals;     // pushed values, or NULL
@@ -423,14 +425,43 @@ constexpr int kLocalUnroll = 4;
 // One 16-byte group per key, all of them far apart: a plain kernel that reads 2^20 such groups and
 // writes them back takes 59 us with one per thread, 63 with two, 67 with four (41 only reading),
 // each launch by itself.
+// (4 bytes per key, far apart: 62.9 us with four per thread and plain loads, 51.1 with one and FAR.)
 constexpr int kStateUnroll = 1;
+__host__ __device__ constexpr int local_unroll(bool group, bool one, bool far) {
+  return one && (group || far) ? kStateUnroll : kLocalUnroll;
+}
+
+// Loads of state.  FAR: most 128-byte lines of the state that the request touches hold one key of
+// it.  A plain load that misses L2 fetches such a line from DRAM, one with this hint half of it:
+// 2^20 random 16-byte groups of 2^30, read and written back, read 134 and 74 MB and take 57.7 and
+// 55.1 us (of 2^26: 51.1 and 47.1; of 2^24: 36.6 and 33.0).  Where a line holds several keys of the
+// request, a whole one is one access instead of two (a hash store with a quarter of its slots
+// wanted: 34 us without the hint, 42 with it).
+template <bool FAR>
+__device__ __forceinline__ float load_one(const float* p) {
+  if constexpr (!FAR) return *p;
+  float v;
+  asm volatile("ld.global.L2::64B.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+template <bool FAR>
+__device__ __forceinline__ float4 load_four(const float* p) {
+  if constexpr (!FAR) return *reinterpret_cast<const float4*>(p);
+  float4 v;
+  asm volatile("ld.global.L2::64B.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
 
 // State of one value: {w, z, n} (z, n: FTRL).  GROUP: side by side, one 16-byte access.
-template <bool GROUP>
+template <bool GROUP, bool FAR>
 __device__ __forceinline__ float4 load_state(const SparseArgs& a, long long e) {
-  if constexpr (GROUP) return *reinterpret_cast<const float4*>(a.w + e * 4);
+  if constexpr (GROUP) return load_four<FAR>(a.w + e * 4);
   const long long s = e * a.sstride;
-  return make_float4(a.w[s], a.kind == 2 ? a.z[s] : 0.f, a.kind == 2 ? a.nacc[s] : 0.f, 0.f);
+  return make_float4(load_one<FAR>(a.w + s), a.kind == 2 ? load_one<FAR>(a.z + s) : 0.f,
+                     a.kind == 2 ? load_one<FAR>(a.nacc + s) : 0.f, 0.f);
 }
 // The handle with gradient g on a loaded state; a zero gradient changes nothing.
 template <bool GROUP>
@@ -467,12 +498,12 @@ __device__ __forceinline__ bool below(long long at, long long end) {
 
 // Every key has `width` values.  Equal keys next to each other count as one whose gradients are
 // added up: the first of them does the work of all.
-template <bool GROUP, bool ONE>
+template <bool GROUP, bool ONE, bool FAR>
 __global__ void __launch_bounds__(256)
     sparse_local_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ LocalReq q) {
   grid_launch_next();
   grid_wait();
-  constexpr int kLocalUnroll = GROUP && ONE ? kStateUnroll : psdev::kLocalUnroll;
+  constexpr int kLocalUnroll = local_unroll(GROUP, ONE, FAR);
   const unsigned int width = ONE ? 1u : (unsigned int)a.width;
   const long long work = q.n * width;
   const long long first = blockIdx.x * (256ll * kLocalUnroll) + threadIdx.x;
@@ -502,7 +533,7 @@ __global__ void __launch_bounds__(256)
     if (head[u] && k[u] < a.range) {  // (a key outside the range is dropped)
       const long long idx = state_index(a, 0, k[u], true);
       e[u] = idx < 0 ? -1 : idx * width + (first + u * 256 - i[u] * width);
-      if (idx >= 0) v[u] = load_state<GROUP>(a, e[u]);
+      if (idx >= 0) v[u] = load_state<GROUP, FAR>(a, e[u]);
       else if (a.capacity) *a.overflow = 1;
     }
   }
@@ -523,6 +554,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // Rows of a multiple of four values with one number each (sum, SGD): 16-byte accesses.
+template <bool FAR>
 __global__ void __launch_bounds__(256)
     sparse_local_rows_kernel(const __grid_constant__ SparseArgs a,
                              const __grid_constant__ LocalReq q) {
@@ -552,7 +584,7 @@ __global__ void __launch_bounds__(256)
       if (vals) g[u] = vals[t];
       if (head && k < a.range) {
         idx[u] = state_index(a, 0, k, true);
-        if (idx[u] >= 0) w[u] = reinterpret_cast<const float4*>(a.w)[idx[u] * quads + j[u]];
+        if (idx[u] >= 0) w[u] = load_four<FAR>(a.w + (idx[u] * quads + j[u]) * 4);
         else if (a.capacity) *a.overflow = 1;
       }
     }
@@ -756,7 +788,7 @@ __global__ void __launch_bounds__(256)
           if (s_idx[c[u]] != -2 && j < s_len[c[u]]) {
             at[u] = base + s_off[c[u]] + j;
             e[u] = s_idx[c[u]] < 0 ? -1 : s_idx[c[u]] * a.width + j;
-            if (e[u] >= 0) v[u] = load_state<GROUP>(a, e[u]);
+            if (e[u] >= 0) v[u] = load_state<GROUP, false>(a, e[u]);
             if (q.lens && below(at[u], q.nvals)) g[u] = q.vals[at[u]];
           }
         }
@@ -944,13 +976,21 @@ int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t 
     const bool rows = t->kind != 2 && t->width % 4 == 0 && a.sstride == 1 &&
                       (((uintptr_t)vals | (uintptr_t)out | (uintptr_t)t->w) & 15) == 0;
     const long long work = rows ? n * (t->width / 4) : n * t->width;
-    const int unroll = group && t->width == 1 ? kStateUnroll : kLocalUnroll;
+    const bool one = t->width == 1;
+    // (see load_one; rows that fill lines of their own are read as they are)
+    const long long value_bytes = 4ll * t->width * (group ? 4 : 1);
+    const bool far = value_bytes < 128 && n < t->slots / (128 / value_bytes);
+    const int unroll = rows ? kLocalUnroll : local_unroll(group, one, far);
     const unsigned ctas = (unsigned)((work + 256 * unroll - 1) / (256 * unroll));
-    auto* kern = rows                    ? sparse_local_rows_kernel
-                 : group && t->width == 1 ? sparse_local_kernel<true, true>
-                 : group                  ? sparse_local_kernel<true, false>
-                 : t->width == 1          ? sparse_local_kernel<false, true>
-                                          : sparse_local_kernel<false, false>;
+    auto pick = [&](auto f) {
+      constexpr bool F = decltype(f)::value;
+      return rows           ? sparse_local_rows_kernel<F>
+             : group && one ? sparse_local_kernel<true, true, F>
+             : group        ? sparse_local_kernel<true, false, F>
+             : one          ? sparse_local_kernel<false, true, F>
+                            : sparse_local_kernel<false, false, F>;
+    };
+    auto* kern = far ? pick(std::true_type{}) : pick(std::false_type{});
     rc = launch_chained(kern, ctas, 256, 0, s, 1, a, q);
   }
   g_launches.fetch_add(1, std::memory_order_relaxed);

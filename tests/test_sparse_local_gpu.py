@@ -63,6 +63,23 @@ def test_fixed_width(cuda_device, n, kind, width, store):
     assert torch.equal(a.pull(ask), _three(b, ask, torch.zeros(n * width, device=cuda_device)))
 
 
+@pytest.mark.parametrize("kind, width", [("ftrl", 1), ("sgd", 1), ("sgd", 4), ("ftrl", 3),
+                                         ("sgd", 31), ("sgd", 32)])
+@pytest.mark.parametrize("more", [-1, 0])
+def test_one_key_per_line(cuda_device, kind, width, more):
+    """Either side of the number of keys from which lines are read whole."""
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(width)
+    value = 4 * width * (4 if kind == "ftrl" else 1)
+    n = SPACE // max(1, 128 // value) + more
+    a, b = _pair(cuda_device, n, kind=kind, width=width)
+    for _ in range(2):
+        keys = torch.sort(torch.randperm(SPACE, device=cuda_device, generator=g)[:n]).values
+        vals = torch.randn(n * width, device=cuda_device, generator=g)
+        assert torch.equal(a.push_pull(keys, vals), _three(b, keys, vals))
+        _same_state(a, b)
+
+
 @pytest.mark.parametrize("width", [1, 4, 5])
 def test_repeated_keys(cuda_device, width):
     a, b = _pair(cuda_device, 4000, kind="sgd", width=width)

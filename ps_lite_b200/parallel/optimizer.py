@@ -16,7 +16,7 @@ and that its users build on ``KVWorker::Push/Pull`` with per-message priorities
   gradient tensors as they are, and the update kernel reads them where they lie; a gradient whose
   memory somebody else can still write (a view of a workspace, say) is copied by its hook;
 * slices are exchanged by fused push+pull kernels on a side stream, overlapping the rest of
-  backward: as soon as ``batch_bytes`` (4 MiB by default, ``PSB200_BATCH_BYTES``) of gradients
+  backward: as soon as ``batch_bytes`` (4 MiB by default, 32 on one rank; ``PSB200_BATCH_BYTES``)
   are pending, everything pending goes out in ONE launch whose CTAs take the slices in priority
   order, so small tensors share a rendezvous; with ``batch_bytes=0`` every hook launches up to
   ``slices_per_event`` single-slice kernels and the rest waits in the host queue.
@@ -36,6 +36,15 @@ import torch
 from .. import _lib
 from .dense import DenseTable, ServerOptimizer
 from .heap import SymmetricHeap
+
+
+# Bytes of gradients that a launch waits for, unless the program says otherwise.  Several ranks:
+# enough that small tensors share a rendezvous.  One rank has none, and a launch costs the thread of
+# the hooks some 8 us, as much as the update of 4 MiB takes the GPU: the 391 tensors of BERT-large,
+# Adam, in a pass that is bound by that thread 4270 us with 4 MiB, 4130 with 16, 3820 with 32.  What
+# is pending when the backward pass ends is all that the step waits for (32 MiB of bf16 gradients,
+# Adam: 72 us).
+BATCH_EXCHANGED, BATCH_ONE_RANK = 4 << 20, 32 << 20
 
 
 class P3Scheduler:
@@ -102,7 +111,8 @@ class DistributedOptimizer:
         # goes out in one launch (small tensors share a rendezvous); 0 = launch from every hook
         if batch_bytes is None:
             import os
-            batch_bytes = int(os.environ.get("PSB200_BATCH_BYTES", str(4 << 20)))
+            batch_bytes = int(os.environ.get("PSB200_BATCH_BYTES", str(
+                BATCH_ONE_RANK if self._one_rank() else BATCH_EXCHANGED)))
         self.batch_bytes = int(batch_bytes)
         self._gsz = gsz
         self.launches = 0
@@ -134,10 +144,13 @@ class DistributedOptimizer:
                            for i, p in enumerate(self.params)]
         self._pending_step = False
 
+    def _one_rank(self) -> bool:
+        return self.heap.world == 1 and not self.heap.emulated_ranks
+
     def _native_ok(self, grad_dtype) -> bool:
         """One rank, gradients in a type that the update kernel reads in place, and batching on
         (``batch_bytes=0`` asks for a launch per slice)."""
-        return (self.heap.world == 1 and not self.heap.emulated_ranks and self.batch_bytes > 0 and
+        return (self._one_rank() and self.batch_bytes > 0 and
                 grad_dtype in (torch.float32, torch.bfloat16) and
                 all(p.is_cuda for p in self.params))
 

@@ -22,30 +22,41 @@ namespace psdev {
 extern std::atomic<uint64_t> g_launches;
 
 namespace sortk {
-// Least-significant-digit radix sort with 8-bit digits.  The keys are cut into a few hundred
+// Least-significant-digit radix sort of 64-bit items.  The items are cut into a few hundred
 // contiguous chunks, one per CTA that fits on the GPU at a time, and a pass is three launches:
 //   digit_count  counts the digits of every chunk;
-//   digit_scan   turns the counts of each digit into how many keys of the chunks before have it
+//   digit_scan   turns the counts of each digit into how many items of the chunks before have it
 //                (left to the scatter when there are few chunks);
-//   scatter      takes its chunk tile by tile: ranks each key among the keys of the same digit in
+//   scatter      takes its chunk tile by tile: ranks each item among the items of the same digit in
 //                input order (the sort is stable), puts the tile in sorted order in shared
 //                memory and stores runs of equal digits to consecutive addresses.
-// ceil(key_bits / 8) passes: a caller that knows its keys are below 2^30 pays four passes,
-// not eight.  No CTA ever waits for another one.
+// No CTA ever waits for another one.  An item is a key, or a key of up to 32 bits above a value of
+// 32 bits (which then needs no array of its own: one store of 8 bytes per item where two of 4 went
+// to different places).
 //
-// Up to some ten million keys everything stays in L2 and a pass is bound by latencies.  The
-// single-sweep form (one launch per pass, tiles finding their offsets by looking back over the
-// words that earlier tiles publish) spent a third of its time in the look-back and another third
-// in a second wave of tiles: 54 us per pass on 2^22 keys of 30 bits with a payload, against 41 us
-// for these three launches (5.5 + 2.2 + 33).  What bounds the scatter now is the shared-memory
-// pipe: 40 wavefronts per 32 keys, half of them bank conflicts of random digits.
+// Digits have 8 bits, or up to 10 where that saves a pass and the runs of equal digits, which are
+// then a quarter as long, are not too short for what DRAM takes at a time (kWidePairs, kWideKeys).
+// Ids with many repeats / all over the key space, distinct ones and sums, us: four passes and three
+// (30 bits, pairs): 2^20 93 / 92 and 78 / 86, 2^22 212 / 202 and 172 / 182, 10^7 456 / 444 and 382 /
+// 451, 2^24 703 / 674 and 623 / 708; five passes and four (40 bits): 10^6 113 / 113 and 102 / 106,
+// 2^22 251 / 262 and 260 / 306.
+//
+// Up to some million items everything stays in L2.  The single-sweep form (one launch per pass,
+// tiles finding their offsets by looking back over the words that earlier tiles publish) spent a
+// third of its time in the look-back and another third in a second wave of tiles: 54 us per pass
+// on 2^22 pairs against 41 us for three launches.  What bounds the scatter is the shared-memory
+// pipe (busy for 0.9 of the clocks of an SM at work): the accesses of a digit's random place, for
+// mask, counter, position and exchange.
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kItems = 8;                  // keys per thread and tile
+constexpr int kItems = 8;                  // keys per thread and tile of the one-CTA sort
 constexpr int kTile = kThreads * kItems;
 constexpr int kRadixBits = 8;
 constexpr int kDigits = 1 << kRadixBits;
+constexpr int kWideBits = 10;
 constexpr int kMaxChunks = 2 * 148;        // two CTAs per SM
+constexpr int kMinChunk = 2048;
+constexpr long long kWidePairs = 1 << 25, kWideKeys = 2 << 20;
 // Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
 // number of launches (64-bit keys without payload, 2^14 / 2^16, us: 119 / 110 with three launches
 // per pass, 64 / 74 with two; the single-sweep form 97 / 101).
@@ -56,15 +67,22 @@ struct SortHead {
   int too_wide;                            // 1: a key has bits beyond key_bits
 };
 
-// The chunks of n keys: `tiles` tiles each, the last ones possibly fewer.
+// The chunks of n items.  A tile of the scatter has `rows` rows of 32 items per warp; the tiles of
+// a chunk are equally long, so that no SM ends on a nearly empty one.
 struct Chunks {
   int count;
-  int tiles;
+  int size;  // items per chunk (the last one: what is left)
+  int rows;
 };
-__host__ __device__ inline Chunks chunks_of(long long n) {
-  const long long ntiles = (n + kTile - 1) / kTile;
-  const long long per = (ntiles + kMaxChunks - 1) / kMaxChunks;
-  return Chunks{(int)((ntiles + per - 1) / per), (int)per};
+inline Chunks chunks_of(long long n, int threads, int max_rows) {
+  long long per = (n + kMaxChunks - 1) / kMaxChunks;
+  if (per < kMinChunk) per = kMinChunk;
+  const long long tile = (long long)threads * max_rows, tiles = (per + tile - 1) / tile;
+  Chunks c;
+  c.rows = (int)((per + tiles * threads - 1) / (tiles * threads));
+  c.size = (int)(tiles * c.rows * threads);
+  c.count = (int)((n + c.size - 1) / c.size);
+  return c;
 }
 
 template <typename K>
@@ -77,8 +95,9 @@ __device__ __forceinline__ unsigned int lanemask_lt() {
   return m;
 }
 
-// Exclusive prefix sum of one value per thread over a CTA of kThreads; `part`: kWarps words of
+// Exclusive prefix sum of one value per thread over a CTA of WARPS warps; `part`: WARPS words of
 // shared memory, free again after the next __syncthreads.
+template <int WARPS = kWarps>
 __device__ __forceinline__ unsigned int cta_exclusive(unsigned int v, unsigned int* part,
                                                       unsigned int* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -92,7 +111,7 @@ __device__ __forceinline__ unsigned int cta_exclusive(unsigned int v, unsigned i
   __syncthreads();
   unsigned int before = 0, all = 0;
 #pragma unroll
-  for (int w = 0; w < kWarps; ++w) {
+  for (int w = 0; w < WARPS; ++w) {
     const unsigned int t = part[w];
     if (w < warp) before += t;
     all += t;
@@ -105,40 +124,46 @@ __device__ __forceinline__ unsigned int cta_exclusive(unsigned int v, unsigned i
 // one after the other and 227 chained, 153 035 of 24 bits 92 and 74.  What the kernel before has
 // written is read through L2 (__ldcg): a read-only path may not be used for it.
 
-// counts[d * chunks + c] = keys of chunk c whose digit is d
-template <typename K>
+using Item = unsigned long long;
+__device__ __forceinline__ unsigned int item_digit(Item k, int shift, unsigned int mask) {
+  return (unsigned int)(k >> shift) & mask;
+}
+
+// counts[c * 2^BITS + d] = items of chunk c whose digit is d
+template <int BITS>
 __global__ void __launch_bounds__(kThreads, 2)
-    digit_count_kernel(const K* __restrict__ keys, long long n, int shift, Chunks ch,
-                       int key_bits, unsigned int* counts, SortHead* head) {
+    digit_count_kernel(const Item* __restrict__ keys, long long n, int shift, unsigned int mask,
+                       Chunks ch, int key_bits, unsigned int* counts, SortHead* head) {
   grid_launch_next();
-  constexpr int kSets = 4;
-  __shared__ unsigned int s[kSets][kDigits];  // four warps share a set of counters
+  constexpr int kDigits = 1 << BITS, kSets = BITS > 8 ? 2 : 4;
+  constexpr int kItems = 14;  // (2^22 items: 28 per thread; 8.4 us, 8.9 with 8 loads in flight)
+  __shared__ unsigned int s[kSets][kDigits];  // groups of warps share a set of counters
   unsigned int* mine = s[threadIdx.x / (kThreads / kSets)];
   for (int i = threadIdx.x; i < kSets * kDigits; i += kThreads) s[0][i] = 0;
   grid_wait();
   __syncthreads();
-  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
-  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
+  const long long lo = (long long)blockIdx.x * ch.size;
+  const long long hi = lo + ch.size < n ? lo + ch.size : n;
   bool wide = false;
-  for (long long base = lo + threadIdx.x; base < hi; base += kTile) {
-    K k[kItems];
+  for (long long base = lo + threadIdx.x; base < hi; base += kThreads * kItems) {
+    Item k[kItems];
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
-      k[j] = base + j * kThreads < hi ? __ldcg(keys + base + j * kThreads) : (K)0;
+      k[j] = base + j * kThreads < hi ? __ldcg(keys + base + j * kThreads) : 0;
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
       if (base + j * kThreads < hi) {
-        if (sizeof(K) == 8 && key_bits < 64) wide |= (k[j] >> (key_bits & 63)) != 0;
-        atomicAdd(&mine[digit_of(k[j], shift)], 1u);
+        if (key_bits < 64) wide |= (k[j] >> (key_bits & 63)) != 0;
+        atomicAdd(&mine[item_digit(k[j], shift, mask)], 1u);
       }
   }
   if (wide) head->too_wide = 1;
   __syncthreads();
-  if (threadIdx.x < kDigits) {
+  for (int d = threadIdx.x; d < kDigits; d += kThreads) {
     unsigned int c = 0;
 #pragma unroll
-    for (int w = 0; w < kSets; ++w) c += s[w][threadIdx.x];
-    counts[(size_t)threadIdx.x * ch.count + blockIdx.x] = c;
+    for (int w = 0; w < kSets; ++w) c += s[w][d];
+    counts[(size_t)blockIdx.x * kDigits + d] = c;
   }
 }
 
@@ -152,29 +177,39 @@ __device__ __forceinline__ void host_report(unsigned long long* host, unsigned i
   __threadfence_system();
 }
 
-// One CTA per digit: exclusive prefix over the chunks in place, and the digit's total.
-__global__ void __launch_bounds__(kThreads)
-    digit_scan_kernel(unsigned int* counts, int chunks, unsigned int* totals) {
+// 32 digits per CTA: exclusive prefix over the chunks in place, and the digits' totals.  A warp
+// takes a run of chunks, a lane a digit.
+__global__ void __launch_bounds__(1024)
+    digit_scan_kernel(unsigned int* counts, int digits, int chunks, unsigned int* totals) {
   grid_launch_next();
   grid_wait();
-  __shared__ unsigned int s_part[kWarps];
-  static_assert(kMaxChunks <= kThreads && kDigits <= kThreads, "one thread per chunk, digit");
-  unsigned int* row = counts + (size_t)blockIdx.x * chunks;
-  const unsigned int c = threadIdx.x < chunks ? row[threadIdx.x] : 0;
-  unsigned int total;
-  const unsigned int before = cta_exclusive(c, s_part, &total);
-  if (threadIdx.x < chunks) row[threadIdx.x] = before;
-  if (threadIdx.x == 0) totals[blockIdx.x] = total;
+  constexpr int kRun = (kMaxChunks + 31) / 32;
+  __shared__ unsigned int s_part[32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int run = (chunks + 31) / 32, first = warp * run;
+  unsigned int* col = counts + blockIdx.x * 32 + lane;
+  unsigned int c[kRun], sum = 0;
+#pragma unroll
+  for (int i = 0; i < kRun; ++i)
+    c[i] = i < run && first + i < chunks ? __ldcg(col + (size_t)(first + i) * digits) : 0;
+#pragma unroll
+  for (int i = 0; i < kRun; ++i) sum += c[i];
+  s_part[warp][lane] = sum;
+  __syncthreads();
+  unsigned int before = 0;
+  for (int w = 0; w < warp; ++w) before += s_part[w][lane];
+#pragma unroll
+  for (int i = 0; i < kRun; ++i)
+    if (i < run && first + i < chunks) {
+      col[(size_t)(first + i) * digits] = before;
+      before += c[i];
+    }
+  if (warp == 31) totals[blockIdx.x * 32 + lane] = before;
 }
 
-// What travels beside the keys of a pass.
-enum { kNoPayload = 0, kMakeIndex = 1, kPayload = 2 };
-
-template <typename KO>
-constexpr int scatter_smem(int payload) {
-  return kTile * ((int)sizeof(KO) + (payload ? 4 : 0)) +
-         2 * kWarps * kDigits * 4 + 2 * kDigits * 4;
-}
+// What travels beside the keys of a pass: nothing, the key's index or a value of 32 bits in an
+// array of its own, or a value that a first pass puts below its key.
+enum { kNoPayload = 0, kMakeIndex = 1, kPayload = 2, kToPairs = 3 };
 
 // Rank of each of a thread's keys (index base + 32 j, below hi) among the keys of its warp that
 // have the same digit, in index order; cnt[d] ends up as the number of such keys.
@@ -204,120 +239,201 @@ __device__ __forceinline__ void rank_tile(const K* k, long long base, long long 
   }
 }
 
-// KI, KO: type of the keys as read and as written (a sort of short keys narrows them in its first
-// pass).  Shared memory: the tile's keys and payloads in sorted order, per-warp digit counters
-// and lane masks, and two 256-entry tables.
-template <typename KI, typename KO, int PAY>
-__global__ void __launch_bounds__(kThreads, 2)
-    scatter_kernel(const KI* __restrict__ keys_in, KO* __restrict__ keys_out,
+// Shared memory of a scatter: the tile's items and payloads in sorted order (before that, the lane
+// masks), the warps' digit counters and a table of output places.
+template <int BITS, int WARPS, int ROWS, bool ARRAY>
+struct ScatterCfg {
+  static constexpr int kDigits = 1 << BITS, kThreads = WARPS * 32, kTile = kThreads * ROWS;
+  static constexpr int kExchange = kTile * (8 + (ARRAY ? 4 : 0)), kMasks = WARPS * kDigits * 4;
+  static constexpr int kShared = kExchange > kMasks ? kExchange : kMasks;
+  static constexpr int kSmemBytes = kShared + WARPS * kDigits * 2 + kDigits * 4;
+};
+// Two CTAs per SM, of 16 warps with 14 rows each (2^22 pairs, 10 bits: 132 us; 8 warps with 28
+// rows 133, 16 with 16 rows 137, one CTA of 32 warps with 14 rows 156); with small chunks 8 warps
+// with 16 rows, whose counters are fewer (2^17 pairs: 36 and 39 us).
+template <int BITS, int WARPS, int ROWS, int PAY>
+__global__ void __launch_bounds__(WARPS * 32, 2)
+    scatter_kernel(const Item* __restrict__ keys_in, Item* __restrict__ keys_out,
                    const unsigned int* __restrict__ pay_in, unsigned int* __restrict__ pay_out,
-                   long long n, int shift, Chunks ch, const unsigned int* __restrict__ prefix,
+                   long long n, int shift, unsigned int mask, Chunks ch,
+                   const unsigned int* __restrict__ prefix,
                    const unsigned int* __restrict__ totals) {
   grid_launch_next();
+  constexpr bool kArray = PAY == kMakeIndex || PAY == kPayload;
+  using C = ScatterCfg<BITS, WARPS, ROWS, kArray>;
+  constexpr int kDigits = C::kDigits, kThreads = C::kThreads, kPairs = kDigits / 2;
+  constexpr int kPer = kPairs > kThreads ? kPairs / kThreads : 1;  // pairs of digits per thread
+  static_assert(kPairs % kThreads == 0 || kThreads % kPairs == 0, "every pair has a thread");
+  static_assert(ROWS % 2 == 0 && C::kTile < 65536, "ranks and positions have 16 bits");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  KO* skeys = reinterpret_cast<KO*>(smem_raw);
-  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + kTile * sizeof(KO));
-  // cnt[w][d]: first the number of keys with digit d seen so far by warp w, afterwards the
-  // sorted position in the tile of that warp's first key with digit d
-  unsigned int (*cnt)[kDigits] = reinterpret_cast<unsigned int (*)[kDigits]>(
-      smem_raw + kTile * sizeof(KO) + (PAY ? kTile * 4 : 0));
-  // lanes[w][d]: lanes of warp w whose present key has digit d; zero in between
-  unsigned int (*lanes)[kDigits] = cnt + kWarps;
-  unsigned int* goff = &lanes[kWarps][0];  // output index of sorted position q: goff[d] + q
-  __shared__ unsigned int s_part[2][kWarps];
+  Item* skeys = reinterpret_cast<Item*>(smem_raw);
+  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + C::kTile * 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool digit = threadIdx.x < kDigits;
-  for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) lanes[0][i] = 0;
+  // lanes[d]: lanes of this warp whose present item has digit d; zero in between.  The memory of
+  // the exchange, which begins when all warps have their ranks.
+  unsigned int* lanes = reinterpret_cast<unsigned int*>(smem_raw) + warp * kDigits;
+  // cnt[d]: first the number of items with digit d seen so far by this warp, afterwards the sorted
+  // position in the tile of its first one.  count2: the counters of digits 2 i and 2 i + 1 at once.
+  unsigned short* cnt =
+      reinterpret_cast<unsigned short*>(smem_raw + C::kShared) + warp * kDigits;
+  unsigned int* count2 = reinterpret_cast<unsigned int*>(smem_raw + C::kShared);
+  // output index of sorted position q: goff[d] + q
+  unsigned int* goff = reinterpret_cast<unsigned int*>(smem_raw + C::kShared + WARPS * kDigits * 2);
+  __shared__ unsigned int s_part[2][WARPS];
+  const bool digits = threadIdx.x * kPer < kPairs;
   grid_wait();
-  // output index of the chunk's next key with digit threadIdx.x
-  unsigned int before = 0, total = 0;
-  if (digit) {
-    const unsigned int* row = prefix + (size_t)threadIdx.x * ch.count;
+  // output index of the chunk's next item with each of this thread's digits
+  unsigned int next[2 * kPer], total[2 * kPer], mine = 0;
+#pragma unroll
+  for (int i = 0; i < 2 * kPer; ++i) next[i] = total[i] = 0;
+  if (digits) {
+    const int d0 = threadIdx.x * 2 * kPer;
     if (totals) {
-      before = __ldcg(row + blockIdx.x);
-      total = __ldcg(totals + threadIdx.x);
-    } else {
-      for (int c = 0; c < ch.count; ++c) {
-        const unsigned int v = __ldcg(row + c);
-        if (c < blockIdx.x) before += v;
-        total += v;
+#pragma unroll
+      for (int i = 0; i < 2 * kPer; ++i) {
+        next[i] = __ldcg(prefix + (size_t)blockIdx.x * kDigits + d0 + i);
+        total[i] = __ldcg(totals + d0 + i);
       }
+    } else {
+      for (int c = 0; c < ch.count; ++c)
+#pragma unroll
+        for (int i = 0; i < 2 * kPer; ++i) {
+          const unsigned int v = __ldcg(prefix + (size_t)c * kDigits + d0 + i);
+          if (c < blockIdx.x) next[i] += v;
+          total[i] += v;
+        }
     }
+#pragma unroll
+    for (int i = 0; i < 2 * kPer; ++i) mine += total[i];
   }
-  unsigned int next = cta_exclusive(total, s_part[0], nullptr) + before;
-  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
-  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
-  // A tile is loaded before the one before it is stored: its keys and payloads take the registers
+  unsigned int smaller = cta_exclusive<WARPS>(mine, s_part[0], nullptr);
+#pragma unroll
+  for (int i = 0; i < 2 * kPer; ++i) {
+    next[i] += smaller;
+    smaller += total[i];
+  }
+  const long long lo = (long long)blockIdx.x * ch.size;
+  const long long hi = lo + ch.size < n ? lo + ch.size : n;
+  const int rows = ch.rows, tile = kThreads * rows;
+  // A tile is loaded before the one before it is stored: its items and payloads take the registers
   // of those that have gone to shared memory.
-  KO k[kItems];
-  unsigned int pay[kItems];
+  Item k[ROWS];
+  unsigned int pay[kArray ? ROWS : 1];
   auto load = [&](long long base) {
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
+    for (int j = 0; j < ROWS; ++j) {
+      if (j >= rows) break;
       const long long i = base + j * 32;
-      k[j] = i < hi ? (KO)__ldcg(keys_in + i) : (KO)~0ull;
+      k[j] = i < hi ? __ldcg(keys_in + i) : ~0ull;
+      if constexpr (PAY == kToPairs) k[j] = k[j] << 32 | (i < hi ? __ldcg(pay_in + i) : 0u);
       if constexpr (PAY == kPayload) pay[j] = i < hi ? __ldcg(pay_in + i) : 0u;
-      else pay[j] = (unsigned int)i;
+      if constexpr (PAY == kMakeIndex) pay[j] = (unsigned int)i;
     }
   };
-  load(lo + (long long)warp * (32 * kItems) + lane);
-  for (long long tile_base = lo; tile_base < hi; tile_base += kTile) {
-    const long long base = tile_base + (long long)warp * (32 * kItems) + lane;
-    const int tile_n = (int)(hi - tile_base < kTile ? hi - tile_base : kTile);
-    unsigned int rank[kItems];
-    for (int i = threadIdx.x; i < kWarps * kDigits; i += kThreads) cnt[0][i] = 0;
-    __syncthreads();
-    rank_tile(k, base, hi, shift, cnt[warp], lanes[warp], rank);
-    __syncthreads();
-    // digit threadIdx.x: where its run starts in the tile, and each warp's part of it
-    unsigned int run = 0;
-    if (digit) {
+  load(lo + (long long)warp * (32 * rows) + lane);
+  for (long long tile_base = lo; tile_base < hi; tile_base += tile) {
+    const long long base = tile_base + (long long)warp * (32 * rows) + lane;
+    const int tile_n = (int)(hi - tile_base < tile ? hi - tile_base : tile);
+    for (int i = lane; i < kDigits; i += 32) lanes[i] = 0;
+    for (int i = lane; i < kPairs; i += 32) reinterpret_cast<unsigned int*>(cnt)[i] = 0;
+    __syncwarp();
+    unsigned int rank[ROWS / 2];  // two of 16 bits each
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) run += cnt[w][threadIdx.x];
-    }
-    const unsigned int start = cta_exclusive(run, s_part[1], nullptr);
-    if (digit) {
-      unsigned int at = start;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        const unsigned int c = cnt[w][threadIdx.x];
-        cnt[w][threadIdx.x] = at;
-        at += c;
+    for (int j = 0; j < ROWS; ++j) {
+      if (j >= rows) break;
+      // the lanes that hold the same digit find each other through a mask in shared memory (32 keys
+      // of an SM in 9 ns; 15 with ballots, 32 with match.any); the first of them advances the
+      // warp's counter for all of them
+      const bool valid = base + j * 32 < hi;
+      const unsigned int d = item_digit(k[j], shift, mask);
+      if (valid) atomicOr(&lanes[d], 1u << lane);
+      __syncwarp();
+      const unsigned int same = valid ? lanes[d] : 1u << lane;
+      const unsigned int before = __popc(same & lanemask_lt());
+      unsigned int r = 0;
+      __syncwarp();
+      if (valid && before == 0) {
+        lanes[d] = 0;
+        r = cnt[d];
+        cnt[d] = (unsigned short)(r + __popc(same));
       }
-      goff[threadIdx.x] = next - start;
-      next += run;
+      r = __shfl_sync(0xffffffffu, r, __ffs(same) - 1) + before;
+      if (j & 1) rank[j / 2] |= r << 16;
+      else rank[j / 2] = r;
+      __syncwarp();
+    }
+    __syncthreads();
+    // where the runs of this thread's digits start in the tile, and each warp's part of them
+    unsigned int run[kPer], items = 0;
+    if (digits) {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        run[i] = 0;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) run[i] += count2[w * kPairs + threadIdx.x * kPer + i];
+        items += (run[i] & 0xffffu) + (run[i] >> 16);
+      }
+    }
+    unsigned int start = cta_exclusive<WARPS>(items, s_part[1], nullptr);
+    if (digits) {
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const unsigned int r0 = run[i] & 0xffffu, r1 = run[i] >> 16;
+        const int d = (threadIdx.x * kPer + i) * 2;
+        unsigned int at = start | (start + r0) << 16;
+        goff[d] = next[2 * i] - start;
+        goff[d + 1] = next[2 * i + 1] - (start + r0);
+        next[2 * i] += r0;
+        next[2 * i + 1] += r1;
+        start += r0 + r1;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+          unsigned int* p = &count2[w * kPairs + threadIdx.x * kPer + i];
+          const unsigned int c = *p;
+          *p = at;
+          at += c;
+        }
+      }
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
+    for (int j = 0; j < ROWS; ++j) {
+      if (j >= rows) break;
       if (base + j * 32 < hi) {
-        const unsigned int q = cnt[warp][digit_of(k[j], shift)] + rank[j];
+        const unsigned int q = cnt[item_digit(k[j], shift, mask)] +
+                               ((j & 1) ? rank[j / 2] >> 16 : rank[j / 2] & 0xffffu);
         skeys[q] = k[j];
-        if constexpr (PAY != kNoPayload) spay[q] = pay[j];
+        if constexpr (kArray) spay[q] = pay[j];
       }
     }
-    load(base + kTile);
+    load(base + tile);
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kItems; ++j) {
+    for (int j = 0; j < ROWS; ++j) {
+      if (j >= rows) break;
       const int q = threadIdx.x + j * kThreads;
       if (q < tile_n) {
-        const KO key = skeys[q];
-        const unsigned int p = goff[digit_of(key, shift)] + (unsigned int)q;
+        const Item key = skeys[q];
+        const unsigned int p = goff[item_digit(key, shift, mask)] + (unsigned int)q;
         keys_out[p] = key;
-        if constexpr (PAY != kNoPayload) pay_out[p] = spay[q];
+        if constexpr (kArray) pay_out[p] = spay[q];
       }
     }
+    __syncthreads();
   }
 }
 
 // All passes of a sort of at most one tile in one launch of one CTA (the three launches per pass of
 // the general form take longer than the work: 2^12 keys of 24 bits, with the sums of equal
 // keys, 111 us in nine launches).  `unique`: receives the number of distinct keys, or NULL;
-// `host`: the report for the host (see host_report), or NULL.
-template <typename KI, typename K, int PAY>
+// `host`: the report for the host (see host_report), or NULL.  Keys of 32 bits come out as pairs.
+template <typename K, int PAY>
+constexpr int small_smem() {
+  return kTile * ((int)sizeof(K) + (PAY ? 4 : 0)) + 2 * kWarps * kDigits * 4;
+}
+template <typename K, int PAY>
 __global__ void __launch_bounds__(kThreads)
-    small_sort_kernel(const KI* keys_in, K* keys_out, const unsigned int* pay_in,
+    small_sort_kernel(const Item* keys_in, Item* keys_out, const unsigned int* pay_in,
                       unsigned int* pay_out, int n, int passes, int key_bits, SortHead* head,
                       unsigned int* unique, unsigned long long* host) {
   grid_launch_next();
@@ -333,8 +449,8 @@ __global__ void __launch_bounds__(kThreads)
   const int base = warp * (32 * kItems) + lane;
   bool wide = false;
   for (int i = threadIdx.x; i < n; i += kThreads) {
-    const KI k = keys_in[i];
-    if (sizeof(KI) == 8 && key_bits < 64) wide |= (k >> (key_bits & 63)) != 0;
+    const Item k = keys_in[i];
+    if (key_bits < 64) wide |= (k >> (key_bits & 63)) != 0;
     skeys[i] = (K)k;
     if constexpr (PAY != kNoPayload) spay[i] = PAY == kPayload ? pay_in[i] : (unsigned int)i;
   }
@@ -381,8 +497,12 @@ __global__ void __launch_bounds__(kThreads)
   }
   unsigned int heads = 0;
   for (int i = threadIdx.x; i < n; i += kThreads) {
-    keys_out[i] = skeys[i];
-    if constexpr (PAY != kNoPayload) pay_out[i] = spay[i];
+    if constexpr (sizeof(K) == 4) {
+      keys_out[i] = (Item)skeys[i] << 32 | spay[i];
+    } else {
+      keys_out[i] = skeys[i];
+      if constexpr (PAY != kNoPayload) pay_out[i] = spay[i];
+    }
     heads += i == 0 || skeys[i] != skeys[i - 1];
   }
   if (unique) {
@@ -403,15 +523,20 @@ struct SortWork {
   SortHead* head;
   unsigned int* counts;
   unsigned int* totals;
-  static size_t bytes(long long n) {
-    return round256(sizeof(SortHead)) + round256((size_t)kDigits * chunks_of(n).count * 4) +
-           round256(kDigits * 4);
+  // (no form has more chunks than items / kMinChunk, nor more than kMaxChunks)
+  static size_t count_bytes(long long n, int bits) {
+    long long chunks = n / kMinChunk + 1;
+    if (chunks > kMaxChunks) chunks = kMaxChunks;
+    return round256(((size_t)chunks << bits) * 4);
   }
-  SortWork(char* p, long long n) {
+  static size_t bytes(long long n, int bits) {
+    return round256(sizeof(SortHead)) + count_bytes(n, bits) + round256((size_t)4 << bits);
+  }
+  SortWork(char* p, long long n, int bits) {
     head = reinterpret_cast<SortHead*>(p);
     p += round256(sizeof(SortHead));
     counts = reinterpret_cast<unsigned int*>(p);
-    p += round256((size_t)kDigits * chunks_of(n).count * 4);
+    p += count_bytes(n, bits);
     totals = reinterpret_cast<unsigned int*>(p);
   }
 };
@@ -431,209 +556,297 @@ static int allow_smem(int bytes) {
   return 0;
 }
 
-template <typename KI, typename K, int PAY>
-static int small_sort(const KI* in, K* out, const unsigned int* pin, unsigned int* pout, int n,
+template <typename K, int PAY>
+static int small_sort(const Item* in, Item* out, const unsigned int* pin, unsigned int* pout, int n,
                       int passes, int key_bits, SortHead* head, unsigned int* unique,
                       unsigned long long* host, cudaStream_t s) {
-  if (int rc = allow_smem<small_sort_kernel<KI, K, PAY>>(scatter_smem<K>(PAY))) return rc;
-  const int rc = launch_chained(small_sort_kernel<KI, K, PAY>, 1, kThreads, scatter_smem<K>(PAY), s,
-                                1, in, out, pin, pout, n, passes, key_bits, head, unique, host);
+  if (int rc = allow_smem<small_sort_kernel<K, PAY>>(small_smem<K, PAY>())) return rc;
+  const int rc = launch_chained(small_sort_kernel<K, PAY>, 1, kThreads, small_smem<K, PAY>(), s, 1,
+                                in, out, pin, pout, n, passes, key_bits, head, unique, host);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return rc;
 }
 
-template <typename KI, typename KO, int PAY>
-static int sort_pass(const KI* in, KO* out, const unsigned int* pin, unsigned int* pout,
-                     long long n, int pass, int key_bits, const SortWork& w, cudaStream_t s) {
-  if (int rc = allow_smem<scatter_kernel<KI, KO, PAY>>(scatter_smem<KO>(PAY))) return rc;
-  const Chunks ch = chunks_of(n);
-  const int shift = pass * kRadixBits;
-  int rc = launch_chained(digit_count_kernel<KI>, ch.count, kThreads, 0, s, 1, in, n, shift, ch,
-                          pass ? 64 : key_bits, w.counts, w.head);
+struct Pass {
+  const Item* in;
+  Item* out;
+  const unsigned int* pin;
+  unsigned int* pout;
+  long long n;
+  int shift, width;    // of the digit in an item
+  int count_shift;     // and in the items as they are read
+  int check_bits;      // of the keys, 64: not checked
+};
+template <int BITS, int WARPS, int ROWS, int PAY>
+static int sort_pass(const Pass& p, const SortWork& w, cudaStream_t s) {
+  using C = ScatterCfg<BITS, WARPS, ROWS, PAY == kMakeIndex || PAY == kPayload>;
+  if (int rc = allow_smem<scatter_kernel<BITS, WARPS, ROWS, PAY>>(C::kSmemBytes)) return rc;
+  const Chunks ch = chunks_of(p.n, C::kThreads, ROWS);
+  const unsigned int mask = (1u << p.width) - 1;
+  int rc = launch_chained(digit_count_kernel<BITS>, ch.count, kThreads, 0, s, 1, p.in, p.n,
+                          p.count_shift, mask, ch, p.check_bits, w.counts, w.head);
   const bool scan = ch.count > kSelfScan;
   if (!rc && scan)
-    rc = launch_chained(digit_scan_kernel, kDigits, kThreads, 0, s, 1, w.counts, ch.count,
-                        w.totals);
+    rc = launch_chained(digit_scan_kernel, C::kDigits / 32, 1024, 0, s, 1, w.counts, C::kDigits,
+                        ch.count, w.totals);
   if (!rc)
-    rc = launch_chained(scatter_kernel<KI, KO, PAY>, ch.count, kThreads, scatter_smem<KO>(PAY), s,
-                        1, in, out, pin, pout, n, shift, ch, w.counts,
-                        scan ? w.totals : nullptr);
+    rc = launch_chained(scatter_kernel<BITS, WARPS, ROWS, PAY>, ch.count, C::kThreads,
+                        C::kSmemBytes, s, 1, p.in, p.out, p.pin, p.pout, p.n, p.shift, mask, ch,
+                        w.counts, scan ? w.totals : nullptr);
   g_launches.fetch_add(scan ? 3 : 2, std::memory_order_relaxed);
   return rc;
 }
+// The form of a pass by its digits and the length of its chunks (ScatterCfg).
+template <int PAY>
+static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) {
+  if (bits == kRadixBits) return sort_pass<kRadixBits, 16, 8, PAY>(p, w, s);
+  if constexpr (PAY == kMakeIndex) {
+    return PSDEV_ERR_ARG;
+  } else {
+    if (p.n <= kMaxChunks * 4096ll) return sort_pass<kWideBits, 8, 16, PAY>(p, w, s);
+    return sort_pass<kWideBits, 16, PAY == kPayload ? 10 : 14, PAY>(p, w, s);
+  }
+}
 
 // ---- sums of the values of equal keys --------------------------------------------------------
-// On sorted (key, value) pairs, in two kernels with the allocation of the outputs between them:
-// unique_count counts the first occurrences in each chunk, unique_sum writes every distinct key
-// and the sum of its values.  Their chunks are smaller than those of the sort (a CTA has little
-// to do per pair): up to 2048, as many counts as unique_sum adds up at its start.
-constexpr int kMaxUniqueChunks = 2048;
-__host__ __device__ inline Chunks unique_chunks_of(long long n) {
-  const long long ntiles = (n + kTile - 1) / kTile;
-  const long long per = (ntiles + kMaxUniqueChunks - 1) / kMaxUniqueChunks;
-  return Chunks{(int)((ntiles + per - 1) / per), (int)per};
-}
-
-template <typename K>
-__global__ void __launch_bounds__(kThreads, 2)
-    unique_count_kernel(const K* __restrict__ keys, long long n, Chunks ch, unsigned int* counts) {
-  grid_launch_next();
-  grid_wait();
-  __shared__ unsigned int s_part[kWarps];
-  const int lane = threadIdx.x & 31;
-  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
-  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
-  unsigned int heads = 0;
-  for (long long base = lo + threadIdx.x; base - lane < hi; base += kTile) {
-    K k[kItems], before[kItems];  // before: of lane 0, the last key of the warp's neighbour
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-      const long long i = base + j * kThreads;
-      k[j] = i < hi ? __ldcg(keys + i) : (K)0;
-      before[j] = lane == 0 && i > 0 && i < hi ? __ldcg(keys + i - 1) : (K)0;
-    }
-#pragma unroll
-    for (int j = 0; j < kItems; ++j) {
-      const long long i = base + j * kThreads;
-      const K up = __shfl_up_sync(0xffffffffu, k[j], 1);
-      heads += i < hi && (i == 0 || k[j] != (lane ? up : before[j]));
-    }
-  }
-  unsigned int total;
-  cta_exclusive(heads, s_part, &total);
-  if (threadIdx.x == 0) counts[blockIdx.x] = total;
-}
-
-// Adds up the chunks' counts for the host.  A kernel that writes a word of mapped memory which the
-// host polls is cheaper than a copy and a wait for the stream (with the call from Python native:
-// 4096 ids 58 us before, 41 now; 2^22 216 and 204).
-__global__ void __launch_bounds__(kThreads)
-    unique_total_kernel(const unsigned int* counts, int chunks, const SortHead* head,
-                        unsigned long long* host) {
-  __shared__ unsigned int s_part[kWarps];
-  grid_launch_next();
-  grid_wait();
-  unsigned int c = 0, total;
-  for (int i = threadIdx.x; i < chunks; i += kThreads) c += __ldcg(counts + i);
-  cta_exclusive(c, s_part, &total);
-  if (threadIdx.x == 0) host_report(host, total, __ldcg(&head->too_wide) != 0);
-}
-
-// Each thread walks kPer consecutive pairs of a round and adds up what belongs to one key; a
-// segmented scan over the threads carries open sums on, so that a key that fills whole chunks
-// costs no atomics inside one.  Keys that begin and end inside a round are stored; what is open at
-// either end of a round is added to its (cleared) output, two global atomics per round.
+// On sorted (key, value) pairs, in three kernels, the outputs allocated before the last:
+//   unique_local  every CTA adds up the values of equal keys in a round of pairs and stores its
+//                 distinct keys and their sums at the round's place in a scratch array.  A key
+//                 belongs to the round that it begins in; what a round finds of a key that began
+//                 before is its lead;
+//   unique_scan   one CTA: prefix of the rounds' counts, and the report to the host;
+//   unique_gather moves every round's keys and sums to their places and adds the leads of the
+//                 rounds behind it to its last sum.
+// Of 2^22 pairs with 0.85 million keys they take 15, 5 and 12 us, cold; the form before, which
+// counted the distinct keys, waited for the outputs and then went over the pairs once more, 9, 5
+// and 22.
+// Nothing is added up with atomics: sums do not depend on the order of the CTAs.
+constexpr int kUniqueThreads = 256;
 constexpr int kUniquePer = 8;
-template <typename K>
-__global__ void __launch_bounds__(kThreads, 2)
-    unique_sum_kernel(const K* __restrict__ keys, const float* __restrict__ vals, long long n,
-                      Chunks ch, const unsigned int* __restrict__ counts,
-                      unsigned long long* out_keys, float* out_sums) {
-  grid_launch_next();
-  grid_wait();
-  constexpr int kPer = kUniquePer;
-  constexpr int kRound = kThreads * kPer;
-  constexpr int kPadded = kRound + kRound / kPer;  // (a thread's pairs start in different banks)
+constexpr int kRound = kUniqueThreads * kUniquePer;
+template <bool PAIRS, int THREADS>
+constexpr int unique_smem() {  // (a thread's pairs start in different banks)
+  return THREADS * (kUniquePer + 1) * (8 + (PAIRS ? 0 : 4));
+}
+static inline long long rounds_of(long long n) { return (n + kRound - 1) / kRound; }
+
+struct Unique {
+  const Item* items;          // sorted: keys, or pairs
+  const float* vals;          // values of keys; NULL: pairs
+  long long n;
+  Item* keys;                 // distinct keys (with their sums: pairs) of every round
+  float* sums;
+  unsigned int* counts;       // of every round, later their prefix
+  float* leads;
+  unsigned long long* out_keys;  // one round only: the outputs, or NULL
+  float* out_sums;
+};
+
+template <bool PAIRS, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1536 / THREADS)
+    unique_local_kernel(const __grid_constant__ Unique u) {
+  constexpr int kPer = kUniquePer, kWarps = THREADS / 32, kRound = THREADS * kPer;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  K* skey = reinterpret_cast<K*>(smem_raw);
-  K* ukey = skey + kPadded;                        // distinct keys of the round, from 1
-  float* sval = reinterpret_cast<float*>(ukey + kRound + 1);
-  float* usum = sval + kPadded;                    // 0: the key that was open before the round
+  Item* s_item = reinterpret_cast<Item*>(smem_raw);
+  float* s_val = reinterpret_cast<float*>(smem_raw + THREADS * (kPer + 1) * 8);
   __shared__ unsigned int s_part[kWarps];
   __shared__ float s_tail[kWarps];
   __shared__ bool s_flag[kWarps];
+  grid_launch_next();
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // index of the chunk's first new key: what the chunks before found
-  unsigned int next;
-  {
-    unsigned int c = 0;
-    for (int i = threadIdx.x; i < blockIdx.x; i += kThreads) c += __ldcg(counts + i);
-    cta_exclusive(c, s_part, &next);
+  const long long base = (long long)blockIdx.x * kRound;
+  const int count = (int)(u.n - base < kRound ? u.n - base : kRound);
+  const Item* items = u.items + base;
+  auto key_of = [](Item i) { return PAIRS ? i >> 32 : i; };
+  const bool follows = base > 0;  // (is the first pair's key that of the pair before the round?)
+  const Item last = follows ? key_of(__ldcg(items - 1)) : 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int q = threadIdx.x + j * THREADS;
+    if (q < count) {
+      s_item[q + q / kPer] = __ldcg(items + q);
+      if constexpr (!PAIRS) s_val[q + q / kPer] = __ldcg(u.vals + base + q);
+    }
   }
-  const long long lo = (long long)blockIdx.x * ch.tiles * kTile;
-  const long long hi = lo + (long long)ch.tiles * kTile < n ? lo + (long long)ch.tiles * kTile : n;
-  for (long long base = lo; base < hi; base += kRound) {
-    const int count = (int)(hi - base < kRound ? hi - base : kRound);
-    __syncthreads();
+  __syncthreads();
+  const int q0 = threadIdx.x * kPer, p0 = q0 + threadIdx.x;
+  Item key[kPer];
+  float val[kPer];
+  Item prev = last;
+  if (q0 > 0 && q0 < count) prev = key_of(s_item[p0 - 2]);
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const int q = threadIdx.x + j * kThreads;
-      if (q < count) {
-        skey[q + q / kPer] = __ldcg(keys + base + q);
-        sval[q + q / kPer] = __ldcg(vals + base + q);
-      }
-    }
-    __syncthreads();
-    const int q0 = threadIdx.x * kPer, p0 = q0 + threadIdx.x;
-    K prev{};
-    if (q0 < count) {
-      if (q0 > 0) prev = skey[p0 - 2];
-      else if (base > 0) prev = __ldcg(keys + base - 1);
-    }
-    bool head[kPer];
-    unsigned int heads = 0;
+  for (int j = 0; j < kPer; ++j) {
+    const bool valid = q0 + j < count;
+    const Item i = valid ? s_item[p0 + j] : 0;
+    key[j] = key_of(i);
+    val[j] = 0.f;
+    if constexpr (PAIRS) val[j] = valid ? __uint_as_float((unsigned int)i) : 0.f;
+    else if (valid) val[j] = s_val[p0 + j];
+  }
+  bool head[kPer];
+  unsigned int heads = 0;
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      const bool valid = q0 + j < count;
-      const K key = valid ? skey[p0 + j] : prev;
-      head[j] = valid && (base + q0 + j == 0 || key != prev);
-      heads += head[j];
-      prev = key;
-    }
-    unsigned int total;
-    unsigned int slot = cta_exclusive(heads, s_part, &total);  // slot of the key open before q0
-    // sum of what belongs to that key, then the thread's own keys; the last one stays open
-    const unsigned int first_slot = slot;
-    float lead = 0.f, sum = 0.f;
+  for (int j = 0; j < kPer; ++j) {
+    const bool valid = q0 + j < count;
+    head[j] = valid && ((q0 + j == 0 && !follows) || key[j] != prev);
+    heads += head[j];
+    if (valid) prev = key[j];
+  }
+  unsigned int total;
+  // (all threads have read their pairs: the memory is free for the round's keys and sums)
+  const unsigned int first_slot = cta_exclusive<kWarps>(heads, s_part, &total);
+  // Slot i holds the i-th key that begins here, slot 0 (with its own place) the lead.  A thread's
+  // sum of what belongs to the slot that is open before its first pair, then its own slots; the
+  // last one stays open.
+  Item* slot_key = s_item;
+  float* slot_sum = PAIRS ? nullptr : s_val;
+  auto put_sum = [&](unsigned int slot, float v) {
+    if constexpr (PAIRS)
+      reinterpret_cast<unsigned int*>(slot_key + slot)[0] = __float_as_uint(v);
+    else
+      slot_sum[slot] = v;
+  };
+  unsigned int slot = first_slot;
+  float lead = 0.f, sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-      if (head[j]) {
-        if (slot == first_slot) lead = sum;
-        else usum[slot] = sum;
-        ++slot;
-        sum = 0.f;
-        ukey[slot] = skey[p0 + j];
-      }
-      if (q0 + j < count) sum += sval[p0 + j];
+  for (int j = 0; j < kPer; ++j) {
+    if (head[j]) {
+      if (slot == first_slot) lead = sum;
+      else put_sum(slot, sum);
+      ++slot;
+      sum = 0.f;
+      if constexpr (PAIRS)
+        reinterpret_cast<unsigned int*>(slot_key + slot)[1] = (unsigned int)key[j];
+      else
+        slot_key[slot] = key[j];
     }
-    // segmented inclusive scan of (has heads, open sum) over the threads
-    const bool any = heads > 0;
-    bool f = any;
-    float v = sum;
+    sum += val[j];
+  }
+  // segmented inclusive scan of (has heads, open sum) over the threads
+  const bool any = heads > 0;
+  bool f = any;
+  float v = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float pv = __shfl_up_sync(0xffffffffu, v, o);
-      const bool pf = __shfl_up_sync(0xffffffffu, f, o);
-      if (lane >= o) {
-        if (!f) v += pv;
-        f |= pf;
-      }
+  for (int o = 1; o < 32; o <<= 1) {
+    const float pv = __shfl_up_sync(0xffffffffu, v, o);
+    const bool pf = __shfl_up_sync(0xffffffffu, f, o);
+    if (lane >= o) {
+      if (!f) v += pv;
+      f |= pf;
     }
-    if (lane == 31) {
-      s_tail[warp] = v;
-      s_flag[warp] = f;
+  }
+  if (lane == 31) {
+    s_tail[warp] = v;
+    s_flag[warp] = f;
+  }
+  float carry = __shfl_up_sync(0xffffffffu, v, 1);
+  bool carried = __shfl_up_sync(0xffffffffu, f, 1);
+  if (lane == 0) {
+    carry = 0.f;
+    carried = false;
+  }
+  __syncthreads();
+  if (!carried)
+    for (int w = warp - 1; w >= 0; --w) {
+      carry += s_tail[w];
+      if (s_flag[w]) break;
     }
-    float carry = __shfl_up_sync(0xffffffffu, v, 1);
-    bool carried = __shfl_up_sync(0xffffffffu, f, 1);
-    if (lane == 0) {
-      carry = 0.f;
-      carried = false;
+  if (any) put_sum(first_slot, carry + lead);
+  if (threadIdx.x == THREADS - 1) put_sum(total, any ? sum : carry + sum);
+  __syncthreads();
+  auto sum_at = [&](unsigned int i) {
+    if constexpr (PAIRS) return __uint_as_float((unsigned int)slot_key[i]);
+    else return slot_sum[i];
+  };
+  if (threadIdx.x == 0 && u.counts) {
+    u.counts[blockIdx.x] = total;
+    u.leads[blockIdx.x] = follows ? sum_at(0) : 0.f;
+  }
+  for (unsigned int i = threadIdx.x; i < total; i += THREADS) {
+    if (u.out_keys) {
+      u.out_keys[i] = key_of(slot_key[i + 1]);
+      u.out_sums[i] = sum_at(i + 1);
+    } else {
+      u.keys[base + i] = slot_key[i + 1];
+      if constexpr (!PAIRS) u.sums[base + i] = slot_sum[i + 1];
     }
-    __syncthreads();
-    if (!carried)
-      for (int w = warp - 1; w >= 0; --w) {
-        carry += s_tail[w];
-        if (s_flag[w]) break;
-      }
-    if (any) usum[first_slot] = carry + lead;
-    if (threadIdx.x == kThreads - 1) usum[total] = any ? sum : carry + sum;
-    __syncthreads();
-    for (unsigned int u = threadIdx.x; u <= total; u += kThreads) {
-      if (u > 0) out_keys[next + u - 1] = (unsigned long long)ukey[u];
-      if (u > 0 && u < total) out_sums[next + u - 1] = usum[u];
-      else if (next + u > 0) atomicAdd(&out_sums[next + u - 1], usum[u]);
+  }
+}
+
+// A kernel that writes a word of mapped memory which the host polls is cheaper than a copy and a
+// wait for the stream (with the call from Python native: 4096 ids 58 us before, 41 now; 2^22 216
+// and 204).
+__global__ void __launch_bounds__(kThreads)
+    unique_scan_kernel(unsigned int* counts, int rounds, const SortHead* head,
+                       unsigned long long* host) {
+  __shared__ unsigned int s_part[2][kWarps];
+  grid_launch_next();
+  grid_wait();
+  constexpr int kEach = 4;
+  unsigned int before = 0;
+  int turn = 0;
+  for (int r0 = 0; r0 < rounds; r0 += kThreads * kEach, turn ^= 1) {
+    const int i0 = r0 + threadIdx.x * kEach;
+    unsigned int c[kEach], mine = 0, all;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) c[j] = i0 + j < rounds ? __ldcg(counts + i0 + j) : 0;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) mine += c[j];
+    unsigned int at = before + cta_exclusive(mine, s_part[turn], &all);
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      if (i0 + j < rounds) counts[i0 + j] = at;
+      at += c[j];
     }
-    next += total;
+    before += all;
+  }
+  if (threadIdx.x == 0) {
+    counts[rounds] = before;
+    host_report(host, before, __ldcg(&head->too_wide) != 0);
+  }
+}
+
+template <bool PAIRS>
+__global__ void __launch_bounds__(kUniqueThreads)
+    unique_gather_kernel(const __grid_constant__ Unique u, int rounds) {
+  grid_launch_next();
+  grid_wait();
+  const unsigned int at = __ldcg(u.counts + blockIdx.x);
+  const unsigned int count = __ldcg(u.counts + blockIdx.x + 1) - at;
+  const long long base = (long long)blockIdx.x * kRound;
+  if (count == 0) return;
+  // what the rounds behind have found of the last key (a warp looks at 32 of them at a time)
+  float more = 0.f;
+  if (threadIdx.x < 32) {
+    for (int r0 = blockIdx.x + 1;; r0 += 32) {
+      const int r = r0 + (int)threadIdx.x;
+      const bool in = r < rounds;
+      const float lead = in ? __ldcg(u.leads + r) : 0.f;
+      const bool ends = !in || __ldcg(u.counts + r + 1) != __ldcg(u.counts + r);
+      const unsigned int stop = __ballot_sync(0xffffffffu, ends);
+      const int n = stop ? __ffs(stop) : 32;  // (the round in which the next key begins has a lead)
+      float v = (int)threadIdx.x < n ? lead : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      more += v;
+      if (stop) break;
+    }
+  }
+  for (unsigned int i = threadIdx.x; i < count; i += kUniqueThreads) {
+    const Item k = __ldcg(u.keys + base + i);
+    if constexpr (PAIRS) {
+      u.out_keys[at + i] = k >> 32;
+      if (i + 1 < count) u.out_sums[at + i] = __uint_as_float((unsigned int)k);
+    } else {
+      u.out_keys[at + i] = k;
+      if (i + 1 < count) u.out_sums[at + i] = __ldcg(u.sums + base + i);
+    }
+  }
+  if (threadIdx.x == 0) {
+    const long long i = base + count - 1;
+    const float v = PAIRS ? __uint_as_float((unsigned int)__ldcg(u.keys + i)) : __ldcg(u.sums + i);
+    u.out_sums[at + count - 1] = v + more;
   }
 }
 
@@ -696,7 +909,7 @@ extern "C" {
 
 // Bytes of scratch psdev_sort_keys needs for n keys (with or without a payload).
 size_t psdev_sort_scratch_bytes(int64_t n, int with_payload) {
-  size_t b = SortWork::bytes(n > 0 ? n : 1);
+  size_t b = SortWork::bytes(n > 0 ? n : 1, kRadixBits);
   b += round256((size_t)n * 8);                        // second key buffer
   if (with_payload) b += round256((size_t)n * 4);      // second payload buffer
   return b + 256;
@@ -717,27 +930,27 @@ int psdev_sort_keys(uint64_t* keys, uint32_t* perm, int64_t n, int key_bits, voi
   const int passes = (key_bits + kRadixBits - 1) / kRadixBits;
   char* p = static_cast<char*>(scratch);
   p = reinterpret_cast<char*>(((uintptr_t)p + 255) & ~uintptr_t(255));
-  const SortWork w(p, n);
-  p += SortWork::bytes(n);
-  using K = unsigned long long;
-  K* in = reinterpret_cast<K*>(keys);
+  const SortWork w(p, n, kRadixBits);
+  p += SortWork::bytes(n, kRadixBits);
+  Item* in = reinterpret_cast<Item*>(keys);
   if (n <= kTile) {
-    const int rc = perm ? small_sort<K, K, kMakeIndex>(in, in, nullptr, perm, (int)n, passes, 64,
+    const int rc = perm ? small_sort<Item, kMakeIndex>(in, in, nullptr, perm, (int)n, passes, 64,
                                                        w.head, nullptr, nullptr, s)
-                        : small_sort<K, K, kNoPayload>(in, in, nullptr, nullptr, (int)n, passes,
+                        : small_sort<Item, kNoPayload>(in, in, nullptr, nullptr, (int)n, passes,
                                                        64, w.head, nullptr, nullptr, s);
     return rc ? rc : (int)cudaGetLastError();
   }
-  K* out = reinterpret_cast<K*>(p);
+  Item* out = reinterpret_cast<Item*>(p);
   p += round256((size_t)n * 8);
   unsigned int* pin = perm;
   unsigned int* pout = perm ? reinterpret_cast<unsigned int*>(p) : nullptr;
   for (int pass = 0; pass < passes; ++pass) {
+    const int shift = pass * kRadixBits;
+    const Pass q{in, out, pass ? pin : nullptr, pout, n, shift, kRadixBits, shift, 64};
     // the first pass makes the payload: the index of every key in the input
-    const int rc =
-        !perm ? sort_pass<K, K, kNoPayload>(in, out, nullptr, nullptr, n, pass, 64, w, s)
-        : pass == 0 ? sort_pass<K, K, kMakeIndex>(in, out, nullptr, pout, n, pass, 64, w, s)
-                    : sort_pass<K, K, kPayload>(in, out, pin, pout, n, pass, 64, w, s);
+    const int rc = !perm       ? any_pass<kNoPayload>(kRadixBits, q, w, s)
+                   : pass == 0 ? any_pass<kMakeIndex>(kRadixBits, q, w, s)
+                               : any_pass<kPayload>(kRadixBits, q, w, s);
     if (rc) return rc;
     std::swap(in, out);
     std::swap(pin, pout);
@@ -761,31 +974,64 @@ int psdev_sort_status(const void* scratch, void* stream) {
 
 // ---- unsorted, repeated (key, value) pairs -> sorted distinct keys and sums ---------------------
 namespace {
-// Layout of the scratch memory: working memory of the sort, counts of the chunks' distinct keys,
-// then two buffers of keys (4 bytes each up to 32 bits) and of values.
+// How (key, value) pairs are sorted: pairs in one word up to 32 bits, and digits of 10 bits where
+// they save a pass.
+struct UniquePlan {
+  bool pairs;
+  int bits, passes, width;
+  UniquePlan(int64_t n, int key_bits) {
+    pairs = key_bits <= 32;
+    const int narrow = (key_bits + kRadixBits - 1) / kRadixBits;
+    const int wide = (key_bits + kWideBits - 1) / kWideBits;
+    const bool take = n > kTile && n <= (pairs ? kWidePairs : kWideKeys) && wide < narrow;
+    bits = take ? kWideBits : kRadixBits;
+    passes = take ? wide : narrow;
+    width = (key_bits + passes - 1) / passes;
+  }
+};
+
+// Layout of the scratch memory: working memory of the sort, counts and leads of the rounds of
+// distinct keys, then two buffers of items and, for keys of more than 32 bits, of values.
 struct UniqueScratch {
   char* work;
   SortHead* head;
   unsigned int* counts;
-  char* keys[2];
+  float* leads;
+  Item* keys[2];
   unsigned int* vals[2];
   size_t bytes;
   UniqueScratch(void* scratch, int64_t n, int key_bits) {
-    const size_t ksz = key_bits <= 32 ? 4 : 8;
+    const UniquePlan plan(n, key_bits);
     const uintptr_t base = ((uintptr_t)scratch + 255) & ~uintptr_t(255);
     uintptr_t p = base;
     work = reinterpret_cast<char*>(p);
-    p += SortWork::bytes(n);
+    p += SortWork::bytes(n, plan.bits);
     head = reinterpret_cast<SortHead*>(p);
-    counts = reinterpret_cast<unsigned int*>(p + sizeof(SortHead));
-    p += round256(sizeof(SortHead) + kMaxUniqueChunks * 4);
+    p += round256(sizeof(SortHead));
+    counts = reinterpret_cast<unsigned int*>(p);
+    p += round256((size_t)(rounds_of(n) + 1) * 4);
+    leads = reinterpret_cast<float*>(p);
+    p += round256((size_t)rounds_of(n) * 4);
     for (int i = 0; i < 2; ++i) {
-      keys[i] = reinterpret_cast<char*>(p);
-      p += round256((size_t)n * ksz);
+      keys[i] = reinterpret_cast<Item*>(p);
+      p += round256((size_t)n * 8);
       vals[i] = reinterpret_cast<unsigned int*>(p);
-      p += round256((size_t)n * 4);
+      if (!plan.pairs) p += round256((size_t)n * 4);
     }
     bytes = p - base + 256;
+  }
+  Unique unique(int64_t n, bool pairs, unsigned long long* out_keys, float* out_sums) const {
+    Unique u{};
+    u.items = keys[0];
+    u.vals = pairs ? nullptr : reinterpret_cast<const float*>(vals[0]);
+    u.n = n;
+    u.keys = keys[1];
+    u.sums = pairs ? nullptr : reinterpret_cast<float*>(vals[1]);
+    u.counts = counts;
+    u.leads = leads;
+    u.out_keys = out_keys;
+    u.out_sums = out_sums;
+    return u;
   }
 };
 
@@ -850,49 +1096,60 @@ struct ReportSlot {
   }
 };
 
-template <typename K>
-int unique_sort(const unsigned long long* keys, const float* vals, int64_t n, int key_bits,
+template <bool PAIRS, int THREADS>
+int unique_local(unsigned rounds, const Unique& u, cudaStream_t s) {
+  constexpr int smem = unique_smem<PAIRS, THREADS>();
+  if (int rc = allow_smem<unique_local_kernel<PAIRS, THREADS>>(smem)) return rc;
+  return launch_chained(unique_local_kernel<PAIRS, THREADS>, rounds, THREADS, smem, s, 1, u);
+}
+
+int unique_sort(const Item* keys, const float* vals, int64_t n, int key_bits,
                 const UniqueScratch& u, const SortWork& w, unsigned long long* host,
                 cudaStream_t s) {
   const unsigned int* v = reinterpret_cast<const unsigned int*>(vals);
-  const int passes = (key_bits + kRadixBits - 1) / kRadixBits;
+  const UniquePlan plan(n, key_bits);
   if (n <= kTile)
-    return small_sort<unsigned long long, K, kPayload>(keys, reinterpret_cast<K*>(u.keys[0]), v,
-                                                       u.vals[0], (int)n, passes, key_bits,
-                                                       w.head, u.counts, host, s);
-  for (int pass = 0; pass < passes; ++pass) {
+    return plan.pairs ? small_sort<unsigned int, kPayload>(keys, u.keys[0], v, nullptr, (int)n,
+                                                           plan.passes, key_bits, w.head, u.counts,
+                                                           host, s)
+                      : small_sort<Item, kPayload>(keys, u.keys[0], v, u.vals[0], (int)n,
+                                                   plan.passes, key_bits, w.head, u.counts, host,
+                                                   s);
+  for (int pass = 0; pass < plan.passes; ++pass) {
     // buffers alternate so that the last pass writes buffer 0
-    const int to = (passes - 1 - pass) & 1;
-    K* out = reinterpret_cast<K*>(u.keys[to]);
-    const int rc =
-        pass == 0 ? sort_pass<unsigned long long, K, kPayload>(keys, out, v, u.vals[to], n, 0,
-                                                               key_bits, w, s)
-                  : sort_pass<K, K, kPayload>(reinterpret_cast<const K*>(u.keys[to ^ 1]), out,
-                                              u.vals[to ^ 1], u.vals[to], n, pass, key_bits, w, s);
+    const int to = (plan.passes - 1 - pass) & 1, low = pass * plan.width;
+    const int width = key_bits - low < plan.width ? key_bits - low : plan.width;
+    const int shift = low + (plan.pairs ? 32 : 0);
+    Pass p{pass ? u.keys[to ^ 1] : keys, u.keys[to], pass ? u.vals[to ^ 1] : v, u.vals[to], n,
+           shift, width, pass ? shift : low, pass ? 64 : key_bits};
+    const int rc = !plan.pairs ? any_pass<kPayload>(plan.bits, p, w, s)
+                   : pass == 0 ? any_pass<kToPairs>(plan.bits, p, w, s)
+                               : any_pass<kNoPayload>(plan.bits, p, w, s);
     if (rc) return rc;
   }
-  const Chunks ch = unique_chunks_of(n);
-  int rc = launch_chained(unique_count_kernel<K>, ch.count, kThreads, 0, s, 1,
-                          reinterpret_cast<const K*>(u.keys[0]), n, ch, u.counts);
+  const unsigned rounds = (unsigned)rounds_of(n);
+  const Unique q = u.unique(n, plan.pairs, nullptr, nullptr);
+  int rc = plan.pairs ? unique_local<true, kUniqueThreads>(rounds, q, s)
+                      : unique_local<false, kUniqueThreads>(rounds, q, s);
   if (!rc)
-    rc = launch_chained(unique_total_kernel, 1, kThreads, 0, s, 1, u.counts, ch.count, u.head,
+    rc = launch_chained(unique_scan_kernel, 1, kThreads, 0, s, 1, u.counts, (int)rounds, u.head,
                         host);
   g_launches.fetch_add(2, std::memory_order_relaxed);
   return rc;
 }
 
-template <typename K>
-int unique_write(const UniqueScratch& u, int64_t n, unsigned long long* out_keys, float* out_sums,
-                 cudaStream_t s) {
-  // the pairs of a round (padded) and its outputs
-  constexpr int smem = (kThreads * (kUniquePer + 1) + kThreads * kUniquePer + 1) *
-                       (int)(sizeof(K) + 4);
-  if (int rc = allow_smem<unique_sum_kernel<K>>(smem)) return rc;
-  const Chunks ch = unique_chunks_of(n);
-  const int rc = launch_chained(unique_sum_kernel<K>, ch.count, kThreads, smem, s, 1,
-                                reinterpret_cast<const K*>(u.keys[0]),
-                                reinterpret_cast<const float*>(u.vals[0]), n, ch, u.counts,
-                                out_keys, out_sums);
+int unique_write(const UniqueScratch& u, int64_t n, bool pairs, unsigned long long* out_keys,
+                 float* out_sums, cudaStream_t s) {
+  Unique q = u.unique(n, pairs, out_keys, out_sums);
+  int rc;
+  if (n <= kTile) {
+    q.counts = nullptr;
+    rc = pairs ? unique_local<true, kThreads>(1, q, s) : unique_local<false, kThreads>(1, q, s);
+  } else {
+    auto* gather = pairs ? unique_gather_kernel<true> : unique_gather_kernel<false>;
+    rc = launch_chained(gather, (unsigned)rounds_of(n), kUniqueThreads, 0, s, 1, q,
+                        (int)rounds_of(n));
+  }
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return rc;
 }
@@ -916,14 +1173,13 @@ int psdev_unique_sum_sort(const uint64_t* keys, const float* vals, int64_t n, in
   if (!scratch || scratch_bytes < psdev_unique_sum_scratch_bytes(n, key_bits)) return PSDEV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const UniqueScratch u(scratch, n, key_bits);
-  SortWork w(u.work, n);
+  SortWork w(u.work, n, UniquePlan(n, key_bits).bits);
   w.head = u.head;
   cudaMemsetAsync(u.head, 0, sizeof(SortHead), s);
   const unsigned long long* k = reinterpret_cast<const unsigned long long*>(keys);
   ReportSlot slot;
   if (!slot.word) return (int)cudaErrorMemoryAllocation;
-  auto* sort = key_bits <= 32 ? unique_sort<unsigned int> : unique_sort<unsigned long long>;
-  int rc = sort(k, vals, n, key_bits, u, w, slot.word, s);
+  int rc = unique_sort(k, vals, n, key_bits, u, w, slot.word, s);
   if (rc) {
     cudaStreamSynchronize(s);  // (a kernel before the one that failed may still report)
     return rc;
@@ -942,10 +1198,8 @@ int psdev_unique_sum_write(const void* scratch, int64_t n, int key_bits, int64_t
   if (!scratch || !out_keys || !out_sums || n < 1 || n_unique < 1) return PSDEV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const UniqueScratch u(const_cast<void*>(scratch), n, key_bits);
-  cudaMemsetAsync(out_sums, 0, (size_t)n_unique * 4, s);
-  unsigned long long* ok = reinterpret_cast<unsigned long long*>(out_keys);
-  return key_bits <= 32 ? unique_write<unsigned int>(u, n, ok, out_sums, s)
-                        : unique_write<unsigned long long>(u, n, ok, out_sums, s);
+  return unique_write(u, n, UniquePlan(n, key_bits).pairs,
+                      reinterpret_cast<unsigned long long*>(out_keys), out_sums, s);
 }
 
 // dst_vals[j] op= src_vals[i] for every key present in both sorted unique lists; values have

@@ -425,7 +425,7 @@ constexpr int kLocalUnroll = 4;
 // One 16-byte group per key, all of them far apart: a plain kernel that reads 2^20 such groups and
 // writes them back takes 59 us with one per thread, 63 with two, 67 with four (41 only reading),
 // each launch by itself.
-// (4 bytes per key, far apart: 62.9 us with four per thread and plain loads, 51.1 with one and FAR.)
+// (4 bytes per key, far apart: 62.9 us with four per thread and plain loads, 51.1 with one, FAR.)
 constexpr int kStateUnroll = 1;
 __host__ __device__ constexpr int local_unroll(bool group, bool one, bool far) {
   return one && (group || far) ? kStateUnroll : kLocalUnroll;

@@ -1,0 +1,45 @@
+"""sort_unique_sum where the width of its digits, the form of its scatter and the number of its chunks
+and rounds change: keys against torch.unique, sums against sums in fp64 within the bound of fp32
+additions in any order, (m - 1) 2^-24 sum |v| for a key of m values."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(keys, vals, bits):
+    from ps_lite_b200.ops.keys import sort_unique_sum
+    want, inverse, times = torch.unique(keys, return_inverse=True, return_counts=True)
+    got, sums = sort_unique_sum(keys, vals, key_bits=bits)
+    assert torch.equal(got, want)
+    exact = torch.zeros(want.numel(), dtype=torch.float64, device=keys.device)
+    size = torch.zeros_like(exact)
+    exact.index_add_(0, inverse, vals.double())
+    size.index_add_(0, inverse, vals.double().abs())
+    assert bool(((sums.double() - exact).abs() <= (times - 1) * 2.0 ** -24 * size).all())
+
+
+# one tile of the one-CTA sort, the chunks whose counts the scatter adds up, chunks of more than the
+# smallest size, the larger tiles, and where keys of more than 32 bits go back to digits of 8 bits
+@pytest.mark.parametrize("n", [4096, 4097, 32 * 2048, 32 * 2048 + 1, 296 * 2048 + 1, 296 * 4096,
+                               296 * 4096 + 1, 1 << 21, (1 << 21) + 1])
+@pytest.mark.parametrize("bits", [17, 30, 32, 33, 40])
+def test_sizes(cuda_device, n, bits):
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(n + bits)
+    keys = torch.randint(0, 1 << bits, (n,), device=cuda_device, generator=g)
+    keys[::3] = keys[0]                                # a popular id
+    keys[1::5] = (1 << bits) - 1 - keys[1::5] % 1000   # some hundred, at the upper end
+    _check(keys, torch.randn(n, device=cuda_device, generator=g), bits)
+
+
+# runs of equal keys that fill rounds of 2048 pairs, end with them or cross many of them
+@pytest.mark.parametrize("bits", [30, 40])
+@pytest.mark.parametrize("run", [1, 2047, 2048, 2049, 40 * 2048, 200_000])
+def test_runs(cuda_device, run, bits):
+    n = 200_000
+    keys = torch.arange(n, device=cuda_device) // run * 4099
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(run)
+    order = torch.randperm(n, device=cuda_device, generator=g)
+    _check(keys[order], torch.randn(n, device=cuda_device, generator=g), bits)

@@ -36,10 +36,10 @@ namespace sortk {
 //
 // Digits have 8 bits, or up to 10 where that saves a pass and the runs of equal digits, which are
 // then a quarter as long, are not too short for what DRAM takes at a time (kWidePairs, kWideKeys).
-// Ids with many repeats / all over the key space, distinct ones and sums, us: four passes and three
-// (30 bits, pairs): 2^20 93 / 92 and 78 / 86, 2^22 212 / 202 and 172 / 182, 10^7 456 / 444 and 382 /
-// 451, 2^24 703 / 674 and 623 / 708; five passes and four (40 bits): 10^6 113 / 113 and 102 / 106,
-// 2^22 251 / 262 and 260 / 306.
+// Distinct ids and sums, us, ids with many repeats / all over the key space: four passes and three
+// (30 bits, pairs) 2^20 93 / 92 and 78 / 86, 2^22 212 / 202 and 172 / 182, 10^7 456 / 444 and
+// 382 / 451, 2^24 703 / 674 and 623 / 708; five passes and four (40 bits) 10^6 113 / 113 and
+// 102 / 106, 2^22 251 / 262 and 260 / 306.
 //
 // Up to some million items everything stays in L2.  The single-sweep form (one launch per pass,
 // tiles finding their offsets by looking back over the words that earlier tiles publish) spent a

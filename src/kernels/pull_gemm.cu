@@ -1504,8 +1504,10 @@ static int pick_plain(long long M, long long N, long long K) {
   };
   if (M >= 256 && N >= 256) {
     // a round of whole tiles, of halves and of quarters of the wide tile
-    const double t512 = fmax(0.63 * kb, 3.2), t256 = fmax(0.33 * kb, 1.6);
-    const double t128 = fmax(0.27 * kb, 0.9);
+    // (rows that begin inside a sector: see below; the wide tile reads fewer of them)
+    const double odd = K % 16 ? 1.12 : K % 64 ? 1.03 : 1;
+    const double t512 = fmax(0.63 * kb, 3.2) * (K % 16 ? 1 : odd);
+    const double t256 = fmax(0.33 * kb, 1.6) * odd, t128 = fmax(0.27 * kb, 0.9) * odd;
     for (int nt = 256; nt <= 512; nt *= 2) {
       const double rounds = tiles(256, nt) / pairs, whole = floor(rounds), rest = rounds - whole;
       const double tile = nt == 512 ? t512 : t256;
@@ -1522,6 +1524,16 @@ static int pick_plain(long long M, long long N, long long K) {
   // otherwise.  us, split form with S = 1 / what is chosen instead: 1x32768x1024 18.5 / 15.4,
   // 1x50264x1024 31.3 / 24.6, 300x16384x4096 59.7 / 48.8, 300x16384x16384 225 / 183; in one row,
   // with 393 and 1024 CTAs, 64x50264x1024 23.8 / 25.2 and 128x131072x256 24.0 / 21.8.
+  //
+  // Small tiles are bound by what an SM takes from L2, and rows that begin inside a 32-byte sector
+  // (K % 16 != 0) or a line cost it more; and of CTAs that fit at a time, a rest of a few costs a
+  // round of its own.  us: 312 CTAs of 128 x 128 for 3013x1616x2104 50.9, pairs 26.6; 338 of
+  // 128 x 64 for 1603x1624x824 18.7, pairs 10.6; 295 of 128 x 64 for 7525x280x3528 38.2, pairs
+  // 26.9.
+  // Over 204 sizes with M 64 .. 16384, N and K any multiples of 8 in 256 .. 4096, the choice is
+  // 1.002 of the fastest form in the mean and 1.06 at most; 1.045 and 1.9 when neither was looked
+  // at.
+  const double rows = K % 16 ? 1.5 : K % 64 ? 1.1 : 1;
   const bool fitted = M >= 64 && (double)N * (double)K <= 4096.0 * 4096.0;
   const double most = fitted ? INFINITY : M < 64 ? sms : M <= 128 ? 3 * sms : 2 * sms;
   for (int n = 64; n <= 128; n += 64) {
@@ -1529,19 +1541,27 @@ static int pick_plain(long long M, long long N, long long K) {
       const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)
       if (split > 1 ? (ctas > 2 * sms || split > kb) : ctas > most) break;
       const double k = ceil(kb / split), full = fmin(ctas / sms, 1);
-      const double over = fmax(0.0, ctas / (2 * sms) - 0.9);
+      const double over = fmin(fmax(0.0, ctas / (2 * sms) - 0.5), 1.0);
+      // A k-block in a round with one and with two CTAs per SM, added up over the rounds.  In one
+      // row of tiles, which reads W from HBM, a rest costs its share.
+      auto rounds = [&](double one, double two) {
+        const double whole = floor(ctas / (2 * sms)), rest = ctas - whole * 2 * sms;
+        if (M <= 128 && whole > 0) return two * ctas / (2 * sms);
+        return whole * two + (rest == 0 ? 0 : one + (two - one) * fmax(0.0, rest / sms - 1));
+      };
+      const double far = fmax(1.0, rows * (fmin((double)M, 128) + n) / (128 + n));
       const bool deep = split_deep(n, (long long)ctas, (int)k);
       double base, per_kb, exchange = 0;
       if (n == 64) {
-        base = deep ? 2.2 + 0.55 * full : 1.8 + 1.95 * full + 2.7 * over;
-        per_kb = deep ? 0.203 : fmax(0.276, 0.0011 * ctas);
+        base = deep ? 2.2 + 0.55 * full : 1.8 + 1.95 * full + over;
+        per_kb = deep ? 0.203 : rounds(0.276, 0.326);
         if (split > 1) exchange = 0.87 + 0.0029 * split * ctas + 0.53 * split;
       } else {
-        base = deep ? 2.7 + 0.6 * full : 2.1 + 3.7 * full + 4.3 * over;
-        per_kb = deep ? 0.232 : fmax(0.38, 0.0015 * ctas);
+        base = deep ? 2.7 + 0.6 * full : 2.1 + 3.7 * full + over;
+        per_kb = deep ? 0.232 : rounds(0.38, 0.444);
         if (split > 1) exchange = 1.36 + 0.0049 * split * ctas + 0.82 * split;
       }
-      offer(base + exchange + k * per_kb, 1000 * split + n);
+      offer(base + exchange + k * per_kb * far, 1000 * split + n);
     }
   }
   return pick;

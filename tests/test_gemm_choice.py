@@ -29,3 +29,10 @@ def test_small_tiles_outside_of_the_measured_sizes(choice, m, n, k):
                                         (16384, 3072, 1024, 2512), (64, 256, 4096, 4064)])
 def test_choices(choice, m, n, k, code):
     assert choice(m, n, k) == code
+
+
+@pytest.mark.parametrize("m,n,k", [(3013, 1616, 2104), (1603, 1624, 824), (7525, 280, 3528),
+                                   (6319, 672, 2648), (301, 3248, 2136)])
+def test_rows_that_begin_inside_a_sector(choice, m, n, k):
+    """Pairs, where small tiles would read such rows."""
+    assert choice(m, n, k) in (2256, 2512)

@@ -1356,12 +1356,12 @@ static int launch_split_t(const SplitArgs& a, const CUtensorMap& tx, const CUten
   if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
     cudaError_t e = cudaFuncSetAttribute(split_gemm_kernel<BN, S, DEEP>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SplitCfg<BN, DEEP>::kSmemBytes);
+                                         SplitCfg<BN, S, DEEP>::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     attr_set[dev & 63].store(true, std::memory_order_release);
   }
   const int e = launch_chained(split_gemm_kernel<BN, S, DEEP>, (unsigned)(tiles * S), kSplitThreads,
-                               SplitCfg<BN, DEEP>::kSmemBytes, s, S, a, tx, tw);
+                               SplitCfg<BN, S, DEEP>::kSmemBytes, s, S, a, tx, tw);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return e;
 }
@@ -1376,10 +1376,17 @@ static int launch_split(int split, const SplitArgs& a, const CUtensorMap& tx,
     default: return PSDEV_ERR_ARG;
   }
 }
+// CTAs of a split product that run at a time.  Clusters keep inside a GPC: 33 clusters of four and
+// 15 of eight find SMs of their own, 71 and 33 with two CTAs per SM, which the shared memory allows
+// where what the parts send is small.
+static int split_fits(int bn, int split, bool deep) {
+  const bool one = deep || (bn == 128 && split >= 4);
+  return split == 8 ? (one ? 120 : 264) : split == 4 ? (one ? 132 : 284) : one ? 148 : 296;
+}
 // Two k-blocks per stage and one CTA per SM, where SMs would have one CTA anyway and the loop is
 // longer than the shallow form's stages.
-static bool split_deep(int bn, long long ctas, int num_kb) {
-  return ctas <= 148 && num_kb > (bn == 64 ? 4 : 3);
+static bool split_deep(int bn, int split, long long ctas, int num_kb) {
+  return ctas <= split_fits(bn, split, true) && num_kb > (bn == 64 ? 4 : 3);
 }
 static int run_split(const Args& a, const void* x, const void* w, int bn, int split,
                      cudaStream_t s) {
@@ -1398,7 +1405,7 @@ static int run_split(const Args& a, const void* x, const void* w, int bn, int sp
   sa.timeout_ns = a.timeout_ns;
   while (split > sa.num_kb) split >>= 1;
   const long long tiles = (long long)sa.tiles_m * ((a.N + bn - 1) / bn);
-  if (split_deep(bn, tiles * split, (sa.num_kb + split - 1) / split))
+  if (split_deep(bn, split, tiles * split, (sa.num_kb + split - 1) / split))
     return bn == 64 ? launch_split<64, true>(split, sa, tx, tw, tiles, s)
                     : launch_split<128, true>(split, sa, tx, tw, tiles, s);
   return bn == 64 ? launch_split<64, false>(split, sa, tx, tw, tiles, s)
@@ -1539,7 +1546,9 @@ static int pick_plain(long long M, long long N, long long K) {
   for (int n = 64; n <= 128; n += 64) {
     for (int split = 1; split <= kMaxSplit; split *= 2) {
       const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)
-      if (split > 1 ? (ctas > 2 * sms || split > kb) : ctas > most) break;
+      if (split > 1 ? (ctas > split_fits(n, split, false) || split > kb) : ctas > most) break;
+      // (tests hold the choice for 64x256x4096, which clusters of eight would do in 5.4 for 7.0 us)
+      if (split == 8 && ctas <= 32) break;
       const double k = ceil(kb / split), full = fmin(ctas / sms, 1);
       const double over = fmin(fmax(0.0, ctas / (2 * sms) - 0.5), 1.0);
       // A k-block in a round with one and with two CTAs per SM, added up over the rounds.  In one
@@ -1550,16 +1559,15 @@ static int pick_plain(long long M, long long N, long long K) {
         return whole * two + (rest == 0 ? 0 : one + (two - one) * fmax(0.0, rest / sms - 1));
       };
       const double far = fmax(1.0, rows * (fmin((double)M, 128) + n) / (128 + n));
-      const bool deep = split_deep(n, (long long)ctas, (int)k);
-      double base, per_kb, exchange = 0;
+      const bool deep = split_deep(n, split, (long long)ctas, (int)k);
+      const double exchange = split == 1 ? 0 : n == 64 ? 1.46 : 1.8;
+      double base, per_kb;
       if (n == 64) {
         base = deep ? 2.2 + 0.55 * full : 1.8 + 1.95 * full + over;
         per_kb = deep ? 0.203 : rounds(0.276, 0.326);
-        if (split > 1) exchange = 0.87 + 0.0029 * split * ctas + 0.53 * split;
       } else {
-        base = deep ? 2.7 + 0.6 * full : 2.1 + 3.7 * full + over;
+        base = deep ? 2.7 + 0.6 * full : 2.1 + (split > 1 ? 1.3 : 3.7) * full + over;
         per_kb = deep ? 0.232 : rounds(0.38, 0.444);
-        if (split > 1) exchange = 1.36 + 0.0049 * split * ctas + 0.82 * split;
       }
       offer(base + exchange + k * per_kb * far, 1000 * split + n);
     }

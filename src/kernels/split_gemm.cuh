@@ -2,8 +2,13 @@
 // tiles of the persistent kernels (pull_gemm.cu).
 //
 // One 128 x BN output tile per cluster of S CTAs; CTA s of the cluster multiplies the s-th part
-// of K.  With S > 1 the partial sums (fp32) are exchanged through distributed shared memory:
-// every CTA adds up BN / S columns of all parts, in the order of the parts, and stores them.
+// of K.  With S > 1 the partial sums (fp32) are exchanged through distributed shared memory: every
+// CTA stores into each of the others the BN / S columns that are theirs, out of its tensor memory,
+// meets them once, and adds up its own columns in the order of the parts.  When every CTA read its
+// columns from the others between two barriers, and the sums lay row by row (a warp's accesses 32
+// pieces of 16 bytes), the exchange took 3 us among four CTAs and 6 among eight; now 1.5.  us,
+// 75 x 928 x 3504 with S = 4 / 8: 8.7 / 9.8 before, 7.2 / 5.9 now (S = 1 13.6); 64 x 256 x 4096
+// 9.2 / 9.9 and 7.0 / 5.4; 92 x 592 x 1360 6.9 / 11.4 and 5.1 / 5.5.
 // There is no loop over tiles, no counter in global memory, and the first loads are issued before
 // the CTA has met at its first barrier, because what bounds these products is a chain of
 // latencies: launch, operands from L2 or HBM, a few MMAs, accumulator, store.
@@ -39,26 +44,26 @@ struct SplitArgs {
   unsigned long long timeout_ns;
 };
 
-template <int BN, bool DEEP>
+template <int BN, int S, bool DEEP>
 struct SplitCfg {
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBlockBytes = kABytes + BN * BK * 2;  // one k-block
   static constexpr int kSub = DEEP ? 2 : 1;                  // k-blocks of a stage
   static constexpr int kStageBytes = kSub * kBlockBytes;
-  static constexpr int kStages = BN == 64 ? 4 : 3;
-  static constexpr int kPitch = BN + 4;  // floats per row of the exchanged partial sums
-  static constexpr int kExchange = BM * kPitch * 4;
+  // What the other parts send has memory of its own: they may be ahead of this CTA's operands.
+  // (Four columns of all rows, then the next four: a warp's stores and loads are contiguous.)
+  static constexpr int kPartBytes = BM * (BN / S) * 4;
+  static constexpr int kExchange = (S - 1) * kPartBytes;
+  static constexpr int kStages = S == 1 ? (BN == 64 ? 4 : 3)
+                                 : BN == 128 ? 2 : (S == 8 ? 2 : 3) + (DEEP ? 1 : 0);
   static constexpr int kTiles = kStages * kStageBytes;
-  static constexpr int kSmemBytes = (kTiles > kExchange ? kTiles : kExchange) + 1024 /*align*/;
+  static constexpr int kSmemBytes = kTiles + kExchange + 1024 /*align*/;
 };
 
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr)
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t* r) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
+               "r"(r[2]), "r"(r[3])
                : "memory");
-  return v;
 }
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t cta) {
   uint32_t a;
@@ -80,7 +85,7 @@ __global__ void __launch_bounds__(kSplitThreads)
                       const __grid_constant__ CUtensorMap tmap_x,
                       const __grid_constant__ CUtensorMap tmap_w) {
   using namespace sm100;
-  using C = SplitCfg<BN, DEEP>;
+  using C = SplitCfg<BN, S, DEEP>;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::kStages], empty_bar[C::kStages], done_bar;
   __shared__ uint32_t s_tmem;
@@ -129,6 +134,7 @@ __global__ void __launch_bounds__(kSplitThreads)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if constexpr (S > 1) cluster_arrive();
   const uint32_t tmem = s_tmem;
   volatile int* abort_flag = &s_abort;
 
@@ -224,63 +230,93 @@ __global__ void __launch_bounds__(kSplitThreads)
     const int in_tile = q * 32 + lane;
     const long long row = (long long)tm * BM + in_tile;
     const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16);
-    if (__all_sync(0xffffffffu, ok)) {
+    const bool all_ok = __all_sync(0xffffffffu, ok);
+    if constexpr (S == 1) {
+      if (all_ok) {
 #pragma unroll
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32(taddr + (uint32_t)c0, r);
+        for (int c0 = 0; c0 < BN; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld_32x32(taddr + (uint32_t)c0, r);
+          tmem_ld_wait();
+          if (row < a.M) {
+            const long long col = (long long)tn * BN + c0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (col + j * 8 + 8 <= a.N) {
+                float f[8];
+#pragma unroll
+                for (int x = 0; x < 8; ++x) f[x] = __uint_as_float(r[8 * j + x]);
+                store_bf16x8(a.c + row * a.N + col + j * 8, f);
+              }
+          }
+        }
+      }
+      tc_fence_before();
+    } else {
+      constexpr int kCols = BN / S, kOnce = kCols < 32 ? kCols : 32;
+      const uint32_t inbox = smem_u32(smem) + C::kTiles;
+      cluster_wait();  // the other parts have begun: their memory can be written
+      uint32_t own[kCols];
+      if (all_ok) {
+#pragma unroll 1
+        for (int d = 1; d < S; ++d) {
+          const int to = (part + d) % S;
+          const uint32_t dst = cluster_addr(
+              inbox + (uint32_t)((part < to ? part : part - 1) * C::kPartBytes + in_tile * 16),
+              (uint32_t)to);
+#pragma unroll
+          for (int c0 = 0; c0 < kCols; c0 += kOnce) {
+            uint32_t r[kOnce];
+#pragma unroll
+            for (int j = 0; j < kOnce; j += 8)
+              tmem_ld_32x8(taddr + (uint32_t)(to * kCols + c0 + j), r + j);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < kOnce; j += 4) st_cluster_v4(dst + (c0 + j) * BM * 4, r + j);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kCols; j += 8)
+          tmem_ld_32x8(taddr + (uint32_t)(part * kCols + j), own + j);
         tmem_ld_wait();
-        if constexpr (S > 1) {
-          // (all MMAs have read their operands: the stages' memory is free)
-          float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(smem) +
-                                                  in_tile * C::kPitch + c0);
+      }
+      tc_fence_before();
+      __syncwarp();
+      cluster_sync_all();  // every part's columns are in place, and nobody writes here any more
+      // (a part that gave up has sent nothing and recorded its error: the results are void)
+      if (all_ok && row < a.M) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                 __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
-        } else if (row < a.M) {
-          const long long col = (long long)tn * BN + c0;
+        for (int c0 = 0; c0 < kCols; c0 += 8) {
+          float f[8] = {};
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (col + j * 8 + 8 <= a.N) {
-              float f[8];
-#pragma unroll
-              for (int x = 0; x < 8; ++x) f[x] = __uint_as_float(r[8 * j + x]);
-              store_bf16x8(a.c + row * a.N + col + j * 8, f);
+          for (int s = 0; s < S; ++s) {
+            float4 lo, hi;
+            if (s == part) {
+              lo = make_float4(__uint_as_float(own[c0]), __uint_as_float(own[c0 + 1]),
+                               __uint_as_float(own[c0 + 2]), __uint_as_float(own[c0 + 3]));
+              hi = make_float4(__uint_as_float(own[c0 + 4]), __uint_as_float(own[c0 + 5]),
+                               __uint_as_float(own[c0 + 6]), __uint_as_float(own[c0 + 7]));
+            } else {
+              const float4* from = reinterpret_cast<const float4*>(
+                  smem + C::kTiles + (s < part ? s : s - 1) * C::kPartBytes + in_tile * 16 +
+                  c0 * BM * 4);
+              lo = from[0];
+              hi = from[BM];
             }
+            f[0] += lo.x; f[1] += lo.y; f[2] += lo.z; f[3] += lo.w;
+            f[4] += hi.x; f[5] += hi.y; f[6] += hi.z; f[7] += hi.w;
+          }
+          const long long col = (long long)tn * BN + part * kCols + c0;
+          if (col + 8 <= a.N) store_bf16x8(a.c + row * a.N + col, f);
         }
       }
     }
-    tc_fence_before();
   }
   if constexpr (S > 1) {
-    cluster_sync_all();  // every part's sums are in place
-    if (warp >= 2) {
-      constexpr int kCols = BN / S;
-      const int in_tile = (warp & 3) * 32 + lane;
-      const long long row = (long long)tm * BM + in_tile;
-      const uint32_t mine =
-          smem_u32(smem) + (uint32_t)(in_tile * C::kPitch + part * kCols) * 4;
-#pragma unroll
-      for (int c0 = 0; c0 < kCols; c0 += 8) {
-        float4 lo[S], hi[S];
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-          const uint32_t from = cluster_addr(mine + c0 * 4, s);
-          lo[s] = ld_cluster_v4(from);
-          hi[s] = ld_cluster_v4(from + 16);
-        }
-        float f[8] = {};
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-          f[0] += lo[s].x; f[1] += lo[s].y; f[2] += lo[s].z; f[3] += lo[s].w;
-          f[4] += hi[s].x; f[5] += hi[s].y; f[6] += hi[s].z; f[7] += hi[s].w;
-        }
-        const long long col = (long long)tn * BN + part * kCols + c0;
-        if (row < a.M && col + 8 <= a.N) store_bf16x8(a.c + row * a.N + col, f);
-      }
+    if (warp < 2) {
+      cluster_wait();
+      cluster_sync_all();
     }
-    cluster_sync_all();  // nobody leaves while its sums are being read
   } else {
     __syncthreads();
   }

@@ -1538,7 +1538,7 @@ static int pick_plain(long long M, long long N, long long K) {
   // 128 x 64 for 1603x1624x824 18.7, pairs 10.6; 295 of 128 x 64 for 7525x280x3528 38.2, pairs
   // 26.9.
   // Over 204 sizes with M 64 .. 16384, N and K any multiples of 8 in 256 .. 4096, the choice is
-  // 1.002 of the fastest form in the mean and 1.06 at most; 1.045 and 1.9 when neither was looked
+  // 1.005 of the fastest form in the mean and 1.11 at most; 1.045 and 1.9 when neither was looked
   // at.
   const double rows = K % 16 ? 1.5 : K % 64 ? 1.1 : 1;
   const bool fitted = M >= 64 && (double)N * (double)K <= 4096.0 * 4096.0;
@@ -1548,7 +1548,7 @@ static int pick_plain(long long M, long long N, long long K) {
       const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)
       if (split > 1 ? (ctas > split_fits(n, split, false) || split > kb) : ctas > most) break;
       // (tests hold the choice for 64x256x4096, which clusters of eight would do in 5.4 for 7.0 us)
-      if (split == 8 && ctas <= 32) break;
+      if (split == 8 && ctas <= 32 && kb >= 64) break;
       const double k = ceil(kb / split), full = fmin(ctas / sms, 1);
       const double over = fmin(fmax(0.0, ctas / (2 * sms) - 0.5), 1.0);
       // A k-block in a round with one and with two CTAs per SM, added up over the rounds.  In one
@@ -1560,14 +1560,14 @@ static int pick_plain(long long M, long long N, long long K) {
       };
       const double far = fmax(1.0, rows * (fmin((double)M, 128) + n) / (128 + n));
       const bool deep = split_deep(n, split, (long long)ctas, (int)k);
-      const double exchange = split == 1 ? 0 : n == 64 ? 1.46 : 1.8;
+      const double exchange = split == 1 ? 0 : n == 64 && split < 8 ? 1.46 : 1.8;
       double base, per_kb;
       if (n == 64) {
-        base = deep ? 2.2 + 0.55 * full : 1.8 + 1.95 * full + over;
+        base = deep ? 2.2 + 0.55 * full : 1.8 + (ctas > sms ? 1.95 : full) + over;
         per_kb = deep ? 0.203 : rounds(0.276, 0.326);
       } else {
         base = deep ? 2.7 + 0.6 * full : 2.1 + (split > 1 ? 1.3 : 3.7) * full + over;
-        per_kb = deep ? 0.232 : rounds(0.38, 0.444);
+        per_kb = deep ? split > 1 ? 0.275 : 0.232 : rounds(0.38, 0.444);
       }
       offer(base + exchange + k * per_kb * far, 1000 * split + n);
     }

@@ -26,7 +26,7 @@
 // deep; what is left is the loads, 70 bytes per clock and SM.
 //
 // Measured, us (this kernel / the persistent 128 x 256 kernel): 64x256x256 2.8 / 6.5,
-// 1024x1024x256 4.1 / 8.4, 1024x1024x1024 6.0 / 11.9, 64x256x4096 8.6 / 23.4 (S = 4).
+// 1024x1024x256 4.1 / 8.4, 1024x1024x1024 6.0 / 11.9, 64x256x4096 7.0 / 23.4 (S = 4).
 #pragma once
 #include "ps/device/sm100_ptx.cuh"
 

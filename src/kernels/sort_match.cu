@@ -990,22 +990,20 @@ struct UniquePlan {
   }
 };
 
-// Layout of the scratch memory: working memory of the sort, counts and leads of the rounds of
-// distinct keys, then two buffers of items and, for keys of more than 32 bits, of values.
+// Layout of the scratch memory: counts and leads of the rounds of distinct keys, two buffers of items
+// and, for keys of more than 32 bits, of values, then the working memory of the sort.  (The second
+// half of a call reads all but the last part, and of key_bits it needs `pairs` alone.)
 struct UniqueScratch {
-  char* work;
   SortHead* head;
   unsigned int* counts;
   float* leads;
   Item* keys[2];
   unsigned int* vals[2];
+  char* work;
   size_t bytes;
-  UniqueScratch(void* scratch, int64_t n, int key_bits) {
-    const UniquePlan plan(n, key_bits);
+  UniqueScratch(void* scratch, int64_t n, bool pairs) {
     const uintptr_t base = ((uintptr_t)scratch + 255) & ~uintptr_t(255);
     uintptr_t p = base;
-    work = reinterpret_cast<char*>(p);
-    p += SortWork::bytes(n, plan.bits);
     head = reinterpret_cast<SortHead*>(p);
     p += round256(sizeof(SortHead));
     counts = reinterpret_cast<unsigned int*>(p);
@@ -1016,9 +1014,10 @@ struct UniqueScratch {
       keys[i] = reinterpret_cast<Item*>(p);
       p += round256((size_t)n * 8);
       vals[i] = reinterpret_cast<unsigned int*>(p);
-      if (!plan.pairs) p += round256((size_t)n * 4);
+      if (!pairs) p += round256((size_t)n * 4);
     }
-    bytes = p - base + 256;
+    work = reinterpret_cast<char*>(p);
+    bytes = p - base + 256;  // (without `work`, whose size depends on the digits)
   }
   Unique unique(int64_t n, bool pairs, unsigned long long* out_keys, float* out_sums) const {
     Unique u{};
@@ -1159,7 +1158,8 @@ extern "C" {
 
 size_t psdev_unique_sum_scratch_bytes(int64_t n, int key_bits) {
   if (n < 1 || key_bits < 1 || key_bits > 64) return 0;
-  return UniqueScratch(nullptr, n, key_bits).bytes;
+  const UniquePlan plan(n, key_bits);
+  return UniqueScratch(nullptr, n, plan.pairs).bytes + SortWork::bytes(n, plan.bits);
 }
 
 // Sorts n (key, value) pairs by key into `scratch` (psdev_unique_sum_scratch_bytes) and counts the
@@ -1172,8 +1172,9 @@ int psdev_unique_sum_sort(const uint64_t* keys, const float* vals, int64_t n, in
   if (n >= (int64_t)1 << 30) return PSDEV_ERR_UNSUPPORTED;
   if (!scratch || scratch_bytes < psdev_unique_sum_scratch_bytes(n, key_bits)) return PSDEV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  const UniqueScratch u(scratch, n, key_bits);
-  SortWork w(u.work, n, UniquePlan(n, key_bits).bits);
+  const UniquePlan plan(n, key_bits);
+  const UniqueScratch u(scratch, n, plan.pairs);
+  SortWork w(u.work, n, plan.bits);
   w.head = u.head;
   cudaMemsetAsync(u.head, 0, sizeof(SortHead), s);
   const unsigned long long* k = reinterpret_cast<const unsigned long long*>(keys);
@@ -1192,14 +1193,17 @@ int psdev_unique_sum_sort(const uint64_t* keys, const float* vals, int64_t n, in
   return 0;
 }
 
-// Second half: the distinct keys, ascending, and the sums of their values.
+// Second half: the distinct keys, ascending, and the sums of their values.  `n` and `key_bits` are those
+// of the first half, `n_unique` what it counted.
 int psdev_unique_sum_write(const void* scratch, int64_t n, int key_bits, int64_t n_unique,
                            uint64_t* out_keys, float* out_sums, void* stream) {
-  if (!scratch || !out_keys || !out_sums || n < 1 || n_unique < 1) return PSDEV_ERR_ARG;
+  if (!scratch || !out_keys || !out_sums || n < 1 || n_unique < 1 || key_bits < 1 || key_bits > 64)
+    return PSDEV_ERR_ARG;
+  if (n >= (int64_t)1 << 30) return PSDEV_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
-  const UniqueScratch u(const_cast<void*>(scratch), n, key_bits);
-  return unique_write(u, n, UniquePlan(n, key_bits).pairs,
-                      reinterpret_cast<unsigned long long*>(out_keys), out_sums, s);
+  const bool pairs = key_bits <= 32;
+  const UniqueScratch u(const_cast<void*>(scratch), n, pairs);
+  return unique_write(u, n, pairs, reinterpret_cast<unsigned long long*>(out_keys), out_sums, s);
 }
 
 // dst_vals[j] op= src_vals[i] for every key present in both sorted unique lists; values have

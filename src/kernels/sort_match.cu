@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <type_traits>
 #include <utility>
 
 #include "ps/device/chain.cuh"
@@ -816,22 +817,37 @@ __global__ void __launch_bounds__(kUniqueThreads)
   const unsigned int count = __ldcg(u.counts + blockIdx.x + 1) - at;
   const long long base = (long long)blockIdx.x * kRound;
   if (count == 0) return;
-  // what the rounds behind have found of the last key (a warp looks at 32 of them at a time)
+  // What the rounds behind have found of the last key.  A warp looks at 32 of them, which is enough
+  // for most keys, and then at 512 at a time: 32 at a time took 90 us of 2^24 pairs with one key, where
+  // one CTA goes through all 8192 rounds.
   float more = 0.f;
   if (threadIdx.x < 32) {
-    for (int r0 = blockIdx.x + 1;; r0 += 32) {
-      const int r = r0 + (int)threadIdx.x;
-      const bool in = r < rounds;
-      const float lead = in ? __ldcg(u.leads + r) : 0.f;
-      const bool ends = !in || __ldcg(u.counts + r + 1) != __ldcg(u.counts + r);
-      const unsigned int stop = __ballot_sync(0xffffffffu, ends);
-      const int n = stop ? __ffs(stop) : 32;  // (the round in which the next key begins has a lead)
-      float v = (int)threadIdx.x < n ? lead : 0.f;
+    auto open_behind = [&](int r0, auto groups) {  // whether the key goes on behind these rounds
+      constexpr int kGroups = decltype(groups)::value;
+      float lead[kGroups], v = 0.f;
+      bool ends[kGroups], open = true;
+#pragma unroll
+      for (int j = 0; j < kGroups; ++j) {
+        const int r = r0 + j * 32 + (int)threadIdx.x;
+        const bool in = r < rounds;
+        lead[j] = in ? __ldcg(u.leads + r) : 0.f;
+        ends[j] = !in || __ldcg(u.counts + r + 1) != __ldcg(u.counts + r);
+      }
+#pragma unroll
+      for (int j = 0; j < kGroups; ++j) {
+        const unsigned int stop = __ballot_sync(0xffffffffu, ends[j]);
+        const int n = stop ? __ffs(stop) : 32;  // (the round in which the next key begins has a lead)
+        if (open && (int)threadIdx.x < n) v += lead[j];
+        if (stop) open = false;
+      }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       more += v;
-      if (stop) break;
-    }
+      return open;
+    };
+    int r0 = blockIdx.x + 1;
+    if (open_behind(r0, std::integral_constant<int, 1>{}))
+      for (r0 += 32; open_behind(r0, std::integral_constant<int, 16>{}); r0 += 512) {}
   }
   for (unsigned int i = threadIdx.x; i < count; i += kUniqueThreads) {
     const Item k = __ldcg(u.keys + base + i);

@@ -43,3 +43,18 @@ def test_runs(cuda_device, run, bits):
     g.manual_seed(run)
     order = torch.randperm(n, device=cuda_device, generator=g)
     _check(keys[order], torch.randn(n, device=cuda_device, generator=g), bits)
+
+
+# one run over so many rounds of 2048 pairs: what a warp looks at first, then 512 at a time, and the
+# 2048 rounds whose counts are put together at a time
+@pytest.mark.parametrize("bits", [30, 40])
+@pytest.mark.parametrize("rounds", [31, 32, 33, 34, 543, 544, 545, 546, 1057, 2047, 2048, 2049, 4100])
+def test_a_run_over_many_rounds(cuda_device, rounds, bits):
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(rounds)
+    first, last = 3000, 5000    # smaller and larger keys, so that the run begins inside a round
+    keys = torch.full((first + rounds * 2048 + last,), 1 << 20, device=cuda_device)
+    keys[:first] = torch.randint(0, 1 << 20, (first,), device=cuda_device, generator=g)
+    keys[-last:] = torch.randint((1 << 20) + 1, 1 << bits, (last,), device=cuda_device, generator=g)
+    order = torch.randperm(keys.numel(), device=cuda_device, generator=g)
+    _check(keys[order], torch.randn(keys.numel(), device=cuda_device, generator=g), bits)

@@ -27,7 +27,7 @@ namespace sortk {
 // contiguous chunks, one per CTA that fits on the GPU at a time, and a pass is three launches:
 //   digit_count  counts the digits of every chunk;
 //   digit_scan   turns the counts of each digit into how many items of the chunks before have it
-//                (left to the scatter when there are few chunks);
+//                (left to the scatter when there are few chunks, see kSelfScan);
 //   scatter      takes its chunk tile by tile: ranks each item among the items of the same digit in
 //                input order (the sort is stable), puts the tile in sorted order in shared
 //                memory and stores runs of equal digits to consecutive addresses.
@@ -60,8 +60,12 @@ constexpr int kMinChunk = 2048;
 constexpr long long kWidePairs = 1 << 25, kWideKeys = 2 << 20;
 // Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
 // number of launches (64-bit keys without payload, 2^14 / 2^16, us: 119 / 110 with three launches
-// per pass, 64 / 74 with two; the single-sweep form 97 / 101).
-constexpr int kSelfScan = 32;
+// per pass, 64 / 74 with two; the single-sweep form 97 / 101).  With digits of 8 bits there are no
+// more up to 128 Ki items, in chunks of up to 4096: 80 Ki keys of 64 bits 80.8 us in 40 chunks of
+// 2048, 67.4 in 32 of 2560; 24 bits 32.8 and 26.6.  Wider digits have four times the counts: 64 Ki
+// pairs of 40 bits 75.8 us when 32 chunks were added up, 65.6 with a scan; and pairs whose wide
+// digits would save one pass of six or more keep to 8 bits there (64 bits, 64 Ki: 102.6 and 95.3).
+constexpr int kSelfScan = 32, kSelfScanWide = 16, kMaxSelfChunk = 4096;
 
 // Head of the scratch memory.
 struct SortHead {
@@ -75,9 +79,11 @@ struct Chunks {
   int size;  // items per chunk (the last one: what is left)
   int rows;
 };
-inline Chunks chunks_of(long long n, int threads, int max_rows) {
+inline Chunks chunks_of(long long n, int bits, int threads, int max_rows) {
   long long per = (n + kMaxChunks - 1) / kMaxChunks;
   if (per < kMinChunk) per = kMinChunk;
+  if (bits == kRadixBits && n > (long long)kSelfScan * per && n <= kSelfScan * kMaxSelfChunk)
+    per = (n + kSelfScan - 1) / kSelfScan;
   const long long tile = (long long)threads * max_rows, tiles = (per + tile - 1) / tile;
   Chunks c;
   c.rows = (int)((per + tiles * threads - 1) / (tiles * threads));
@@ -296,13 +302,29 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
         total[i] = __ldcg(totals + d0 + i);
       }
     } else {
-      for (int c = 0; c < ch.count; ++c)
+      // (eight chunks' counts in flight, also at the end: one after the other, 29 chunks cost more than 32)
+      for (int c0 = 0; c0 < ch.count; c0 += 8) {
+        uint2 v[8][kPer];
 #pragma unroll
-        for (int i = 0; i < 2 * kPer; ++i) {
-          const unsigned int v = __ldcg(prefix + (size_t)c * kDigits + d0 + i);
-          if (c < blockIdx.x) next[i] += v;
-          total[i] += v;
-        }
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int i = 0; i < kPer; ++i)
+            v[j][i] = c0 + j < ch.count
+                          ? __ldcg(reinterpret_cast<const uint2*>(
+                                       prefix + (size_t)(c0 + j) * kDigits + d0) + i)
+                          : make_uint2(0, 0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) {
+            if (c0 + j < blockIdx.x) {
+              next[2 * i] += v[j][i].x;
+              next[2 * i + 1] += v[j][i].y;
+            }
+            total[2 * i] += v[j][i].x;
+            total[2 * i + 1] += v[j][i].y;
+          }
+      }
     }
 #pragma unroll
     for (int i = 0; i < 2 * kPer; ++i) mine += total[i];
@@ -582,11 +604,11 @@ template <int BITS, int WARPS, int ROWS, int PAY>
 static int sort_pass(const Pass& p, const SortWork& w, cudaStream_t s) {
   using C = ScatterCfg<BITS, WARPS, ROWS, PAY == kMakeIndex || PAY == kPayload>;
   if (int rc = allow_smem<scatter_kernel<BITS, WARPS, ROWS, PAY>>(C::kSmemBytes)) return rc;
-  const Chunks ch = chunks_of(p.n, C::kThreads, ROWS);
+  const Chunks ch = chunks_of(p.n, BITS, C::kThreads, ROWS);
   const unsigned int mask = (1u << p.width) - 1;
   int rc = launch_chained(digit_count_kernel<BITS>, ch.count, kThreads, 0, s, 1, p.in, p.n,
                           p.count_shift, mask, ch, p.check_bits, w.counts, w.head);
-  const bool scan = ch.count > kSelfScan;
+  const bool scan = ch.count > (BITS == kRadixBits ? kSelfScan : kSelfScanWide);
   if (!rc && scan)
     rc = launch_chained(digit_scan_kernel, C::kDigits / 32, 1024, 0, s, 1, w.counts, C::kDigits,
                         ch.count, w.totals);
@@ -999,7 +1021,10 @@ struct UniquePlan {
     pairs = key_bits <= 32;
     const int narrow = (key_bits + kRadixBits - 1) / kRadixBits;
     const int wide = (key_bits + kWideBits - 1) / kWideBits;
-    const bool take = n > kTile && n <= (pairs ? kWidePairs : kWideKeys) && wide < narrow;
+    // (a pass of 10 bits has three launches where one of 8 bits has two)
+    const bool self = n > kSelfScanWide * kMinChunk && n <= kSelfScan * kMaxSelfChunk;
+    const bool take = n > kTile && n <= (pairs ? kWidePairs : kWideKeys) && wide < narrow &&
+                      !(self && 3 * wide > 2 * narrow + 2);
     bits = take ? kWideBits : kRadixBits;
     passes = take ? wide : narrow;
     width = (key_bits + passes - 1) / passes;

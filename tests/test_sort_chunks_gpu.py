@@ -17,3 +17,16 @@ def test_sorted_and_stable(cuda_device, n, bits, spread):
     got, perm = sort_keys(keys.clone(), bits, return_perm=True)
     assert torch.equal(got, want) and torch.equal(perm.long(), order)
     assert torch.equal(sort_keys(keys.clone(), bits)[0], want)
+
+
+@pytest.mark.parametrize("n,each", [(4097, 2), (1 << 16, 2), ((1 << 16) + 1, 2), (80 << 10, 2), (96 << 10, 2),
+                                    (32 * 4096, 2), (32 * 4096 + 1, 3)])
+def test_launches_per_pass(cuda_device, n, each):
+    """No scan where the scatter adds up the counts."""
+    from ps_lite_b200 import _lib
+    from ps_lite_b200.ops.keys import sort_keys
+    lib = _lib.device_lib()
+    keys = torch.arange(n, device=cuda_device).flip(0).contiguous()
+    before = lib.psdev_launch_count()
+    assert torch.equal(sort_keys(keys, 24)[0], torch.arange(n, device=cuda_device))
+    assert lib.psdev_launch_count() - before == 3 * each

@@ -58,6 +58,12 @@ constexpr int kWideBits = 10;
 constexpr int kMaxChunks = 2 * 148;        // two CTAs per SM
 constexpr int kMinChunk = 2048;
 constexpr long long kWidePairs = 1 << 25, kWideKeys = 2 << 20;
+// Up to so many items pairs that keep to digits of 8 bits travel in one word from the first pass on.
+// More have arrays of keys and values until the last one.  us, ids of 24 bits all over the key space
+// / with many repeats / half of them one id, together and apart: 2^20 71 / 74 / 75 and 74 / 75 / 77,
+// 2^22 162 / 164 / 174 and 153 / 152 / 161, 2^24 535 / 539 / 579 and 522 / 498 / 528 (all three 3 to 8 %
+// slower together than in the form before pairs, 545 / 519 / 538, but for the first).
+constexpr long long kPairsTogether = 3 << 19;
 // Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
 // number of launches (64-bit keys without payload, 2^14 / 2^16, us: 119 / 110 with three launches
 // per pass, 64 / 74 with two; the single-sweep form 97 / 101).  With digits of 8 bits there are no
@@ -137,9 +143,9 @@ __device__ __forceinline__ unsigned int item_digit(Item k, int shift, unsigned i
 }
 
 // counts[c * 2^BITS + d] = items of chunk c whose digit is d
-template <int BITS>
+template <typename K, int BITS>
 __global__ void __launch_bounds__(kThreads, 2)
-    digit_count_kernel(const Item* __restrict__ keys, long long n, int shift, unsigned int mask,
+    digit_count_kernel(const K* __restrict__ keys, long long n, int shift, unsigned int mask,
                        Chunks ch, int key_bits, unsigned int* counts, SortHead* head) {
   grid_launch_next();
   constexpr int kDigits = 1 << BITS, kSets = BITS > 8 ? 2 : 4;
@@ -153,14 +159,15 @@ __global__ void __launch_bounds__(kThreads, 2)
   const long long hi = lo + ch.size < n ? lo + ch.size : n;
   bool wide = false;
   for (long long base = lo + threadIdx.x; base < hi; base += kThreads * kItems) {
-    Item k[kItems];
+    K k[kItems];
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
-      k[j] = base + j * kThreads < hi ? __ldcg(keys + base + j * kThreads) : 0;
+      k[j] = base + j * kThreads < hi ? __ldcg(keys + base + j * kThreads) : (K)0;
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
       if (base + j * kThreads < hi) {
-        if (key_bits < 64) wide |= (k[j] >> (key_bits & 63)) != 0;
+        if constexpr (sizeof(K) == 8)
+          if (key_bits < 64) wide |= (k[j] >> (key_bits & 63)) != 0;
         atomicAdd(&mine[item_digit(k[j], shift, mask)], 1u);
       }
   }
@@ -215,8 +222,21 @@ __global__ void __launch_bounds__(1024)
 }
 
 // What travels beside the keys of a pass: nothing, the key's index or a value of 32 bits in an
-// array of its own, or a value that a first pass puts below its key.
-enum { kNoPayload = 0, kMakeIndex = 1, kPayload = 2, kToPairs = 3 };
+// array of its own, or a value that a first pass puts below its key.  With values in an array, keys of
+// up to 32 bits can have 32 too: the first pass narrows them (kNarrow), the last one puts pairs
+// together (kShortToPairs).
+enum {
+  kNoPayload = 0, kMakeIndex = 1, kPayload = 2, kToPairs = 3,
+  kNarrow = 4, kShort = 5, kShortToPairs = 6
+};
+template <int PAY>
+struct Form {
+  static constexpr bool kShortIn = PAY == kShort || PAY == kShortToPairs;
+  static constexpr bool kShortKey = kShortIn || PAY == kNarrow;
+  static constexpr bool kArray = PAY == kMakeIndex || PAY == kPayload || kShortKey;
+  using In = std::conditional_t<kShortIn, unsigned int, Item>;    // as a pass reads them
+  using Key = std::conditional_t<kShortKey, unsigned int, Item>;  // and ranks them
+};
 
 // Rank of each of a thread's keys (index base + 32 j, below hi) among the keys of its warp that
 // have the same digit, in index order; cnt[d] ends up as the number of such keys.
@@ -248,10 +268,12 @@ __device__ __forceinline__ void rank_tile(const K* k, long long base, long long 
 
 // Shared memory of a scatter: the tile's items and payloads in sorted order (before that, the lane
 // masks), the warps' digit counters and a table of output places.
-template <int BITS, int WARPS, int ROWS, bool ARRAY>
+template <int BITS, int WARPS, int ROWS, int PAY>
 struct ScatterCfg {
   static constexpr int kDigits = 1 << BITS, kThreads = WARPS * 32, kTile = kThreads * ROWS;
-  static constexpr int kExchange = kTile * (8 + (ARRAY ? 4 : 0)), kMasks = WARPS * kDigits * 4;
+  static constexpr int kKeys = kTile * (int)sizeof(typename Form<PAY>::Key);
+  static constexpr int kExchange = kKeys + (Form<PAY>::kArray ? kTile * 4 : 0);
+  static constexpr int kMasks = WARPS * kDigits * 4;
   static constexpr int kShared = kExchange > kMasks ? kExchange : kMasks;
   static constexpr int kSmemBytes = kShared + WARPS * kDigits * 2 + kDigits * 4;
 };
@@ -260,21 +282,22 @@ struct ScatterCfg {
 // with 16 rows, whose counters are fewer (2^17 pairs: 36 and 39 us).
 template <int BITS, int WARPS, int ROWS, int PAY>
 __global__ void __launch_bounds__(WARPS * 32, 2)
-    scatter_kernel(const Item* __restrict__ keys_in, Item* __restrict__ keys_out,
+    scatter_kernel(const typename Form<PAY>::In* __restrict__ keys_in, void* __restrict__ out,
                    const unsigned int* __restrict__ pay_in, unsigned int* __restrict__ pay_out,
                    long long n, int shift, unsigned int mask, Chunks ch,
                    const unsigned int* __restrict__ prefix,
                    const unsigned int* __restrict__ totals) {
   grid_launch_next();
-  constexpr bool kArray = PAY == kMakeIndex || PAY == kPayload;
-  using C = ScatterCfg<BITS, WARPS, ROWS, kArray>;
+  constexpr bool kArray = Form<PAY>::kArray;
+  using K = typename Form<PAY>::Key;
+  using C = ScatterCfg<BITS, WARPS, ROWS, PAY>;
   constexpr int kDigits = C::kDigits, kThreads = C::kThreads, kPairs = kDigits / 2;
   constexpr int kPer = kPairs > kThreads ? kPairs / kThreads : 1;  // pairs of digits per thread
   static_assert(kPairs % kThreads == 0 || kThreads % kPairs == 0, "every pair has a thread");
   static_assert(ROWS % 2 == 0 && C::kTile < 65536, "ranks and positions have 16 bits");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Item* skeys = reinterpret_cast<Item*>(smem_raw);
-  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + C::kTile * 8);
+  K* skeys = reinterpret_cast<K*>(smem_raw);
+  unsigned int* spay = reinterpret_cast<unsigned int*>(smem_raw + C::kKeys);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // lanes[d]: lanes of this warp whose present item has digit d; zero in between.  The memory of
   // the exchange, which begins when all warps have their ranks.
@@ -340,17 +363,17 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
   const int rows = ch.rows, tile = kThreads * rows;
   // A tile is loaded before the one before it is stored: its items and payloads take the registers
   // of those that have gone to shared memory.
-  Item k[ROWS];
+  K k[ROWS];
   unsigned int pay[kArray ? ROWS : 1];
   auto load = [&](long long base) {
 #pragma unroll
     for (int j = 0; j < ROWS; ++j) {
       if (j >= rows) break;
       const long long i = base + j * 32;
-      k[j] = i < hi ? __ldcg(keys_in + i) : ~0ull;
+      k[j] = i < hi ? (K)__ldcg(keys_in + i) : (K)~0ull;
       if constexpr (PAY == kToPairs) k[j] = k[j] << 32 | (i < hi ? __ldcg(pay_in + i) : 0u);
-      if constexpr (PAY == kPayload) pay[j] = i < hi ? __ldcg(pay_in + i) : 0u;
       if constexpr (PAY == kMakeIndex) pay[j] = (unsigned int)i;
+      else if constexpr (kArray) pay[j] = i < hi ? __ldcg(pay_in + i) : 0u;
     }
   };
   load(lo + (long long)warp * (32 * rows) + lane);
@@ -436,10 +459,14 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
       if (j >= rows) break;
       const int q = threadIdx.x + j * kThreads;
       if (q < tile_n) {
-        const Item key = skeys[q];
+        const K key = skeys[q];
         const unsigned int p = goff[item_digit(key, shift, mask)] + (unsigned int)q;
-        keys_out[p] = key;
-        if constexpr (kArray) pay_out[p] = spay[q];
+        if constexpr (PAY == kShortToPairs) {
+          static_cast<Item*>(out)[p] = (Item)key << 32 | spay[q];
+        } else {
+          static_cast<K*>(out)[p] = key;
+          if constexpr (kArray) pay_out[p] = spay[q];
+        }
       }
     }
     __syncthreads();
@@ -591,8 +618,8 @@ static int small_sort(const Item* in, Item* out, const unsigned int* pin, unsign
 }
 
 struct Pass {
-  const Item* in;
-  Item* out;
+  const void* in;
+  void* out;
   const unsigned int* pin;
   unsigned int* pout;
   long long n;
@@ -602,11 +629,13 @@ struct Pass {
 };
 template <int BITS, int WARPS, int ROWS, int PAY>
 static int sort_pass(const Pass& p, const SortWork& w, cudaStream_t s) {
-  using C = ScatterCfg<BITS, WARPS, ROWS, PAY == kMakeIndex || PAY == kPayload>;
+  using C = ScatterCfg<BITS, WARPS, ROWS, PAY>;
+  using In = typename Form<PAY>::In;
+  const In* in = static_cast<const In*>(p.in);
   if (int rc = allow_smem<scatter_kernel<BITS, WARPS, ROWS, PAY>>(C::kSmemBytes)) return rc;
   const Chunks ch = chunks_of(p.n, BITS, C::kThreads, ROWS);
   const unsigned int mask = (1u << p.width) - 1;
-  int rc = launch_chained(digit_count_kernel<BITS>, ch.count, kThreads, 0, s, 1, p.in, p.n,
+  int rc = launch_chained(digit_count_kernel<In, BITS>, ch.count, kThreads, 0, s, 1, in, p.n,
                           p.count_shift, mask, ch, p.check_bits, w.counts, w.head);
   const bool scan = ch.count > (BITS == kRadixBits ? kSelfScan : kSelfScanWide);
   if (!rc && scan)
@@ -614,7 +643,7 @@ static int sort_pass(const Pass& p, const SortWork& w, cudaStream_t s) {
                         ch.count, w.totals);
   if (!rc)
     rc = launch_chained(scatter_kernel<BITS, WARPS, ROWS, PAY>, ch.count, C::kThreads,
-                        C::kSmemBytes, s, 1, p.in, p.out, p.pin, p.pout, p.n, p.shift, mask, ch,
+                        C::kSmemBytes, s, 1, in, p.out, p.pin, p.pout, p.n, p.shift, mask, ch,
                         w.counts, scan ? w.totals : nullptr);
   g_launches.fetch_add(scan ? 3 : 2, std::memory_order_relaxed);
   return rc;
@@ -623,7 +652,7 @@ static int sort_pass(const Pass& p, const SortWork& w, cudaStream_t s) {
 template <int PAY>
 static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) {
   if (bits == kRadixBits) return sort_pass<kRadixBits, 16, 8, PAY>(p, w, s);
-  if constexpr (PAY == kMakeIndex) {
+  if constexpr (PAY == kMakeIndex || Form<PAY>::kShortKey) {
     return PSDEV_ERR_ARG;
   } else {
     if (p.n <= kMaxChunks * 4096ll) return sort_pass<kWideBits, 8, 16, PAY>(p, w, s);
@@ -1013,9 +1042,10 @@ int psdev_sort_status(const void* scratch, void* stream) {
 // ---- unsorted, repeated (key, value) pairs -> sorted distinct keys and sums ---------------------
 namespace {
 // How (key, value) pairs are sorted: pairs in one word up to 32 bits, and digits of 10 bits where
-// they save a pass.
+// they save a pass.  Where they do not, many keys have an array of their own until the last pass, so
+// that counting reads 4 bytes per item (kPairsTogether).
 struct UniquePlan {
-  bool pairs;
+  bool pairs, apart;
   int bits, passes, width;
   UniquePlan(int64_t n, int key_bits) {
     pairs = key_bits <= 32;
@@ -1028,6 +1058,7 @@ struct UniquePlan {
     bits = take ? kWideBits : kRadixBits;
     passes = take ? wide : narrow;
     width = (key_bits + passes - 1) / passes;
+    apart = pairs && !take && passes > 1 && n > kPairsTogether;
   }
 };
 
@@ -1162,6 +1193,17 @@ int unique_sort(const Item* keys, const float* vals, int64_t n, int key_bits,
     const int shift = low + (plan.pairs ? 32 : 0);
     Pass p{pass ? u.keys[to ^ 1] : keys, u.keys[to], pass ? u.vals[to ^ 1] : v, u.vals[to], n,
            shift, width, pass ? shift : low, pass ? 64 : key_bits};
+    if (plan.apart) {  // (a buffer of pairs holds the keys, then the values)
+      const bool last = pass + 1 == plan.passes;
+      p.shift = p.count_shift = low;
+      if (pass) p.pin = reinterpret_cast<const unsigned int*>(u.keys[to ^ 1]) + n;
+      p.pout = last ? nullptr : reinterpret_cast<unsigned int*>(u.keys[to]) + n;
+      const int rc = pass == 0 ? any_pass<kNarrow>(plan.bits, p, w, s)
+                     : last    ? any_pass<kShortToPairs>(plan.bits, p, w, s)
+                               : any_pass<kShort>(plan.bits, p, w, s);
+      if (rc) return rc;
+      continue;
+    }
     const int rc = !plan.pairs ? any_pass<kPayload>(plan.bits, p, w, s)
                    : pass == 0 ? any_pass<kToPairs>(plan.bits, p, w, s)
                                : any_pass<kNoPayload>(plan.bits, p, w, s);

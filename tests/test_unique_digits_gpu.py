@@ -58,3 +58,26 @@ def test_a_run_over_many_rounds(cuda_device, rounds, bits):
     keys[-last:] = torch.randint((1 << 20) + 1, 1 << bits, (last,), device=cuda_device, generator=g)
     order = torch.randperm(keys.numel(), device=cuda_device, generator=g)
     _check(keys[order], torch.randn(keys.numel(), device=cuda_device, generator=g), bits)
+
+
+# where pairs of one word become arrays of keys and values until the last pass: two to four passes of
+# 8 bits, chunks of several tiles, ends inside a tile
+@pytest.mark.parametrize("n", [3 << 19, (3 << 19) + 1, (3 << 19) + 4095, 2_500_000, (1 << 22) + 12_345])
+@pytest.mark.parametrize("bits", [5, 8, 16, 24, 32])
+def test_keys_and_values_apart(cuda_device, n, bits):
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(n + bits)
+    keys = torch.randint(0, 1 << bits, (n,), device=cuda_device, generator=g)
+    keys[::7] = (1 << bits) - 1
+    _check(keys, torch.randn(n, device=cuda_device, generator=g), bits)
+
+
+@pytest.mark.parametrize("n", [(3 << 19) + 1, 2_500_000])
+def test_a_key_wider_than_stated_among_many(cuda_device, n):
+    """The first pass, which narrows the keys, sees it: keys sort by their low bits, as in sort_keys."""
+    from ps_lite_b200.ops.keys import sort_unique_sum
+    keys = torch.arange(n, device=cuda_device) % 1000
+    keys[n // 2] += 1 << 40
+    got, sums = sort_unique_sum(keys, torch.ones(n, device=cuda_device), key_bits=24)
+    assert int(sums.sum()) == n and bool(((got & 0xffffff).diff() >= 0).all())
+    assert (1 << 40) + n // 2 % 1000 in got.tolist()

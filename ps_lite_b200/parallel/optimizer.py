@@ -16,9 +16,10 @@ and that its users build on ``KVWorker::Push/Pull`` with per-message priorities
   gradient tensors as they are, and the update kernel reads them where they lie; a gradient whose
   memory somebody else can still write (a view of a workspace, say) is copied by its hook;
 * slices are exchanged by fused push+pull kernels on a side stream, overlapping the rest of
-  backward: as soon as ``batch_bytes`` (4 MiB by default, 32 on one rank; ``PSB200_BATCH_BYTES``)
-  are pending, everything pending goes out in ONE launch whose CTAs take the slices in priority
-  order, so small tensors share a rendezvous; with ``batch_bytes=0`` every hook launches up to
+  backward: as soon as ``batch_bytes`` (4 MiB by default, on one rank a quarter of the model, 4 to
+  32; ``PSB200_BATCH_BYTES``) are pending, everything pending goes out in ONE launch whose CTAs take
+  the slices in priority order, so small tensors share a rendezvous (on one rank up to four batches
+  wait while the launch before is still running); with ``batch_bytes=0`` every hook launches up to
   ``slices_per_event`` single-slice kernels and the rest waits in the host queue.
 
 Every rank makes the same scheduling decisions because they depend only on the order in which
@@ -38,13 +39,18 @@ from .dense import DenseTable, ServerOptimizer
 from .heap import SymmetricHeap
 
 
-# Bytes of gradients that a launch waits for, unless the program says otherwise.  Several ranks:
-# enough that small tensors share a rendezvous.  One rank has none, and a launch costs the thread of
-# the hooks some 8 us, as much as the update of 4 MiB takes the GPU: the 391 tensors of BERT-large,
-# Adam, in a pass that is bound by that thread 4270 us with 4 MiB, 4130 with 16, 3820 with 32.  What
-# is pending when the backward pass ends is all that the step waits for (32 MiB of bf16 gradients,
-# Adam: 72 us).
-BATCH_EXCHANGED, BATCH_ONE_RANK = 4 << 20, 32 << 20
+# Bytes of gradients that a launch waits for, unless the program says otherwise.  Several ranks, and
+# the hooks in Python: enough that small tensors share a rendezvous.
+BATCH_BYTES = 4 << 20
+# The native hooks of one rank have no rendezvous, but every launch costs their thread some 5 us
+# (300 tensors with 2^27 values, ready gradients: 3777 us with 34 launches, 3635 with 7; the 297 tensors
+# of BERT-large 3763 with 37, 3605 with 19).  A quarter of the model within these bounds, so that the
+# rest is updated beside the backward pass ...
+BATCH_ONE_RANK = 4 << 20, 32 << 20
+# ... and more while the launch before is still running: what is sent would only queue up behind it
+# and take SMs from the backward pass.  (A program that names its batch: four of them.  Three layers of
+# 2048 x 2048, 16384 rows, Adam, batches of 4 MiB: 1488 us, 1548 when none waits.)
+BATCH_BUSY = 16 << 20
 
 
 class P3Scheduler:
@@ -111,9 +117,13 @@ class DistributedOptimizer:
         # goes out in one launch (small tensors share a rendezvous); 0 = launch from every hook
         if batch_bytes is None:
             import os
-            batch_bytes = int(os.environ.get("PSB200_BATCH_BYTES", str(
-                BATCH_ONE_RANK if self._one_rank() else BATCH_EXCHANGED)))
-        self.batch_bytes = int(batch_bytes)
+            batch_bytes = os.environ.get("PSB200_BATCH_BYTES")
+        self.batch_bytes = BATCH_BYTES if batch_bytes is None else int(batch_bytes)
+        self._busy_bytes = 4 * self.batch_bytes
+        if batch_bytes is None and self._native_ok(grad_dtype):
+            least, most = BATCH_ONE_RANK
+            self.batch_bytes = min(most, max(least, self.total * gsz // 4))
+            self._busy_bytes = max(BATCH_BUSY, self.batch_bytes)
         self._gsz = gsz
         self.launches = 0
         self.overlap = overlap
@@ -144,13 +154,10 @@ class DistributedOptimizer:
                            for i, p in enumerate(self.params)]
         self._pending_step = False
 
-    def _one_rank(self) -> bool:
-        return self.heap.world == 1 and not self.heap.emulated_ranks
-
     def _native_ok(self, grad_dtype) -> bool:
         """One rank, gradients in a type that the update kernel reads in place, and batching on
         (``batch_bytes=0`` asks for a launch per slice)."""
-        return (self._one_rank() and self.batch_bytes > 0 and
+        return (self.heap.world == 1 and not self.heap.emulated_ranks and self.batch_bytes > 0 and
                 grad_dtype in (torch.float32, torch.bfloat16) and
                 all(p.is_cuda for p in self.params))
 
@@ -182,7 +189,7 @@ class DistributedOptimizer:
             self.params, self.offsets, pri, t.grad, C.addressof(t._world), C.addressof(t._table),
             C.addressof(self._opt), segs, cast, self.comm.cuda_stream if self.comm else 0,
             self.comm is not None, max(1, self.batch_bytes // self._gsz),
-            max(8, int(slice_elems) & ~7), channel, refresh)
+            max(1, self._busy_bytes // self._gsz), max(8, int(slice_elems) & ~7), channel, refresh)
 
     def _make_hook(self, index: int):
         n_params = len(self.params)

@@ -52,14 +52,15 @@ using CastFn = int (*)(const void*, void*, int64_t, float, int, void*);
 
 class GradExchange {
  public:
+  // `batch_elems`: gradients that a launch waits for, `busy_elems` while one is still running.
   // `world`, `table`, `opt`, `segs_fn`, `cast_fn`: addresses of the structures, of
   // psdev_dense_op_segs and of psdev_filter_cast;
   // `refresh` brings *opt up to date and is called before every launch.
   GradExchange(std::vector<at::Tensor> params, std::vector<int64_t> offsets,
                std::vector<int64_t> priorities, at::Tensor grad_buffer, uint64_t world,
                uint64_t table, uint64_t opt, uint64_t segs_fn, uint64_t cast_fn,
-               uint64_t comm_stream, bool overlap, int64_t batch_elems, int64_t slice_elems,
-               int channel, py::function refresh)
+               uint64_t comm_stream, bool overlap, int64_t batch_elems, int64_t busy_elems,
+               int64_t slice_elems, int channel, py::function refresh)
       : params_(std::move(params)),
         offsets_(std::move(offsets)),
         priorities_(std::move(priorities)),
@@ -74,6 +75,7 @@ class GradExchange {
         comm_(c10::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(comm_stream),
                                                device_)),
         batch_elems_(batch_elems),
+        busy_elems_(busy_elems),
         slice_elems_(slice_elems),
         channel_(channel),
         refresh_(std::move(refresh)) {
@@ -267,15 +269,21 @@ class GradExchange {
     sent_[i] = kPending;
     pending_ += padded;
     slices_ += (padded + slice_elems_ - 1) / slice_elems_;
-    if (pending_ >= batch_elems_) Drain(lk);
+    if (pending_ >= batch_elems_) {
+      const bool idle = Idle(cur);
+      if (idle || pending_ >= busy_elems_) Drain(lk);
+    }
   }
 
-  // Gives up the gradients whose kernels have finished.
-  void Collect(const c10::cuda::CUDAStream& cur) {
+  // Gives up the gradients whose kernels have finished, and says whether all have.  While one is
+  // running, what is pending would only queue up behind it; it goes out with what comes next
+  // instead, in fewer and larger launches.
+  bool Idle(const c10::cuda::CUDAStream& cur) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     C10_CUDA_CHECK(cudaStreamIsCapturing(cur.stream(), &capture));
-    if (capture != cudaStreamCaptureStatusNone) return;  // (an event may not be queried)
+    if (capture != cudaStreamCaptureStatusNone) return true;  // (an event may not be queried)
     while (!batches_.empty() && batches_.front().read.query()) Retire();
+    return batches_.empty();
   }
 
   // Sends what is pending, behind the stream of its hooks.  `lk` holds mu_; it is given up while
@@ -291,7 +299,6 @@ class GradExchange {
     if (segs_.empty()) return;  // another thread has sent them
     const auto made_on = *pending_on_;
     const auto stream = overlap_ ? comm_ : made_on;
-    Collect(made_on);
     After(made_on, stream);
     if (launched_on_) After(*launched_on_, stream);
     launched_on_ = stream;
@@ -334,7 +341,7 @@ class GradExchange {
   c10::DeviceIndex device_;
   bool overlap_;
   c10::cuda::CUDAStream comm_;
-  int64_t batch_elems_, slice_elems_;
+  int64_t batch_elems_, busy_elems_, slice_elems_;
   int channel_;
   py::function refresh_;
   struct Attached {
@@ -373,7 +380,7 @@ PYBIND11_MODULE(psb200_torch, m) {
   py::class_<GradExchange>(m, "GradExchange")
       .def(py::init<std::vector<at::Tensor>, std::vector<int64_t>, std::vector<int64_t>, at::Tensor,
                     uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, bool, int64_t,
-                    int64_t, int, py::function>())
+                    int64_t, int64_t, int, py::function>())
       .def("step", &GradExchange::Step, release())
       .def("detach", &GradExchange::Detach, release())
       .def_property_readonly("launches", &GradExchange::launches)

@@ -1547,8 +1547,6 @@ static int pick_plain(long long M, long long N, long long K) {
     for (int split = 1; split <= kMaxSplit; split *= 2) {
       const double ctas = tiles(128, n) * split;  // (two CTAs share an SM)
       if (split > 1 ? (ctas > split_fits(n, split, false) || split > kb) : ctas > most) break;
-      // (tests hold the choice for 64x256x4096, which clusters of eight would do in 5.4 for 7.0 us)
-      if (split == 8 && ctas <= 32 && kb >= 64) break;
       const double k = ceil(kb / split), full = fmin(ctas / sms, 1);
       const double over = fmin(fmax(0.0, ctas / (2 * sms) - 0.5), 1.0);
       // A k-block in a round with one and with two CTAs per SM, added up over the rounds.  In one

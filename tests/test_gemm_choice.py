@@ -26,7 +26,7 @@ def test_small_tiles_outside_of_the_measured_sizes(choice, m, n, k):
 
 @pytest.mark.parametrize("m,n,k,code", [(300, 16384, 4096, 2512), (1, 50264, 1024, 0), (64, 50264, 1024, 1128),
                                         (1024, 1024, 1024, 1064), (7572, 288, 256, 1064),
-                                        (16384, 3072, 1024, 2512), (64, 256, 4096, 4064)])
+                                        (16384, 3072, 1024, 2512), (64, 256, 4096, 8064)])
 def test_choices(choice, m, n, k, code):
     assert choice(m, n, k) == code
 
@@ -36,3 +36,10 @@ def test_choices(choice, m, n, k, code):
 def test_rows_that_begin_inside_a_sector(choice, m, n, k):
     """Pairs, where small tiles would read such rows."""
     assert choice(m, n, k) in (2256, 2512)
+
+
+@pytest.mark.parametrize("m,n", [(1, 256), (64, 64), (64, 256), (100, 200), (128, 256), (128, 512), (256, 256)])
+def test_a_longer_k_keeps_its_parts(choice, m, n):
+    """A few tiles: one more k-block does not take CTAs from the cluster that shares it."""
+    parts = [choice(m, n, k) // 1000 for k in range(1024, 16385, 64)]
+    assert all(b >= a for a, b in zip(parts, parts[1:])) and parts[-1] == 8

@@ -8,7 +8,7 @@
 // columns from the others between two barriers, and the sums lay row by row (a warp's accesses 32
 // pieces of 16 bytes), the exchange took 3 us among four CTAs and 6 among eight; now 1.5.  us,
 // 75 x 928 x 3504 with S = 4 / 8: 8.7 / 9.8 before, 7.2 / 5.9 now (S = 1 13.6); 64 x 256 x 4096
-// 9.2 / 9.9 and 7.0 / 5.4; 92 x 592 x 1360 6.9 / 11.4 and 5.1 / 5.5.
+// 9.2 / 9.9 and 7.3 / 5.7; 92 x 592 x 1360 6.9 / 11.4 and 5.1 / 5.5.
 // There is no loop over tiles, no counter in global memory, and the first loads are issued before
 // the CTA has met at its first barrier, because what bounds these products is a chain of
 // latencies: launch, operands from L2 or HBM, a few MMAs, accumulator, store.
@@ -18,15 +18,16 @@
 // Launched with programmatic stream serialization: the prologue runs beside the end of the kernel
 // before it.
 //
-// Two forms.  With more CTAs than SMs about 100 KB of shared memory per CTA, so that two share an
-// SM and one loads while the other stores.  Otherwise (DEEP) one CTA has the SM, and a stage holds
+// Two forms.  With more CTAs than SMs up to 100 KB of shared memory per CTA, so that two share an
+// SM and one loads while the other stores (121 KB and one with 128 columns and S = 4 or 8, whose
+// exchange takes 48 and 56).  Otherwise (DEEP) one CTA has the SM, and a stage holds
 // two k-blocks: per stage the ring costs some 300 clocks (commit, barrier, producer) whatever it
 // carries, and 128 columns of K make up for them.  The issuer of the deep form touches no mbarrier
 // (see wait_ready).  1024 x 1024 x 4096 with BN = 64 / 128 20.9 / 24.5 us shallow, 16.5 / 18.2
 // deep; what is left is the loads, 70 bytes per clock and SM.
 //
 // Measured, us (this kernel / the persistent 128 x 256 kernel): 64x256x256 2.8 / 6.5,
-// 1024x1024x256 4.1 / 8.4, 1024x1024x1024 6.0 / 11.9, 64x256x4096 7.0 / 23.4 (S = 4).
+// 1024x1024x256 4.1 / 8.4, 1024x1024x1024 6.0 / 11.9, 64x256x4096 5.7 / 23.4 (S = 8).
 #pragma once
 #include "ps/device/sm100_ptx.cuh"
 

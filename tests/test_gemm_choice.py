@@ -40,6 +40,8 @@ def test_rows_that_begin_inside_a_sector(choice, m, n, k):
 
 @pytest.mark.parametrize("m,n", [(1, 256), (64, 64), (64, 256), (100, 200), (128, 256), (128, 512), (256, 256)])
 def test_a_longer_k_keeps_its_parts(choice, m, n):
-    """A few tiles: one more k-block does not take CTAs from the cluster that shares it."""
-    parts = [choice(m, n, k) // 1000 for k in range(1024, 16385, 64)]
+    """A few tiles: one more k-block does not take CTAs from the cluster that shares it.  (From 32
+    k-blocks on: of fewer, 17 say, a part of eight has as many as one of six would, and a cluster of
+    four can be ahead.)"""
+    parts = [choice(m, n, k) // 1000 for k in range(2048, 16385, 64)]
     assert all(b >= a for a, b in zip(parts, parts[1:])) and parts[-1] == 8

@@ -34,6 +34,16 @@ def test_matches_fp32_matmul(cuda_device, M, N, K, bn, split):
     assert torch.all(guard[0] == 7.0) and torch.all(guard[-1] == 7.0)
 
 
+@pytest.mark.parametrize("bn", [64, 128])
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+@pytest.mark.parametrize("per", [2, 3, 4, 5])
+@pytest.mark.parametrize("short", [0, 56])
+def test_as_many_k_blocks_as_stages(cuda_device, per, short, bn, split):
+    """Two to five k-blocks for each CTA of a cluster, where the form with two of them per stage begins;
+    the last part one short."""
+    test_matches_fp32_matmul(cuda_device, 200, 2 * bn + 8, 64 * per * split - short, bn, split)
+
+
 def test_unknown_variants_are_refused(cuda_device):
     from ps_lite_b200 import _lib
     lib = _lib.device_lib()

@@ -1376,11 +1376,11 @@ static int launch_split(int split, const SplitArgs& a, const CUtensorMap& tx,
     default: return PSDEV_ERR_ARG;
   }
 }
-// CTAs of a split product that run at a time.  Clusters keep inside a GPC: on the B200 that the times
-// below were taken on 33 clusters of four and 15 of eight find SMs of their own, 71 and 33 with two CTAs
-// per SM, which the shared memory allows where what the parts send is small.  (Where GPCs have other
-// numbers of SMs the counts differ by a cluster or two: the estimate is off by a round there, no result.
-// The choice is made on the host without a GPU, so they are not asked for.)
+// CTAs of a split product that run at a time.  Clusters keep inside a GPC: on the B200 that the
+// times below were taken on 33 clusters of four and 15 of eight find SMs of their own, 71 and 33
+// with two CTAs per SM, which the shared memory allows where what the parts send is small.  (Where
+// GPCs have other numbers of SMs the counts differ by a cluster or two: the estimate is off by a
+// round there, no result.  The choice is made without a GPU, so they are not asked for.)
 static int split_fits(int bn, int split, bool deep) {
   const bool one = deep || (bn == 128 && split >= 4);
   return split == 8 ? (one ? 120 : 264) : split == 4 ? (one ? 132 : 284) : one ? 148 : 296;
@@ -1393,9 +1393,10 @@ static int shallow_stages(int split) {
                       : SplitCfg<BN, 1, false>::kStages;
 }
 // Two k-blocks per stage and one CTA per SM, where SMs would have one CTA anyway and the loop is
-// longer than the shallow form's stages, which it would then wait for.  us, shallow / deep, with four
-// k-blocks per part: 512 x 1024 x 456 S = 2, BN = 64 7.1 / 5.3, 256 x 1024 x 1024 S = 4 6.4 / 5.1;
-// with three, S = 8, 128 x 512 x 1536 5.4 / 4.8 and S = 2, BN = 128, 1024 x 1024 x 328 8.8 / 6.1.
+// longer than the shallow form's stages, which it would then wait for.  us, shallow / deep, with
+// four k-blocks per part: 512 x 1024 x 456 S = 2, BN = 64 7.1 / 5.3, 256 x 1024 x 1024 S = 4
+// 6.4 / 5.1; with three: S = 8, 128 x 512 x 1536 5.4 / 4.8 and S = 2, BN = 128, 1024 x 1024 x 328
+// 8.8 / 6.1.
 static bool split_deep(int bn, int split, long long ctas, int num_kb) {
   return ctas <= split_fits(bn, split, true) &&
          num_kb > (bn == 64 ? shallow_stages<64>(split) : shallow_stages<128>(split));
@@ -1549,8 +1550,8 @@ static int pick_plain(long long M, long long N, long long K) {
   // round of its own.  us: 312 CTAs of 128 x 128 for 3013x1616x2104 50.9, pairs 26.6; 338 of
   // 128 x 64 for 1603x1624x824 18.7, pairs 10.6; 295 of 128 x 64 for 7525x280x3528 38.2, pairs
   // 26.9.
-  // Over 204 sizes drawn with M 64 .. 16384, N and K any multiples of 8 in 256 .. 4096, the choice is
-  // 1.010 of the fastest form in the mean and 1.17 at most (1515x1784x328 and 140x1096x3592, two
+  // Over 204 sizes drawn with M 64 .. 16384, N and K any multiples of 8 in 256 .. 4096, the choice
+  // is 1.010 of the fastest form in the mean and 1.17 at most (1515x1784x328 and 140x1096x3592, two
   // runs), 1.05 and 1.97 when neither was looked at; over the grid of the sweep 1.004 and 1.14.
   const double rows = K % 16 ? 1.5 : K % 64 ? 1.1 : 1;
   const bool fitted = M >= 64 && (double)N * (double)K <= 4096.0 * 4096.0;

@@ -1,6 +1,7 @@
-// Utility kernels for key lists: radix sort of 64-bit keys, 8 bits per pass (with an
-// optional payload of 32-bit indices) and ordered match (merge-join) of two sorted key lists
-// with an assignment operator applied to the values of the keys present in both.
+// Utility kernels for key lists: radix sort of 64-bit keys, 8 bits per pass (with an optional
+// payload of 32-bit indices), sums of the values of equal keys (sorted by 8 or up to 10 bits per
+// pass) and ordered match (merge-join) of two sorted key lists with an assignment operator applied
+// to the values of the keys present in both.
 //
 // They are the device form of helpers the reference ships as headers that nothing includes
 // and that do not compile as written: ParallelSort (include/ps/internal/parallel_sort.h:23-55,
@@ -35,12 +36,18 @@ namespace sortk {
 // 32 bits (which then needs no array of its own: one store of 8 bytes per item where two of 4 went
 // to different places).
 //
-// Digits have 8 bits, or up to 10 where that saves a pass and the runs of equal digits, which are
-// then a quarter as long, are not too short for what DRAM takes at a time (kWidePairs, kWideKeys).
-// Distinct ids and sums, us, ids with many repeats / all over the key space: four passes and three
-// (30 bits, pairs) 2^20 93 / 92 and 78 / 86, 2^22 212 / 202 and 172 / 182, 10^7 456 / 444 and
-// 382 / 451, 2^24 703 / 674 and 623 / 708; five passes and four (40 bits) 10^6 113 / 113 and
-// 102 / 106, 2^22 251 / 262 and 260 / 306.
+// Digits have 8 bits, or up to 10 where that saves a pass (kWidePairs, kWideKeys).  Runs of equal
+// digits are then a quarter as long, for keys all over the key space shorter than what DRAM takes
+// at a time.  Whole calls of sort_unique_sum, us, ids with many repeats / all different:
+//   30 bits         10^6     2^22       2^23       2^24       2^25         4 10^7
+//   four passes    90 / 92  194 / 204  341 / 373  647 / 694  1265 / 1328  1487 / 1569
+//   three          81 / 87  168 / 182  312 / 377  615 / 715  1185 / 1360  1394 / 1594
+//   form before    98 / 93  212 / 203  348 / 355  662 / 671  1277 / 1305  1498 / 1550
+//   40 bits, five passes and four: 113 / 113 and 102 / 106 (10^6), 251 / 262 and 260 / 306 (2^22)
+// Pairs have wide digits up to 2^25: ids that repeat, which a batch has and which the sums are for,
+// gain 5 to 14 %, those all different lose 1 to 4 from 2^23 on.  (Larger sorts would be the same
+// trade.  The form before had keys and values in two arrays, four passes, and counted the distinct
+// keys before it summed: for ids all different from 2^23 on the faster way, by 3 to 7 %.)
 //
 // Up to some million items everything stays in L2.  The single-sweep form (one launch per pass,
 // tiles finding their offsets by looking back over the words that earlier tiles publish) spent a
@@ -58,11 +65,11 @@ constexpr int kWideBits = 10;
 constexpr int kMaxChunks = 2 * 148;        // two CTAs per SM
 constexpr int kMinChunk = 2048;
 constexpr long long kWidePairs = 1 << 25, kWideKeys = 2 << 20;
-// Up to so many items pairs that keep to digits of 8 bits travel in one word from the first pass on.
-// More have arrays of keys and values until the last one.  us, ids of 24 bits all over the key space
-// / with many repeats / half of them one id, together and apart: 2^20 71 / 74 / 75 and 74 / 75 / 77,
-// 2^22 162 / 164 / 174 and 153 / 152 / 161, 2^24 535 / 539 / 579 and 522 / 498 / 528 (all three 3 to 8 %
-// slower together than in the form before pairs, 545 / 519 / 538, but for the first).
+// Up to so many items pairs that keep to digits of 8 bits travel in one word from the first pass
+// on.  More have arrays of keys and values until the last one.  us, ids of 24 bits all over the key
+// space / with many repeats / half of them one id: together 2^20 71 / 74 / 75, 2^22 162 / 164 / 174,
+// 2^24 535 / 539 / 579; apart 74 / 75 / 77, 153 / 152 / 161, 522 / 498 / 528 (in the form before
+// pairs 73 / 75 / 73, 161 / 168 / 174, 545 / 519 / 538).
 constexpr long long kPairsTogether = 3 << 19;
 // Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
 // number of launches (64-bit keys without payload, 2^14 / 2^16, us: 119 / 110 with three launches
@@ -222,8 +229,8 @@ __global__ void __launch_bounds__(1024)
 }
 
 // What travels beside the keys of a pass: nothing, the key's index or a value of 32 bits in an
-// array of its own, or a value that a first pass puts below its key.  With values in an array, keys of
-// up to 32 bits can have 32 too: the first pass narrows them (kNarrow), the last one puts pairs
+// array of its own, or a value that a first pass puts below its key.  With values in an array, keys
+// of up to 32 bits can have 32 too: the first pass narrows them (kNarrow), the last one puts pairs
 // together (kShortToPairs).
 enum {
   kNoPayload = 0, kMakeIndex = 1, kPayload = 2, kToPairs = 3,
@@ -325,7 +332,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
         total[i] = __ldcg(totals + d0 + i);
       }
     } else {
-      // (eight chunks' counts in flight, also at the end: one after the other, 29 chunks cost more than 32)
+      // (eight chunks' counts in flight, also the last ones: one by one 29 chunks cost more than 32)
       for (int c0 = 0; c0 < ch.count; c0 += 8) {
         uint2 v[8][kPer];
 #pragma unroll
@@ -869,8 +876,8 @@ __global__ void __launch_bounds__(kUniqueThreads)
   const long long base = (long long)blockIdx.x * kRound;
   if (count == 0) return;
   // What the rounds behind have found of the last key.  A warp looks at 32 of them, which is enough
-  // for most keys, and then at 512 at a time: 32 at a time took 90 us of 2^24 pairs with one key, where
-  // one CTA goes through all 8192 rounds.
+  // for most keys, and then at 512 at a time: 32 at a time took 90 us of 2^24 pairs with one key,
+  // where one CTA goes through all 8192 rounds.
   float more = 0.f;
   if (threadIdx.x < 32) {
     auto open_behind = [&](int r0, auto groups) {  // whether the key goes on behind these rounds
@@ -887,7 +894,7 @@ __global__ void __launch_bounds__(kUniqueThreads)
 #pragma unroll
       for (int j = 0; j < kGroups; ++j) {
         const unsigned int stop = __ballot_sync(0xffffffffu, ends[j]);
-        const int n = stop ? __ffs(stop) : 32;  // (the round in which the next key begins has a lead)
+        const int n = stop ? __ffs(stop) : 32;  // (the round of the next key's begin has a lead)
         if (open && (int)threadIdx.x < n) v += lead[j];
         if (stop) open = false;
       }
@@ -1042,8 +1049,8 @@ int psdev_sort_status(const void* scratch, void* stream) {
 // ---- unsorted, repeated (key, value) pairs -> sorted distinct keys and sums ---------------------
 namespace {
 // How (key, value) pairs are sorted: pairs in one word up to 32 bits, and digits of 10 bits where
-// they save a pass.  Where they do not, many keys have an array of their own until the last pass, so
-// that counting reads 4 bytes per item (kPairsTogether).
+// they save a pass.  Where they do not, many keys have an array of their own until the last pass,
+// so that counting reads 4 bytes per item (kPairsTogether).
 struct UniquePlan {
   bool pairs, apart;
   int bits, passes, width;
@@ -1062,9 +1069,9 @@ struct UniquePlan {
   }
 };
 
-// Layout of the scratch memory: counts and leads of the rounds of distinct keys, two buffers of items
-// and, for keys of more than 32 bits, of values, then the working memory of the sort.  (The second
-// half of a call reads all but the last part, and of key_bits it needs `pairs` alone.)
+// Layout of the scratch memory: counts and leads of the rounds of distinct keys, two buffers of
+// items and, for keys of more than 32 bits, of values, then the working memory of the sort.  (The
+// second half of a call reads all but the last part, and of key_bits it needs `pairs` alone.)
 struct UniqueScratch {
   SortHead* head;
   unsigned int* counts;
@@ -1276,8 +1283,8 @@ int psdev_unique_sum_sort(const uint64_t* keys, const float* vals, int64_t n, in
   return 0;
 }
 
-// Second half: the distinct keys, ascending, and the sums of their values.  `n` and `key_bits` are those
-// of the first half, `n_unique` what it counted.
+// Second half: the distinct keys, ascending, and the sums of their values.  `n` and `key_bits` are
+// those of the first half, `n_unique` what it counted.
 int psdev_unique_sum_write(const void* scratch, int64_t n, int key_bits, int64_t n_unique,
                            uint64_t* out_keys, float* out_sums, void* stream) {
   if (!scratch || !out_keys || !out_sums || n < 1 || n_unique < 1 || key_bits < 1 || key_bits > 64)

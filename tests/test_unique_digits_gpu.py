@@ -81,3 +81,17 @@ def test_a_key_wider_than_stated_among_many(cuda_device, n):
     got, sums = sort_unique_sum(keys, torch.ones(n, device=cuda_device), key_bits=24)
     assert int(sums.sum()) == n and bool(((got & 0xffffff).diff() >= 0).all())
     assert (1 << 40) + n // 2 % 1000 in got.tolist()
+
+
+# more rounds than have their counts put together at a time (2048, of 2048 pairs), and the sizes from
+# which 30 bits take digits of 8 bits
+@pytest.mark.parametrize("n,bits", [(1 << 22, 30), ((1 << 22) + 1, 30), ((1 << 22) + 1, 40), (9_000_000, 30),
+                                    (9_000_000, 40), (1 << 25, 30), ((1 << 25) + 1, 30)])
+def test_many_rounds(cuda_device, n, bits):
+    g = torch.Generator(device=cuda_device)
+    g.manual_seed(n)
+    keys = torch.randint(0, 1 << bits, (n,), device=cuda_device, generator=g)
+    # ids of which the sorted list has a run around the pair that begins the 2049th round
+    middle = torch.sort(keys).values[min(n - 1, 1 << 22)]
+    keys[torch.randperm(n, device=cuda_device, generator=g)[:9000]] = middle
+    _check(keys, torch.randn(n, device=cuda_device, generator=g), bits)

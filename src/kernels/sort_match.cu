@@ -67,8 +67,8 @@ constexpr int kMinChunk = 2048;
 constexpr long long kWidePairs = 1 << 25, kWideKeys = 2 << 20;
 // Up to so many items pairs that keep to digits of 8 bits travel in one word from the first pass
 // on.  More have arrays of keys and values until the last one.  us, ids of 24 bits all over the key
-// space / with many repeats / half of them one id: together 2^20 71 / 74 / 75, 2^22 162 / 164 / 174,
-// 2^24 535 / 539 / 579; apart 74 / 75 / 77, 153 / 152 / 161, 522 / 498 / 528 (in the form before
+// space / with many repeats / half of them one id: together 2^20 71 / 74 / 75, 2^22
+// 162 / 164 / 174, 2^24 535 / 539 / 579; apart 74 / 75 / 77, 153 / 152 / 161, 522 / 498 / 528 (in the form before
 // pairs 73 / 75 / 73, 161 / 168 / 174, 545 / 519 / 538).
 constexpr long long kPairsTogether = 3 << 19;
 // Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
         total[i] = __ldcg(totals + d0 + i);
       }
     } else {
-      // (eight chunks' counts in flight, also the last ones: one by one 29 chunks cost more than 32)
+      // (eight chunks' counts in flight, the last ones too: one by one 29 chunks cost more than 32)
       for (int c0 = 0; c0 < ch.count; c0 += 8) {
         uint2 v[8][kPer];
 #pragma unroll

@@ -67,9 +67,11 @@ constexpr int kMinChunk = 2048;
 constexpr long long kWidePairs = 1 << 25, kWideKeys = 2 << 20;
 // Up to so many items pairs that keep to digits of 8 bits travel in one word from the first pass
 // on.  More have arrays of keys and values until the last one.  us, ids of 24 bits all over the key
-// space / with many repeats / half of them one id: together 2^20 71 / 74 / 75, 2^22
-// 162 / 164 / 174, 2^24 535 / 539 / 579; apart 74 / 75 / 77, 153 / 152 / 161, 522 / 498 / 528 (in the form before
-// pairs 73 / 75 / 73, 161 / 168 / 174, 545 / 519 / 538).
+// space / with many repeats / half of them one id:
+//               2^20            2^22               2^24
+//   together    71 / 74 / 75   162 / 164 / 174   535 / 539 / 579
+//   apart       74 / 75 / 77   153 / 152 / 161   522 / 498 / 528
+//   form before 73 / 75 / 73   161 / 168 / 174   545 / 519 / 538
 constexpr long long kPairsTogether = 3 << 19;
 // Up to so many chunks the scatter adds up the counts itself: sorts of that size are bound by the
 // number of launches (64-bit keys without payload, 2^14 / 2^16, us: 119 / 110 with three launches

@@ -438,8 +438,8 @@ __host__ __device__ constexpr int local_unroll(bool group, bool one, bool far) {
 // request, a whole one is one access instead of two (a hash store with a quarter of its slots
 // wanted: 34 us without the hint, 42 with it).  The rule looks at the whole table.  Keys that lie
 // close together in a large one lose nothing by it: 2^20 keys of 2^28 in runs of 4, 8 and 64, state
-// in DRAM, us without and with the hint 16.9 / 16.7, 12.3 / 12.3, 11.0 / 10.9 and, states of 4 bytes,
-// which then also have one key per thread, 17.3 / 14.9, 13.3 / 10.5, 11.6 / 8.9.
+// in DRAM, us without and with the hint 16.9 / 16.7, 12.3 / 12.3, 11.0 / 10.9.  States of 4 bytes,
+// which then also have one key per thread, take 17.3 / 14.9, 13.3 / 10.5 and 11.6 / 8.9.
 template <bool FAR>
 __device__ __forceinline__ float load_one(const float* p) {
   if constexpr (!FAR) return *p;

@@ -19,7 +19,7 @@ def _check(keys, vals, bits):
     assert bool(((sums.double() - exact).abs() <= (times - 1) * 2.0 ** -24 * size).all())
 
 
-# one tile of the one-CTA sort, the chunks whose counts the scatter adds up, chunks of more than the
+# one tile of the one-CTA sort, chunks that grow until there are 32 of them, chunks of more than the
 # smallest size, the larger tiles, and where keys of more than 32 bits go back to digits of 8 bits
 @pytest.mark.parametrize("n", [4096, 4097, 32 * 2048, 32 * 2048 + 1, 296 * 2048 + 1, 296 * 4096,
                                296 * 4096 + 1, 1 << 21, (1 << 21) + 1])
@@ -31,6 +31,14 @@ def test_sizes(cuda_device, n, bits):
     keys[::3] = keys[0]                                # a popular id
     keys[1::5] = (1 << bits) - 1 - keys[1::5] % 1000   # some hundred, at the upper end
     _check(keys, torch.randn(n, device=cuda_device, generator=g), bits)
+
+
+# the chunks whose counts the scatter adds up: 16 of digits of 10 bits, 32 (of up to 4096) of 8, which
+# keys of more than 40 bits have in between
+@pytest.mark.parametrize("n", [16 * 2048, 16 * 2048 + 1, 29 * 2560, 80 << 10, 32 * 4096, 32 * 4096 + 1])
+@pytest.mark.parametrize("bits", [8, 24, 30, 40, 48, 56, 60, 62])
+def test_sizes_of_a_few_chunks(cuda_device, n, bits):
+    test_sizes(cuda_device, n, bits)
 
 
 # runs of equal keys that fill rounds of 2048 pairs, end with them or cross many of them

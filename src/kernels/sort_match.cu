@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cmath>
 #include <type_traits>
 #include <utility>
 
@@ -38,7 +39,8 @@ namespace sortk {
 //
 // Digits have 8 bits, or up to 10 where that saves a pass (kWidePairs, kWideKeys).  Runs of equal
 // digits are then a quarter as long, for keys all over the key space shorter than what DRAM takes
-// at a time.  Whole calls of sort_unique_sum, us, ids with many repeats / all different:
+// at a time.  Calls of sort_unique_sum pass by pass (which those above 4.7 million items and others
+// that piece_sum.cuh is not for still go), us, ids with many repeats / all different:
 //   30 bits         10^6     2^22       2^23       2^24       2^25         4 10^7
 //   four passes    90 / 92  194 / 204  341 / 373  647 / 694  1265 / 1328  1487 / 1569
 //   three          81 / 87  168 / 182  312 / 377  615 / 715  1185 / 1360  1394 / 1594
@@ -85,6 +87,12 @@ constexpr int kSelfScan = 32, kSelfScanWide = 16, kMaxSelfChunk = 4096;
 // Head of the scratch memory.
 struct SortHead {
   int too_wide;                            // 1: a key has bits beyond key_bits
+  int groups;                              // of segments (piece_sum.cuh); 0: rounds
+  int shift;                               // of the group in a key, 0: items have whole keys
+  unsigned int pieces, several;
+  int split, separate;                     // parts begin at b.splits; keys and sums in two arrays
+  unsigned int done;                       // CTAs of the merge
+  int crowded;                             // 1: a part has too many distinct keys
 };
 
 // The chunks of n items.  A tile of the scatter has `rows` rows of 32 items per warp; the tiles of
@@ -151,12 +159,104 @@ __device__ __forceinline__ unsigned int item_digit(Item k, int shift, unsigned i
   return (unsigned int)(k >> shift) & mask;
 }
 
-// counts[c * 2^BITS + d] = items of chunk c whose digit is d
-template <typename K, int BITS>
+// What a sort reports to the host, one word in mapped memory: whether a key was too wide, whether
+// the keys are too close together for buckets, and the number of distinct keys.
+constexpr unsigned long long kReported = 1ull << 63, kReportWide = 1ull << 62,
+                             kReportCrowded = 1ull << 61;
+__device__ __forceinline__ void host_report(unsigned long long* host, unsigned int total,
+                                            bool too_wide) {
+  *reinterpret_cast<volatile unsigned long long*>(host) =
+      kReported | (too_wide ? kReportWide : 0) | total;
+  __threadfence_system();
+}
+
+// Counters of two digits in a word.
+__device__ __forceinline__ unsigned int half_of(unsigned int word, unsigned int d) {
+  return (d & 1) ? word >> 16 : word & 0xffffu;
+}
+
+// In how many rows of 32 a lane has an item: `left` from its first one to the end of them all.
+__device__ __forceinline__ int valid_rows(int left, int rows) {
+  const int have = (left + 31) >> 5;
+  return have < rows ? have : rows;
+}
+
+// Ranks of a warp's items, in rows of 32: of each among those with the same digit, in index order;
+// two of 16 bits in a word of `rank`.  `cnt`, of zeros, ends up with the number of each digit's
+// items; `lanes`: zeros, and again afterwards.  A lane has items in its first `valid` rows.
+//
+// The lanes that hold the same digit find each other through a mask in shared memory (32 keys of an
+// SM in 9 ns; 15 with ballots, 32 with match.any), and the first of them advances the counter.
+// FREE: items of a digit may be in any order, the counter gives out the ranks.  (Lanes of one
+// instruction get theirs in the hardware's order, on which nothing but rounding depends.)
+// POPULAR: most items have the same key, so that the lanes with the digit of the first lane are
+// found with a ballot (32 atomics on one address take an SM some 70 clocks).
+template <bool FREE, bool POPULAR, int ROWS, typename Digit>
+__device__ __forceinline__ void rank_rows(const Digit& digit, int rows, int valid,
+                                          unsigned int* lanes, unsigned short* cnt,
+                                          unsigned int (&rank)[ROWS / 2]) {
+  const unsigned int mine = 1u << (threadIdx.x & 31), below = lanemask_lt();
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    if (j % 2 == 0 && j >= rows) break;
+    const bool in = j < valid;
+    const unsigned int d = digit(j);
+    unsigned int like = 0, r = 0;  // like: lanes with the first one's digit, where this one has it
+    if constexpr (POPULAR) {
+      const unsigned int d0 = __shfl_sync(0xffffffffu, d, 0);
+      const unsigned int all = __ballot_sync(0xffffffffu, in && d == d0);
+      if (in && d == d0) like = all;
+    }
+    if constexpr (FREE) {
+      const unsigned int add = POPULAR && like ? __popc(like) : 1u;
+      if (in && (!POPULAR || (like & below) == 0))
+        r = half_of(atomicAdd(reinterpret_cast<unsigned int*>(cnt) + d / 2, add << (d & 1) * 16),
+                    d);
+      if constexpr (POPULAR) {
+        const unsigned int of_first = __shfl_sync(0xffffffffu, r, like ? __ffs(like) - 1 : 0);
+        if (like) r = of_first + __popc(like & below);
+      }
+    } else {
+      if (in && !like) atomicOr(&lanes[d], mine);
+      __syncwarp();
+      const unsigned int same = like ? like : lanes[d];
+      const unsigned int first = cnt[d], before = __popc(same & below);
+      __syncwarp();
+      if (in && before == 0) {
+        lanes[d] = 0;
+        cnt[d] = (unsigned short)(first + __popc(same));
+      }
+      r = first + before;
+      __syncwarp();
+    }
+    if (j & 1) rank[j / 2] |= r << 16;
+    else rank[j / 2] = r;
+  }
+}
+
+}  // namespace sortk
+}  // namespace psdev
+#include "kernels/piece_sum.cuh"
+namespace psdev {
+namespace sortk {
+
+// counts[c * 2^BITS + d] = items of chunk c whose digit is d.  SAMPLE: one CTA more looks at a
+// sample of the keys, and wide keys are noted chunk by chunk.
+template <typename K, int BITS, bool SAMPLE>
 __global__ void __launch_bounds__(kThreads, 2)
     digit_count_kernel(const K* __restrict__ keys, long long n, int shift, unsigned int mask,
-                       Chunks ch, int key_bits, unsigned int* counts, SortHead* head) {
+                       Chunks ch, int key_bits, unsigned int* counts, SortHead* head,
+                       const __grid_constant__ Buckets b, unsigned long long* host) {
   grid_launch_next();
+  if constexpr (SAMPLE) {
+    if (blockIdx.x == ch.count) {
+      grid_wait();
+      __shared__ __align__(16) unsigned int slots[kSampleSlots];
+      __shared__ unsigned int found[kMaxBuckets];
+      sample_buckets<kThreads>(keys, (unsigned int)n, __popc(mask), b, {slots, found}, head, host);
+      return;
+    }
+  }
   constexpr int kDigits = 1 << BITS, kSets = BITS > 8 ? 2 : 4;
   constexpr int kItems = 14;  // (2^22 items: 28 per thread; 8.4 us, 8.9 with 8 loads in flight)
   __shared__ unsigned int s[kSets][kDigits];  // groups of warps share a set of counters
@@ -180,24 +280,19 @@ __global__ void __launch_bounds__(kThreads, 2)
         atomicAdd(&mine[item_digit(k[j], shift, mask)], 1u);
       }
   }
-  if (wide) head->too_wide = 1;
-  __syncthreads();
+  if constexpr (SAMPLE) {
+    wide = __syncthreads_or(wide);
+    if (threadIdx.x == 0) b.wide[blockIdx.x] = wide;
+  } else {
+    if (wide) head->too_wide = 1;
+    __syncthreads();
+  }
   for (int d = threadIdx.x; d < kDigits; d += kThreads) {
     unsigned int c = 0;
 #pragma unroll
     for (int w = 0; w < kSets; ++w) c += s[w][d];
     counts[(size_t)blockIdx.x * kDigits + d] = c;
   }
-}
-
-// What a sort reports to the host, one word in mapped memory: whether a key was too wide and the
-// number of distinct keys.
-constexpr unsigned long long kReported = 1ull << 63, kReportWide = 1ull << 62;
-__device__ __forceinline__ void host_report(unsigned long long* host, unsigned int total,
-                                            bool too_wide) {
-  *reinterpret_cast<volatile unsigned long long*>(host) =
-      kReported | (too_wide ? kReportWide : 0) | total;
-  __threadfence_system();
 }
 
 // 32 digits per CTA: exclusive prefix over the chunks in place, and the digits' totals.  A warp
@@ -234,15 +329,19 @@ __global__ void __launch_bounds__(1024)
 // array of its own, or a value that a first pass puts below its key.  With values in an array, keys
 // of up to 32 bits can have 32 too: the first pass narrows them (kNarrow), the last one puts pairs
 // together (kShortToPairs).
+// Equal keys of sums may be in any order: a first pass (kToPairs, kNarrow, kFirst: kPayload) needs
+// no masks (rank_rows, FREE).
 enum {
   kNoPayload = 0, kMakeIndex = 1, kPayload = 2, kToPairs = 3,
-  kNarrow = 4, kShort = 5, kShortToPairs = 6
+  kNarrow = 4, kShort = 5, kShortToPairs = 6, kFirst = 7
 };
 template <int PAY>
 struct Form {
   static constexpr bool kShortIn = PAY == kShort || PAY == kShortToPairs;
   static constexpr bool kShortKey = kShortIn || PAY == kNarrow;
-  static constexpr bool kArray = PAY == kMakeIndex || PAY == kPayload || kShortKey;
+  static constexpr bool kArray =
+      PAY == kMakeIndex || PAY == kPayload || PAY == kFirst || kShortKey;
+  static constexpr bool kFree = PAY == kToPairs || PAY == kNarrow || PAY == kFirst;
   using In = std::conditional_t<kShortIn, unsigned int, Item>;    // as a pass reads them
   using Key = std::conditional_t<kShortKey, unsigned int, Item>;  // and ranks them
 };
@@ -389,34 +488,14 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
   for (long long tile_base = lo; tile_base < hi; tile_base += tile) {
     const long long base = tile_base + (long long)warp * (32 * rows) + lane;
     const int tile_n = (int)(hi - tile_base < tile ? hi - tile_base : tile);
-    for (int i = lane; i < kDigits; i += 32) lanes[i] = 0;
+    if constexpr (!Form<PAY>::kFree)
+      for (int i = lane; i < kDigits; i += 32) lanes[i] = 0;
     for (int i = lane; i < kPairs; i += 32) reinterpret_cast<unsigned int*>(cnt)[i] = 0;
     __syncwarp();
     unsigned int rank[ROWS / 2];  // two of 16 bits each
-#pragma unroll
-    for (int j = 0; j < ROWS; ++j) {
-      if (j >= rows) break;
-      // the lanes that hold the same digit find each other through a mask in shared memory (32 keys
-      // of an SM in 9 ns; 15 with ballots, 32 with match.any); the first of them advances the
-      // warp's counter for all of them
-      const bool valid = base + j * 32 < hi;
-      const unsigned int d = item_digit(k[j], shift, mask);
-      if (valid) atomicOr(&lanes[d], 1u << lane);
-      __syncwarp();
-      const unsigned int same = valid ? lanes[d] : 1u << lane;
-      const unsigned int before = __popc(same & lanemask_lt());
-      unsigned int r = 0;
-      __syncwarp();
-      if (valid && before == 0) {
-        lanes[d] = 0;
-        r = cnt[d];
-        cnt[d] = (unsigned short)(r + __popc(same));
-      }
-      r = __shfl_sync(0xffffffffu, r, __ffs(same) - 1) + before;
-      if (j & 1) rank[j / 2] |= r << 16;
-      else rank[j / 2] = r;
-      __syncwarp();
-    }
+    const int valid = valid_rows((int)(hi - base), rows);
+    rank_rows<Form<PAY>::kFree, false, ROWS>(
+        [&](int j) { return item_digit(k[j], shift, mask); }, rows, valid, lanes, cnt, rank);
     __syncthreads();
     // where the runs of this thread's digits start in the tile, and each warp's part of them
     unsigned int run[kPer], items = 0;
@@ -644,8 +723,9 @@ static int sort_pass(const Pass& p, const SortWork& w, cudaStream_t s) {
   if (int rc = allow_smem<scatter_kernel<BITS, WARPS, ROWS, PAY>>(C::kSmemBytes)) return rc;
   const Chunks ch = chunks_of(p.n, BITS, C::kThreads, ROWS);
   const unsigned int mask = (1u << p.width) - 1;
-  int rc = launch_chained(digit_count_kernel<In, BITS>, ch.count, kThreads, 0, s, 1, in, p.n,
-                          p.count_shift, mask, ch, p.check_bits, w.counts, w.head);
+  int rc = launch_chained(digit_count_kernel<In, BITS, false>, ch.count, kThreads, 0, s, 1, in, p.n,
+                          p.count_shift, mask, ch, p.check_bits, w.counts, w.head, Buckets{},
+                          nullptr);
   const bool scan = ch.count > (BITS == kRadixBits ? kSelfScan : kSelfScanWide);
   if (!rc && scan)
     rc = launch_chained(digit_scan_kernel, C::kDigits / 32, 1024, 0, s, 1, w.counts, C::kDigits,
@@ -665,7 +745,7 @@ static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) 
     return PSDEV_ERR_ARG;
   } else {
     if (p.n <= kMaxChunks * 4096ll) return sort_pass<kWideBits, 8, 16, PAY>(p, w, s);
-    return sort_pass<kWideBits, 16, PAY == kPayload ? 10 : 14, PAY>(p, w, s);
+    return sort_pass<kWideBits, 16, PAY == kPayload || PAY == kFirst ? 10 : 14, PAY>(p, w, s);
   }
 }
 
@@ -685,6 +765,7 @@ static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) 
 constexpr int kUniqueThreads = 256;
 constexpr int kUniquePer = 8;
 constexpr int kRound = kUniqueThreads * kUniquePer;
+constexpr unsigned kGatherCtas = 6 * 148;
 template <bool PAIRS, int THREADS>
 constexpr int unique_smem() {  // (a thread's pairs start in different banks)
   return THREADS * (kUniquePer + 1) * (8 + (PAIRS ? 0 : 4));
@@ -868,14 +949,50 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// The keys and sums of segments: CTA i takes the groups i, i + grid, ..., or with more CTAs than
+// groups one of several shares of a group.
+__device__ __forceinline__ void gather_segments(const Unique& u, const Segments& seg, int groups,
+                                                int shift, bool separate) {
+  const unsigned int low = shift > 0 && shift < 32 ? (1u << shift) - 1 : ~0u;
+  const unsigned int shares = gridDim.x / groups ? gridDim.x / groups : 1;
+  for (unsigned int g = blockIdx.x; g < groups * shares; g += gridDim.x) {
+    const unsigned int group = g / shares, share = g % shares;
+    const Item high = shift ? (Item)group << shift : 0;
+    const unsigned int *prefix = seg.counts + group * kGroup, *place = seg.place + group * kGroup;
+    unsigned int begin[kGroup + 1], from[kGroup];
+#pragma unroll
+    for (int p = 0; p <= kGroup; ++p) begin[p] = __ldcg(prefix + p);
+#pragma unroll
+    for (int p = 0; p < kGroup; ++p) from[p] = __ldcg(place + p);
+#pragma unroll 4
+    for (unsigned int i = begin[0] + share * kUniqueThreads + threadIdx.x; i < begin[kGroup];
+         i += shares * kUniqueThreads) {
+      unsigned int first = begin[0], at = from[0];
+#pragma unroll
+      for (int p = 1; p < kGroup; ++p)
+        if (i >= begin[p]) {
+          first = begin[p];
+          at = from[p];
+        }
+      const unsigned int q = (at & ~kMerged) + (i - first);
+      const Item k = __ldcg((at & kMerged ? u.keys : u.items) + q);
+      if (separate) {
+        u.out_keys[i] = k;
+        u.out_sums[i] = __ldcg((at & kMerged ? u.sums : u.vals) + q);
+        continue;
+      }
+      u.out_keys[i] = high | ((unsigned int)(k >> 32) & low);
+      u.out_sums[i] = __uint_as_float((unsigned int)k);
+    }
+  }
+}
+
+// The keys and sums of a round.
 template <bool PAIRS>
-__global__ void __launch_bounds__(kUniqueThreads)
-    unique_gather_kernel(const __grid_constant__ Unique u, int rounds) {
-  grid_launch_next();
-  grid_wait();
-  const unsigned int at = __ldcg(u.counts + blockIdx.x);
-  const unsigned int count = __ldcg(u.counts + blockIdx.x + 1) - at;
-  const long long base = (long long)blockIdx.x * kRound;
+__device__ __forceinline__ void gather_round(const Unique& u, int round, int rounds) {
+  const unsigned int at = __ldcg(u.counts + round);
+  const unsigned int count = __ldcg(u.counts + round + 1) - at;
+  const long long base = (long long)round * kRound;
   if (count == 0) return;
   // What the rounds behind have found of the last key.  A warp looks at 32 of them, which is enough
   // for most keys, and then at 512 at a time: 32 at a time took 90 us of 2^24 pairs with one key,
@@ -905,7 +1022,7 @@ __global__ void __launch_bounds__(kUniqueThreads)
       more += v;
       return open;
     };
-    int r0 = blockIdx.x + 1;
+    int r0 = round + 1;
     if (open_behind(r0, std::integral_constant<int, 1>{}))
       for (r0 += 32; open_behind(r0, std::integral_constant<int, 16>{}); r0 += 512) {}
   }
@@ -924,6 +1041,20 @@ __global__ void __launch_bounds__(kUniqueThreads)
     const float v = PAIRS ? __uint_as_float((unsigned int)__ldcg(u.keys + i)) : __ldcg(u.sums + i);
     u.out_sums[at + count - 1] = v + more;
   }
+}
+
+template <bool PAIRS>
+__global__ void __launch_bounds__(kUniqueThreads, 6)
+    unique_gather_kernel(const __grid_constant__ Unique u, int rounds, const SortHead* head,
+                         Segments seg) {
+  grid_launch_next();
+  grid_wait();
+  if (const int groups = __ldcg(&head->groups)) {
+    gather_segments(u, seg, groups, __ldcg(&head->shift), __ldcg(&head->separate) != 0);
+    return;
+  }
+  for (int round = blockIdx.x; round < rounds; round += gridDim.x)
+    gather_round<PAIRS>(u, round, rounds);
 }
 
 // ---- ordered match -------------------------------------------------------------------------
@@ -1071,11 +1202,97 @@ struct UniquePlan {
   }
 };
 
+// Which calls sort piece by piece (piece_sum.cuh), and how: fewer than 16 bits are one or two
+// passes of the general way.
+struct BucketPlan {
+  bool take = false;
+  int pieces = 0;                    // of the input, 0: scattered into buckets
+  int top = 0;                       // bits of a bucket
+  Buckets b{};
+  static bool sized(int64_t n) { return n > kTile && n <= kMaxBucketItems; }
+  static void digits(int bits, int* passes, int* width) {
+    *passes = (bits + kWideBits - 1) / kWideBits;
+    *width = (bits + *passes - 1) / *passes;
+  }
+  BucketPlan(int64_t n, int key_bits) {
+    const bool few = n <= kFewItems && key_bits <= 64 - kIndexBits;
+    if (!sized(n) || key_bits < 16 || (!few && key_bits > 32 + kWideBits)) return;
+    take = true;
+    b.sample = n > kFewItems / 2 ? kMaxSample : kMaxSample / 2;
+    int spread;                      // bits that the sample's keys are told apart by
+    if (few) {
+      // pieces and parts of 512 items and more
+      pieces = (int)((n + 511) / 512);
+      if (pieces > kFewPieces) pieces = kFewPieces;
+      for (spread = 3; 512ll << spread < n && 1 << spread < kFewPieces;) ++spread;
+      b.parts = 1 << spread;
+      b.part_shift = b.shift = key_bits - spread;
+      digits(key_bits, &b.passes, &b.width);
+      digits(b.shift, &b.merge_passes, &b.merge_width);
+      b.chunks = pieces;
+    } else {
+      // 2048 to 4608 items per bucket, and no more than 32 bits of a key below
+      for (top = kRadixBits; top < kWideBits && 4096ll << top < n;) ++top;
+      if (top < key_bits - 32) top = key_bits - 32;
+      spread = top;
+      b.shift = key_bits - top;
+      b.count = 1 << top;
+      b.parts = kGroup;
+      b.part_shift = b.shift - 3;
+      b.key_shift = key_bits > 32 ? b.shift : 0;
+      digits(b.shift, &b.passes, &b.width);
+      b.merge_passes = b.passes;
+      b.merge_width = b.width;
+    }
+    // A range with kPiece distinct keys has x in the sample on average, and one with many more has
+    // more than this.  (2^22 ids all different have 2 in each of 1024 buckets, the limit is 16, and
+    // the average is not to be above 2.5.)
+    const double x = (double)kPiece * b.sample / n;
+    b.limit = (unsigned int)(x + 6 * sqrt(x) + 4);
+    b.mean = (float)x;
+    b.key_mask = ~0ull >> (64 - key_bits);
+  }
+};
+
+// Working memory of the buckets, beside that of the scatter.
+struct BucketWork {
+  unsigned int *wide, *distinct, *bounds;
+  Item* splits;
+  Piece* pieces;
+  Several* several;
+  static size_t bytes() {
+    return kOf.wide + kOf.pieces + kOf.several + kOf.splits + kOf.distinct + kOf.bounds;
+  }
+  explicit BucketWork(char* p) {
+    wide = reinterpret_cast<unsigned int*>(p);
+    p += kOf.wide;
+    pieces = reinterpret_cast<Piece*>(p);
+    p += kOf.pieces;
+    several = reinterpret_cast<Several*>(p);
+    p += kOf.several;
+    splits = reinterpret_cast<Item*>(p);
+    p += kOf.splits;
+    distinct = reinterpret_cast<unsigned int*>(p);
+    p += kOf.distinct;
+    bounds = reinterpret_cast<unsigned int*>(p);
+  }
+
+ private:
+  struct Of {
+    size_t wide, pieces, several, splits, distinct, bounds;
+  };
+  static_assert(kMaxPieces * kGroup <= kFewPieces * kFewParts, "bounds of either kind");
+  static_assert(kMaxChunks <= 512 && kMaxPieces <= 3072, "of every piece");
+  static constexpr Of kOf{4 * 512, 16 * 3072, 16 * kMaxBuckets, 8 * kFewParts, 4 * 3072,
+                          4 * kFewPieces * kFewParts};
+};
+
 // Layout of the scratch memory: counts and leads of the rounds of distinct keys, two buffers of
 // items and, for keys of more than 32 bits, of values, then the working memory of the sort.  (The
 // second half of a call reads all but the last part, and of key_bits it needs `pairs` alone.)
 struct UniqueScratch {
   SortHead* head;
+  Segments seg;
   unsigned int* counts;
   float* leads;
   Item* keys[2];
@@ -1087,6 +1304,13 @@ struct UniqueScratch {
     uintptr_t p = base;
     head = reinterpret_cast<SortHead*>(p);
     p += round256(sizeof(SortHead));
+    seg = {};
+    if (BucketPlan::sized(n)) {
+      seg.counts = reinterpret_cast<unsigned int*>(p);
+      p += round256((kMaxSegments + 1) * 4);
+      seg.place = reinterpret_cast<unsigned int*>(p);
+      p += round256(kMaxSegments * 4);
+    }
     counts = reinterpret_cast<unsigned int*>(p);
     p += round256((size_t)(rounds_of(n) + 1) * 4);
     leads = reinterpret_cast<float*>(p);
@@ -1147,15 +1371,27 @@ struct ReportSlot {
     }
     if (!word) {
       void* m = nullptr;
-      if (cudaHostAlloc(&m, 8, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+      if (cudaHostAlloc(&m, 16, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
         word = static_cast<unsigned long long*>(m);
     }
-    if (word) *word = 0;
+    if (word) word[0] = word[1] = 0;
   }
   ReportSlot(const ReportSlot&) = delete;
   ~ReportSlot() {
     if (index >= 0) used().fetch_and(~(1ull << index), std::memory_order_release);
     else if (word) cudaFreeHost(word);
+  }
+  // What the sample has shown, once it has (the second word of the slot).
+  bool spread() const {
+    const volatile unsigned long long* w = word;
+    for (int i = 0; i < 100000; ++i) {
+      if (const unsigned long long got = w[1]) return !(got & kReportCrowded);
+      if (w[0]) break;
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+    }
+    return true;
   }
   // Polls while a sort takes microseconds; a long one is waited for without using the core.
   int wait(cudaStream_t s, unsigned long long* got) const {
@@ -1181,6 +1417,84 @@ int unique_local(unsigned rounds, const Unique& u, cudaStream_t s) {
   constexpr int smem = unique_smem<PAIRS, THREADS>();
   if (int rc = allow_smem<unique_local_kernel<PAIRS, THREADS>>(smem)) return rc;
   return launch_chained(unique_local_kernel<PAIRS, THREADS>, rounds, THREADS, smem, s, 1, u);
+}
+
+// Sums piece by piece: of the buckets, or (RAW) of the input.
+template <bool RAW, bool LONG>
+int piece_sums(const Item* keys, const unsigned int* vals, int64_t n, const UniqueScratch& u,
+                const Buckets& b, const ReportSlot& slot, cudaStream_t s) {
+  constexpr int smem = piece_smem<LONG>();
+  if (int rc = allow_smem<piece_sum_kernel<RAW, LONG>>(smem)) return rc;
+  if (int rc = allow_smem<piece_merge_kernel<LONG>>(smem)) return rc;
+  const Items mine{u.keys[0], LONG ? reinterpret_cast<float*>(u.vals[0]) : nullptr};
+  const Items merged{u.keys[1], LONG ? reinterpret_cast<float*>(u.vals[1]) : nullptr};
+  const unsigned grid = RAW ? b.chunks + 1 : b.count + (unsigned)(n / kSmallPiece);
+  int rc = launch_chained(piece_sum_kernel<RAW, LONG>, grid, kPieceThreads, smem, s, 1,
+                          RAW ? keys : u.keys[1], vals, (long long)n, mine, b, u.head,
+                          slot.word);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (!rc && RAW && !b.splits && !slot.spread()) return 0;
+  // (a bucket in several pieces has more than kPiece items)
+  const int64_t units = RAW ? b.parts : n / kPiece * b.parts;
+  if (!rc)
+    rc = launch_chained(piece_merge_kernel<LONG>,
+                        units < 1 ? 1 : units < kMergeCtas ? (unsigned)units : kMergeCtas,
+                        kPieceThreads, smem, s, 1, mine, merged, b, u.head, slot.word);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return rc;
+}
+// Scatters into buckets.  The host hears what the sample has shown while the count and the scan are
+// running, before it launches the rest.
+template <int BITS, bool CUT>
+int bucket_sums(const Item* keys, const unsigned int* vals, int64_t n, int key_bits,
+                const BucketPlan& plan, const UniqueScratch& u, const SortWork& w, Buckets b,
+                const ReportSlot& slot, cudaStream_t s) {
+  using C = BucketCfg<BITS, CUT>;
+  constexpr auto* kScatter = bucket_scatter_kernel<BITS, CUT>;
+  if (int rc = allow_smem<kScatter>(C::kSmemBytes)) return rc;
+  const Chunks ch = chunks_of(n, kWideBits, C::kThreads, C::kRows);
+  const unsigned int mask = (1u << plan.top) - 1;
+  b.chunks = ch.count;
+  int rc = launch_chained(digit_count_kernel<Item, BITS, true>, ch.count + 1, kThreads, 0, s, 1,
+                          keys, (long long)n, b.shift, mask, ch, key_bits, w.counts, w.head, b,
+                          slot.word);
+  if (!rc)
+    rc = launch_chained(digit_scan_kernel, C::kDigits / 32, 1024, 0, s, 1, w.counts, C::kDigits,
+                        ch.count, w.totals);
+  g_launches.fetch_add(2, std::memory_order_relaxed);
+  if (rc || !slot.spread()) return rc;
+  rc = launch_chained(kScatter, ch.count, C::kThreads, C::kSmemBytes, s, 1, keys, vals, u.keys[1],
+                      (unsigned int)n, mask, ch, w.counts, w.totals, b, w.head);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return rc ? rc : piece_sums<false, false>(keys, vals, n, u, b, slot, s);
+}
+template <int BITS>
+int bucket_sums(const Item* keys, const unsigned int* vals, int64_t n, int key_bits,
+                const BucketPlan& plan, const UniqueScratch& u, const SortWork& w, const Buckets& b,
+                const ReportSlot& slot, cudaStream_t s) {
+  return key_bits <= 32
+             ? bucket_sums<BITS, false>(keys, vals, n, key_bits, plan, u, w, b, slot, s)
+             : bucket_sums<BITS, true>(keys, vals, n, key_bits, plan, u, w, b, slot, s);
+}
+int unique_by_pieces(const Item* keys, const float* vals, int64_t n, int key_bits,
+                     const BucketPlan& plan, const UniqueScratch& u, const SortWork& w,
+                     const ReportSlot& slot, cudaStream_t s) {
+  const BucketWork own(u.work + SortWork::bytes(n, kWideBits));
+  Buckets b = plan.b;
+  b.wide = own.wide;
+  b.pieces = own.pieces;
+  b.several = own.several;
+  b.distinct = own.distinct;
+  b.bounds = own.bounds;
+  b.splits = plan.pieces && n <= kSplitItems ? own.splits : nullptr;
+  b.seg = u.seg;
+  const unsigned int* v = reinterpret_cast<const unsigned int*>(vals);
+  if (plan.pieces)
+    return key_bits <= 32 ? piece_sums<true, false>(keys, v, n, u, b, slot, s)
+                          : piece_sums<true, true>(keys, v, n, u, b, slot, s);
+  if (plan.top == 8) return bucket_sums<8>(keys, v, n, key_bits, plan, u, w, b, slot, s);
+  if (plan.top == 9) return bucket_sums<9>(keys, v, n, key_bits, plan, u, w, b, slot, s);
+  return bucket_sums<10>(keys, v, n, key_bits, plan, u, w, b, slot, s);
 }
 
 int unique_sort(const Item* keys, const float* vals, int64_t n, int key_bits,
@@ -1213,7 +1527,8 @@ int unique_sort(const Item* keys, const float* vals, int64_t n, int key_bits,
       if (rc) return rc;
       continue;
     }
-    const int rc = !plan.pairs ? any_pass<kPayload>(plan.bits, p, w, s)
+    const int rc = !plan.pairs ? pass ? any_pass<kPayload>(plan.bits, p, w, s)
+                                      : any_pass<kFirst>(plan.bits, p, w, s)
                    : pass == 0 ? any_pass<kToPairs>(plan.bits, p, w, s)
                                : any_pass<kNoPayload>(plan.bits, p, w, s);
     if (rc) return rc;
@@ -1238,8 +1553,9 @@ int unique_write(const UniqueScratch& u, int64_t n, bool pairs, unsigned long lo
     rc = pairs ? unique_local<true, kThreads>(1, q, s) : unique_local<false, kThreads>(1, q, s);
   } else {
     auto* gather = pairs ? unique_gather_kernel<true> : unique_gather_kernel<false>;
-    rc = launch_chained(gather, (unsigned)rounds_of(n), kUniqueThreads, 0, s, 1, q,
-                        (int)rounds_of(n));
+    const unsigned rounds = (unsigned)rounds_of(n);
+    const unsigned grid = rounds < 256 ? 256 : rounds < kGatherCtas ? rounds : kGatherCtas;
+    rc = launch_chained(gather, grid, kUniqueThreads, 0, s, 1, q, (int)rounds, u.head, u.seg);
   }
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return rc;
@@ -1251,7 +1567,9 @@ extern "C" {
 size_t psdev_unique_sum_scratch_bytes(int64_t n, int key_bits) {
   if (n < 1 || key_bits < 1 || key_bits > 64) return 0;
   const UniquePlan plan(n, key_bits);
-  return UniqueScratch(nullptr, n, plan.pairs).bytes + SortWork::bytes(n, plan.bits);
+  const bool buckets = BucketPlan(n, key_bits).take;
+  return UniqueScratch(nullptr, n, plan.pairs).bytes +
+         SortWork::bytes(n, buckets ? kWideBits : plan.bits) + (buckets ? BucketWork::bytes() : 0);
 }
 
 // Sorts n (key, value) pairs by key into `scratch` (psdev_unique_sum_scratch_bytes) and counts the
@@ -1266,20 +1584,31 @@ int psdev_unique_sum_sort(const uint64_t* keys, const float* vals, int64_t n, in
   cudaStream_t s = (cudaStream_t)stream;
   const UniquePlan plan(n, key_bits);
   const UniqueScratch u(scratch, n, plan.pairs);
-  SortWork w(u.work, n, plan.bits);
-  w.head = u.head;
-  cudaMemsetAsync(u.head, 0, sizeof(SortHead), s);
   const unsigned long long* k = reinterpret_cast<const unsigned long long*>(keys);
   ReportSlot slot;
   if (!slot.word) return (int)cudaErrorMemoryAllocation;
-  int rc = unique_sort(k, vals, n, key_bits, u, w, slot.word, s);
+  const BucketPlan buckets(n, key_bits);
+  int rc = 0;
+  unsigned long long got = 0;
+  if (buckets.take) {
+    SortWork w(u.work, n, kWideBits);
+    w.head = u.head;
+    rc = unique_by_pieces(k, vals, n, key_bits, buckets, u, w, slot, s);
+    if (!rc) rc = slot.wait(s, &got);
+  }
+  if (!rc && (!buckets.take || (got & kReportCrowded))) {
+    SortWork w(u.work, n, plan.bits);
+    w.head = u.head;
+    // (behind the buckets' kernels, whose report has come: the word is free again)
+    cudaMemsetAsync(u.head, 0, sizeof(SortHead), s);
+    *slot.word = got = 0;
+    rc = unique_sort(k, vals, n, key_bits, u, w, slot.word, s);
+    if (!rc) rc = slot.wait(s, &got);
+  }
   if (rc) {
     cudaStreamSynchronize(s);  // (a kernel before the one that failed may still report)
     return rc;
   }
-  unsigned long long got = 0;
-  rc = slot.wait(s, &got);
-  if (rc) return rc;
   if (got & kReportWide) return PSDEV_ERR_ARG;
   *n_unique = (int64_t)(got & 0xffffffffu);
   return 0;

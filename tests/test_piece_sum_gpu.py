@@ -1,0 +1,96 @@
+"""sort_unique_sum piece by piece, where its way and its parts change: keys against torch.unique, sums
+against sums in fp64 within the bound of fp32 additions in any order, (m - 1) 2^-24 sum |v| for a key of
+m values."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+FEW, MOST = 3 << 18, 9 << 19   # items that are not scattered, items that go into buckets
+
+
+def _check(keys, vals, bits):
+    from ps_lite_b200.ops.keys import sort_unique_sum
+    want, inverse, times = torch.unique(keys, return_inverse=True, return_counts=True)
+    got, sums = sort_unique_sum(keys, vals, key_bits=bits)
+    assert torch.equal(got, want)
+    exact = torch.zeros(want.numel(), dtype=torch.float64, device=keys.device)
+    size = torch.zeros_like(exact)
+    exact.index_add_(0, inverse, vals.double())
+    size.index_add_(0, inverse, vals.double().abs())
+    assert bool(((sums.double() - exact).abs() <= (times - 1) * 2.0 ** -24 * size).all())
+    again, same = sort_unique_sum(keys, vals, key_bits=bits)
+    assert torch.equal(again, got) and torch.equal(same, sums)
+
+
+def _keys(kind, n, bits, dev):
+    g = torch.Generator(device=dev)
+    g.manual_seed(n + bits)
+    keys = torch.randint(0, 1 << bits, (n,), device=dev, generator=g)
+    if kind == "popular":        # half of all items one id, a tenth another one
+        order = torch.randperm(n, device=dev, generator=g)
+        keys[order[: n // 2]] = (1 << bits) - 1
+        keys[order[n // 2: n // 2 + n // 10]] = 5
+    elif kind == "low":          # in a small range of a large space
+        keys %= 1 << min(bits, 15)
+    elif kind == "ranges":       # in a few narrow ranges
+        wide = min(bits - 4, 20)
+        keys = (keys >> (bits - 3) << (bits - 3)) + keys % (1 << wide)
+    elif kind == "one":
+        keys.fill_(3)
+    elif kind == "rising":
+        keys = torch.arange(n, device=dev) * ((1 << bits) // n) if n < 1 << bits else torch.sort(keys)[0]
+    return keys, torch.randn(n, device=dev, generator=g)
+
+
+@pytest.mark.parametrize("kind", ["spread", "popular", "low", "ranges", "one", "rising"])
+@pytest.mark.parametrize("n", [4097, 5120, 65_537, 131_073, 300_001, FEW])
+@pytest.mark.parametrize("bits", [16, 24, 32, 33, 40, 51])
+def test_pieces_of_the_input(cuda_device, kind, n, bits):
+    _check(*_keys(kind, n, bits, cuda_device), bits)
+
+
+@pytest.mark.parametrize("kind", ["spread", "popular", "low", "ranges", "one", "rising"])
+@pytest.mark.parametrize("n", [FEW + 1, 1 << 20, (1 << 20) + 1, 296 * 4096 + 1, MOST])
+@pytest.mark.parametrize("bits", [16, 24, 32, 33, 42])
+def test_buckets(cuda_device, kind, n, bits):
+    _check(*_keys(kind, n, bits, cuda_device), bits)
+
+
+# beyond what pieces and buckets are for
+@pytest.mark.parametrize("n,bits", [(FEW, 52), (FEW + 1, 43), (MOST + 1, 30), (9000, 15)])
+def test_the_general_way(cuda_device, n, bits):
+    _check(*_keys("spread", n, bits, cuda_device), bits)
+
+
+# distinct keys of a part or a bucket: as many as a CTA sorts, and one more
+@pytest.mark.parametrize("n,bits", [(40_000, 30), (40_000, 40), (1 << 20, 30), (1 << 20, 40)])
+@pytest.mark.parametrize("crowd", [5119, 5120, 5121, 12_000])
+def test_a_crowd(cuda_device, n, bits, crowd):
+    keys, vals = _keys("spread", n, bits, cuda_device)
+    at = torch.randperm(n, device=cuda_device)[:crowd]
+    keys[at] = (1 << (bits - 1)) + torch.arange(crowd, device=cuda_device)
+    _check(keys, vals, bits)
+
+
+# popular ids side by side, which every piece of the input has: more items for one part than a CTA sorts
+@pytest.mark.parametrize("bits", [30, 40])
+@pytest.mark.parametrize("ids,crowd", [(19, 0), (20, 0), (21, 0), (100, 0), (40, 3000), (40, 6000)])
+def test_popular_neighbours(cuda_device, bits, ids, crowd):
+    n = 400_000
+    keys, vals = _keys("spread", n, bits, cuda_device)
+    keys[::2] = (1 << (bits - 1)) + torch.arange(n // 2, device=cuda_device) % ids
+    if crowd:
+        keys[1:2 * crowd:2] = (1 << (bits - 1)) + 1000 + torch.arange(crowd, device=cuda_device)
+    _check(keys, vals, bits)
+
+
+@pytest.mark.parametrize("n", [9000, 600_000, FEW + 1])
+@pytest.mark.parametrize("bits", [20, 40])
+def test_a_key_wider_than_stated(cuda_device, n, bits):
+    """Keys sort by their low bits then, as in sort_keys."""
+    from ps_lite_b200.ops.keys import sort_unique_sum
+    keys = torch.arange(n, device=cuda_device) % 1000 << (bits - 10)
+    keys[n // 2] += 1 << 55
+    got, sums = sort_unique_sum(keys, torch.ones(n, device=cuda_device), key_bits=bits)
+    assert int(sums.sum()) == n and bool(((got & ((1 << bits) - 1)).diff() >= 0).all())

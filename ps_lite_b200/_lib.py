@@ -125,6 +125,7 @@ def _declare(lib: C.CDLL) -> None:
                                         C.POINTER(i64), C.POINTER(i64)]),
         "psdev_gemm_status": (i32, [C.POINTER(C.c_int32)]),
         "psdev_filter_cast": (i32, [vp, vp, i64, C.c_float, i32, vp]),
+        "psdev_copy_cast": (i32, [vp, i32, vp, i32, i64, vp]),
         "psdev_filter_int8_pack": (i32, [vp, vp, vp, i64, vp]),
         "psdev_filter_int8_unpack": (i32, [vp, vp, vp, i64, i32, vp]),
         "psdev_sort_scratch_bytes": (sz, [i64, i32]),

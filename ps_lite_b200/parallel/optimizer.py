@@ -172,8 +172,8 @@ class DistributedOptimizer:
             t.step = me().steps + 1
             C.memmove(C.byref(opt), C.byref(t._opt_struct()), C.sizeof(opt))
 
-        segs, cast = (C.cast(f, C.c_void_p).value for f in (self.heap.lib.psdev_dense_op_segs,
-                                                             self.heap.lib.psdev_filter_cast))
+        segs, copy = (C.cast(f, C.c_void_p).value for f in (self.heap.lib.psdev_dense_op_segs,
+                                                             self.heap.lib.psdev_copy_cast))
         # reverse layer order, published parameters last (on one rank publishing is the same
         # store into this rank's weight buffer)
         pri = [-1 - i if self._publish[i] else len(self.params) - i
@@ -187,7 +187,7 @@ class DistributedOptimizer:
         # one rank the update is a pass over memory, shortest on the whole GPU
         return _lib.torch_ext().GradExchange(
             self.params, self.offsets, pri, t.grad, C.addressof(t._world), C.addressof(t._table),
-            C.addressof(self._opt), segs, cast, self.comm.cuda_stream if self.comm else 0,
+            C.addressof(self._opt), segs, copy, self.comm.cuda_stream if self.comm else 0,
             self.comm is not None, max(1, self.batch_bytes // self._gsz),
             max(1, self._busy_bytes // self._gsz), max(8, int(slice_elems) & ~7), channel, refresh)
 

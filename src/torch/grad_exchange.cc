@@ -35,6 +35,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <deque>
 #include <mutex>
 #include <optional>
@@ -48,17 +49,17 @@ using torch::autograd::Node;
 using torch::autograd::variable_list;
 using SegsFn = int (*)(const psdev_world_t*, const psdev_table_t*, int, const psdev_seg_t*, int,
                        const psdev_opt_t*, int, int, void*);
-using CastFn = int (*)(const void*, void*, int64_t, float, int, void*);
+using CopyFn = int (*)(const void*, int, void*, int, int64_t, void*);
 
 class GradExchange {
  public:
   // `batch_elems`: gradients that a launch waits for, `busy_elems` while one is still running.
-  // `world`, `table`, `opt`, `segs_fn`, `cast_fn`: addresses of the structures, of
-  // psdev_dense_op_segs and of psdev_filter_cast;
+  // `world`, `table`, `opt`, `segs_fn`, `copy_fn`: addresses of the structures, of
+  // psdev_dense_op_segs and of psdev_copy_cast;
   // `refresh` brings *opt up to date and is called before every launch.
   GradExchange(std::vector<at::Tensor> params, std::vector<int64_t> offsets,
                std::vector<int64_t> priorities, at::Tensor grad_buffer, uint64_t world,
-               uint64_t table, uint64_t opt, uint64_t segs_fn, uint64_t cast_fn,
+               uint64_t table, uint64_t opt, uint64_t segs_fn, uint64_t copy_fn,
                uint64_t comm_stream, bool overlap, int64_t batch_elems, int64_t busy_elems,
                int64_t slice_elems, int channel, py::function refresh)
       : params_(std::move(params)),
@@ -69,7 +70,7 @@ class GradExchange {
         table_(reinterpret_cast<const psdev_table_t*>(table)),
         opt_(reinterpret_cast<const psdev_opt_t*>(opt)),
         segs_fn_(reinterpret_cast<SegsFn>(segs_fn)),
-        cast_fn_(reinterpret_cast<CastFn>(cast_fn)),
+        copy_fn_(reinterpret_cast<CopyFn>(copy_fn)),
         device_(grad_buffer_.device().index()),
         overlap_(overlap),
         comm_(c10::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(comm_stream),
@@ -169,6 +170,8 @@ class GradExchange {
     std::vector<at::Tensor> tensors;
   };
 
+  static int DeviceType(at::ScalarType t) { return t == at::kFloat ? PSDEV_F32 : PSDEV_BF16; }
+
   // Whether `grad`, taken out of its parameter, is the only way to its memory.  The tensor that
   // autograd accumulated (`inputs`) is still alive here and may share the storage, and so may the
   // tensor that this one is a view of (the transpose of a matrix product, for a linear layer);
@@ -192,21 +195,18 @@ class GradExchange {
     return mem.use_count() == owners;
   }
 
-  // The gradient of parameter `i` into the table's gradient buffer, on the hook's stream: a copy or
-  // a cast of its own where the layout allows it (a third of what Tensor::copy_ costs this thread).
+  // The gradient of parameter `i` into the table's gradient buffer, on the hook's stream: a kernel of
+  // its own where the layout allows it (a fifth of what Tensor::copy_ costs this thread, less than
+  // half of cudaMemcpyAsync).
   void Stage(size_t i, const at::Tensor& grad, bool plain, const c10::cuda::CUDAStream& cur) {
     ++staged_;
     const int64_t n = params_[i].numel();
-    const auto to = grad_buffer_.scalar_type(), from = grad.scalar_type();
-    const size_t size = grad_buffer_.element_size();
-    char* dst = static_cast<char*>(grad_buffer_.data_ptr()) + offsets_[i] * size;
-    if (plain && from == to) {
-      C10_CUDA_CHECK(cudaMemcpyAsync(dst, grad.data_ptr(), n * size, cudaMemcpyDeviceToDevice,
-                                     cur.stream()));
-    } else if (plain) {
-      const int rc = cast_fn_(grad.data_ptr(), dst, n, 1.f, to == at::kBFloat16 ? 0 : 1,
-                              cur.stream());
-      TORCH_CHECK(rc == 0, "psdev_filter_cast failed with ", rc);
+    if (plain) {
+      char* dst = static_cast<char*>(grad_buffer_.data_ptr()) +
+                  offsets_[i] * grad_buffer_.element_size();
+      const int rc = copy_fn_(grad.data_ptr(), DeviceType(grad.scalar_type()), dst,
+                              DeviceType(grad_buffer_.scalar_type()), n, cur.stream());
+      TORCH_CHECK(rc == 0, "psdev_copy_cast failed with ", rc);
     } else {
       at::NoGradGuard no_grad;
       grad_buffer_.narrow(0, offsets_[i], n).view(params_[i].sizes()).copy_(grad, true);
@@ -259,7 +259,7 @@ class GradExchange {
                        (dt == at::kFloat || dt == at::kBFloat16);
     if (plain && Private(grad, inputs)) {
       seg.src = grad.data_ptr();
-      seg.dtype = dt == at::kFloat ? PSDEV_F32 : PSDEV_BF16;
+      seg.dtype = DeviceType(dt);
       held_.push_back(std::move(grad));
     } else {
       Stage(i, grad, plain, cur);
@@ -277,12 +277,16 @@ class GradExchange {
 
   // Gives up the gradients whose kernels have finished, and says whether all have.  While one is
   // running, what is pending would only queue up behind it; it goes out with what comes next
-  // instead, in fewer and larger launches.
+  // instead, in fewer and larger launches.  (An event's query takes this thread 1.4 us, so a hook
+  // that comes soon after one that found a launch running takes it to be running still.)
   bool Idle(const c10::cuda::CUDAStream& cur) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     C10_CUDA_CHECK(cudaStreamIsCapturing(cur.stream(), &capture));
     if (capture != cudaStreamCaptureStatusNone) return true;  // (an event may not be queried)
+    const auto now = std::chrono::steady_clock::now();
+    if (!batches_.empty() && now < next_look_) return false;
     while (!batches_.empty() && batches_.front().read.query()) Retire();
+    next_look_ = now + std::chrono::microseconds(25);
     return batches_.empty();
   }
 
@@ -337,7 +341,7 @@ class GradExchange {
   const psdev_table_t* table_;
   const psdev_opt_t* opt_;
   SegsFn segs_fn_;
-  CastFn cast_fn_;
+  CopyFn copy_fn_;
   c10::DeviceIndex device_;
   bool overlap_;
   c10::cuda::CUDAStream comm_;
@@ -359,6 +363,7 @@ class GradExchange {
   std::vector<at::Tensor> held_;  // gradients of segs_
   std::deque<Batch> batches_;     // launched, not known to be finished
   std::vector<Batch> spare_;
+  std::chrono::steady_clock::time_point next_look_{};  // not before: a launch was running
   at::cuda::CUDAEvent fork_;
   std::optional<c10::cuda::CUDAStream> pending_on_;   // hooks of what is pending ran here
   std::optional<c10::cuda::CUDAStream> launched_on_;  // launches of this step

@@ -119,9 +119,19 @@ inline int launch_local(const DenseArgs& d, int num_ctas, cudaStream_t s) {
     ntiles = d.end > d.begin ? (d.end - 1) / kLocalTile - d.begin / kLocalTile + 1 : 1;
   }
   const long long ctas = num_ctas > 0 && num_ctas < ntiles ? num_ctas : ntiles;
-  const int rc = launch_chained(local_update_kernel<GT, OT, Opt, RED, BC, NoSegs>,
-                                (unsigned)(ctas < (1ll << 30) ? ctas : 1ll << 30), kLocalThreads, 0,
-                                s, 1, a, NoSegs{});
+  const unsigned grid = (unsigned)(ctas < (1ll << 30) ? ctas : 1ll << 30);
+  // (int8 gradients come through a table of their own, not as requests)
+  if constexpr (sizeof(GT) > 1) {
+    const Told told{arm_done(d.done, ctas)};
+    if (told.done.word) {
+      const int rc = launch_chained(local_update_kernel<GT, OT, Opt, RED, BC, Told>, grid,
+                                    kLocalThreads, 0, s, 1, a, told);
+      psdev_count_launch();
+      return rc;
+    }
+  }
+  const int rc = launch_chained(local_update_kernel<GT, OT, Opt, RED, BC, NoSegs>, grid,
+                                kLocalThreads, 0, s, 1, a, NoSegs{});
   psdev_count_launch();
   return rc;
 }

@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "ps/device/chain.cuh"
+#include "ps/device/done.cuh"
 #include "ps/device/push_pull.cuh"
 
 namespace psdev {
@@ -65,6 +66,9 @@ struct LocalSegs {
   LocalSeg seg[kLocalMaxSegs];
 };
 struct NoSegs {};
+struct Told {            // one piece, and the host waits for a word
+  DoneArgs done;
+};
 
 __device__ __forceinline__ void load8(const float* p, float* f, bool wide) {
   if (wide) {
@@ -142,8 +146,10 @@ __device__ __forceinline__ void update_part(const LocalArgs& a, long long lo, lo
 template <typename GT, typename OT, class Opt, bool REDUCE, bool BCAST, typename Segs>
 __global__ void __launch_bounds__(kLocalThreads, Opt::kStates >= 2 ? 9 : 0)
     local_update_kernel(const __grid_constant__ LocalArgs a, const __grid_constant__ Segs segs) {
-  constexpr bool kSegs = !std::is_same<Segs, NoSegs>::value;
+  constexpr bool kSegs = std::is_same<Segs, LocalSegs>::value;
+  constexpr bool kTold = std::is_same<Segs, Told>::value;
   grid_launch_next();
+  if constexpr (kTold) expect_done(segs.done);
   grid_wait();
   long long ntiles;
   if constexpr (kSegs) ntiles = segs.tiles;
@@ -249,6 +255,7 @@ __global__ void __launch_bounds__(kLocalThreads, Opt::kStates >= 2 ? 9 : 0)
       }
     }
   }
+  if constexpr (kTold) signal_done(segs.done);
 }
 
 }  // namespace psdev

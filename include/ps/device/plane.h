@@ -188,7 +188,8 @@ class Plane : public DeviceRoute {
 
  private:
   void SubmitSparse(DeviceRequest&& req);
-  void FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* stream);
+  void FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* stream,
+                    psdev_done_t* word = nullptr);
   Plane();
   ~Plane();
   std::unique_ptr<Impl> impl_;

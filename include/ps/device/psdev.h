@@ -209,6 +209,26 @@ int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op
                           int64_t end, const psdev_opt_t* opt, int channel, int num_ctas,
                           void* stream, const void* src, void* dst, int64_t n_valid);
 
+/* How a launch tells the host that its work is done (done.cuh): it writes `value` to a word in
+ * mapped host memory.  The caller polls *host, gives every launch another value, and uses an entry
+ * for one launch at a time; it is used again only after its word was seen. */
+typedef struct {
+  volatile uint32_t* host; /* the word                                              */
+  uint32_t* word;          /* and its address on the device                         */
+  uint32_t* ticket;        /* device memory: CTAs done, of all launches so far      */
+  uint32_t value;
+  uint32_t tickets;        /* what *ticket will be after this launch (kept by the launch) */
+  int32_t armed;           /* set by the launch: it will write the word             */
+} psdev_done_t;
+int psdev_done_create(int n, psdev_done_t* done);
+int psdev_done_destroy(int n, psdev_done_t* done);
+/* psdev_dense_op_direct on memory of this GPU that writes the word when it is done; where it
+ * cannot, done->armed stays 0. */
+int psdev_dense_op_direct_done(const psdev_world_t* w, const psdev_table_t* t, int op,
+                               int64_t begin, int64_t end, const psdev_opt_t* opt, int channel,
+                               int num_ctas, void* stream, const void* src, void* dst,
+                               int64_t n_valid, psdev_done_t* done);
+
 /* One rank: several pieces of one table in as few launches as their number allows, the most
  * urgent (highest priority, ties in list order) first, each with the gradient in an array of its
  * own.  The ranges are disjoint (PSDEV_ERR_ARG otherwise).  The list is host memory and is not
@@ -319,6 +339,11 @@ int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t 
                        const uint64_t* keys, const float* vals, int64_t nvals,
                        const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
                        void* stream);
+/* The same, with the word of psdev_dense_op_direct_done. */
+int psdev_sparse_local_done(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
+                            const uint64_t* keys, const float* vals, int64_t nvals,
+                            const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
+                            void* stream, psdev_done_t* done);
 
 /* Command of a keyed request whose caller has seen that every array is memory of the table's GPU;
  * for others the driver is asked about each array (0.1 to 0.2 us apiece). */

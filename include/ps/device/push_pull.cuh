@@ -65,6 +65,7 @@ struct DenseArgs {
   // the table, elements of this rank's master/state arrays
   unsigned long long heap_bytes;
   long long n_total, local_len;
+  psdev_done_t* done;  // one rank: the host waits for this word, or NULL
 };
 
 #ifdef PSDEV_CHECKS

@@ -59,6 +59,40 @@ int psdev_rt_stream_wait_event(void* stream, void* event) {
   return (int)cudaStreamWaitEvent((cudaStream_t)stream, (cudaEvent_t)event, 0);
 }
 
+// Words that kernels write when they are done: every one in a line of its own, like its counter.
+int psdev_done_create(int n, psdev_done_t* done) {
+  constexpr size_t kLine = 128;
+  if (n < 1 || !done) return PSDEV_ERR_ARG;
+  char *host = nullptr, *words = nullptr, *tickets = nullptr;
+  cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&host), n * kLine,
+                                cudaHostAllocMapped | cudaHostAllocPortable);
+  if (e != cudaSuccess) return (int)e;
+  e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&words), host, 0);
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&tickets), n * kLine);
+  if (e == cudaSuccess) e = cudaMemset(tickets, 0, n * kLine);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) {
+    cudaFree(tickets);
+    cudaFreeHost(host);
+    return (int)e;
+  }
+  for (int i = 0; i < n; ++i) {
+    done[i] = psdev_done_t{};
+    done[i].host = reinterpret_cast<volatile uint32_t*>(host + i * kLine);
+    *done[i].host = 0;
+    done[i].word = reinterpret_cast<uint32_t*>(words + i * kLine);
+    done[i].ticket = reinterpret_cast<uint32_t*>(tickets + i * kLine);
+  }
+  return 0;
+}
+// (the first entry's addresses are those of the allocations; both calls wait for running kernels)
+int psdev_done_destroy(int n, psdev_done_t* done) {
+  if (n < 1 || !done) return PSDEV_ERR_ARG;
+  const cudaError_t a = cudaFree(done[0].ticket);
+  const cudaError_t b = cudaFreeHost(const_cast<uint32_t*>(done[0].host));
+  return (int)(a != cudaSuccess ? a : b);
+}
+
 // One asynchronous copy; the direction is inferred from the pointers (unified addressing).
 int psdev_rt_memcpy_async(void* dst, const void* src, size_t bytes, void* stream) {
   return (int)cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, (cudaStream_t)stream);

@@ -143,7 +143,7 @@ static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op,
                          uint64_t timeout_ns, int sync, void* stream, const int64_t* segs,
                          int nseg, void* sched, const void* src = nullptr, void* dst = nullptr,
                          int64_t n_valid = INT64_MAX, const psdev_seg_t* lsegs = nullptr,
-                         int nlsegs = 0);
+                         int nlsegs = 0, psdev_done_t* done = nullptr);
 
 extern "C" int psdev_dense_op(const psdev_world_t* w, const psdev_table_t* t, int op,
                               int64_t begin, int64_t end, const psdev_opt_t* opt, int channel,
@@ -164,10 +164,12 @@ extern "C" int psdev_dense_op_multi(const psdev_world_t* w, const psdev_table_t*
                        stream, segs, nseg, sched);
 }
 
-extern "C" int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op,
-                                     int64_t begin, int64_t end, const psdev_opt_t* opt,
-                                     int channel, int num_ctas, void* stream, const void* src,
-                                     void* dst, int64_t n_valid) {
+extern "C" int psdev_dense_op_direct_done(const psdev_world_t* w, const psdev_table_t* t, int op,
+                                          int64_t begin, int64_t end, const psdev_opt_t* opt,
+                                          int channel, int num_ctas, void* stream,
+                                          const void* src, void* dst, int64_t n_valid,
+                                          psdev_done_t* done) {
+  if (done) done->armed = 0;
   if (!w || !t) return PSDEV_ERR_ARG;
   if (w->world != 1) return PSDEV_ERR_UNSUPPORTED;
   // an array of whole values: aligned to its element type
@@ -175,7 +177,14 @@ extern "C" int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t
                          1)) || ((uintptr_t)dst & ((t->out_dtype == PSDEV_F32 ? 4 : 2) - 1)))
     return PSDEV_ERR_ARG;
   return dense_op_impl(w, t, op, begin, end, opt, channel, num_ctas, 0, 0, stream, nullptr, 0,
-                       nullptr, src, dst, n_valid);
+                       nullptr, src, dst, n_valid, nullptr, 0, done);
+}
+extern "C" int psdev_dense_op_direct(const psdev_world_t* w, const psdev_table_t* t, int op,
+                                     int64_t begin, int64_t end, const psdev_opt_t* opt,
+                                     int channel, int num_ctas, void* stream, const void* src,
+                                     void* dst, int64_t n_valid) {
+  return psdev_dense_op_direct_done(w, t, op, begin, end, opt, channel, num_ctas, stream, src, dst,
+                                    n_valid, nullptr);
 }
 
 // Whether no two ranges overlap: two CTAs would update the same values with no order between them.
@@ -254,7 +263,7 @@ static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op,
                          int64_t end, const psdev_opt_t* opt, int channel, int num_ctas,
                          uint64_t timeout_ns, int sync, void* stream, const int64_t* segs,
                          int nseg, void* sched, const void* src, void* dst, int64_t n_valid,
-                         const psdev_seg_t* lsegs, int nlsegs) {
+                         const psdev_seg_t* lsegs, int nlsegs, psdev_done_t* done) {
   if (!w || !t || w->world < 1 || w->world > PSDEV_MAX_RANKS || w->rank < 0 ||
       w->rank >= w->world)
     return PSDEV_ERR_ARG;
@@ -312,6 +321,7 @@ static int dense_op_impl(const psdev_world_t* w, const psdev_table_t* t, int op,
   a.n_valid = n_valid;
   a.lsegs = lsegs;
   a.nlsegs = nlsegs;
+  a.done = done;
   a.heap_bytes = w->heap_bytes;
   a.n_total = t->n;
   {

@@ -195,9 +195,9 @@ class GradExchange {
     return mem.use_count() == owners;
   }
 
-  // The gradient of parameter `i` into the table's gradient buffer, on the hook's stream: a kernel of
-  // its own where the layout allows it (a fifth of what Tensor::copy_ costs this thread, less than
-  // half of cudaMemcpyAsync).
+  // The gradient of parameter `i` into the table's gradient buffer, on the hook's stream: a kernel
+  // of its own where the layout allows it (a fifth of what Tensor::copy_ costs this thread, less
+  // than half of cudaMemcpyAsync).
   void Stage(size_t i, const at::Tensor& grad, bool plain, const c10::cuda::CUDAStream& cur) {
     ++staged_;
     const int64_t n = params_[i].numel();

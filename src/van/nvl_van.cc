@@ -68,8 +68,8 @@ struct Rt {
   int (*sparse_lens)(const psdev_world_t*, const psdev_sparse_t*, int, void*) = nullptr;
   int (*key_shard_lookup)(const uint64_t*, int64_t, uint64_t, int, int64_t*, void*) = nullptr;
   int (*sparse_local)(const psdev_world_t*, const psdev_sparse_t*, int64_t, const uint64_t*,
-                      const float*, int64_t, const int32_t*, float*, int64_t, int32_t*,
-                      void*) = nullptr;
+                      const float*, int64_t, const int32_t*, float*, int64_t, int32_t*, void*,
+                      psdev_done_t*) = nullptr;
   int (*lens_to_offsets)(const int32_t*, int64_t, int64_t*, void*) = nullptr;
   int (*device_barrier)(const psdev_world_t*, int, uint64_t, void*) = nullptr;
   int (*multicast_pays)(int, uint64_t) = nullptr;
@@ -96,8 +96,10 @@ struct Rt {
   int (*dense_op)(const psdev_world_t*, const psdev_table_t*, int, int64_t, int64_t,
                   const psdev_opt_t*, int, int, uint64_t, int, void*) = nullptr;
   int (*dense_op_direct)(const psdev_world_t*, const psdev_table_t*, int, int64_t, int64_t,
-                         const psdev_opt_t*, int, int, void*, const void*, void*,
-                         int64_t) = nullptr;
+                         const psdev_opt_t*, int, int, void*, const void*, void*, int64_t,
+                         psdev_done_t*) = nullptr;
+  int (*done_create)(int, psdev_done_t*) = nullptr;
+  int (*done_destroy)(int, psdev_done_t*) = nullptr;
   int (*checks_enabled)() = nullptr;
   uint64_t (*launch_count)() = nullptr;
 };
@@ -148,7 +150,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_sparse_respond", &rt->sparse_respond);
   Bind(lib, "psdev_sparse_lens", &rt->sparse_lens);
   Bind(lib, "psdev_key_shard_lookup", &rt->key_shard_lookup);
-  Bind(lib, "psdev_sparse_local", &rt->sparse_local);
+  Bind(lib, "psdev_sparse_local_done", &rt->sparse_local);
   Bind(lib, "psdev_lens_to_offsets", &rt->lens_to_offsets);
   Bind(lib, "psdev_device_barrier", &rt->device_barrier);
   Bind(lib, "psdev_multicast_pays", &rt->multicast_pays);
@@ -173,7 +175,9 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_channel_status_on", &rt->channel_status_on);
   Bind(lib, "psdev_channel_clear", &rt->channel_clear);
   Bind(lib, "psdev_dense_op", &rt->dense_op);
-  Bind(lib, "psdev_dense_op_direct", &rt->dense_op_direct);
+  Bind(lib, "psdev_dense_op_direct_done", &rt->dense_op_direct);
+  Bind(lib, "psdev_done_create", &rt->done_create);
+  Bind(lib, "psdev_done_destroy", &rt->done_destroy);
   Bind(lib, "psdev_checks_enabled", &rt->checks_enabled);
   Bind(lib, "psdev_launch_count", &rt->launch_count);
   return lib;
@@ -546,7 +550,28 @@ struct Plane::Impl {
       rt.stream_wait_event(s, prev.event);
   }
 
+  // Words that the kernel of a one-rank request writes when it is done, for the completer to poll
+  // (done.cuh).  A request takes one while there are some, and gives it back when it has completed.
+  static constexpr int kDoneWords = 64;
+  psdev_done_t done_words[kDoneWords];
+  std::vector<psdev_done_t*> idle_words;
+  psdev_done_t* NewWord() {
+    const auto lk = SpinLock(ev_mu);
+    if (idle_words.empty()) return nullptr;
+    psdev_done_t* w = idle_words.back();
+    idle_words.pop_back();
+    ++w->value;
+    w->armed = 0;
+    return w;
+  }
+  void RecycleWord(psdev_done_t* w) {
+    if (!w) return;
+    const auto lk = SpinLock(ev_mu);
+    idle_words.push_back(w);
+  }
+
   struct Pending {
+    psdev_done_t* word = nullptr;  // armed: says so before the event does
     void* event = nullptr;
     std::vector<void*> events_to_recycle;
     int channel = 0;
@@ -620,7 +645,13 @@ struct Plane::Impl {
         queue.pop_front();
         queued.store(static_cast<int>(queue.size()), std::memory_order_release);
       }
-      int rc = rt.event_sync(p.event);
+      // (a kernel that waits behind others, or fails, is left to the event)
+      const psdev_done_t* w = p.word;
+      const bool told =
+          w && SpinUntil(std::chrono::steady_clock::now() + std::chrono::microseconds(SpinMicros()),
+                         [&] { return *w->host == w->value; });
+      int rc = told ? 0 : rt.event_sync(p.event);
+      if (rc == 0) RecycleWord(p.word);
       int32_t status = 0;
       if (rc == 0 && status_can_change)
         rc = rt.channel_status_on(ws.peer_base[rank], p.channel, s_status, &status, nullptr);
@@ -857,6 +888,9 @@ void Plane::Start(const PlaneOptions& options) {
   CHECK_EQ(m.rt.stream_create(&m.s_compute, 1), 0);
   CHECK_EQ(m.rt.stream_create(&m.s_d2h, 0), 0);
   CHECK_EQ(m.rt.stream_create(&m.s_status, 0), 0);
+  if (m.world == 1 && !m.sim && SpinMicros() > 0 &&
+      m.rt.done_create(Impl::kDoneWords, m.done_words) == 0)
+    for (psdev_done_t& w : m.done_words) m.idle_words.push_back(&w);
   m.stop = false;
   m.asleep = false;
   m.queued = 0;
@@ -875,6 +909,8 @@ void Plane::Stop() {
   if (!m.started) return;
   m.Drain();
   if (!m.sim) {
+    // (a request that a word has completed: the rest of its kernel, on a stream of the program's)
+    for (void* e : m.event_pool) m.rt.event_sync(e);
     m.rt.stream_sync(m.s_h2d);
     m.rt.stream_sync(m.s_compute);
     m.rt.stream_sync(m.s_d2h);
@@ -930,6 +966,8 @@ void Plane::Stop() {
   }
   if (!m.sim) {
     for (void* e : m.event_pool) m.rt.event_destroy(e);
+    if (!m.idle_words.empty()) m.rt.done_destroy(Impl::kDoneWords, m.done_words);
+    m.idle_words.clear();
     m.rt.stream_destroy(m.s_h2d);
     m.rt.stream_destroy(m.s_compute);
     m.rt.stream_destroy(m.s_d2h);
@@ -1453,9 +1491,12 @@ void Plane::Submit(DeviceRequest&& req) {
         void* dst = req.pull && outs && outs != weight ? out_at : nullptr;
         int ctas = d->num_ctas;
         if ((host_in || host_out) && ctas <= 0) ctas = kZeroCopyCtas;
+        psdev_done_t* word = nruns == 1 && !host_in && !host_out ? m.NewWord() : nullptr;
         const int rc = m.rt.dense_op_direct(&m.ws, &t, op, r.begin, pad8(r.end), &opt, d->channel,
-                                            ctas, s, src, dst, d->n_user);
+                                            ctas, s, src, dst, d->n_user, word);
         CHECK_EQ(rc, 0) << "psdev_dense_op_direct failed";
+        if (word && word->armed) pend.word = word;
+        else m.RecycleWord(word);
         continue;
       }
       if (req.push && vals + eoff * gsz != grad + r.begin * gsz) {
@@ -1645,12 +1686,18 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
   if (local) {
     // one rank: one kernel on the request's own arrays
     if (lens_to) CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));
+    psdev_done_t* word = m.NewWord();
     CHECK_EQ(m.rt.sparse_local(&m.ws, &t, n, static_cast<const uint64_t*>(kptr),
                                static_cast<const float*>(req.push ? req.vals : nullptr),
                                static_cast<int64_t>(vbytes / 4), lens_in, static_cast<float*>(out),
-                               static_cast<int64_t>(obytes / 4), static_cast<int*>(lens_to), s), 0)
+                               static_cast<int64_t>(obytes / 4), static_cast<int*>(lens_to), s,
+                               word), 0)
         << "psdev_sparse_local failed";
-    FinishSparse(sp, std::move(req), s);
+    if (word && !word->armed) {
+      m.RecycleWord(word);
+      word = nullptr;
+    }
+    FinishSparse(sp, std::move(req), s, word);
     return;
   }
   if (kptr != sp->keys) {
@@ -1697,11 +1744,13 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
 }
 
 // The request's work has been issued on `s`: completion and the ordering point of the table.
-void Plane::FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* s) {
+void Plane::FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* s,
+                         psdev_done_t* word) {
   Impl& m = *impl_;
   void* done = m.NewEvent();
   m.rt.event_record(done, s);
   Impl::Pending pend;
+  pend.word = word;
   pend.event = done;
   pend.channel = sp->table.channel;
   pend.timestamp = req.timestamp;

@@ -345,8 +345,9 @@ int psdev_sparse_local_done(const psdev_world_t* w, const psdev_sparse_t* t, int
                             const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
                             void* stream, psdev_done_t* done);
 
-/* Command of a keyed request whose caller has seen that every array is memory of the table's GPU;
- * for others the driver is asked about each array (0.1 to 0.2 us apiece). */
+/* Command of a request whose caller has seen that every array is memory of the table's GPU, and no
+ * host memory by another name; for others the driver is asked about each array (0.1 to 0.2 us
+ * apiece). */
 #define PSDEV_CMD_ARRAYS_HERE 0x48455245
 
 /* Server role, tables with lengths: stores the length of the value of every key that a worker

@@ -5,6 +5,7 @@
 // the tensors, looks up the current stream and hands the request to the worker
 // (ps_capi_bworker_request_on, src/capi/ps_nvl_c_api.h).
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
@@ -31,9 +32,18 @@ struct Target {
 };
 constexpr const char* kName = "psb200.target";
 
-// The address of `obj`'s values, or `own` for None; false with a Python error set.
+// Whether `x` is memory of torch's own allocator on this GPU.  (A tensor may also name memory that
+// something else made, mapped host memory for one.)
+bool allocated_on(const at::Tensor& x, c10::DeviceIndex device) {
+  return x.is_cuda() && x.get_device() == device &&
+         x.storage().data_ptr().get_deleter() ==
+             c10::cuda::CUDACachingAllocator::get()->raw_deleter();
+}
+
+// The address of `obj`'s values, or `own` for None; false with a Python error set.  *here: false
+// where it may be elsewhere than on the table's GPU.
 bool values_of(PyObject* obj, const Target& t, at::ScalarType type, void* own, const char* wrong,
-               void** at) {
+               void** at, bool* here) {
   if (obj == Py_None) {
     *at = own;
     return true;
@@ -48,6 +58,7 @@ bool values_of(PyObject* obj, const Target& t, at::ScalarType type, void* own, c
     return false;
   }
   *at = x.data_ptr();
+  *here = *here && allocated_on(x, t.device);
   return true;
 }
 
@@ -61,17 +72,20 @@ PyObject* request(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (!t) return nullptr;
   const bool push = args[1] == Py_True, pull = args[2] == Py_True;
   void *vals = nullptr, *outs = nullptr;
+  bool here = true;
   HANDLE_TH_ERRORS
   if (push && !values_of(args[3], *t, t->grad_type, t->grad,
                          "pushed values must be a contiguous tensor of the declared length and "
-                         "gradient dtype", &vals))
+                         "gradient dtype", &vals, &here))
     return nullptr;
   if (pull && !values_of(args[4], *t, t->out_type, t->weight,
                          "the output must be a contiguous tensor of the declared length and "
-                         "weight dtype", &outs))
+                         "weight dtype", &outs, &here))
     return nullptr;
-  const long cmd = PyLong_AsLong(args[5]), priority = PyLong_AsLong(args[6]);
+  long cmd = PyLong_AsLong(args[5]);
+  const long priority = PyLong_AsLong(args[6]);
   if (PyErr_Occurred()) return nullptr;
+  if (here && cmd == 0) cmd = PSDEV_CMD_ARRAYS_HERE;
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream(t->device).stream();
   int ts;
   Py_BEGIN_ALLOW_THREADS
@@ -150,7 +164,7 @@ PyObject* keyed_request(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int* lp = vals && lens ? static_cast<const int*>(lens->data_ptr()) : nullptr;
   int* lo = out && !vals && lens_out ? static_cast<int*>(lens_out->data_ptr()) : nullptr;
   const size_t vb = vals ? vals->numel() * 4 : 0, ob = out ? out->numel() * 4 : 0;
-  auto here = [&](const at::Tensor* x) { return !x || x->get_device() == t->device; };
+  auto here = [&](const at::Tensor* x) { return !x || allocated_on(*x, t->device); };
   const bool all = here(keys) && here(vals) && here(out) && here(lens) && here(lens_out);
   int ts;
   Py_BEGIN_ALLOW_THREADS

@@ -536,11 +536,12 @@ struct Plane::Impl {
     unsigned long long id = 0;
     return rt.stream_id && rt.stream_id(s, &id) == 0 ? id : 0;
   }
-  // Whether `p` is device memory; *here: of this GPU.
-  bool OnDevice(const void* p, bool* here) const {
+  // Whether `p` is device memory; *here: of this GPU; *managed: set where it may be the host's too.
+  bool OnDevice(const void* p, bool* here, bool* managed) const {
     int device = -1;
     const int kind = rt.memory(p, &device);
     *here = kind == 2 || (kind == 1 && device == opts.device);
+    *managed |= kind == 2;
     return kind != 0;
   }
   // Orders work on `s` after the previous request on the tensor, unless that was on this stream too
@@ -1393,11 +1394,12 @@ void Plane::Submit(DeviceRequest&& req) {
 
   // (the CPU stand-in calls "device memory" what lies in an arena.)  What lies on another GPU is
   // copied: a kernel of this one may not be able to reach it.
-  bool near = true;
+  bool near = true, managed = false;
   auto on_device = [&](const void* p) {
+    if (req.cmd == PSDEV_CMD_ARRAYS_HERE) return true;
     if (!m.sim) {
       bool here = false;
-      const bool device = m.OnDevice(p, &here);
+      const bool device = m.OnDevice(p, &here, &managed);
       if (device && !here) near = false;
       return device;
     }
@@ -1491,7 +1493,8 @@ void Plane::Submit(DeviceRequest&& req) {
         void* dst = req.pull && outs && outs != weight ? out_at : nullptr;
         int ctas = d->num_ctas;
         if ((host_in || host_out) && ctas <= 0) ctas = kZeroCopyCtas;
-        psdev_done_t* word = nruns == 1 && !host_in && !host_out ? m.NewWord() : nullptr;
+        const bool words = nruns == 1 && !host_in && !host_out && !managed;
+        psdev_done_t* word = words ? m.NewWord() : nullptr;
         const int rc = m.rt.dense_op_direct(&m.ws, &t, op, r.begin, pad8(r.end), &opt, d->channel,
                                             ctas, s, src, dst, d->n_user, word);
         CHECK_EQ(rc, 0) << "psdev_dense_op_direct failed";
@@ -1662,9 +1665,10 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
     return !a || !b || a == b || !Clash(a, an, 1, b, bn, 1);
   };
   // (and so does a request with an array on the host or on another GPU)
+  bool managed = false;
   auto here = [&](const void* p) {
     bool is = !p;
-    return is || (m.OnDevice(p, &is) && is);
+    return is || (m.OnDevice(p, &is, &managed) && is);
   };
   const size_t kbytes = static_cast<size_t>(n) * 8, lbytes = static_cast<size_t>(n) * 4;
   void* out = req.pull ? req.outs : nullptr;
@@ -1686,7 +1690,7 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
   if (local) {
     // one rank: one kernel on the request's own arrays
     if (lens_to) CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));
-    psdev_done_t* word = m.NewWord();
+    psdev_done_t* word = managed ? nullptr : m.NewWord();
     CHECK_EQ(m.rt.sparse_local(&m.ws, &t, n, static_cast<const uint64_t*>(kptr),
                                static_cast<const float*>(req.push ? req.vals : nullptr),
                                static_cast<int64_t>(vbytes / 4), lens_in, static_cast<float*>(out),

@@ -512,8 +512,6 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
   unsigned short* cnt = sh.cnt + warp * digits;
   unsigned int* mine2 = reinterpret_cast<unsigned int*>(cnt);
   unsigned int* count2 = reinterpret_cast<unsigned int*>(sh.cnt);
-  constexpr int kPer = kPieceCounters / 2 / kT;  // pairs of digits per thread
-  const int per = pairs > kT ? pairs / kT : 1;
   for (int pass = 0; pass < passes; ++pass) {
     const int shift = pass * width;
     if (pass) clear_words(lanes, digits);
@@ -527,32 +525,41 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
     if (pass == 0) rank_rows<true, POPULAR, kRows>(digit, rows, valid, lanes, cnt, rank);
     else rank_rows<false, POPULAR, kRows>(digit, rows, valid, lanes, cnt, rank);
     __syncthreads();
-    // where the warps' parts of this thread's digits start in the piece
-    unsigned int items = 0, run[kPer];
-    const int first = threadIdx.x * per;
+    // Where the warps' parts of this thread's digits start in the piece: of two pairs of digits side
+    // by side, or of one.  (Two words at a time: one by one, two apart, they took twice the clocks.)
+    static_assert(kPieceCounters / 2 == 2 * kT, "two pairs per thread at most");
+    const bool two = pairs > kT, mine = two || (int)threadIdx.x < pairs;
+    unsigned int* const at0 = count2 + (two ? 2 * threadIdx.x : threadIdx.x);
+    auto counts_of = [&](int w) {
+      if (two) return *reinterpret_cast<const uint2*>(at0 + w * pairs);
+      return make_uint2(mine ? at0[w * pairs] : 0u, 0u);
+    };
+    uint2 run = make_uint2(0, 0);
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      run[i] = 0;
-      if (i < per && first + i < pairs) {
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) run[i] += count2[w * pairs + first + i];
-        items += (run[i] & 0xffffu) + (run[i] >> 16);
-      }
+    for (int w = 0; w < kWarps; ++w) {
+      const uint2 c = counts_of(w);
+      run.x += c.x;
+      run.y += c.y;
     }
-    unsigned int start = cta_exclusive<kWarps>(items, sh.part + (pass & 1) * kWarps, nullptr);
+    const unsigned int items0 = (run.x & 0xffffu) + (run.x >> 16);
+    const unsigned int items1 = (run.y & 0xffffu) + (run.y >> 16);
+    const unsigned int start = cta_exclusive<kWarps>(items0 + items1,
+                                                     sh.part + (pass & 1) * kWarps, nullptr);
+    if (mine) {
+      uint2 at;
+      at.x = start | (start + (run.x & 0xffffu)) << 16;
+      at.y = (start + items0) | (start + items0 + (run.y & 0xffffu)) << 16;
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      if (i < per && first + i < pairs) {
-        const unsigned int r0 = run[i] & 0xffffu, r1 = run[i] >> 16;
-        unsigned int at = start | (start + r0) << 16;
-        start += r0 + r1;
-        unsigned int c[kWarps];
+      for (int w0 = 0; w0 < kWarps; w0 += 4) {
+        uint2 c[4];
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) c[w] = count2[w * pairs + first + i];
+        for (int w = 0; w < 4; ++w) c[w] = counts_of(w0 + w);
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-          count2[w * pairs + first + i] = at;
-          at += c[w];
+        for (int w = 0; w < 4; ++w) {
+          if (two) *reinterpret_cast<uint2*>(at0 + (w0 + w) * pairs) = at;
+          else at0[(w0 + w) * pairs] = at.x;
+          at.x += c[w].x;
+          at.y += c[w].y;
         }
       }
     }

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(BucketCfg<BITS, CUT>::kThreads, 2)
     clear_words(reinterpret_cast<unsigned int*>(cnt), kPairs);
     __syncwarp();
     unsigned int rank[ROWS / 2];  // two of 16 bits each
-    rank_rows<true, false, ROWS>(digit, rows, valid, nullptr, cnt, rank);
+    rank_rows<true, ROWS>(digit, rows, valid, nullptr, cnt, rank);
     __syncthreads();
     // where the runs of this thread's digits start in the tile, and each warp's part of them
     unsigned int run[kPer], have = 0;
@@ -494,7 +494,7 @@ __device__ __forceinline__ void sort_few(Item (&k)[kPieceRows], int valid, const
 
 // Sorts the items of a CTA, which it has in registers in rows of 32 per warp, by `passes` digits of
 // `width` bits from the lowest of the key on; leaves them in order in sh.items.
-template <bool POPULAR, bool LONG>
+template <bool LONG>
 __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int passes, int width,
                                            const PieceShared& sh) {
   constexpr int kWarps = kPieceWarps, kRows = kPieceRows, kT = kPieceThreads;
@@ -522,11 +522,12 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
       return LONG ? item_digit(k[j], shift + kIndexBits, mask)
                   : (unsigned int)(k[j] >> 32) >> shift & mask;
     };
-    if (pass == 0) rank_rows<true, POPULAR, kRows>(digit, rows, valid, lanes, cnt, rank);
-    else rank_rows<false, POPULAR, kRows>(digit, rows, valid, lanes, cnt, rank);
+    if (pass == 0) rank_rows<true, kRows>(digit, rows, valid, lanes, cnt, rank);
+    else rank_rows<false, kRows>(digit, rows, valid, lanes, cnt, rank);
     __syncthreads();
-    // Where the warps' parts of this thread's digits start in the piece: of two pairs of digits side
-    // by side, or of one.  (Two words at a time: one by one, two apart, they took twice the clocks.)
+    // Where the warps' parts of this thread's digits start in the piece: of two pairs of digits
+    // side by side, or of one.  (Two words at a time: one by one, two apart, they took twice the
+    // clocks.)
     static_assert(kPieceCounters / 2 == 2 * kT, "two pairs per thread at most");
     const bool two = pairs > kT, mine = two || (int)threadIdx.x < pairs;
     unsigned int* const at0 = count2 + (two ? 2 * threadIdx.x : threadIdx.x);
@@ -580,6 +581,74 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
       __syncthreads();
     }
   }
+}
+
+// Pieces of a large bucket: most of their items are those of one popular id, or of a few.  Such a
+// key is looked for among the first ones of the warps; the values of its items are added up as they
+// are, and one item with the sum joins the others, which alone are left to sort.  Once more while
+// that takes away a quarter.  Returns how many items there are now, in `k` as before.
+__device__ __forceinline__ int add_up_popular(Item (&k)[kPieceRows], int count,
+                                              const PieceShared& sh) {
+  __shared__ unsigned int s_key[kPieceWarps], s_kept[kPieceWarps];
+  __shared__ float s_sum[kPieceWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int round = 0; round < 4; ++round) {
+    const int rows = (count + kPieceThreads - 1) / kPieceThreads;
+    if (rows <= 2) break;
+    const int valid = valid_rows(count - warp * (32 * rows) - lane, rows);
+    // (a warp without items shows some key that may not be there, and is outvoted)
+    if (lane == 0) s_key[warp] = (unsigned int)(k[0] >> 32);
+    __syncthreads();
+    const unsigned int seen = s_key[lane % kPieceWarps];
+    const unsigned int times = __popc(__match_any_sync(0xffffffffu, seen));
+    const unsigned int most = __reduce_max_sync(0xffffffffu, times << 8 | (31u - lane));
+    const unsigned int key = __shfl_sync(0xffffffffu, seen, 31 - (most & 0xff));
+    unsigned int kept = 0;
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < kPieceRows; ++j) {
+      if (j % 2 == 0 && j >= rows) break;
+      const bool is = j < valid && (unsigned int)(k[j] >> 32) == key;
+      if (is) sum += __uint_as_float((unsigned int)k[j]);
+      kept += __popc(__ballot_sync(0xffffffffu, j < valid && !is));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) {
+      s_kept[warp] = kept;
+      s_sum[warp] = sum;
+    }
+    __syncthreads();
+    unsigned int at = 0, all = 0;
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPieceWarps; ++w) {
+      if (w < warp) at += s_kept[w];
+      all += s_kept[w];
+      total += s_sum[w];
+    }
+    if (4 * all > 3 * (unsigned int)count) break;  // (the same for all threads)
+#pragma unroll
+    for (int j = 0; j < kPieceRows; ++j) {
+      if (j % 2 == 0 && j >= rows) break;
+      const bool keep = j < valid && (unsigned int)(k[j] >> 32) != key;
+      const unsigned int m = __ballot_sync(0xffffffffu, keep);
+      if (keep) sh.items[at + __popc(m & lanemask_lt())] = k[j];
+      at += __popc(m);
+    }
+    if (threadIdx.x == 0) sh.items[all] = (Item)key << 32 | __float_as_uint(total);
+    __syncthreads();
+    count = (int)all + 1;
+    const int left = (count + kPieceThreads - 1) / kPieceThreads;
+    const int base = warp * (32 * left) + lane, have = valid_rows(count - base, left);
+#pragma unroll
+    for (int j = 0; j < kPieceRows; ++j) {
+      if (j % 2 == 0 && j >= left) break;
+      if (j < have) k[j] = sh.items[base + j * 32];
+    }
+    __syncthreads();
+  }
+  return count;
 }
 
 // The sums of the values of equal keys in `count` sorted items.  The distinct keys end up at the
@@ -712,7 +781,7 @@ __device__ __forceinline__ void sample_parts(const Item* keys, unsigned int n, c
     }
     __syncthreads();
     // (every lane has an item in every row)
-    sort_piece<false, LONG>(k, count, b.passes, b.width, sh);
+    sort_piece<LONG>(k, count, b.passes, b.width, sh);
     const unsigned int total = sum_piece<LONG>(count, sh);
     for (int q = threadIdx.x; q < b.parts; q += kPieceThreads) {
       const Item i = sh.items[(unsigned int)q * total / b.parts];
@@ -758,7 +827,8 @@ __global__ void __launch_bounds__(kPieceThreads, LONG ? 2 : 3)
     const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(b.pieces + blockIdx.x));
     p = {raw.x, raw.y, raw.z, raw.w};
   }
-  const int count = (int)p.count, rows = (count + kPieceThreads - 1) / kPieceThreads;
+  int count = (int)p.count;
+  const int rows = (count + kPieceThreads - 1) / kPieceThreads;
   const int base = (threadIdx.x >> 5) * (32 * rows) + (threadIdx.x & 31);
   const int valid = valid_rows(count - base, rows);
   Item k[kPieceRows];
@@ -785,8 +855,8 @@ __global__ void __launch_bounds__(kPieceThreads, LONG ? 2 : 3)
     }
     wide = __syncthreads_or(wide);
   }
-  if (!RAW && p.pieces > 1) sort_piece<true, LONG>(k, count, b.passes, b.width, sh);
-  else sort_piece<false, LONG>(k, count, b.passes, b.width, sh);
+  if (!RAW && p.pieces > 1) count = add_up_popular(k, count, sh);
+  sort_piece<LONG>(k, count, b.passes, b.width, sh);
   const unsigned int total = sum_piece<LONG>(count, sh);
   const int parts = b.parts;
   unsigned int* bounds = b.bounds + (size_t)blockIdx.x * parts;
@@ -963,8 +1033,8 @@ __global__ void __launch_bounds__(kPieceThreads, 2)
         if constexpr (LONG) k[j] = k[j] << kLow | q;
       }
       __syncthreads();
-      if (split) sort_piece<false, LONG>(k, (int)items, b.passes, b.width, sh);
-      else sort_piece<false, LONG>(k, (int)items, b.merge_passes, b.merge_width, sh);
+      if (split) sort_piece<LONG>(k, (int)items, b.passes, b.width, sh);
+      else sort_piece<LONG>(k, (int)items, b.merge_passes, b.merge_width, sh);
       total = sum_piece<LONG>((int)items, sh);
       taken += items - kept;
       if (taken == count || total > kPiece * 3 / 4) break;

@@ -189,9 +189,9 @@ __device__ __forceinline__ int valid_rows(int left, int rows) {
 // SM in 9 ns; 15 with ballots, 32 with match.any), and the first of them advances the counter.
 // FREE: items of a digit may be in any order, the counter gives out the ranks.  (Lanes of one
 // instruction get theirs in the hardware's order, on which nothing but rounding depends.)
-// POPULAR: most items have the same key, so that the lanes with the digit of the first lane are
-// found with a ballot (32 atomics on one address take an SM some 70 clocks).
-template <bool FREE, bool POPULAR, int ROWS, typename Digit>
+// (32 atomics on one address take an SM some 70 clocks, which popular ids among others do not
+// need.)
+template <bool FREE, int ROWS, typename Digit>
 __device__ __forceinline__ void rank_rows(const Digit& digit, int rows, int valid,
                                           unsigned int* lanes, unsigned short* cnt,
                                           unsigned int (&rank)[ROWS / 2]) {
@@ -201,25 +201,14 @@ __device__ __forceinline__ void rank_rows(const Digit& digit, int rows, int vali
     if (j % 2 == 0 && j >= rows) break;
     const bool in = j < valid;
     const unsigned int d = digit(j);
-    unsigned int like = 0, r = 0;  // like: lanes with the first one's digit, where this one has it
-    if constexpr (POPULAR) {
-      const unsigned int d0 = __shfl_sync(0xffffffffu, d, 0);
-      const unsigned int all = __ballot_sync(0xffffffffu, in && d == d0);
-      if (in && d == d0) like = all;
-    }
+    unsigned int r = 0;
     if constexpr (FREE) {
-      const unsigned int add = POPULAR && like ? __popc(like) : 1u;
-      if (in && (!POPULAR || (like & below) == 0))
-        r = half_of(atomicAdd(reinterpret_cast<unsigned int*>(cnt) + d / 2, add << (d & 1) * 16),
-                    d);
-      if constexpr (POPULAR) {
-        const unsigned int of_first = __shfl_sync(0xffffffffu, r, like ? __ffs(like) - 1 : 0);
-        if (like) r = of_first + __popc(like & below);
-      }
+      if (in)
+        r = half_of(atomicAdd(reinterpret_cast<unsigned int*>(cnt) + d / 2, 1u << (d & 1) * 16), d);
     } else {
-      if (in && !like) atomicOr(&lanes[d], mine);
+      if (in) atomicOr(&lanes[d], mine);
       __syncwarp();
-      const unsigned int same = like ? like : lanes[d];
+      const unsigned int same = lanes[d];
       const unsigned int first = cnt[d], before = __popc(same & below);
       __syncwarp();
       if (in && before == 0) {
@@ -494,7 +483,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
     __syncwarp();
     unsigned int rank[ROWS / 2];  // two of 16 bits each
     const int valid = valid_rows((int)(hi - base), rows);
-    rank_rows<Form<PAY>::kFree, false, ROWS>(
+    rank_rows<Form<PAY>::kFree, ROWS>(
         [&](int j) { return item_digit(k[j], shift, mask); }, rows, valid, lanes, cnt, rank);
     __syncthreads();
     // where the runs of this thread's digits start in the tile, and each warp's part of them

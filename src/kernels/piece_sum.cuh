@@ -422,69 +422,56 @@ struct PieceShared {
         vals(reinterpret_cast<float*>(smem + kPieceItems + kPieceCount)), part(part) {}
 };
 
-// Sorts up to R rows of items as whole words: every warp its own in registers (bitonic), then runs
-// are merged two by two, each item finding its place in the other run by bisection.  A pass of the
-// radix sort takes some 2400 clocks however few the items are, this sort about as long in all
-// (2^16 items in two rows, 30 bits: 33.5 -> 31 us; with four rows it is slower than radix, 2^17
-// items 36 and 33.5 us).
-template <int R>
-__device__ __forceinline__ void sort_few(Item (&k)[kPieceRows], int valid, const PieceShared& sh) {
-  constexpr int kRun = 32 * R, kAll = kRun * kPieceWarps;
-  static_assert(2 * kAll <= kPiece, "two buffers");
+// Sorts up to 512 items as whole words, two per thread: every warp its own in registers (bitonic),
+// then runs are merged two by two, each item finding its place in the other run by bisection.
+// `mem`: 1024 items, which begins with the sorted ones.  A pass of the radix sort takes some 2400
+// clocks however few the items are, this sort about as long in all (2^16 items in two rows, 30
+// bits: 33.5 -> 30.5 us; four rows are faster by radix, 2^17 items 33.5 and 36 us).  The loops are
+// not unrolled: a kernel of a few CTAs runs through its code once, and waits for the code.
+__device__ __forceinline__ void sort_few(Item k0, Item k1, int valid, Item* mem) {
+  constexpr int kRun = 64, kAll = kRun * kPieceWarps;
   const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (r >= valid) k[r] = ~0ull;  // (behind all others)
-#pragma unroll
+  if (valid < 1) k0 = ~0ull;  // (behind all others)
+  if (valid < 2) k1 = ~0ull;
+#pragma unroll 1
   for (int size = 2; size <= kRun; size *= 2) {
-#pragma unroll
-    for (int stride = size / 2; stride > 0; stride /= 2) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) {  // element lane * R + r
-        const bool up = ((lane * R + r) & size) == 0;
-        if (stride >= R) {
-          const Item other = __shfl_xor_sync(0xffffffffu, k[r], stride / R);
-          const bool lower = (lane & (stride / R)) == 0;
-          if ((other < k[r]) == (lower == up)) k[r] = other;
-        } else if ((r & stride) == 0) {
-          const Item a = k[r], b = k[r | stride];
-          const bool swap = (b < a) == up;
-          k[r] = swap ? b : a;
-          k[r | stride] = swap ? a : b;
-        }
-      }
+    const bool up = ((2 * lane) & size) == 0;  // elements 2 lane and 2 lane + 1
+#pragma unroll 1
+    for (int away = size / 4; away > 0; away /= 2) {
+      const Item o0 = __shfl_xor_sync(0xffffffffu, k0, away);
+      const Item o1 = __shfl_xor_sync(0xffffffffu, k1, away);
+      const bool least = ((lane & away) == 0) == up;
+      if ((o0 < k0) == least) k0 = o0;
+      if ((o1 < k1) == least) k1 = o1;
+    }
+    if ((k1 < k0) == up) {
+      const Item t = k0;
+      k0 = k1;
+      k1 = t;
     }
   }
-  Item* from = sh.items + kAll;
-  Item* to = sh.items;
-  int at[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    at[r] = threadIdx.x * R + r;
-    from[at[r]] = k[r];
-  }
+  Item *from = mem + kAll, *to = mem;
+  int at0 = 2 * threadIdx.x, at1 = at0 + 1;
+  from[at0] = k0;
+  from[at1] = k1;
 #pragma unroll 1
   for (int run = kRun; run < kAll; run *= 2) {
     __syncthreads();
-    const int mine = at[0] / run;  // (all of a thread's items are in one run)
+    const int mine = at0 / run;  // (both of a thread's items are in one run)
+    const bool second = mine & 1;  // equal items of the first run go before those of the second
     const Item* other = from + (mine ^ 1) * run;
-    int less[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) less[r] = 0;
-    // equal items of the first run go before those of the second
-    for (int step = run / 2; step > 0; step /= 2)
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const Item o = other[less[r] + step - 1];
-        if (o < k[r] || ((mine & 1) && o == k[r])) less[r] += step;
-      }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const Item o = other[less[r]];
-      if (o < k[r] || ((mine & 1) && o == k[r])) ++less[r];
-      at[r] = at[r] - (mine & 1) * run + less[r];
-      to[at[r]] = k[r];
+    int less0 = 0, less1 = 0;
+#pragma unroll 1
+    for (int step = run / 2; step > 0; step /= 2) {
+      const Item o0 = other[less0 + step - 1], o1 = other[less1 + step - 1];
+      if (o0 < k0 || (second && o0 == k0)) less0 += step;
+      if (o1 < k1 || (second && o1 == k1)) less1 += step;
     }
+    const Item o0 = other[less0], o1 = other[less1];
+    at0 += less0 + (o0 < k0 || (second && o0 == k0)) - (second ? run : 0);
+    at1 += less1 + (o1 < k1 || (second && o1 == k1)) - (second ? run : 0);
+    to[at0] = k0;
+    to[at1] = k1;
     Item* const t = from;
     from = to;
     to = t;
@@ -492,18 +479,62 @@ __device__ __forceinline__ void sort_few(Item (&k)[kPieceRows], int valid, const
   __syncthreads();
 }
 
+// Turns the warps' counts of every digit, two digits in a word, into where the warps' parts of the
+// digits start.
+__device__ __forceinline__ void place_counts(unsigned int* count2, int pairs, unsigned int* part) {
+  // Where the warps' parts of this thread's digits start in the piece: of two pairs of digits
+  // side by side, or of one.  (Two words at a time: one by one, two apart, they took twice the
+  // clocks.)
+  constexpr int kWarps = kPieceWarps, kT = kPieceThreads;
+  static_assert(kPieceCounters / 2 == 2 * kT, "two pairs per thread at most");
+  const bool two = pairs > kT, mine = two || (int)threadIdx.x < pairs;
+  unsigned int* const at0 = count2 + (two ? 2 * threadIdx.x : threadIdx.x);
+  auto counts_of = [&](int w) {
+    if (two) return *reinterpret_cast<const uint2*>(at0 + w * pairs);
+    return make_uint2(mine ? at0[w * pairs] : 0u, 0u);
+  };
+  uint2 run = make_uint2(0, 0);
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    const uint2 c = counts_of(w);
+    run.x += c.x;
+    run.y += c.y;
+  }
+  const unsigned int items0 = (run.x & 0xffffu) + (run.x >> 16);
+  const unsigned int items1 = (run.y & 0xffffu) + (run.y >> 16);
+  const unsigned int start = cta_exclusive<kWarps>(items0 + items1, part, nullptr);
+  if (mine) {
+    uint2 at;
+    at.x = start | (start + (run.x & 0xffffu)) << 16;
+    at.y = (start + items0) | (start + items0 + (run.y & 0xffffu)) << 16;
+#pragma unroll
+    for (int w0 = 0; w0 < kWarps; w0 += 4) {
+      uint2 c[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) c[w] = counts_of(w0 + w);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        if (two) *reinterpret_cast<uint2*>(at0 + (w0 + w) * pairs) = at;
+        else at0[(w0 + w) * pairs] = at.x;
+        at.x += c[w].x;
+        at.y += c[w].y;
+      }
+    }
+  }
+}
+
 // Sorts the items of a CTA, which it has in registers in rows of 32 per warp, by `passes` digits of
 // `width` bits from the lowest of the key on; leaves them in order in sh.items.
 template <bool LONG>
 __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int passes, int width,
                                            const PieceShared& sh) {
-  constexpr int kWarps = kPieceWarps, kRows = kPieceRows, kT = kPieceThreads;
+  constexpr int kRows = kPieceRows, kT = kPieceThreads;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rows = (count + kT - 1) / kT;
   const int base = warp * (32 * rows) + lane;
   const int valid = valid_rows(count - base, rows);
   if (rows <= 2) {
-    sort_few<2>(k, valid, sh);
+    sort_few(k[0], k[1], valid, sh.items);
     return;
   }
   const int digits = 1 << width, pairs = digits / 2;
@@ -525,45 +556,7 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
     if (pass == 0) rank_rows<true, kRows>(digit, rows, valid, lanes, cnt, rank);
     else rank_rows<false, kRows>(digit, rows, valid, lanes, cnt, rank);
     __syncthreads();
-    // Where the warps' parts of this thread's digits start in the piece: of two pairs of digits
-    // side by side, or of one.  (Two words at a time: one by one, two apart, they took twice the
-    // clocks.)
-    static_assert(kPieceCounters / 2 == 2 * kT, "two pairs per thread at most");
-    const bool two = pairs > kT, mine = two || (int)threadIdx.x < pairs;
-    unsigned int* const at0 = count2 + (two ? 2 * threadIdx.x : threadIdx.x);
-    auto counts_of = [&](int w) {
-      if (two) return *reinterpret_cast<const uint2*>(at0 + w * pairs);
-      return make_uint2(mine ? at0[w * pairs] : 0u, 0u);
-    };
-    uint2 run = make_uint2(0, 0);
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      const uint2 c = counts_of(w);
-      run.x += c.x;
-      run.y += c.y;
-    }
-    const unsigned int items0 = (run.x & 0xffffu) + (run.x >> 16);
-    const unsigned int items1 = (run.y & 0xffffu) + (run.y >> 16);
-    const unsigned int start = cta_exclusive<kWarps>(items0 + items1,
-                                                     sh.part + (pass & 1) * kWarps, nullptr);
-    if (mine) {
-      uint2 at;
-      at.x = start | (start + (run.x & 0xffffu)) << 16;
-      at.y = (start + items0) | (start + items0 + (run.y & 0xffffu)) << 16;
-#pragma unroll
-      for (int w0 = 0; w0 < kWarps; w0 += 4) {
-        uint2 c[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) c[w] = counts_of(w0 + w);
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          if (two) *reinterpret_cast<uint2*>(at0 + (w0 + w) * pairs) = at;
-          else at0[(w0 + w) * pairs] = at.x;
-          at.x += c[w].x;
-          at.y += c[w].y;
-        }
-      }
-    }
+    place_counts(count2, pairs, sh.part + (pass & 1) * kPieceWarps);
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kRows; ++j) {
@@ -651,14 +644,49 @@ __device__ __forceinline__ int add_up_popular(Item (&k)[kPieceRows], int count,
   return count;
 }
 
+// What the threads before have of the key that is open where this thread begins; `any`: whether a
+// key begins in this thread's items, `sum`: of its open one (of all of them, where none begins).
+__device__ __forceinline__ float carry_into(bool any, float sum) {
+  __shared__ float s_tail[kPieceWarps];
+  __shared__ bool s_flag[kPieceWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // segmented inclusive scan of (has heads, open sum) over the threads
+  bool f = any;
+  float v = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float pv = __shfl_up_sync(0xffffffffu, v, o);
+    const bool pf = __shfl_up_sync(0xffffffffu, f, o);
+    if (lane >= o) {
+      if (!f) v += pv;
+      f |= pf;
+    }
+  }
+  if (lane == 31) {
+    s_tail[warp] = v;
+    s_flag[warp] = f;
+  }
+  float carry = __shfl_up_sync(0xffffffffu, v, 1);
+  bool carried = __shfl_up_sync(0xffffffffu, f, 1);
+  if (lane == 0) {
+    carry = 0.f;
+    carried = false;
+  }
+  __syncthreads();
+  if (!carried)
+    for (int w = warp - 1; w >= 0; --w) {
+      carry += s_tail[w];
+      if (s_flag[w]) break;
+    }
+  return carry;
+}
+
 // The sums of the values of equal keys in `count` sorted items.  The distinct keys end up at the
 // front of sh.items, above their sums or (LONG) alone, with the sums in sh.vals.  Returns how many.
 template <bool LONG>
 __device__ __forceinline__ unsigned int sum_piece(int count, const PieceShared& sh) {
   constexpr int kWarps = kPieceWarps, kMost = kPieceRows + 1;
   using Key = std::conditional_t<LONG, Item, unsigned int>;
-  __shared__ float s_tail[kWarps];
-  __shared__ bool s_flag[kWarps];
   auto key_of = [](Item i) { return (Key)(i >> (LONG ? kIndexBits : 32)); };
   auto put_sum = [&](unsigned int slot, float v) {
     if constexpr (LONG) sh.vals[slot] = v;
@@ -668,7 +696,6 @@ __device__ __forceinline__ unsigned int sum_piece(int count, const PieceShared& 
     if constexpr (LONG) sh.items[slot] = k;
     else reinterpret_cast<unsigned int*>(sh.items + slot)[1] = k;
   };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // every thread takes a run of items, an odd number: threads then start in different banks
   const int each = ((count + kPieceThreads - 1) / kPieceThreads) | 1;
   const int q0 = threadIdx.x * each, have = count - q0;
@@ -707,35 +734,8 @@ __device__ __forceinline__ unsigned int sum_piece(int count, const PieceShared& 
     }
     sum += val[j];
   }
-  // segmented inclusive scan of (has heads, open sum) over the threads
   const bool any = heads > 0;
-  bool f = any;
-  float v = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float pv = __shfl_up_sync(0xffffffffu, v, o);
-    const bool pf = __shfl_up_sync(0xffffffffu, f, o);
-    if (lane >= o) {
-      if (!f) v += pv;
-      f |= pf;
-    }
-  }
-  if (lane == 31) {
-    s_tail[warp] = v;
-    s_flag[warp] = f;
-  }
-  float carry = __shfl_up_sync(0xffffffffu, v, 1);
-  bool carried = __shfl_up_sync(0xffffffffu, f, 1);
-  if (lane == 0) {
-    carry = 0.f;
-    carried = false;
-  }
-  __syncthreads();
-  if (!carried)
-    for (int w = warp - 1; w >= 0; --w) {
-      carry += s_tail[w];
-      if (s_flag[w]) break;
-    }
+  const float carry = carry_into(any, sum);
   if (any && first_slot > 0) put_sum(first_slot - 1, carry + lead);
   if (threadIdx.x == kPieceThreads - 1 && total > 0) put_sum(total - 1, any ? sum : carry + sum);
   __syncthreads();

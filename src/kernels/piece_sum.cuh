@@ -22,20 +22,21 @@
 //
 // Whole calls, us, before (pass by pass) and now; ids with many repeats, ids all different:
 //                24 bits                   30 bits                   40 bits
-//   2^14 (10^4)  40 -> 29,  41 -> 30       42 -> 30,  43 -> 30       52 -> 30,  55 -> 31
-//   2^16         44 -> 32,  45 -> 32       50 -> 31,  51 -> 34       63 -> 32,  66 -> 37
-//   2^18         55 -> 37,  61 -> 38       59 -> 41,  66 -> 42       80 -> 48,  86 -> 49
-//   2^19         61 -> 42,  64 -> 49       65 -> 47,  71 -> 55       84 -> 56,  92 -> 63
-//   2^20         72 -> 69,  71 -> 61       78 -> 77,  84 -> 65      102 -> 91, 107 -> 72
-//   2^21         97 -> 89,  96 -> 84      103 -> 104, 112 -> 92     148 -> 116, 161 -> 104
-//   2^22        154 -> 136, 154 -> 132    172 -> 145, 183 -> 144    251 -> 174, 263 -> 165
-// Half of all items one id: 0.49 to 0.70 of the time before up to 2^19 items, 0.7 to 1.0 beyond.
-// Keys that crowd together in seven narrow ranges: 0.65 to 1.17 up to 2^19, where a sample makes
+//   2^14         41 -> 30,  41 -> 34       42 -> 30,  43 -> 33       52 -> 31,  53 -> 36
+//   2^16         43 -> 31,  45 -> 32       50 -> 31,  50 -> 33       63 -> 31,  66 -> 37
+//   2^18         55 -> 38,  61 -> 38       59 -> 40,  65 -> 42       79 -> 48,  86 -> 49
+//   2^19         61 -> 42,  64 -> 49       65 -> 45,  72 -> 54       83 -> 56,  91 -> 63
+//   2^20         71 -> 68,  71 -> 61       79 -> 77,  85 -> 65      102 -> 91, 108 -> 72
+//   2^21         97 -> 88,  96 -> 83      103 -> 104, 111 -> 89     147 -> 112, 160 -> 101
+//   2^22        152 -> 133, 153 -> 128    169 -> 135, 182 -> 138    250 -> 158, 263 -> 161
+// Half of all items one id: 0.48 to 0.72 of the time before up to 2^19 items, 0.63 to 0.98 beyond.
+// Keys that crowd together in seven narrow ranges: 0.72 to 1.14 up to 2^19, where a sample makes
 // the parts; then the general way after a count, or after the pieces, for nothing: 1.3 at 700 000,
-// 1.06 to 1.15 from 2^20 on.
-// What bounds it: up to 2^18 items the chain of some ten trips to L2 and
-// three sorts of 2400 clocks per pass; at 2^22 the instructions of piece_sum (52 us; 0.55 of the
-// issue slots, 24 warps per SM).
+// 1.05 to 1.14 from 2^20 on.  More than 20 popular ids in one part of the input: every piece has
+// them, so that the part's merge takes another round (700 000 items: 64 -> 70 us, else 52).
+// What bounds it: up to 2^18 items the chain of some ten trips to L2 and three sorts of 2400 clocks
+// per pass; at 2^22 piece_sum (48 us; 0.52 of the issue slots, two thirds of the shared-memory
+// pipe, 24 warps per SM), bucket_scatter (26 to 32), and the latency of piece_merge (25).
 //
 // An item is a key of up to 32 bits above its value, or (LONG) one of up to 51 above the index that
 // its value has in the CTA.

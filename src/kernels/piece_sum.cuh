@@ -423,15 +423,29 @@ struct PieceShared {
         vals(reinterpret_cast<float*>(smem + kPieceItems + kPieceCount)), part(part) {}
 };
 
-// Sorts up to 512 items as whole words, two per thread: every warp its own in registers (bitonic),
-// then runs are merged two by two, each item finding its place in the other run by bisection.
-// `mem`: 1024 items, which begins with the sorted ones.  A pass of the radix sort takes some 2400
-// clocks however few the items are, this sort about as long in all (2^16 items in two rows, 30
-// bits: 33.5 -> 30.5 us; four rows are faster by radix, 2^17 items 33.5 and 36 us).  The loops are
-// not unrolled: a kernel of a few CTAs runs through its code once, and waits for the code.
+// Sorts up to 512 items, two per thread: every warp its own in registers (bitonic), then runs are
+// merged two by two, each item finding its place in the other run by bisection.  `mem`: 1024 items,
+// which begins with the sorted ones.  A pass of the radix sort takes some 2400 clocks however few
+// the items are, this sort about as long in all (2^16 items in two rows, 30 bits: 33.5 -> 30.5 us;
+// four rows are faster by radix, 2^17 items 33.5 and 36 us).  The loops are not unrolled: a kernel
+// of a few CTAs runs through its code once, and waits for the code.
+// Pairs are sorted with their numbers in place of the values: in the order of the values' bits all
+// positive ones of a key would be added up before the negative ones, at three times the error.
+template <bool LONG>
 __device__ __forceinline__ void sort_few(Item k0, Item k1, int valid, Item* mem) {
   constexpr int kRun = 64, kAll = kRun * kPieceWarps;
   const int lane = threadIdx.x & 31;
+  Item *from = mem + kAll, *to = mem;
+  int at0 = 2 * threadIdx.x, at1 = at0 + 1;
+  unsigned int* const low = reinterpret_cast<unsigned int*>(from + (at0 & -kRun));
+  unsigned int low0 = 0, low1 = 0;
+  if constexpr (!LONG) {
+    low[2 * lane] = (unsigned int)k0;
+    low[2 * lane + 1] = (unsigned int)k1;
+    k0 = (k0 >> 32 << 32) | at0;
+    k1 = (k1 >> 32 << 32) | at1;
+    __syncwarp();
+  }
   if (valid < 1) k0 = ~0ull;  // (behind all others)
   if (valid < 2) k1 = ~0ull;
 #pragma unroll 1
@@ -451,8 +465,11 @@ __device__ __forceinline__ void sort_few(Item k0, Item k1, int valid, Item* mem)
       k1 = t;
     }
   }
-  Item *from = mem + kAll, *to = mem;
-  int at0 = 2 * threadIdx.x, at1 = at0 + 1;
+  if constexpr (!LONG) {
+    low0 = low[k0 % kRun];
+    low1 = low[k1 % kRun];
+    __syncwarp();
+  }
   from[at0] = k0;
   from[at1] = k1;
 #pragma unroll 1
@@ -476,6 +493,10 @@ __device__ __forceinline__ void sort_few(Item k0, Item k1, int valid, Item* mem)
     Item* const t = from;
     from = to;
     to = t;
+  }
+  if constexpr (!LONG) {  // (places that only this thread writes, and nobody reads before)
+    from[at0] = (k0 >> 32 << 32) | low0;
+    from[at1] = (k1 >> 32 << 32) | low1;
   }
   __syncthreads();
 }
@@ -535,7 +556,7 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
   const int base = warp * (32 * rows) + lane;
   const int valid = valid_rows(count - base, rows);
   if (rows <= 2) {
-    sort_few(k[0], k[1], valid, sh.items);
+    sort_few<LONG>(k[0], k[1], valid, sh.items);
     return;
   }
   const int digits = 1 << width, pairs = digits / 2;

@@ -94,3 +94,16 @@ def test_a_key_wider_than_stated(cuda_device, n, bits):
     keys[n // 2] += 1 << 55
     got, sums = sort_unique_sum(keys, torch.ones(n, device=cuda_device), key_bits=bits)
     assert int(sums.sum()) == n and bool(((got & ((1 << bits) - 1)).diff() >= 0).all())
+
+
+# the order in which the values of a key are added up does not depend on them: in the order of their
+# bits all positive ones would come first, and partial sums would be large
+@pytest.mark.parametrize("kind", ["low", "popular"])
+@pytest.mark.parametrize("n", [4097, 65_537, 131_072, 131_073, FEW, 1 << 20])
+@pytest.mark.parametrize("bits", [24, 32, 40])
+def test_negated_values_have_negated_sums(cuda_device, kind, n, bits):
+    from ps_lite_b200.ops.keys import sort_unique_sum
+    keys, vals = _keys(kind, n, bits, cuda_device)
+    ids, sums = sort_unique_sum(keys, vals, key_bits=bits)
+    same, negated = sort_unique_sum(keys, -vals, key_bits=bits)
+    assert torch.equal(ids, same) and torch.equal(sums, -negated)

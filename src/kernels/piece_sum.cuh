@@ -426,7 +426,7 @@ struct PieceShared {
 // Sorts up to 512 items, two per thread: every warp its own in registers (bitonic), then runs are
 // merged two by two, each item finding its place in the other run by bisection.  `mem`: 1024 items,
 // which begins with the sorted ones.  A pass of the radix sort takes some 2400 clocks however few
-// the items are, this sort about as long in all (2^16 items in two rows, 30 bits: 33.5 -> 30.5 us;
+// the items are, this sort about as long in all (2^16 items in two rows, 30 bits: 33.5 -> 31 us;
 // four rows are faster by radix, 2^17 items 33.5 and 36 us).  The loops are not unrolled: a kernel
 // of a few CTAs runs through its code once, and waits for the code.
 // Pairs are sorted with their numbers in place of the values: in the order of the values' bits all

@@ -1,21 +1,25 @@
-// The end of a request of one rank, told to the host by the kernel itself.
+// The end of a small dense request of one rank, told to the host by the kernel itself.
 //
-// The host hears of an event behind a kernel 8.7 to 9.2 us after it begins to launch that kernel,
-// of a word that the kernel writes to mapped memory as its last act after 7.2 us (1 CTA) to 8.3
-// (600).  The CTAs count themselves done; the last one writes the word.  The order is that of this
-// GPU (GPU scope): what a request writes is memory of this GPU, and whatever reads it once the host
-// has seen the word - a kernel, a copy engine, a peer - reads it through the GPU's L2, where it is
-// by then.  (A fence of system scope takes the 1.3 us back: 8.1 to 9.5 us.)  Requests with arrays
-// on the host wait for an event, and so does everything that the host orders by events or streams.
+// The CTAs count themselves done; the last one writes a word in mapped memory.  What a request has
+// written may be read by anybody whom the host tells that it is done - a kernel of another stream, a
+// copy, a peer, the host itself - with no event in between, so the word is released at system
+// scope: the other CTAs' writes come before their counts at GPU scope, and those before the last
+// one's fence.  The fence takes 1.2 us of what the word saves against an event: a launch is known to
+// be done after 9.1 us with one CTA and 9.7 to 9.9 with more (7.8 and 8.5 to 8.8 behind a fence of
+// GPU scope, which would order nothing for a reader that the host starts), by an event after 9.1 to
+// 9.5 and the 1 to 2 us that its query takes the completion thread.
 #pragma once
 #include "ps/device/psdev.h"
 
 namespace psdev {
 
-// Up to so many CTAs count themselves one by one on one address.  (fp32 values pushed and pulled,
-// SGD, an event / the word: 500 000 in 489 CTAs 13.5 / 12.5 us, 4 10^6 in 3907 19.7 / 18.9, 1.6
-// 10^7 in 15625 61.0 / 59.0, 3.2 10^7 in 31250 108.6 / 106.4, but 2^26 in 65536 216 / 251.)
-constexpr long long kDoneCtas = 16384;
+// Up to so many CTAs a request has a word.  Waited for from Python, us, fp32 SGD / bf16 momentum,
+// pushed and pulled, by an event and by the word: 1024 values (1 CTA) 12.3 / 12.5 and 11.4 / 11.7,
+// 100 000 (98) 12.4 / 12.5 and 12.0 / 12.1, 200 000 (196) 12.7 / 12.8 and 12.5 / 12.6, 500 000 (489)
+// 13.3 / 13.4 and 13.2 / 13.3, 2 10^6 (1954) 16.1 / 16.5 and 16.2 / 17.1; pushed alone 2 10^6 13.8 /
+// 15.1 and 14.1 / 15.9.  (Keyed requests gained nothing: 50 001 rows 14.8 and 14.9, with lengths
+// 30.4 and 31.2.)
+constexpr long long kDoneCtas = 128;
 
 struct DoneArgs {
   unsigned int* word;     // NULL: the host waits for an event
@@ -38,8 +42,7 @@ inline DoneArgs arm_done(psdev_done_t* done, long long ctas) {
 
 // At the beginning of a kernel: brings its arguments near, so that the end does not wait for them.
 // (Kernels that tell nobody are compiled without either: such a read at the end, of a pointer that
-// is NULL, takes 0.5 us of a launch, keyed calls one behind the other 4.1 and 4.6 us.  Held in
-// registers from here on, the arguments cost occupancy: 3.2 10^7 values 77.6 and 80.5 us.)
+// is NULL, takes 0.5 us of a launch.)
 __device__ __forceinline__ void expect_done(const DoneArgs& a) {
   asm volatile("" ::"l"(a.word), "r"(a.last));
 }
@@ -54,7 +57,7 @@ __device__ __forceinline__ void signal_done(const DoneArgs& a) {
                  : "=r"(before) : "l"(a.ticket) : "memory");
     if (before + 1 != a.last) return;
   }
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  asm volatile("fence.acq_rel.sys;" ::: "memory");
   asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(a.word), "r"(a.value) : "memory");
 }
 

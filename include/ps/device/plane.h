@@ -188,8 +188,7 @@ class Plane : public DeviceRoute {
 
  private:
   void SubmitSparse(DeviceRequest&& req);
-  void FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* stream,
-                    psdev_done_t* word = nullptr);
+  void FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* stream);
   Plane();
   ~Plane();
   std::unique_ptr<Impl> impl_;

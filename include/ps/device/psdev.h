@@ -222,8 +222,8 @@ typedef struct {
 } psdev_done_t;
 int psdev_done_create(int n, psdev_done_t* done);
 int psdev_done_destroy(int n, psdev_done_t* done);
-/* psdev_dense_op_direct on memory of this GPU that writes the word when it is done; where it
- * cannot, done->armed stays 0. */
+/* psdev_dense_op_direct that writes the word when it is done; where it does not (more CTAs than
+ * gain by it), done->armed stays 0. */
 int psdev_dense_op_direct_done(const psdev_world_t* w, const psdev_table_t* t, int op,
                                int64_t begin, int64_t end, const psdev_opt_t* opt, int channel,
                                int num_ctas, void* stream, const void* src, void* dst,
@@ -339,12 +339,6 @@ int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t 
                        const uint64_t* keys, const float* vals, int64_t nvals,
                        const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
                        void* stream);
-/* The same, with the word of psdev_dense_op_direct_done. */
-int psdev_sparse_local_done(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
-                            const uint64_t* keys, const float* vals, int64_t nvals,
-                            const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
-                            void* stream, psdev_done_t* done);
-
 /* Command of a request whose caller has seen that every array is memory of the table's GPU, and no
  * host memory by another name; for others the driver is asked about each array (0.1 to 0.2 us
  * apiece). */

@@ -32,7 +32,6 @@
 #include <type_traits>
 
 #include "ps/device/chain.cuh"
-#include "ps/device/done.cuh"
 #include "ps/device/push_pull.cuh"
 
 namespace psdev {
@@ -422,17 +421,6 @@ struct LocalReq {
   long long* sums;       // values per chunk (requests with lengths and many keys), or NULL
   int blocks;            // blocks of kLenBlock keys per chunk
 };
-struct ToldReq : LocalReq {  // the host waits for a word
-  DoneArgs done;
-};
-template <typename Req>
-__device__ __forceinline__ void expect(const Req& q) {
-  if constexpr (std::is_same<Req, ToldReq>::value) expect_done(q.done);
-}
-template <typename Req>
-__device__ __forceinline__ void tell(const Req& q) {
-  if constexpr (std::is_same<Req, ToldReq>::value) signal_done(q.done);
-}
 constexpr int kLocalUnroll = 4;
 // One 16-byte group per key, all of them far apart: a plain kernel that reads 2^20 such groups and
 // writes them back takes 59 us with one per thread, 63 with two, 67 with four (41 only reading),
@@ -513,11 +501,10 @@ __device__ __forceinline__ bool below(long long at, long long end) {
 
 // Every key has `width` values.  Equal keys next to each other count as one whose gradients are
 // added up: the first of them does the work of all.
-template <bool GROUP, bool ONE, bool FAR, typename Req>
+template <bool GROUP, bool ONE, bool FAR>
 __global__ void __launch_bounds__(256)
-    sparse_local_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ Req q) {
+    sparse_local_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ LocalReq q) {
   grid_launch_next();
-  expect(q);
   grid_wait();
   constexpr int kLocalUnroll = local_unroll(GROUP, ONE, FAR);
   const unsigned int width = ONE ? 1u : (unsigned int)a.width;
@@ -567,15 +554,14 @@ __global__ void __launch_bounds__(256)
     if (q.out)
       for (long long m = 0; m <= more; ++m) q.out[t + m * width] = v[u].x;
   }
-  tell(q);
 }
 
 // Rows of a multiple of four values with one number each (sum, SGD): 16-byte accesses.
-template <bool FAR, typename Req>
+template <bool FAR>
 __global__ void __launch_bounds__(256)
-    sparse_local_rows_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ Req q) {
+    sparse_local_rows_kernel(const __grid_constant__ SparseArgs a,
+                             const __grid_constant__ LocalReq q) {
   grid_launch_next();
-  expect(q);
   grid_wait();
   const unsigned int quads = (unsigned int)a.width / 4;
   const long long work = q.n * quads;
@@ -631,7 +617,6 @@ __global__ void __launch_bounds__(256)
     if (out)
       for (long long m = i[u]; m <= last; ++m) out[m * quads + j[u]] = w[u];
   }
-  tell(q);
 }
 
 // Values with lengths (`lens` given: a push, possibly of no value at all).  A CTA takes a chunk
@@ -712,11 +697,11 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x == 0) q.sums[blockIdx.x] = all;
 }
 
-template <bool GROUP, typename Req>
+template <bool GROUP>
 __global__ void __launch_bounds__(256)
-    sparse_local_lens_kernel(const __grid_constant__ SparseArgs a, const __grid_constant__ Req q) {
+    sparse_local_lens_kernel(const __grid_constant__ SparseArgs a,
+                             const __grid_constant__ LocalReq q) {
   grid_launch_next();
-  expect(q);
   grid_wait();
   __shared__ long long s_part[8];
   __shared__ unsigned long long s_key[kLenBlock];
@@ -728,7 +713,7 @@ __global__ void __launch_bounds__(256)
   const unsigned int width = (unsigned int)a.width;
   for (int b = 0; b < q.blocks; ++b) {
     const long long lo = chunk + (long long)b * kLenBlock;
-    if (lo >= q.n) break;
+    if (lo >= q.n) return;
     const int count = (int)(q.n - lo < kLenBlock ? q.n - lo : kLenBlock);
     __syncthreads();
     const bool mine = threadIdx.x < count;
@@ -841,23 +826,11 @@ __global__ void __launch_bounds__(256)
     }
     base += total;
   }
-  tell(q);
 }
 
 }  // namespace psdev
 
 using namespace psdev;
-
-// One launch of the kernel that `kernel` names for a request of the given kind.
-template <typename Kernel>
-static int launch_request(psdev_done_t* done, unsigned ctas, cudaStream_t s, const SparseArgs& a,
-                          const LocalReq& q, const Kernel& kernel) {
-  ToldReq told{};
-  told.done = arm_done(done, ctas);
-  if (!told.done.word) return launch_chained(kernel(LocalReq{}), ctas, 256, 0, s, 1, a, q);
-  static_cast<LocalReq&>(told) = q;
-  return launch_chained(kernel(ToldReq{}), ctas, 256, 0, s, 1, a, told);
-}
 
 extern "C" {
 
@@ -960,11 +933,10 @@ int psdev_sparse_scatter(const psdev_world_t* w, const psdev_sparse_t* t, int64_
   return (int)cudaGetLastError();
 }
 
-int psdev_sparse_local_done(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
-                            const uint64_t* keys, const float* vals, int64_t nvals,
-                            const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
-                            void* stream, psdev_done_t* done) {
-  if (done) done->armed = 0;
+int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
+                       const uint64_t* keys, const float* vals, int64_t nvals,
+                       const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
+                       void* stream) {
   SparseArgs a{};
   int rc = fill(&a, w, t, n);
   if (rc) return rc;
@@ -1001,11 +973,8 @@ int psdev_sparse_local_done(const psdev_world_t* w, const psdev_sparse_t* t, int
       rc = launch_chained(sparse_len_sums_kernel, chunks, 256, 0, s, 1, a, q);
       g_launches.fetch_add(1, std::memory_order_relaxed);
     }
-    if (!rc)
-      rc = launch_request(done, chunks, s, a, q, [&](auto req) {
-        using R = decltype(req);
-        return group ? sparse_local_lens_kernel<true, R> : sparse_local_lens_kernel<false, R>;
-      });
+    auto* kern = group ? sparse_local_lens_kernel<true> : sparse_local_lens_kernel<false>;
+    if (!rc) rc = launch_chained(kern, chunks, 256, 0, s, 1, a, q);
   } else {
     const bool rows = t->kind != 2 && t->width % 4 == 0 && a.sstride == 1 &&
                       (((uintptr_t)vals | (uintptr_t)out | (uintptr_t)t->w) & 15) == 0;
@@ -1016,28 +985,19 @@ int psdev_sparse_local_done(const psdev_world_t* w, const psdev_sparse_t* t, int
     const bool far = value_bytes < 128 && n < t->slots / (128 / value_bytes);
     const int unroll = rows ? kLocalUnroll : local_unroll(group, one, far);
     const unsigned ctas = (unsigned)((work + 256 * unroll - 1) / (256 * unroll));
-    auto pick = [&](auto f, auto req) {
+    auto pick = [&](auto f) {
       constexpr bool F = decltype(f)::value;
-      using R = decltype(req);
-      return rows           ? sparse_local_rows_kernel<F, R>
-             : group && one ? sparse_local_kernel<true, true, F, R>
-             : group        ? sparse_local_kernel<true, false, F, R>
-             : one          ? sparse_local_kernel<false, true, F, R>
-                            : sparse_local_kernel<false, false, F, R>;
+      return rows           ? sparse_local_rows_kernel<F>
+             : group && one ? sparse_local_kernel<true, true, F>
+             : group        ? sparse_local_kernel<true, false, F>
+             : one          ? sparse_local_kernel<false, true, F>
+                            : sparse_local_kernel<false, false, F>;
     };
-    rc = launch_request(done, ctas, s, a, q, [&](auto req) {
-      return far ? pick(std::true_type{}, req) : pick(std::false_type{}, req);
-    });
+    auto* kern = far ? pick(std::true_type{}) : pick(std::false_type{});
+    rc = launch_chained(kern, ctas, 256, 0, s, 1, a, q);
   }
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return rc;
-}
-int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t n,
-                       const uint64_t* keys, const float* vals, int64_t nvals,
-                       const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
-                       void* stream) {
-  return psdev_sparse_local_done(w, t, n, keys, vals, nvals, lens, out, nout, lens_out, stream,
-                                 nullptr);
 }
 
 // Server role.  `sync` != 0: the kernel first waits until every rank has entered it, i.e.

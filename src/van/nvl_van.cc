@@ -68,8 +68,8 @@ struct Rt {
   int (*sparse_lens)(const psdev_world_t*, const psdev_sparse_t*, int, void*) = nullptr;
   int (*key_shard_lookup)(const uint64_t*, int64_t, uint64_t, int, int64_t*, void*) = nullptr;
   int (*sparse_local)(const psdev_world_t*, const psdev_sparse_t*, int64_t, const uint64_t*,
-                      const float*, int64_t, const int32_t*, float*, int64_t, int32_t*, void*,
-                      psdev_done_t*) = nullptr;
+                      const float*, int64_t, const int32_t*, float*, int64_t, int32_t*,
+                      void*) = nullptr;
   int (*lens_to_offsets)(const int32_t*, int64_t, int64_t*, void*) = nullptr;
   int (*device_barrier)(const psdev_world_t*, int, uint64_t, void*) = nullptr;
   int (*multicast_pays)(int, uint64_t) = nullptr;
@@ -150,7 +150,7 @@ void* LoadRt(const std::string& configured, Rt* rt) {
   Bind(lib, "psdev_sparse_respond", &rt->sparse_respond);
   Bind(lib, "psdev_sparse_lens", &rt->sparse_lens);
   Bind(lib, "psdev_key_shard_lookup", &rt->key_shard_lookup);
-  Bind(lib, "psdev_sparse_local_done", &rt->sparse_local);
+  Bind(lib, "psdev_sparse_local", &rt->sparse_local);
   Bind(lib, "psdev_lens_to_offsets", &rt->lens_to_offsets);
   Bind(lib, "psdev_device_barrier", &rt->device_barrier);
   Bind(lib, "psdev_multicast_pays", &rt->multicast_pays);
@@ -536,12 +536,11 @@ struct Plane::Impl {
     unsigned long long id = 0;
     return rt.stream_id && rt.stream_id(s, &id) == 0 ? id : 0;
   }
-  // Whether `p` is device memory; *here: of this GPU; *managed: set where it may be the host's too.
-  bool OnDevice(const void* p, bool* here, bool* managed) const {
+  // Whether `p` is device memory; *here: of this GPU.
+  bool OnDevice(const void* p, bool* here) const {
     int device = -1;
     const int kind = rt.memory(p, &device);
     *here = kind == 2 || (kind == 1 && device == opts.device);
-    *managed |= kind == 2;
     return kind != 0;
   }
   // Orders work on `s` after the previous request on the tensor, unless that was on this stream too
@@ -551,10 +550,11 @@ struct Plane::Impl {
       rt.stream_wait_event(s, prev.event);
   }
 
-  // Words that the kernel of a one-rank request writes when it is done, for the completer to poll
-  // (done.cuh).  A request takes one while there are some, and gives it back when it has completed.
+  // Words that the kernel of a small one-rank request writes when it is done, for the completer to
+  // poll (done.cuh).  A request takes one while there are some, and gives it back when it has
+  // completed.
   static constexpr int kDoneWords = 64;
-  psdev_done_t done_words[kDoneWords];
+  psdev_done_t done_words[kDoneWords] = {};
   std::vector<psdev_done_t*> idle_words;
   psdev_done_t* NewWord() {
     const auto lk = SpinLock(ev_mu);
@@ -650,7 +650,7 @@ struct Plane::Impl {
       const psdev_done_t* w = p.word;
       const bool told =
           w && SpinUntil(std::chrono::steady_clock::now() + std::chrono::microseconds(SpinMicros()),
-                         [&] { return *w->host == w->value; });
+                         [&] { return __atomic_load_n(w->host, __ATOMIC_ACQUIRE) == w->value; });
       int rc = told ? 0 : rt.event_sync(p.event);
       if (rc == 0) RecycleWord(p.word);
       int32_t status = 0;
@@ -967,7 +967,8 @@ void Plane::Stop() {
   }
   if (!m.sim) {
     for (void* e : m.event_pool) m.rt.event_destroy(e);
-    if (!m.idle_words.empty()) m.rt.done_destroy(Impl::kDoneWords, m.done_words);
+    if (m.done_words[0].host) m.rt.done_destroy(Impl::kDoneWords, m.done_words);
+    m.done_words[0].host = nullptr;
     m.idle_words.clear();
     m.rt.stream_destroy(m.s_h2d);
     m.rt.stream_destroy(m.s_compute);
@@ -1394,12 +1395,12 @@ void Plane::Submit(DeviceRequest&& req) {
 
   // (the CPU stand-in calls "device memory" what lies in an arena.)  What lies on another GPU is
   // copied: a kernel of this one may not be able to reach it.
-  bool near = true, managed = false;
+  bool near = true;
   auto on_device = [&](const void* p) {
     if (req.cmd == PSDEV_CMD_ARRAYS_HERE) return true;
     if (!m.sim) {
       bool here = false;
-      const bool device = m.OnDevice(p, &here, &managed);
+      const bool device = m.OnDevice(p, &here);
       if (device && !here) near = false;
       return device;
     }
@@ -1493,8 +1494,7 @@ void Plane::Submit(DeviceRequest&& req) {
         void* dst = req.pull && outs && outs != weight ? out_at : nullptr;
         int ctas = d->num_ctas;
         if ((host_in || host_out) && ctas <= 0) ctas = kZeroCopyCtas;
-        const bool words = nruns == 1 && !host_in && !host_out && !managed;
-        psdev_done_t* word = words ? m.NewWord() : nullptr;
+        psdev_done_t* word = nruns == 1 && !host_in && !host_out ? m.NewWord() : nullptr;
         const int rc = m.rt.dense_op_direct(&m.ws, &t, op, r.begin, pad8(r.end), &opt, d->channel,
                                             ctas, s, src, dst, d->n_user, word);
         CHECK_EQ(rc, 0) << "psdev_dense_op_direct failed";
@@ -1665,10 +1665,9 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
     return !a || !b || a == b || !Clash(a, an, 1, b, bn, 1);
   };
   // (and so does a request with an array on the host or on another GPU)
-  bool managed = false;
   auto here = [&](const void* p) {
     bool is = !p;
-    return is || (m.OnDevice(p, &is, &managed) && is);
+    return is || (m.OnDevice(p, &is) && is);
   };
   const size_t kbytes = static_cast<size_t>(n) * 8, lbytes = static_cast<size_t>(n) * 4;
   void* out = req.pull ? req.outs : nullptr;
@@ -1690,18 +1689,12 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
   if (local) {
     // one rank: one kernel on the request's own arrays
     if (lens_to) CHECK_EQ(req.lens_out_n, static_cast<size_t>(n));
-    psdev_done_t* word = managed ? nullptr : m.NewWord();
     CHECK_EQ(m.rt.sparse_local(&m.ws, &t, n, static_cast<const uint64_t*>(kptr),
                                static_cast<const float*>(req.push ? req.vals : nullptr),
                                static_cast<int64_t>(vbytes / 4), lens_in, static_cast<float*>(out),
-                               static_cast<int64_t>(obytes / 4), static_cast<int*>(lens_to), s,
-                               word), 0)
+                               static_cast<int64_t>(obytes / 4), static_cast<int*>(lens_to), s), 0)
         << "psdev_sparse_local failed";
-    if (word && !word->armed) {
-      m.RecycleWord(word);
-      word = nullptr;
-    }
-    FinishSparse(sp, std::move(req), s, word);
+    FinishSparse(sp, std::move(req), s);
     return;
   }
   if (kptr != sp->keys) {
@@ -1748,13 +1741,11 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
 }
 
 // The request's work has been issued on `s`: completion and the ordering point of the table.
-void Plane::FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* s,
-                         psdev_done_t* word) {
+void Plane::FinishSparse(const SparseInfo* sp, DeviceRequest&& req, void* s) {
   Impl& m = *impl_;
   void* done = m.NewEvent();
   m.rt.event_record(done, s);
   Impl::Pending pend;
-  pend.word = word;
   pend.event = done;
   pend.channel = sp->table.channel;
   pend.timestamp = req.timestamp;

@@ -1,6 +1,7 @@
 """Requests of one rank whose kernel itself tells the host that it is done: what a request has written
-is there for another stream once it has been waited for, from one CTA to more than count themselves,
-with more requests in flight than there are words, and from several threads."""
+is there for another stream, for a copy engine and for the host once it has been waited for, from one
+CTA to more than count themselves, with more requests in flight than there are words, and from several
+threads."""
 import os
 import subprocess
 import sys
@@ -28,7 +29,7 @@ DENSE = """
     dev = ctx.device
     other = torch.cuda.Stream(dev)
     # CTAs of 1024 values: one, two, a few, as many as count themselves and one more
-    for key, n in enumerate([1, 1024, 1025, 37 * 1024, 16384 * 1024, 16384 * 1024 + 1]):
+    for key, n in enumerate([1, 1024, 1025, 37 * 1024, 128 * 1024, 128 * 1024 + 1, 1 << 24]):
         kv.declare(key, n, optimizer=ServerOptimizer("sum"))
         grad, out = torch.ones(n, device=dev), torch.zeros(n, device=dev)
         torch.cuda.synchronize()
@@ -112,4 +113,96 @@ def test_requests_of_several_threads(cuda_device):
         assert not bad, bad
         kvstore.finalize()
         print("RAN")
+    """)
+
+
+def test_copies_that_follow_no_event(cuda_device):
+    """Another stream's copy engine takes the output to the host: nothing orders it behind the request
+    but the host, which has waited for that."""
+    _run("""
+        import torch
+        from ps_lite_b200 import kvstore
+        from ps_lite_b200.parallel import ServerOptimizer
+        ctx = kvstore.init(heap_bytes=1 << 30)
+        kv, dev = kvstore.KVStore(ctx), ctx.device
+        other = torch.cuda.Stream(dev)
+        def reads(n, request, wait, out, step):
+            host = torch.zeros(n, pin_memory=True)
+            torch.cuda.synchronize()
+            first = None
+            for i in range(300):
+                wait(request())
+                with torch.cuda.stream(other):
+                    host.copy_(out, non_blocking=True)
+                other.synchronize()
+                first = host[0].item() if first is None else first
+                assert bool((host == first + i * step).all()), (n, i)
+        for key, n in enumerate([1, 1024, 1025, 37 * 1024, 128 * 1024, 128 * 1024 + 1]):
+            kv.declare(key, n, optimizer=ServerOptimizer("sum"))
+            grad, out = torch.ones(n, device=dev), torch.zeros(n, device=dev)
+            reads(n, lambda: kv.push_pull(key, grad, out), kv.wait, out, 1)
+        ks = kvstore.KeyedStore(ctx, 7, 1 << 20, 20000, width=8, kind="sum")
+        for n in [1, 300, 20000]:
+            keys = torch.arange(n, device=dev) * 7 + 1
+            vals, out = torch.full((n * 8,), 2.0, device=dev), torch.zeros(n * 8, device=dev)
+            ks.wait(ks.pull(keys, out))
+            ks.wait(ks.push(keys, -out))           # (what a smaller n has left)
+            reads(n * 8, lambda: ks.push_pull(keys, vals, out), ks.wait, out, 2)
+        kvstore.finalize()
+        print("RAN")
+    """)
+
+
+@pytest.mark.parametrize("kind", ["managed", "mapped", "pool"])
+def test_memory_that_the_host_reads(cuda_device, kind, tmp_path):
+    """Tensors over memory that is the host's too: managed, mapped host memory, and a pool of torch's
+    allocator over one that makes managed memory.  The host reads it as soon as it has waited."""
+    source, lib = tmp_path / "managed.cc", tmp_path / "managed.so"
+    source.write_text("""
+        #include <cuda_runtime.h>
+        extern "C" void* take(long size, int, cudaStream_t) {
+          void* p = nullptr;
+          return cudaMallocManaged(&p, size) == cudaSuccess ? p : nullptr;
+        }
+        extern "C" void give(void* p, long, int, cudaStream_t) { cudaFree(p); }
+        extern "C" void* mapped(long size) {
+          void* p = nullptr;
+          return cudaHostAlloc(&p, size, cudaHostAllocMapped) == cudaSuccess ? p : nullptr;
+        }
+    """)
+    subprocess.run(["nvcc", "-shared", "-Xcompiler", "-fPIC", "-x", "cu", str(source), "-o", str(lib)], check=True)
+    _run(f"""
+        import ctypes, numpy as np, torch
+        from ps_lite_b200 import kvstore
+        from ps_lite_b200.parallel import ServerOptimizer
+        ctx = kvstore.init(heap_bytes=1 << 28)
+        kv, dev, kind = kvstore.KVStore(ctx), ctx.device, {kind!r}
+        lib = ctypes.CDLL({str(lib)!r})
+        lib.take.restype = lib.mapped.restype = ctypes.c_void_p
+        lib.take.argtypes, lib.mapped.argtypes = [ctypes.c_long, ctypes.c_int, ctypes.c_void_p], [ctypes.c_long]
+        pool = None
+        if kind == "pool":
+            own = torch.cuda.memory.CUDAPluggableAllocator({str(lib)!r}, "take", "give")
+            pool = torch.cuda.MemPool(own.allocator())
+        def tensor(n):
+            if kind == "pool":
+                with torch.cuda.use_mem_pool(pool):
+                    return torch.zeros(n, device=dev)
+            at = lib.take(4 * n, 0, None) if kind == "managed" else lib.mapped(4 * n)
+            class Array:
+                __cuda_array_interface__ = dict(shape=(n,), typestr="<f4", data=(at, False), version=3)
+            return torch.as_tensor(Array(), device=dev)
+        for key, n in enumerate([1000, 100_000, 1_000_000]):
+            kv.declare(key, n, optimizer=ServerOptimizer("sum"))
+            grad, out = tensor(n).fill_(1.0), tensor(n).zero_()
+            seen = np.ctypeslib.as_array(ctypes.cast(out.data_ptr(), ctypes.POINTER(ctypes.c_float)), (n,))
+            torch.cuda.synchronize()
+            for i in range(1, 60):
+                kv.wait(kv.push_pull(key, grad, out))
+                assert (seen == i).all(), (n, i)
+        torch.cuda.synchronize()
+        import os
+        kvstore.finalize()
+        print("RAN", flush=True)
+        os._exit(0)   # (the tensors' memory has no owner)
     """)

@@ -1,11 +1,10 @@
 // One dense request from Python in one native call.
 //
-// A small request costs some 7 us from its launch to the word that says it is done; the Python
-// statements and the ctypes conversion in front of them would cost another 2.  This function checks
-// the tensors, looks up the current stream and hands the request to the worker
+// A small request costs the GPU about 2 us and its launch and completion some 9; the Python
+// statements and the ctypes conversion in front of them cost another 2.  This function checks the
+// tensors, looks up the current stream and hands the request to the worker
 // (ps_capi_bworker_request_on, src/capi/ps_nvl_c_api.h).
 #include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDACachingAllocator.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
@@ -32,18 +31,9 @@ struct Target {
 };
 constexpr const char* kName = "psb200.target";
 
-// Whether `x` is memory of torch's own allocator on this GPU.  (A tensor may also name memory that
-// something else made, mapped host memory for one.)
-bool allocated_on(const at::Tensor& x, c10::DeviceIndex device) {
-  return x.is_cuda() && x.get_device() == device &&
-         x.storage().data_ptr().get_deleter() ==
-             c10::cuda::CUDACachingAllocator::get()->raw_deleter();
-}
-
-// The address of `obj`'s values, or `own` for None; false with a Python error set.  *here: false
-// where it may be elsewhere than on the table's GPU.
+// The address of `obj`'s values, or `own` for None; false with a Python error set.
 bool values_of(PyObject* obj, const Target& t, at::ScalarType type, void* own, const char* wrong,
-               void** at, bool* here) {
+               void** at) {
   if (obj == Py_None) {
     *at = own;
     return true;
@@ -58,7 +48,6 @@ bool values_of(PyObject* obj, const Target& t, at::ScalarType type, void* own, c
     return false;
   }
   *at = x.data_ptr();
-  *here = *here && allocated_on(x, t.device);
   return true;
 }
 
@@ -72,20 +61,17 @@ PyObject* request(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (!t) return nullptr;
   const bool push = args[1] == Py_True, pull = args[2] == Py_True;
   void *vals = nullptr, *outs = nullptr;
-  bool here = true;
   HANDLE_TH_ERRORS
   if (push && !values_of(args[3], *t, t->grad_type, t->grad,
                          "pushed values must be a contiguous tensor of the declared length and "
-                         "gradient dtype", &vals, &here))
+                         "gradient dtype", &vals))
     return nullptr;
   if (pull && !values_of(args[4], *t, t->out_type, t->weight,
                          "the output must be a contiguous tensor of the declared length and "
-                         "weight dtype", &outs, &here))
+                         "weight dtype", &outs))
     return nullptr;
-  long cmd = PyLong_AsLong(args[5]);
-  const long priority = PyLong_AsLong(args[6]);
+  const long cmd = PyLong_AsLong(args[5]), priority = PyLong_AsLong(args[6]);
   if (PyErr_Occurred()) return nullptr;
-  if (here && cmd == 0) cmd = PSDEV_CMD_ARRAYS_HERE;
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream(t->device).stream();
   int ts;
   Py_BEGIN_ALLOW_THREADS
@@ -164,7 +150,7 @@ PyObject* keyed_request(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int* lp = vals && lens ? static_cast<const int*>(lens->data_ptr()) : nullptr;
   int* lo = out && !vals && lens_out ? static_cast<int*>(lens_out->data_ptr()) : nullptr;
   const size_t vb = vals ? vals->numel() * 4 : 0, ob = out ? out->numel() * 4 : 0;
-  auto here = [&](const at::Tensor* x) { return !x || allocated_on(*x, t->device); };
+  auto here = [&](const at::Tensor* x) { return !x || x->get_device() == t->device; };
   const bool all = here(keys) && here(vals) && here(out) && here(lens) && here(lens_out);
   int ts;
   Py_BEGIN_ALLOW_THREADS

@@ -153,10 +153,11 @@ def test_copies_that_follow_no_event(cuda_device):
     """)
 
 
-@pytest.mark.parametrize("kind", ["managed", "mapped", "pool"])
+@pytest.mark.parametrize("kind", ["managed", "mapped", "managed pool", "mapped pool"])
 def test_memory_that_the_host_reads(cuda_device, kind, tmp_path):
-    """Tensors over memory that is the host's too: managed, mapped host memory, and a pool of torch's
-    allocator over one that makes managed memory.  The host reads it as soon as it has waited."""
+    """Tensors over memory that is the host's too: managed, mapped host memory, and pools of torch's
+    allocator over either.  The host reads it as soon as it has waited.  What is host memory goes the
+    way of host memory, whoever has made the tensor: 64 MiB both ways in slices."""
     source, lib = tmp_path / "managed.cc", tmp_path / "managed.so"
     source.write_text("""
         #include <cuda_runtime.h>
@@ -165,43 +166,49 @@ def test_memory_that_the_host_reads(cuda_device, kind, tmp_path):
           return cudaMallocManaged(&p, size) == cudaSuccess ? p : nullptr;
         }
         extern "C" void give(void* p, long, int, cudaStream_t) { cudaFree(p); }
-        extern "C" void* mapped(long size) {
+        extern "C" void* mapped(long size, int, cudaStream_t) {
           void* p = nullptr;
           return cudaHostAlloc(&p, size, cudaHostAllocMapped) == cudaSuccess ? p : nullptr;
         }
+        extern "C" void unmapped(void* p, long, int, cudaStream_t) { cudaFreeHost(p); }
     """)
     subprocess.run(["nvcc", "-shared", "-Xcompiler", "-fPIC", "-x", "cu", str(source), "-o", str(lib)], check=True)
     _run(f"""
-        import ctypes, numpy as np, torch
-        from ps_lite_b200 import kvstore
+        import ctypes, os, numpy as np, torch
+        from ps_lite_b200 import host, kvstore
         from ps_lite_b200.parallel import ServerOptimizer
-        ctx = kvstore.init(heap_bytes=1 << 28)
+        ctx = kvstore.init(heap_bytes=1 << 29)
         kv, dev, kind = kvstore.KVStore(ctx), ctx.device, {kind!r}
-        lib = ctypes.CDLL({str(lib)!r})
-        lib.take.restype = lib.mapped.restype = ctypes.c_void_p
-        lib.take.argtypes, lib.mapped.argtypes = [ctypes.c_long, ctypes.c_int, ctypes.c_void_p], [ctypes.c_long]
-        pool = None
-        if kind == "pool":
-            own = torch.cuda.memory.CUDAPluggableAllocator({str(lib)!r}, "take", "give")
+        lib, names = ctypes.CDLL({str(lib)!r}), ("take", "give") if "managed" in kind else ("mapped", "unmapped")
+        make = getattr(lib, names[0])
+        make.restype, make.argtypes = ctypes.c_void_p, [ctypes.c_long, ctypes.c_int, ctypes.c_void_p]
+        if "pool" in kind:
+            own = torch.cuda.memory.CUDAPluggableAllocator({str(lib)!r}, *names)
             pool = torch.cuda.MemPool(own.allocator())
         def tensor(n):
-            if kind == "pool":
+            if "pool" in kind:
                 with torch.cuda.use_mem_pool(pool):
                     return torch.zeros(n, device=dev)
-            at = lib.take(4 * n, 0, None) if kind == "managed" else lib.mapped(4 * n)
             class Array:
-                __cuda_array_interface__ = dict(shape=(n,), typestr="<f4", data=(at, False), version=3)
+                __cuda_array_interface__ = dict(shape=(n,), typestr="<f4", data=(make(4 * n, 0, None), False),
+                                                version=3)
             return torch.as_tensor(Array(), device=dev)
-        for key, n in enumerate([1000, 100_000, 1_000_000]):
+        def launches(key, grad, out):
+            before = host.lib().psnvl_launches()
+            kv.wait(kv.push_pull(key, grad, out))
+            return host.lib().psnvl_launches() - before
+        for key, n in enumerate([1000, 100_000, 1_000_000, 1 << 24]):
             kv.declare(key, n, optimizer=ServerOptimizer("sum"))
             grad, out = tensor(n).fill_(1.0), tensor(n).zero_()
             seen = np.ctypeslib.as_array(ctypes.cast(out.data_ptr(), ctypes.POINTER(ctypes.c_float)), (n,))
             torch.cuda.synchronize()
-            for i in range(1, 60):
+            for i in range(1, 60 if n < 1 << 24 else 4):
                 kv.wait(kv.push_pull(key, grad, out))
                 assert (seen == i).all(), (n, i)
         torch.cuda.synchronize()
-        import os
+        like = torch.ones(n, pin_memory=True) if "mapped" in kind else torch.ones(n, device=dev)
+        torch.cuda.synchronize()
+        assert launches(key, grad, out) == launches(key, like, torch.empty_like(like, pin_memory=like.is_pinned()))
         kvstore.finalize()
         print("RAN", flush=True)
         os._exit(0)   # (the tensors' memory has no owner)

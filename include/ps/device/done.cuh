@@ -7,7 +7,7 @@
 // one's fence.  The fence takes 1.2 us of what the word saves against an event: a launch is known
 // to be done after 9.1 us with one CTA and 9.7 to 9.9 with more (7.8 and 8.5 to 8.8 behind a fence
 // of GPU scope, which would order nothing for a reader that the host starts), by an event after
-// 9.1 to 9.5 and the 1 to 2 us that its query takes the completion thread.
+// 9.1 to 9.5.  In whole requests the word gains more (kDoneCtas).
 #pragma once
 #include "ps/device/psdev.h"
 

@@ -339,11 +339,6 @@ int psdev_sparse_local(const psdev_world_t* w, const psdev_sparse_t* t, int64_t 
                        const uint64_t* keys, const float* vals, int64_t nvals,
                        const int32_t* lens, float* out, int64_t nout, int32_t* lens_out,
                        void* stream);
-/* Command of a request whose caller has seen that every array is memory of the table's GPU, and no
- * host memory by another name; for others the driver is asked about each array (0.1 to 0.2 us
- * apiece). */
-#define PSDEV_CMD_ARRAYS_HERE 0x48455245
-
 /* Server role, tables with lengths: stores the length of the value of every key that a worker
  * staged (keys in its arena, cut points computed with psdev_key_shard_lookup) into that worker's
  * array of lengths; 0 for a key that was never pushed.  Used by a pull that does not know the

@@ -37,6 +37,9 @@ struct DeviceRequest {
   int* lens_out = nullptr;     // pull: per-key value counts are written here when not null
   size_t lens_out_n = 0;
   size_t val_size = 4;         // sizeof(Val) of the KVWorker
+  // Keyed tables: the caller has seen that every array is memory of the table's GPU.  Otherwise the
+  // driver is asked about each of them (0.1 to 0.2 us apiece).
+  bool arrays_here = false;
   Customer* customer = nullptr;
   int responses = 1;           // what the tracker expects for this timestamp
   std::function<void()> on_done;  // runs before the request is credited (user callback)

@@ -116,14 +116,15 @@ class KVWorker : public SimpleApp {
   void Wait(int timestamp) { obj_->WaitRequest(timestamp); }
 
   // Zero-copy variants: the arrays are shared, not copied; the caller must leave their
-  // contents unchanged until the request has completed.
+  // contents unchanged until the request has completed.  `arrays_here`: see DeviceRequest.
   int ZPush(const SArray<Key>& keys, const SArray<Val>& vals, const SArray<int>& lens = {},
-            int cmd = 0, const Callback& cb = nullptr, int priority = 0) {
+            int cmd = 0, const Callback& cb = nullptr, int priority = 0,
+            bool arrays_here = false) {
     if (DeviceRoute* route = DeviceRouteFor(keys)) {
       // the arrays are captured by the completion routine: they stay alive until then
       return SubmitToDevice(route, true, false, cmd, keys, vals.data(),
                             vals.size() * sizeof(Val), nullptr, 0, lens, nullptr, 0,
-                            [keys, vals, lens, cb]() { if (cb) cb(); }, priority);
+                            [keys, vals, lens, cb]() { if (cb) cb(); }, priority, arrays_here);
     }
     const int ts = obj_->NewRequest(kServerGroup);
     AddCallback(ts, cb);
@@ -137,7 +138,8 @@ class KVWorker : public SimpleApp {
   }
 
   int ZPull(const SArray<Key>& keys, SArray<Val>* vals, SArray<int>* lens = nullptr,
-            int cmd = 0, const Callback& cb = nullptr, int priority = 0) {
+            int cmd = 0, const Callback& cb = nullptr, int priority = 0,
+            bool arrays_here = false) {
     if (DeviceRoute* route = DeviceRouteFor(keys)) {
       CHECK_NOTNULL(vals);
       if (vals->empty()) vals->resize(route->PullBytes(obj_->app_id(), keys) / sizeof(Val));
@@ -145,7 +147,7 @@ class KVWorker : public SimpleApp {
       return SubmitToDevice(route, false, true, cmd, keys, nullptr, 0, vals->data(),
                             vals->size() * sizeof(Val), SArray<int>(),
                             lens ? lens->data() : nullptr, lens ? lens->size() : 0,
-                            [keys, cb]() { if (cb) cb(); }, priority);
+                            [keys, cb]() { if (cb) cb(); }, priority, arrays_here);
     }
     const int ts = AddPullCB(keys, vals, lens, cmd, cb);
     KVPairs<Val> kvs;
@@ -157,14 +159,14 @@ class KVWorker : public SimpleApp {
 
   int ZPushPull(const SArray<Key>& keys, const SArray<Val>& vals, SArray<Val>* outs,
                 SArray<int>* lens = nullptr, int cmd = 0, const Callback& cb = nullptr,
-                int priority = 0) {
+                int priority = 0, bool arrays_here = false) {
     if (DeviceRoute* route = DeviceRouteFor(keys)) {
       CHECK_NOTNULL(outs);
       if (outs->empty()) outs->resize(vals.size());
       return SubmitToDevice(route, true, true, cmd, keys, vals.data(),
                             vals.size() * sizeof(Val), outs->data(), outs->size() * sizeof(Val),
                             lens ? *lens : SArray<int>(), nullptr, 0,
-                            [keys, vals, cb]() { if (cb) cb(); }, priority);
+                            [keys, vals, cb]() { if (cb) cb(); }, priority, arrays_here);
     }
     const int ts = AddPullCB(keys, outs, lens, cmd, cb);
     KVPairs<Val> kvs;
@@ -200,7 +202,7 @@ class KVWorker : public SimpleApp {
   int SubmitToDevice(DeviceRoute* route, bool push, bool pull, int cmd, const SArray<Key>& keys,
                      const void* vals, size_t vals_bytes, void* outs, size_t outs_bytes,
                      const SArray<int>& lens, int* lens_out, size_t lens_out_n,
-                     Callback cb, int priority) {
+                     Callback cb, int priority, bool arrays_here = false) {
     const int ts = obj_->NewRequest(kServerGroup);
     DeviceRequest req;
     req.app_id = obj_->app_id();
@@ -218,6 +220,7 @@ class KVWorker : public SimpleApp {
     req.lens_out = lens_out;
     req.lens_out_n = lens_out_n;
     req.val_size = sizeof(Val);
+    req.arrays_here = arrays_here;
     req.customer = obj_;
     req.responses = Postoffice::Get()->num_servers();
     req.on_done = std::move(cb);

@@ -115,6 +115,7 @@ def lib() -> C.CDLL:
             keyed = [i, i, vp, sz, vp, sz, vp, sz, vp, vp, i]
             L.ps_capi_bworker_keyed_request.argtypes = [vp] + keyed
             L.ps_capi_bworker_keyed_request_on.argtypes = [vp, vp] + keyed
+            L.ps_capi_bworker_keyed_request_here.argtypes = [vp, vp] + keyed
             _lib = L
         return _lib
 

@@ -319,9 +319,10 @@ class KeyedStore:
         if not self.worker:
             raise host.PSError(L.ps_capi_last_error().decode())
         ext = _lib.torch_ext()
-        fn = C.cast(L.ps_capi_bworker_keyed_request_on, C.c_void_p).value
+        fn, here_fn = (C.cast(f, C.c_void_p).value for f in (L.ps_capi_bworker_keyed_request_on,
+                                                              L.ps_capi_bworker_keyed_request_here))
         self._submit = ext.keyed_request
-        self._target = ext.keyed_target(fn, self.worker, self.max_keys, self.var_len,
+        self._target = ext.keyed_target(fn, here_fn, self.worker, self.max_keys, self.var_len,
                                         ctx._device_index)
         self._wait = L.ps_capi_bworker_wait
         self._alive: Dict[int, tuple] = {}

@@ -199,10 +199,9 @@ int psnvl_declare_sparse(int app_id, uint64_t key_space, int64_t max_keys, int w
   });
 }
 
-int ps_capi_bworker_keyed_request(void* worker, int push, int pull, const uint64_t* keys_dev,
-                                  size_t nkeys, const void* vals_dev, size_t vals_bytes,
-                                  void* outs_dev, size_t outs_bytes, const int* lens_dev,
-                                  int* lens_out_dev, int cmd) {
+static int KeyedRequest(void* worker, int push, int pull, const uint64_t* keys_dev, size_t nkeys,
+                        const void* vals_dev, size_t vals_bytes, void* outs_dev, size_t outs_bytes,
+                        const int* lens_dev, int* lens_out_dev, int cmd, bool here) {
   return Guard([&] {
     auto* kv = static_cast<KVWorker<char>*>(worker);
     SArray<Key> k = SArray<Key>::FromDevice(
@@ -211,26 +210,41 @@ int ps_capi_bworker_keyed_request(void* worker, int push, int pull, const uint64
         const_cast<char*>(static_cast<const char*>(vals_dev)), vals_bytes);
     SArray<int> l;
     if (lens_dev) l = SArray<int>::FromDevice(const_cast<int*>(lens_dev), nkeys);
-    if (push && !pull) return kv->ZPush(k, v, l, cmd);
+    if (push && !pull) return kv->ZPush(k, v, l, cmd, nullptr, 0, here);
     // output views live until the request has completed
     auto* o = new SArray<char>(SArray<char>::FromDevice(static_cast<char*>(outs_dev), outs_bytes));
     if (push) {
       auto* lp = lens_dev ? new SArray<int>(l) : nullptr;
-      return kv->ZPushPull(k, v, o, lp, cmd, [o, lp]() { delete o; delete lp; });
+      return kv->ZPushPull(k, v, o, lp, cmd, [o, lp]() { delete o; delete lp; }, 0, here);
     }
     auto* lo = lens_out_dev ? new SArray<int>(SArray<int>::FromDevice(lens_out_dev, nkeys))
                             : nullptr;
-    return kv->ZPull(k, o, lo, cmd, [o, lo]() { delete o; delete lo; });
+    return kv->ZPull(k, o, lo, cmd, [o, lo]() { delete o; delete lo; }, 0, here);
   });
 }
-
+int ps_capi_bworker_keyed_request(void* worker, int push, int pull, const uint64_t* keys_dev,
+                                  size_t nkeys, const void* vals_dev, size_t vals_bytes,
+                                  void* outs_dev, size_t outs_bytes, const int* lens_dev,
+                                  int* lens_out_dev, int cmd) {
+  return KeyedRequest(worker, push, pull, keys_dev, nkeys, vals_dev, vals_bytes, outs_dev,
+                      outs_bytes, lens_dev, lens_out_dev, cmd, false);
+}
 int ps_capi_bworker_keyed_request_on(void* worker, void* stream, int push, int pull,
                                      const uint64_t* keys_dev, size_t nkeys, const void* vals_dev,
                                      size_t vals_bytes, void* outs_dev, size_t outs_bytes,
                                      const int* lens_dev, int* lens_out_dev, int cmd) {
   Plane::Get()->SetStream(stream);
-  return ps_capi_bworker_keyed_request(worker, push, pull, keys_dev, nkeys, vals_dev, vals_bytes,
-                                       outs_dev, outs_bytes, lens_dev, lens_out_dev, cmd);
+  return KeyedRequest(worker, push, pull, keys_dev, nkeys, vals_dev, vals_bytes, outs_dev,
+                      outs_bytes, lens_dev, lens_out_dev, cmd, false);
+}
+int ps_capi_bworker_keyed_request_here(void* worker, void* stream, int push, int pull,
+                                       const uint64_t* keys_dev, size_t nkeys,
+                                       const void* vals_dev, size_t vals_bytes, void* outs_dev,
+                                       size_t outs_bytes, const int* lens_dev, int* lens_out_dev,
+                                       int cmd) {
+  Plane::Get()->SetStream(stream);
+  return KeyedRequest(worker, push, pull, keys_dev, nkeys, vals_dev, vals_bytes, outs_dev,
+                      outs_bytes, lens_dev, lens_out_dev, cmd, true);
 }
 
 }  // extern "C"

@@ -79,7 +79,7 @@ int psnvl_declare_sparse(int app_id, uint64_t key_space, int64_t max_keys, int w
 /* One keyed request of a worker created for that app; every array is DEVICE memory and stays
  * valid until the wait returns.  keys: sorted unique uint64.  Push: vals (fp32) and, on a table
  * with lengths, lens (int32 per key).  Pull: outs, and on a table with lengths lens_out receives
- * the stored length of every key.  cmd: 0, or PSDEV_CMD_ARRAYS_HERE.  Returns the timestamp. */
+ * the stored length of every key.  Returns the timestamp. */
 int ps_capi_bworker_keyed_request(void* worker, int push, int pull, const uint64_t* keys_dev,
                                   size_t nkeys, const void* vals_dev, size_t vals_bytes,
                                   void* outs_dev, size_t outs_bytes, const int* lens_dev,
@@ -88,6 +88,13 @@ int ps_capi_bworker_keyed_request_on(void* worker, void* stream, int push, int p
                                      const uint64_t* keys_dev, size_t nkeys, const void* vals_dev,
                                      size_t vals_bytes, void* outs_dev, size_t outs_bytes,
                                      const int* lens_dev, int* lens_out_dev, int cmd);
+/* The same where the caller has seen that every array is memory of the table's GPU, about which the
+ * driver is then not asked (0.1 to 0.2 us apiece). */
+int ps_capi_bworker_keyed_request_here(void* worker, void* stream, int push, int pull,
+                                       const uint64_t* keys_dev, size_t nkeys,
+                                       const void* vals_dev, size_t vals_bytes, void* outs_dev,
+                                       size_t outs_bytes, const int* lens_dev, int* lens_out_dev,
+                                       int cmd);
 
 #ifdef __cplusplus
 }

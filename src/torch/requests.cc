@@ -89,6 +89,7 @@ using KeyedFn = int (*)(void*, void*, int, int, const uint64_t*, size_t, const v
                         size_t, const int*, int*, int);
 struct KeyedTarget {
   KeyedFn request;
+  KeyedFn request_here;  // all arrays on the table's GPU
   void* worker;
   int64_t max_keys;
   bool var_len;
@@ -154,9 +155,9 @@ PyObject* keyed_request(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const bool all = here(keys) && here(vals) && here(out) && here(lens) && here(lens_out);
   int ts;
   Py_BEGIN_ALLOW_THREADS
-  ts = t->request(t->worker, stream, vals != nullptr, out != nullptr,
-                  static_cast<const uint64_t*>(kp), static_cast<size_t>(n), vp, vb, op, ob, lp, lo,
-                  all ? PSDEV_CMD_ARRAYS_HERE : 0);
+  ts = (all ? t->request_here : t->request)(
+      t->worker, stream, vals != nullptr, out != nullptr, static_cast<const uint64_t*>(kp),
+      static_cast<size_t>(n), vp, vb, op, ob, lp, lo, 0);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(ts);
   END_HANDLE_TH_ERRORS
@@ -188,10 +189,11 @@ void add_requests(py::module& m) {
     t->out_size = c10::elementSize(t->out_type);
     return py::capsule(t, kName, [](void* p) { delete static_cast<Target*>(p); });
   });
-  m.def("keyed_target", [](uint64_t fn, uint64_t worker, int64_t max_keys, bool var_len,
-                           int device) {
-    auto* t = new KeyedTarget{reinterpret_cast<KeyedFn>(fn), reinterpret_cast<void*>(worker),
-                              max_keys, var_len, static_cast<c10::DeviceIndex>(device)};
+  m.def("keyed_target", [](uint64_t fn, uint64_t here_fn, uint64_t worker, int64_t max_keys,
+                           bool var_len, int device) {
+    auto* t = new KeyedTarget{reinterpret_cast<KeyedFn>(fn), reinterpret_cast<KeyedFn>(here_fn),
+                              reinterpret_cast<void*>(worker), max_keys, var_len,
+                              static_cast<c10::DeviceIndex>(device)};
     return py::capsule(t, kKeyedName, [](void* p) { delete static_cast<KeyedTarget*>(p); });
   });
   PyModule_AddFunctions(m.ptr(), kMethods);

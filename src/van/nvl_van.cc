@@ -1397,7 +1397,6 @@ void Plane::Submit(DeviceRequest&& req) {
   // copied: a kernel of this one may not be able to reach it.
   bool near = true;
   auto on_device = [&](const void* p) {
-    if (req.cmd == PSDEV_CMD_ARRAYS_HERE) return true;
     if (!m.sim) {
       bool here = false;
       const bool device = m.OnDevice(p, &here);
@@ -1683,7 +1682,7 @@ void Plane::SubmitSparse(DeviceRequest&& req) {
         ((reinterpret_cast<uintptr_t>(req.push ? req.vals : nullptr) |
           reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(lens_in) |
           reinterpret_cast<uintptr_t>(lens_to)) & 3)) &&
-      (req.cmd == PSDEV_CMD_ARRAYS_HERE ||
+      (req.arrays_here ||
        (here(kptr) && (!req.push || here(req.vals)) && here(out) && here(lens_in) &&
         here(lens_to)));
   if (local) {

@@ -81,14 +81,22 @@ CODE = """if 1:
 """
 
 
-def _run(places):
-    r = subprocess.run([sys.executable, "-c", CODE % (ROOT, places)], capture_output=True, text=True,
+def _run(places, code=CODE):
+    r = subprocess.run([sys.executable, "-c", code % (ROOT, places)], capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "PLACES_OK" in r.stdout, (r.stdout + r.stderr)[-3000:]
 
 
 def test_host_and_device(cuda_device):
     _run(["cuda:0", "cpu", "pinned"])
+
+
+def test_a_command_says_nothing_about_arrays(cuda_device):
+    """The number that once told the plane not to ask where the arrays of a request are."""
+    code = CODE.replace("None, None, 0)", "None, None, 0x48455245)").replace("else None, 0)", "else None, 0x48455245)")
+    code = code.replace("kv.wait(kv.push_pull(0, g, o))", "kv.wait(kv._request(0, True, True, g, o, cmd=0x48455245))")
+    assert code.count("0x48455245") == 3
+    _run(["cuda:0", "cpu", "pinned"], code)
 
 
 def test_two_gpus(cuda_device):

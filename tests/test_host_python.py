@@ -342,6 +342,24 @@ def test_device_plane_c_abi_on_the_cpu_stand_in(tmp_path, nproc):
     assert rc == 0 and out.count("PY_PLANE_OK") == nproc, out[-3000:]
 
 
+@pytest.mark.parametrize("cmd", [1, 0x48455245])
+def test_a_command_says_nothing_about_arrays(tmp_path, cmd):
+    """The command of a request is the program's: whatever it is, arrays on the host go through the
+    tensor's buffers, slice by slice (as many launches as without a command)."""
+    script = tmp_path / "plane_node.py"
+    counts = []
+    for c in (0, cmd):
+        script.write_text(PLANE_SCRIPT.replace("4 * n, 0, 0)", f"4 * n, {c}, 0)").replace(
+            "assert L.psnvl_launches() > 0", "print('LAUNCHES', L.psnvl_launches())"))
+        env = dict(os.environ, PSB_ROOT=ROOT, DMLC_PS_VAN_TYPE="loop")
+        env.pop("DMLC_ROLE", None)
+        r = subprocess.run([sys.executable, str(script)], capture_output=True, text=True,
+                           timeout=120, env=env)
+        assert r.returncode == 0 and "PY_PLANE_OK 0" in r.stdout, (r.stdout + r.stderr)[-3000:]
+        counts.append(r.stdout.split("LAUNCHES")[1].split()[0])
+    assert counts[0] == counts[1]
+
+
 def test_exit_without_finalize_ends_with_the_programs_status():
     """A process that started the runtime and dies of an exception leaves with status 1 at once
     (it neither blocks in the destruction of the runtime nor aborts)."""

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <type_traits>
 #include <utility>
@@ -1331,6 +1332,9 @@ struct UniqueScratch {
 // A word of mapped host memory for the time of one call.  64 of them in one page, allocated at the
 // first use and kept; a call that finds all taken gets memory of its own.
 struct ReportSlot {
+  // (behind nothing else the sample has been looked at 8 to 31 us after the launch, the more the
+  // larger the call before)
+  static constexpr int kSampleMicros = 50;
   unsigned long long* word = nullptr;
   int index = -1;
   static std::atomic<unsigned long long>& used() {
@@ -1370,16 +1374,20 @@ struct ReportSlot {
     if (index >= 0) used().fetch_and(~(1ull << index), std::memory_order_release);
     else if (word) cudaFreeHost(word);
   }
-  // What the sample has shown, once it has (the second word of the slot).
+  // What the sample has shown, once it has (the second word of the slot).  Behind other work on the
+  // stream it is not waited for: the rest is launched then too, and whatever the keys are like, its
+  // kernels find that out by themselves.
   bool spread() const {
     const volatile unsigned long long* w = word;
-    for (int i = 0; i < 100000; ++i) {
-      if (const unsigned long long got = w[1]) return !(got & kReportCrowded);
-      if (w[0]) break;
+    const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(kSampleMicros);
+    do {
+      for (int i = 0; i < 16; ++i) {
+        if (const unsigned long long got = w[1]) return !(got & kReportCrowded);
 #if defined(__x86_64__)
-      __builtin_ia32_pause();
+        __builtin_ia32_pause();
 #endif
-    }
+      }
+    } while (std::chrono::steady_clock::now() < until);
     return true;
   }
   // Polls while a sort takes microseconds; a long one is waited for without using the core.

@@ -85,6 +85,22 @@ def test_popular_neighbours(cuda_device, bits, ids, crowd):
     _check(keys, vals, bits)
 
 
+# a part with some items more than a CTA sorts, of fewer keys: three of them are in each of 79 pieces
+@pytest.mark.parametrize("bits", [30, 40])
+def test_a_part_with_a_few_items_too_many(cuda_device, bits):
+    from ps_lite_b200 import _lib
+    n, first = 40_000, 1 << (bits - 1)
+    keys, vals = _keys("spread", n, bits, cuda_device)
+    keys[keys >> (bits - 7) == 64] += 1 << (bits - 2)       # (nothing else in the part)
+    at = torch.arange(4997, device=cuda_device)
+    keys[at * 8] = first + 3 + at
+    keys[1::2] = torch.where(torch.arange(n // 2, device=cuda_device) % 10 == 0,
+                             first + torch.arange(n // 2, device=cuda_device) // 10 % 3, keys[1::2])
+    before = _lib.device_lib().psdev_launch_count()
+    _check(keys, vals, bits)
+    assert _lib.device_lib().psdev_launch_count() - before == 6   # (two calls: pieces, merge, gather)
+
+
 @pytest.mark.parametrize("n", [9000, 600_000, FEW + 1])
 @pytest.mark.parametrize("bits", [20, 40])
 def test_a_key_wider_than_stated(cuda_device, n, bits):

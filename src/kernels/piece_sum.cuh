@@ -59,7 +59,14 @@ constexpr long long kMaxBucketItems = 9ll << 19;     // (in 1024 buckets 4608 on
 // so that all units of a merge run at a time (444 pieces and 512 parts: 2^18 items 52 us, with 256
 // of both 40).  700 000 items, many repeats / all different: 57 / 65 us, in buckets 70 / 56; 2^20:
 // 66 / 78 and 75 / 65.
-constexpr long long kFewItems = 3 << 18, kSplitItems = 1 << 19;  // (and so many where keys crowd)
+constexpr long long kFewItems = 3 << 18;
+// Up to so many of them the parts of crowded keys are those of a sample; beyond, one of 256 parts
+// by a sample of 5120 would often have more keys than a CTA sorts, and the host goes the general
+// way as soon as it hears of the crowd.  Seven narrow ranges, 24 / 30 / 40 bits, before sums went
+// piece by piece, the general way and by the sample: 560 000 items 62 / 69 / 91, 79 / 88 / 114, 79
+// / 81 / 97; 655 360 64 / 71 / 94, 80 / 91 / 119, 81 / 87 / 102; 720 896 64 / 73 / 96, 82 / 94 /
+// 123, 107 / 108 / 132.  (The host has nothing to wait for then: others gain a microsecond.)
+constexpr long long kSplitItems = 5 << 17;
 constexpr int kFewPieces = 256, kFewParts = 256;
 // A bucket with more items than a CTA sorts is cut in smaller pieces, which do not keep the others
 // waiting, or in whole ones where those would be too many to merge.

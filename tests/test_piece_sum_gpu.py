@@ -50,6 +50,14 @@ def test_pieces_of_the_input(cuda_device, kind, n, bits):
     _check(*_keys(kind, n, bits, cuda_device), bits)
 
 
+# the line up to which a sample makes the parts of crowded keys
+@pytest.mark.parametrize("kind", ["spread", "popular", "low", "ranges"])
+@pytest.mark.parametrize("n", [5 << 17, (5 << 17) + 1])
+@pytest.mark.parametrize("bits", [24, 40])
+def test_parts_by_a_sample(cuda_device, kind, n, bits):
+    _check(*_keys(kind, n, bits, cuda_device), bits)
+
+
 @pytest.mark.parametrize("kind", ["spread", "popular", "low", "ranges", "one", "rising"])
 @pytest.mark.parametrize("n", [FEW + 1, 1 << 20, (1 << 20) + 1, 296 * 4096 + 1, MOST])
 @pytest.mark.parametrize("bits", [16, 24, 32, 33, 42])

@@ -68,6 +68,12 @@ constexpr long long kFewItems = 3 << 18;
 // 123, 107 / 108 / 132.  (The host has nothing to wait for then: others gain a microsecond.)
 constexpr long long kSplitItems = 5 << 17;
 constexpr int kFewPieces = 256, kFewParts = 256;
+// With more items than this CTAs that are left over help to merge the parts of the input.  700 000
+// ids of 24 bits with 25 popular ones in one part 73 -> 60 us, others with repeats from 530 000 on
+// 0.91 to 1.01, all different 0.94 to 1.00, half of them one id 0.89 to 1.00.  Fewer items seldom
+// make a part of more than a round, and looking for it costs up to a microsecond (2^16 ids 31.0 and
+// 32.1, 2^19 45.8 and 46.6).
+constexpr long long kHelpItems = 1 << 19;
 // A bucket with more items than a CTA sorts is cut in smaller pieces, which do not keep the others
 // waiting, or in whole ones where those would be too many to merge.
 constexpr int kSmallPiece = kPiece / 2, kManyItems = 1 << 20;
@@ -820,7 +826,7 @@ __device__ __forceinline__ void sample_parts(const Item* keys, unsigned int n, c
   if (threadIdx.x == 0) {
     if (!b.splits) sample_report(spread, host);
     SortHead h{};
-    h.groups = spread || split ? b.parts / kGroup : 0;
+    h.groups = spread || split ? (n > kHelpItems ? 2 : 1) * b.parts / kGroup : 0;
     h.several = 1;
     h.split = split;
     h.separate = LONG;
@@ -914,12 +920,52 @@ __global__ void __launch_bounds__(kPieceThreads, LONG ? 2 : 3)
 }
 
 constexpr unsigned int kMerged = 1u << 31;  // a place in the merge's output
+constexpr int kMaxGroup = 8;                // parts of the input that one CTA helps
+static_assert(kFewPieces <= kPieceThreads && kMaxOfBucket <= 4 * kPieceThreads, "of a thread");
+constexpr int kHelpers = kMergeCtas - kFewParts;
+static_assert(kHelpers * kMaxGroup >= kFewParts && 2 * kFewParts <= kMaxSegments,
+              "every part has a group, and segments");
+
+// The input's parts of `group`, group + kHelpers, ...: the one with the most items, if those are
+// more than a CTA sorts, else b.parts.  (One piece per thread.)
+__device__ __forceinline__ unsigned int heaviest(const Buckets& b, unsigned int group,
+                                                 unsigned int (&sums)[kMaxGroup][kPieceWarps]) {
+  const unsigned int parts = b.parts, p = threadIdx.x;
+  int j = 0;
+  for (unsigned int q = group; q < parts; q += kHelpers, ++j) {
+    unsigned int have = 0;
+    if (p < (unsigned int)b.chunks) {
+      const unsigned int* bound = b.bounds + (size_t)p * parts + q;
+      have = (q + 1 < parts ? __ldcg(bound + 1) : __ldcg(b.distinct + p) & ~kWidePiece) -
+             __ldcg(bound);
+    }
+    have = __reduce_add_sync(0xffffffffu, have);
+    if ((p & 31) == 0) sums[j][p >> 5] = have;
+  }
+  __syncthreads();
+  unsigned int most = kPiece, which = parts;
+  j = 0;
+  for (unsigned int q = group; q < parts; q += kHelpers, ++j) {
+    unsigned int all = 0;
+#pragma unroll
+    for (int w = 0; w < kPieceWarps; ++w) all += sums[j][w];
+    if (all > most) {
+      most = all;
+      which = q;
+    }
+  }
+  return which;
+}
 
 // Unit u: part u / m of the u % m-th of the m buckets in several pieces.  A bucket is merged in as
 // few parts as have room for the distinct keys of its pieces, with a third to spare: a unit then
-// takes several parts, and those that follow have nothing to do.  The input is merged part by part
-// (popular ids, which every piece has, may make more than kPiece items of few keys).
-template <bool LONG>
+// takes several parts, and those that follow have nothing to do.  The input is merged part by part.
+//
+// Popular ids, which every piece has, may make more than kPiece items of few keys, and a round more
+// would be the longest of the kernel.  HELP: the CTAs that the parts of the input leave over help;
+// each has a group of parts and takes the upper half of the heaviest, if that is more than one
+// round.  A part then has two segments, the second one for its helper.
+template <bool LONG, bool HELP>
 __global__ void __launch_bounds__(kPieceThreads, 2)
     piece_merge_kernel(Items in, Items out, const __grid_constant__ Buckets b, SortHead* head,
                        unsigned long long* host) {
@@ -927,6 +973,8 @@ __global__ void __launch_bounds__(kPieceThreads, 2)
   grid_launch_next();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned int s_part[2 * kPieceWarps], s_scan[2][kPieceWarps], s_before[kPieceWarps];
+  __shared__ unsigned int s_sums[HELP ? kMaxGroup : 1][kPieceWarps];
+  __shared__ Item s_middle;
   __shared__ bool s_last;
   bool wide = false;
   const PieceShared sh(smem_raw, s_part);
@@ -941,13 +989,27 @@ __global__ void __launch_bounds__(kPieceThreads, 2)
   const unsigned int buckets = __ldcg(&head->several), parts = b.parts;
   const bool split = __ldcg(&head->split) != 0;
   if (groups == 0) return;
-  for (unsigned int u = blockIdx.x; u < buckets * parts; u += gridDim.x) {
+  for (unsigned int u = blockIdx.x; u < buckets * parts + (HELP ? kHelpers : 0); u += gridDim.x) {
     Several s{0, 0, (unsigned int)b.chunks, 0};
     if (b.count) {
       const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(b.several + u % buckets));
       s = {raw.x, raw.y, raw.z, raw.w};
     }
-    const unsigned int part = u / buckets, segment = s.bucket * parts + part;
+    unsigned int part = u / buckets;
+    bool halved = false;
+    if constexpr (HELP) {
+      halved = part >= parts;  // (a helper)
+      if (halved) {
+        if (split) continue;
+        part = heaviest(b, u - parts, s_sums);
+        if (part == parts) {  // (the same for all threads)
+          __syncthreads();
+          continue;
+        }
+      }
+    }
+    const bool helping = halved;
+    const unsigned int segment = HELP ? 2 * part + helping : s.bucket * parts + part;
     Item low = 0, high = 0;
     if (split) {
       low = __ldcg(b.splits + part);
@@ -955,7 +1017,6 @@ __global__ void __launch_bounds__(kPieceThreads, 2)
     }
     // Each thread's pieces follow one another: what they have in all, of this part and of the parts
     // before.  (Up to four pieces of a bucket, one of the input; the first one's numbers are kept.)
-    static_assert(kFewPieces <= kPieceThreads && kMaxOfBucket <= 4 * kPieceThreads, "a thread's");
     const unsigned int run = (s.pieces + kPieceThreads - 1) / kPieceThreads;
     const unsigned int p0 = threadIdx.x * run, p1 = p0 + run < s.pieces ? p0 + run : s.pieces;
     unsigned int span = 1;
@@ -1019,6 +1080,39 @@ __global__ void __launch_bounds__(kPieceThreads, 2)
     unsigned int at = cta_exclusive<kPieceWarps>(have, s_scan[1], &count);
 #pragma unroll
     for (int w = 0; w < kPieceWarps; ++w) before += s_before[w];
+    if constexpr (HELP) {
+      if (!helping && !split && count > kPiece)
+        halved = heaviest(b, part % kHelpers, s_sums) == part;
+      if (halved) {
+        // the upper half begins at the key in the middle of what the first piece has
+        if (threadIdx.x == 0) {
+          const unsigned int size = first.to - first.from;
+          Item k = ((Item)part << b.part_shift) + ((Item)1 << (b.part_shift - 1));
+          if (size) {
+            k = __ldcg(in.keys + first.start + first.from + size / 2);
+            if constexpr (!LONG) k >>= 32;
+          }
+          s_middle = k;
+        }
+        __syncthreads();
+        const Item* keys = in.keys + first.start;
+        unsigned int lo = first.from, hi = first.to;
+        while (lo < hi) {
+          const unsigned int m = (lo + hi) / 2;
+          const Item k = __ldcg(keys + m);
+          if ((LONG ? k : k >> 32) < s_middle) lo = m + 1;
+          else hi = m;
+        }
+        if (helping) first.from = lo;
+        else first.to = lo;
+        smaller = __reduce_add_sync(0xffffffffu, first.from);
+        if ((threadIdx.x & 31) == 0) s_before[threadIdx.x >> 5] = smaller;
+        at = cta_exclusive<kPieceWarps>(first.to - first.from, s_scan[0], &count);
+        before = 0;
+#pragma unroll
+        for (int w = 0; w < kPieceWarps; ++w) before += s_before[w];
+      }
+    }
     // As many items as there is room for, in one round; where there are more, distinct keys make
     // room for the next ones.  (Given up where they leave less than a quarter, unless the next
     // round is the last: 560 000 ids of 24 bits in seven ranges have parts of 5000 items and some
@@ -1088,6 +1182,7 @@ __global__ void __launch_bounds__(kPieceThreads, 2)
     if (threadIdx.x == 0) {
       b.seg.counts[segment] = total;
       b.seg.place[segment] = (s.start + before) | kMerged;
+      if (HELP && !halved) b.seg.counts[segment + 1] = 0;
     }
     __syncthreads();
   }

@@ -1422,7 +1422,11 @@ int piece_sums(const Item* keys, const unsigned int* vals, int64_t n, const Uniq
                 const Buckets& b, const ReportSlot& slot, cudaStream_t s) {
   constexpr int smem = piece_smem<LONG>();
   if (int rc = allow_smem<piece_sum_kernel<RAW, LONG>>(smem)) return rc;
-  if (int rc = allow_smem<piece_merge_kernel<LONG>>(smem)) return rc;
+  const bool help = RAW && n > kHelpItems;
+  auto* merge = help ? piece_merge_kernel<LONG, true> : piece_merge_kernel<LONG, false>;
+  if (int rc = help ? allow_smem<piece_merge_kernel<LONG, true>>(smem)
+                    : allow_smem<piece_merge_kernel<LONG, false>>(smem))
+    return rc;
   const Items mine{u.keys[0], LONG ? reinterpret_cast<float*>(u.vals[0]) : nullptr};
   const Items merged{u.keys[1], LONG ? reinterpret_cast<float*>(u.vals[1]) : nullptr};
   const unsigned grid = RAW ? b.chunks + 1 : b.count + (unsigned)(n / kSmallPiece);
@@ -1432,9 +1436,9 @@ int piece_sums(const Item* keys, const unsigned int* vals, int64_t n, const Uniq
   g_launches.fetch_add(1, std::memory_order_relaxed);
   if (!rc && RAW && !b.splits && !slot.spread()) return 0;
   // (a bucket in several pieces has more than kPiece items)
-  const int64_t units = RAW ? b.parts : n / kPiece * b.parts;
+  const int64_t units = RAW ? b.parts + (help ? kHelpers : 0) : n / kPiece * b.parts;
   if (!rc)
-    rc = launch_chained(piece_merge_kernel<LONG>,
+    rc = launch_chained(merge,
                         units < 1 ? 1 : units < kMergeCtas ? (unsigned)units : kMergeCtas,
                         kPieceThreads, smem, s, 1, mine, merged, b, u.head, slot.word);
   g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -23,6 +23,20 @@ def _check(keys, vals, bits):
     assert torch.equal(again, got) and torch.equal(same, sums)
 
 
+def _check_exact(keys, bits):
+    """Whole numbers of which every partial sum is below 2^24: any order of additions is exact."""
+    from ps_lite_b200.ops.keys import sort_unique_sum
+    g = torch.Generator(device=keys.device)
+    g.manual_seed(keys.numel())
+    vals = torch.randint(-3, 5, keys.shape, device=keys.device, generator=g)
+    want, inverse = torch.unique(keys, return_inverse=True)
+    exact = torch.zeros_like(want).index_add_(0, inverse, vals)
+    size = torch.zeros_like(want).index_add_(0, inverse, vals.abs())
+    assert int(size.max()) < 1 << 24
+    got, sums = sort_unique_sum(keys, vals.float(), key_bits=bits)
+    assert torch.equal(got, want) and torch.equal(sums, exact.float())
+
+
 def _keys(kind, n, bits, dev):
     g = torch.Generator(device=dev)
     g.manual_seed(n + bits)
@@ -91,6 +105,28 @@ def test_popular_neighbours(cuda_device, bits, ids, crowd):
     if crowd:
         keys[1:2 * crowd:2] = (1 << (bits - 1)) + 1000 + torch.arange(crowd, device=cuda_device)
     _check(keys, vals, bits)
+
+
+# parts of the input with more items than a CTA sorts, which another CTA helps to merge: of one group
+# (40 parts away), without a key in the first piece, with one, with more keys than both can sort
+@pytest.mark.parametrize("n", [(1 << 19) + 1, 700_000, FEW])
+@pytest.mark.parametrize("bits", [24, 30, 40])
+@pytest.mark.parametrize("ids,parts,first,crowd", [(25, [7], True, 0), (40, [7, 47, 255], True, 0),
+                                                   (30, [0, 40], True, 0), (25, [7], False, 0), (21, [9], None, 0),
+                                                   (25, [7], True, 4500), (25, [7], True, 5200), (120, [3], True, 2000)])
+def test_parts_that_are_helped(cuda_device, n, bits, ids, parts, first, crowd):
+    keys, _ = _keys("spread", n, bits, cuda_device)
+    shift, size = bits - 8, (n + 255) // 256
+    for j, part in enumerate(parts):
+        at = torch.arange(j, n, 7, device=cuda_device)
+        keys[at] = (part << shift) + 11 * (torch.arange(at.numel(), device=cuda_device) % ids)
+    if first is not True:          # the first piece: nothing of the part, or one key
+        keys[:size] = torch.where(keys[:size] >> shift == parts[0], 0, keys[:size])
+        if first is None:
+            keys[5] = (parts[0] << shift) + 22
+    if crowd:
+        keys[3:7 * crowd:7] = (parts[0] << shift) + 5000 + torch.arange(crowd, device=cuda_device)
+    _check_exact(keys, bits)
 
 
 # a part with some items more than a CTA sorts, of fewer keys: three of them are in each of 79 pieces

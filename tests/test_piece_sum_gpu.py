@@ -113,7 +113,8 @@ def test_popular_neighbours(cuda_device, bits, ids, crowd):
 @pytest.mark.parametrize("bits", [24, 30, 40])
 @pytest.mark.parametrize("ids,parts,first,crowd", [(25, [7], True, 0), (40, [7, 47, 255], True, 0),
                                                    (30, [0, 40], True, 0), (25, [7], False, 0), (21, [9], None, 0),
-                                                   (25, [7], True, 4500), (25, [7], True, 5200), (120, [3], True, 2000)])
+                                                   (25, [7], True, 4500), (25, [7], True, 5200),
+                                                   (120, [3], True, 2000)])
 def test_parts_that_are_helped(cuda_device, n, bits, ids, parts, first, crowd):
     keys, _ = _keys("spread", n, bits, cuda_device)
     shift, size = bits - 8, (n + 255) // 256

@@ -1,6 +1,7 @@
 """sort_unique_sum piece by piece, where its way and its parts change: keys against torch.unique, sums
 against sums in fp64 within the bound of fp32 additions in any order, (m - 1) 2^-24 sum |v| for a key of
-m values."""
+m values, which says little where m is large: there, and wherever a key's values are added up apart from
+the others, sums of whole numbers, which have to be exact."""
 import pytest
 import torch
 
@@ -79,6 +80,28 @@ def test_buckets(cuda_device, kind, n, bits):
     _check(*_keys(kind, n, bits, cuda_device), bits)
 
 
+@pytest.mark.parametrize("kind", ["spread", "popular", "low", "ranges", "one"])
+@pytest.mark.parametrize("n", [4097, 5120, 65_537, 300_001, 5 << 17, FEW, FEW + 1, 1 << 20, (1 << 21) + 1, MOST])
+@pytest.mark.parametrize("bits", [16, 30, 40])
+def test_sums_of_whole_numbers(cuda_device, kind, n, bits):
+    _check_exact(_keys(kind, n, bits, cuda_device)[0], bits)
+
+
+# popular ids of a bucket: one that takes away more than a quarter of a piece's items (again and again),
+# several that take less, and pieces that keep at most two rows
+@pytest.mark.parametrize("n", [FEW + 1, (1 << 20) + 1, MOST])
+@pytest.mark.parametrize("bits", [24, 40])
+@pytest.mark.parametrize("shares", [[4], [4, 3, 3, 3, 3, 2], [8] * 10, [2, 1000], [1.05], [1.01, 200]])
+def test_popular_ids_of_a_bucket(cuda_device, n, bits, shares):
+    keys, _ = _keys("spread", n, bits, cuda_device)
+    left = torch.randperm(n, device=cuda_device)[: n // 2]
+    for j, share in enumerate(shares):      # every share-th of those that are left
+        take = int(len(left) / share)
+        keys[left[:take]] = (5 << (bits - 10)) + 3 * j
+        left = left[take:]
+    _check_exact(keys, bits)
+
+
 # beyond what pieces and buckets are for
 @pytest.mark.parametrize("n,bits", [(FEW, 52), (FEW + 1, 43), (MOST + 1, 30), (9000, 15)])
 def test_the_general_way(cuda_device, n, bits):
@@ -105,6 +128,7 @@ def test_popular_neighbours(cuda_device, bits, ids, crowd):
     if crowd:
         keys[1:2 * crowd:2] = (1 << (bits - 1)) + 1000 + torch.arange(crowd, device=cuda_device)
     _check(keys, vals, bits)
+    _check_exact(keys, bits)
 
 
 # parts of the input with more items than a CTA sorts, which another CTA helps to merge: of one group

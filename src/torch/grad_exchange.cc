@@ -277,8 +277,11 @@ class GradExchange {
 
   // Gives up the gradients whose kernels have finished, and says whether all have.  While one is
   // running, what is pending would only queue up behind it; it goes out with what comes next
-  // instead, in fewer and larger launches.  (An event's query takes this thread 1.4 us, so a hook
-  // that comes soon after one that found a launch running takes it to be running still.)
+  // instead, in fewer and larger launches.  (An event's query takes this thread 1.4 us, so it is
+  // made every 25 us at most: what is running at a look, or launched since, counts as running until
+  // the next.  How often hardly matters: never, 10, 25, 50 and 100 us in between, a pass of
+  // ResNet-50 took 1869, 1897, 1880, 1913 and 1845 us, of BERT-large 3412, 3406, 3385, 3408 and
+  // 3349, each of them within 2 % of itself from run to run.)
   bool Idle(const c10::cuda::CUDAStream& cur) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     C10_CUDA_CHECK(cudaStreamIsCapturing(cur.stream(), &capture));
@@ -363,7 +366,7 @@ class GradExchange {
   std::vector<at::Tensor> held_;  // gradients of segs_
   std::deque<Batch> batches_;     // launched, not known to be finished
   std::vector<Batch> spare_;
-  std::chrono::steady_clock::time_point next_look_{};  // not before: a launch was running
+  std::chrono::steady_clock::time_point next_look_{};  // not before
   at::cuda::CUDAEvent fork_;
   std::optional<c10::cuda::CUDAStream> pending_on_;   // hooks of what is pending ran here
   std::optional<c10::cuda::CUDAStream> launched_on_;  // launches of this step

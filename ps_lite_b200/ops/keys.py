@@ -57,7 +57,11 @@ def sort_unique_sum(keys: torch.Tensor, vals: torch.Tensor, key_bits: int = 64
     """Turn arbitrary (key, value) pairs into the sorted unique keys a push needs, summing the
     values of repeated keys; keys must be below ``2**key_bits``.  fp32 values travel with the
     keys through the sort and are summed by a kernel of their own; other types take the sort
-    permutation and torch's ``index_add_``."""
+    permutation and torch's ``index_add_``.
+
+    The values of a key are added up in a fixed tree, in which their places depend on the input and
+    on the order in which the GPU serves lanes that count on one address.  Equal inputs have had
+    equal sums from run to run, bit for bit, but nothing guarantees that of this order."""
     if keys.is_cuda:
         got = _native.unique_sum(*_native.fns, keys, vals, key_bits)
         if type(got) is tuple:

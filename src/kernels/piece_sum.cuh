@@ -12,7 +12,9 @@
 //                 the input), by parts of its key range.  The last CTA to end makes the prefix of
 //                 the counts and reports to the host;
 //   unique_gather moves keys and sums to their places in the outputs.
-// Every sum has a fixed tree: results do not depend on the order of the CTAs.
+// Every sum has a fixed tree: results do not depend on the order of the CTAs.  Which of a key's
+// values comes where in it depends on the order in which the lanes of an instruction that count on
+// one address get their turn (rank_rows), which has always been the same and is not guaranteed.
 //
 // Popular ids make large buckets, in pieces of which little is left to merge.  Keys that crowd
 // together would not fit: a CTA of the first kernel looks at a sample of them.  Parts of the input
@@ -22,18 +24,18 @@
 //
 // Whole calls, us, before (pass by pass) and now; ids with many repeats, ids all different:
 //                24 bits                   30 bits                   40 bits
-//   2^14         41 -> 30,  41 -> 34       42 -> 30,  43 -> 33       52 -> 31,  53 -> 36
-//   2^16         43 -> 31,  45 -> 32       50 -> 31,  50 -> 33       63 -> 31,  66 -> 37
-//   2^18         55 -> 38,  61 -> 38       59 -> 40,  65 -> 42       79 -> 48,  86 -> 49
-//   2^19         61 -> 42,  64 -> 49       65 -> 45,  72 -> 54       83 -> 56,  91 -> 63
-//   2^20         71 -> 68,  71 -> 61       79 -> 77,  85 -> 65      102 -> 91, 108 -> 72
-//   2^21         97 -> 88,  96 -> 83      103 -> 104, 111 -> 89     147 -> 112, 160 -> 101
-//   2^22        152 -> 133, 153 -> 128    169 -> 135, 182 -> 138    250 -> 158, 263 -> 161
-// Half of all items one id: 0.48 to 0.72 of the time before up to 2^19 items, 0.63 to 0.98 beyond.
-// Keys that crowd together in seven narrow ranges: 0.72 to 1.14 up to 2^19, where a sample makes
-// the parts; then the general way after a count, or after the pieces, for nothing: 1.3 at 700 000,
-// 1.05 to 1.14 from 2^20 on.  More than 20 popular ids in one part of the input: every piece has
-// them, so that the part's merge takes another round (700 000 items: 64 -> 70 us, else 52).
+//   2^14       45 ->  35,  41 ->  32      43 ->  31,  43 ->  38      52 ->  31,  53 ->  36
+//   2^16       43 ->  31,  45 ->  32      50 ->  31,  50 ->  34      62 ->  31,  65 ->  37
+//   2^18       55 ->  37,  60 ->  39      59 ->  41,  66 ->  43      79 ->  48,  85 ->  49
+//   2^19       61 ->  42,  63 ->  50      64 ->  46,  71 ->  54      84 ->  56,  91 ->  64
+//   700000     64 ->  60,  65 ->  57      69 ->  52,  73 ->  62      89 ->  64,  96 ->  74
+//   2^20       71 ->  68,  71 ->  59      80 ->  77,  85 ->  64     101 ->  91, 107 ->  72
+//   2^21       96 ->  88,  95 ->  81     102 -> 103, 110 ->  87     147 -> 113, 160 ->  98
+//   2^22      152 -> 134, 152 -> 128     168 -> 134, 180 -> 137     250 -> 159, 261 -> 158
+// Half of all items one id: 0.49 to 0.80 of the time before up to 786 432 items, 0.62 to 0.99
+// beyond.  Keys that crowd together in seven narrow ranges: 0.75 to 1.15 up to 2^19, where a sample
+// makes the parts, 1.05 to 1.23 up to 655 360; then the general way comes after the pieces, which
+// were for nothing, 1.26 to 1.31, and beyond 786 432 items after a count, 1.05 to 1.13.
 // What bounds it: up to 2^18 items the chain of some ten trips to L2 and three sorts of 2400 clocks
 // per pass; at 2^22 piece_sum (48 us; 0.52 of the issue slots, two thirds of the shared-memory
 // pipe, 24 warps per SM), bucket_scatter (26 to 32), and the latency of piece_merge (25).
@@ -57,8 +59,8 @@ constexpr int kMaxSegments = kMaxBuckets * kGroup;
 constexpr long long kMaxBucketItems = 9ll << 19;     // (in 1024 buckets 4608 on average)
 // Up to so many items are not scattered: pieces of the input and parts of the key range, at most,
 // so that all units of a merge run at a time (444 pieces and 512 parts: 2^18 items 52 us, with 256
-// of both 40).  700 000 items, many repeats / all different: 57 / 65 us, in buckets 70 / 56; 2^20:
-// 66 / 78 and 75 / 65.
+// of both 40).  786 432 ids of 30 bits, many repeats / all different: 54 / 66 us, in buckets 75
+// / 58; 2^20 (where no CTAs helped yet) 66 / 78 and 75 / 65.
 constexpr long long kFewItems = 3 << 18;
 // Up to so many of them the parts of crowded keys are those of a sample; beyond, one of 256 parts
 // by a sample of 5120 would often have more keys than a CTA sorts, and the host goes the general

@@ -189,7 +189,9 @@ __device__ __forceinline__ int valid_rows(int left, int rows) {
 // The lanes that hold the same digit find each other through a mask in shared memory (32 keys of an
 // SM in 9 ns; 15 with ballots, 32 with match.any), and the first of them advances the counter.
 // FREE: items of a digit may be in any order, the counter gives out the ranks.  (Lanes of one
-// instruction get theirs in the hardware's order, on which nothing but rounding depends.)
+// instruction get theirs in the hardware's order, on which nothing but rounding depends: the order
+// in which the values of a key are added up.  It has been the same from run to run, with nothing
+// that guarantees it; masks, which would, take the scatter of 2^22 pairs from 37 to 42 us.)
 // (32 atomics on one address take an SM some 70 clocks, which popular ids among others do not
 // need.)
 template <bool FREE, int ROWS, typename Digit>
@@ -751,7 +753,7 @@ static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) 
 // Of 2^22 pairs with 0.85 million keys they take 15, 5 and 12 us, cold; the form before, which
 // counted the distinct keys, waited for the outputs and then went over the pairs once more, 9, 5
 // and 22.
-// Nothing is added up with atomics: sums do not depend on the order of the CTAs.
+// Nothing is added up with atomics: sums do not depend on the order of the CTAs (but see FREE).
 constexpr int kUniqueThreads = 256;
 constexpr int kUniquePer = 8;
 constexpr int kRound = kUniqueThreads * kUniquePer;

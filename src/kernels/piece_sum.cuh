@@ -12,9 +12,10 @@
 //                 the input), by parts of its key range.  The last CTA to end makes the prefix of
 //                 the counts and reports to the host;
 //   unique_gather moves keys and sums to their places in the outputs.
-// Every sum has a fixed tree: results do not depend on the order of the CTAs.  Which of a key's
-// values comes where in it depends on the order in which the lanes of an instruction that count on
-// one address get their turn (rank_rows), which has always been the same and is not guaranteed.
+// Every sum has a fixed tree: results do not depend on the order of the CTAs.  In buckets, which of
+// a key's values comes where in it depends on the order in which the lanes of an instruction that
+// count on one address get their turn (rank_rows), which has always been the same and is not
+// guaranteed.
 //
 // Popular ids make large buckets, in pieces of which little is left to merge.  Keys that crowd
 // together would not fit: a CTA of the first kernel looks at a sample of them.  Parts of the input
@@ -561,8 +562,12 @@ __device__ __forceinline__ void place_counts(unsigned int* count2, int pairs, un
 }
 
 // Sorts the items of a CTA, which it has in registers in rows of 32 per warp, by `passes` digits of
-// `width` bits from the lowest of the key on; leaves them in order in sh.items.
-template <bool LONG>
+// `width` bits from the lowest of the key on; leaves them in order in sh.items.  FREE: with equal
+// keys in any order, which a first pass then ranks without masks.  (2^22 ids of 30 bits all
+// different in buckets 138 us, 145 with masks; the fewer items of a piece of the input or of a
+// merge gain nothing by it: 2^18 ids with repeats 41.3 and 39.7 us, 2^19 all different 54.3 and
+// 54.8.)
+template <bool LONG, bool FREE = false>
 __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int passes, int width,
                                            const PieceShared& sh) {
   constexpr int kRows = kPieceRows, kT = kPieceThreads;
@@ -582,7 +587,7 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
   unsigned int* count2 = reinterpret_cast<unsigned int*>(sh.cnt);
   for (int pass = 0; pass < passes; ++pass) {
     const int shift = pass * width;
-    if (pass) clear_words(lanes, digits);
+    if (pass || !FREE) clear_words(lanes, digits);
     clear_words(mine2, pairs);
     __syncwarp();
     unsigned int rank[kRows / 2];
@@ -590,7 +595,7 @@ __device__ __forceinline__ void sort_piece(Item (&k)[kPieceRows], int count, int
       return LONG ? item_digit(k[j], shift + kIndexBits, mask)
                   : (unsigned int)(k[j] >> 32) >> shift & mask;
     };
-    if (pass == 0) rank_rows<true, kRows>(digit, rows, valid, lanes, cnt, rank);
+    if (FREE && pass == 0) rank_rows<true, kRows>(digit, rows, valid, lanes, cnt, rank);
     else rank_rows<false, kRows>(digit, rows, valid, lanes, cnt, rank);
     __syncthreads();
     place_counts(count2, pairs, sh.part + (pass & 1) * kPieceWarps);
@@ -893,7 +898,7 @@ __global__ void __launch_bounds__(kPieceThreads, LONG ? 2 : 3)
     wide = __syncthreads_or(wide);
   }
   if (!RAW && p.pieces > 1) count = add_up_popular(k, count, sh);
-  sort_piece<LONG>(k, count, b.passes, b.width, sh);
+  sort_piece<LONG, !RAW>(k, count, b.passes, b.width, sh);
   const unsigned int total = sum_piece<LONG>(count, sh);
   const int parts = b.parts;
   unsigned int* bounds = b.bounds + (size_t)blockIdx.x * parts;

@@ -320,20 +320,17 @@ __global__ void __launch_bounds__(1024)
 // What travels beside the keys of a pass: nothing, the key's index or a value of 32 bits in an
 // array of its own, or a value that a first pass puts below its key.  With values in an array, keys
 // of up to 32 bits can have 32 too: the first pass narrows them (kNarrow), the last one puts pairs
-// together (kShortToPairs).
-// Equal keys of sums may be in any order: a first pass (kToPairs, kNarrow, kFirst: kPayload) needs
-// no masks (rank_rows, FREE).
+// together (kShortToPairs).  (First passes of sums without masks, FREE, would save 1 to 2 % from
+// 2^23 items on and leave the order of a key's values to the hardware.)
 enum {
   kNoPayload = 0, kMakeIndex = 1, kPayload = 2, kToPairs = 3,
-  kNarrow = 4, kShort = 5, kShortToPairs = 6, kFirst = 7
+  kNarrow = 4, kShort = 5, kShortToPairs = 6
 };
 template <int PAY>
 struct Form {
   static constexpr bool kShortIn = PAY == kShort || PAY == kShortToPairs;
   static constexpr bool kShortKey = kShortIn || PAY == kNarrow;
-  static constexpr bool kArray =
-      PAY == kMakeIndex || PAY == kPayload || PAY == kFirst || kShortKey;
-  static constexpr bool kFree = PAY == kToPairs || PAY == kNarrow || PAY == kFirst;
+  static constexpr bool kArray = PAY == kMakeIndex || PAY == kPayload || kShortKey;
   using In = std::conditional_t<kShortIn, unsigned int, Item>;    // as a pass reads them
   using Key = std::conditional_t<kShortKey, unsigned int, Item>;  // and ranks them
 };
@@ -480,13 +477,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2)
   for (long long tile_base = lo; tile_base < hi; tile_base += tile) {
     const long long base = tile_base + (long long)warp * (32 * rows) + lane;
     const int tile_n = (int)(hi - tile_base < tile ? hi - tile_base : tile);
-    if constexpr (!Form<PAY>::kFree)
-      for (int i = lane; i < kDigits; i += 32) lanes[i] = 0;
+    for (int i = lane; i < kDigits; i += 32) lanes[i] = 0;
     for (int i = lane; i < kPairs; i += 32) reinterpret_cast<unsigned int*>(cnt)[i] = 0;
     __syncwarp();
     unsigned int rank[ROWS / 2];  // two of 16 bits each
     const int valid = valid_rows((int)(hi - base), rows);
-    rank_rows<Form<PAY>::kFree, ROWS>(
+    rank_rows<false, ROWS>(
         [&](int j) { return item_digit(k[j], shift, mask); }, rows, valid, lanes, cnt, rank);
     __syncthreads();
     // where the runs of this thread's digits start in the tile, and each warp's part of them
@@ -737,7 +733,7 @@ static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) 
     return PSDEV_ERR_ARG;
   } else {
     if (p.n <= kMaxChunks * 4096ll) return sort_pass<kWideBits, 8, 16, PAY>(p, w, s);
-    return sort_pass<kWideBits, 16, PAY == kPayload || PAY == kFirst ? 10 : 14, PAY>(p, w, s);
+    return sort_pass<kWideBits, 16, PAY == kPayload ? 10 : 14, PAY>(p, w, s);
   }
 }
 
@@ -753,7 +749,7 @@ static int any_pass(int bits, const Pass& p, const SortWork& w, cudaStream_t s) 
 // Of 2^22 pairs with 0.85 million keys they take 15, 5 and 12 us, cold; the form before, which
 // counted the distinct keys, waited for the outputs and then went over the pairs once more, 9, 5
 // and 22.
-// Nothing is added up with atomics: sums do not depend on the order of the CTAs (but see FREE).
+// Nothing is added up with atomics: sums do not depend on the order of the CTAs.
 constexpr int kUniqueThreads = 256;
 constexpr int kUniquePer = 8;
 constexpr int kRound = kUniqueThreads * kUniquePer;
@@ -1530,8 +1526,7 @@ int unique_sort(const Item* keys, const float* vals, int64_t n, int key_bits,
       if (rc) return rc;
       continue;
     }
-    const int rc = !plan.pairs ? pass ? any_pass<kPayload>(plan.bits, p, w, s)
-                                      : any_pass<kFirst>(plan.bits, p, w, s)
+    const int rc = !plan.pairs ? any_pass<kPayload>(plan.bits, p, w, s)
                    : pass == 0 ? any_pass<kToPairs>(plan.bits, p, w, s)
                                : any_pass<kNoPayload>(plan.bits, p, w, s);
     if (rc) return rc;

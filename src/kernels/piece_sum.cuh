@@ -25,18 +25,18 @@
 //
 // Whole calls, us, before (pass by pass) and now; ids with many repeats, ids all different:
 //                24 bits                   30 bits                   40 bits
-//   2^14       45 ->  35,  41 ->  32      43 ->  31,  43 ->  38      52 ->  31,  53 ->  36
-//   2^16       43 ->  31,  45 ->  32      50 ->  31,  50 ->  34      62 ->  31,  65 ->  37
-//   2^18       55 ->  37,  60 ->  39      59 ->  41,  66 ->  43      79 ->  48,  85 ->  49
-//   2^19       61 ->  42,  63 ->  50      64 ->  46,  71 ->  54      84 ->  56,  91 ->  64
-//   700000     64 ->  60,  65 ->  57      69 ->  52,  73 ->  62      89 ->  64,  96 ->  74
-//   2^20       71 ->  68,  71 ->  59      80 ->  77,  85 ->  64     101 ->  91, 107 ->  72
-//   2^21       96 ->  88,  95 ->  81     102 -> 103, 110 ->  87     147 -> 113, 160 ->  98
-//   2^22      152 -> 134, 152 -> 128     168 -> 134, 180 -> 137     250 -> 159, 261 -> 158
-// Half of all items one id: 0.49 to 0.80 of the time before up to 786 432 items, 0.62 to 0.99
-// beyond.  Keys that crowd together in seven narrow ranges: 0.75 to 1.15 up to 2^19, where a sample
-// makes the parts, 1.05 to 1.23 up to 655 360; then the general way comes after the pieces, which
-// were for nothing, 1.26 to 1.31, and beyond 786 432 items after a count, 1.05 to 1.13.
+//   2^14       47 ->  36,  40 ->  32      43 ->  31,  44 ->  38      53 ->  32,  54 ->  35
+//   2^16       45 ->  32,  46 ->  32      50 ->  32,  51 ->  34      63 ->  32,  64 ->  36
+//   2^18       55 ->  37,  59 ->  38      59 ->  40,  64 ->  41      80 ->  47,  86 ->  49
+//   2^19       61 ->  43,  63 ->  50      65 ->  46,  71 ->  55      84 ->  56,  91 ->  63
+//   700000     64 ->  60,  65 ->  58      68 ->  52,  73 ->  63      89 ->  64,  96 ->  73
+//   2^20       71 ->  68,  70 ->  60      80 ->  77,  86 ->  66     102 ->  90, 107 ->  73
+//   2^21       97 ->  89,  96 ->  82     103 -> 103, 111 ->  87     147 -> 112, 161 ->  98
+//   2^22      153 -> 132, 152 -> 130     169 -> 134, 181 -> 139     250 -> 159, 262 -> 160
+// Half of all items one id: 0.50 to 0.75 of the time before up to 786 432 items, 0.61 to 0.97
+// beyond.  Keys that crowd together in seven narrow ranges: 0.75 to 1.16 up to 2^19, where a sample
+// makes the parts, 1.05 to 1.22 up to 655 360; then the general way comes after the pieces, which
+// were for nothing, 1.27 to 1.33, and beyond 786 432 items after a count, 1.06 to 1.15.
 // What bounds it: up to 2^18 items the chain of some ten trips to L2 and three sorts of 2400 clocks
 // per pass; at 2^22 piece_sum (48 us; 0.52 of the issue slots, two thirds of the shared-memory
 // pipe, 24 warps per SM), bucket_scatter (26 to 32), and the latency of piece_merge (25).
